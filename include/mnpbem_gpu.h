@@ -257,6 +257,15 @@ MNPBEM_API mnpbem_status mnpbem_gemm_c64(int32_t device, int32_t path, int64_t M
                                          int64_t lda, const float* B, int64_t ldb,
                                          const float* beta, float* C, int64_t ldc);
 
+/* A <- inv(A) for one w x w diagonal block (row-major, interleaved complex, row
+ * stride lda, host array) by the block inverses of the factorisations:
+ * precision MNPBEM_FP64 complex128, w <= 64 (partial pivoting inside the block);
+ * MNPBEM_FP32 complex64, w <= 64 (the same) or <= 256 (no row interchanges).
+ * cond (may be NULL): max|A| * max|inv(A)|.  MNPBEM_ERR_SINGULAR for a zero or
+ * non-finite pivot.  The building block of MATLAB's inv in initmat.m:27-72.   */
+MNPBEM_API mnpbem_status mnpbem_block_inverse(int32_t device, int32_t precision, int32_t w, void* A,
+                                              int32_t lda, double* cond);
+
 /* Extinction and scattering cross sections of given surface charges and
  * currents, like mnpbem_solve's ext/sca, for callers that cannot allocate GPU
  * memory (a MEX gateway inside a MATLAB session whose GPU memory belongs to

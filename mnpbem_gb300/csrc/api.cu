@@ -809,6 +809,38 @@ mnpbem_status mnpbem_gemm_c64(int32_t device, int32_t path, int64_t M, int64_t N
   return MNPBEM_OK;
 }
 
+mnpbem_status mnpbem_block_inverse(int32_t device, int32_t precision, int32_t w, void* A, int32_t lda,
+                                   double* cond) {
+  const bool fp64 = precision == MNPBEM_FP64;
+  if (!A || w < 1 || lda < w || (!fp64 && precision != MNPBEM_FP32) || w > (fp64 ? 64 : 256)) {
+    set_error("mnpbem_block_inverse: invalid arguments");
+    return MNPBEM_ERR_INVALID_ARG;
+  }
+  MNP_CUDA(cudaSetDevice(device));
+  const size_t es = fp64 ? sizeof(double2) : sizeof(float2);
+  DevBuf dA, dX, ds, pan;
+  MNP_TRY(dA.ensure(es * w * lda));
+  MNP_TRY(dX.ensure(es * w * w));
+  MNP_TRY(ds.ensure(2 * sizeof(int)));
+  MNP_CUDA(cudaMemcpy(dA.ptr, A, es * w * lda, cudaMemcpyHostToDevice));
+  MNP_CUDA(cudaMemset(ds.ptr, 0, 2 * sizeof(int)));
+  if (fp64) MNP_TRY(block_inverse<double>(dA.as<double2>(), lda, w, dX.as<double2>(), ds.as<int>(), pan, nullptr));
+  else MNP_TRY(block_inverse<float>(dA.as<float2>(), lda, w, dX.as<float2>(), ds.as<int>(), pan, nullptr));
+  int hs[2] = {0, 0};
+  MNP_CUDA(cudaMemcpy(hs, ds.ptr, sizeof(hs), cudaMemcpyDeviceToHost));
+  MNP_CUDA(cudaMemcpy(A, dA.ptr, es * w * lda, cudaMemcpyDeviceToHost));
+  if (cond) {
+    float c;
+    memcpy(&c, &hs[1], sizeof(float));
+    *cond = c;
+  }
+  if (hs[0]) {
+    set_error("block inverse: zero or non-finite pivot");
+    return MNPBEM_ERR_SINGULAR;
+  }
+  return MNPBEM_OK;
+}
+
 mnpbem_status mnpbem_geom_stream(const mnpbem_geom* G, void** stream) {
   MNP_TRY(check_geom(G));
   if (!stream) { set_error("null stream pointer"); return MNPBEM_ERR_INVALID_ARG; }
@@ -884,17 +916,17 @@ uint64_t lane_sig(const mnpbem_geom* G, const Lane& L) {
   mixbuf(L.outbuf); mixbuf(L.bsplit); mixbuf(L.lp_dev); mixbuf(G->exbuf);
   mixbuf(L.tc.bexp); mixbuf(L.tc.err);
   auto gj = [&](const auto& w) {
-    mixbuf(w.ccol); mixbuf(w.rrow); mixbuf(w.ncol); mixbuf(w.xblk); mixbuf(w.status);
+    mixbuf(w.ccol); mixbuf(w.rrow); mixbuf(w.ncol); mixbuf(w.xblk); mixbuf(w.status); mixbuf(w.pan);
     mix(nullptr, (size_t)w.nb);
     if (w.inner) {
       mixbuf(w.inner->ccol); mixbuf(w.inner->rrow); mixbuf(w.inner->ncol); mixbuf(w.inner->xblk);
-      mixbuf(w.inner->status);
+      mixbuf(w.inner->status); mixbuf(w.inner->pan);
     }
   };
   gj(L.gj32);
   gj(L.gj64);
   auto lu = [&](const auto& w) {
-    mixbuf(w.ccol); mixbuf(w.rrow); mixbuf(w.xblk); mixbuf(w.tmp);
+    mixbuf(w.ccol); mixbuf(w.rrow); mixbuf(w.xblk); mixbuf(w.tmp); mixbuf(w.pan);
     mix(nullptr, (size_t)w.b);
     mix(nullptr, (size_t)w.m);
   };

@@ -790,95 +790,104 @@ __device__ __forceinline__ void record_cond(int* status, double amax, double xma
   atomicMax(status + 1, __float_as_int((float)c));
 }
 
-// In-place Gauss-Jordan of one w x w block (w <= 64) with partial pivoting
-// inside the block.  256 threads as a 16 x 16 grid; thread (ty, tx) keeps the
-// 16 entries (ty + 16 i, tx + 16 j) in registers.  Pivoting is implicit: step p
-// takes as pivot row r_p the row, among those not yet used, with the largest
-// |a_rp| in column p, and eliminates with (r_p, p) in place of (p, p).  The
-// matrix M this leaves satisfies inv(A)[q][r_k] = M[r_q][k], so the block is
-// written out through the permutation.  Two __syncthreads per step: after the
-// pivot column is published, and after the pivot row is.
-template <typename R>
-__global__ void __launch_bounds__(256) k_block_inv(const cplx<R>* __restrict__ A, int64_t lda, int w,
-                                                   cplx<R>* __restrict__ X, int64_t ldx, int* status) {
-  using Cx = cplx<R>;
-  __shared__ Cx prow[2][64], pcol[2][64];
+// Row of the largest key among 64 candidates, keys of rows lane and lane + 32 in
+// k0 and k1 (0 = not a candidate); the lowest row on ties.  Every lane gets it.
+__device__ __forceinline__ int argmax64(unsigned k0, unsigned k1) {
+  const unsigned mx = __reduce_max_sync(0xffffffffu, max(k0, k1));
+  const unsigned b0 = __ballot_sync(0xffffffffu, k0 == mx), b1 = __ballot_sync(0xffffffffu, k1 == mx);
+  return b0 ? __ffs(b0) - 1 : 31 + __ffs(b1);
+}
+
+// In-place Gauss-Jordan of one w x w complex64 block (w <= 64) with partial
+// pivoting inside the block.  256 threads as a 16 x 16 grid; thread (ty, tx)
+// keeps the 16 entries (ty + 16 i, tx + 16 j) in registers.  Pivoting is
+// implicit: step p takes as pivot row r_p the row, among those not yet used,
+// with the largest |a_rp| in column p, and eliminates with (r_p, p) in place of
+// (p, p).  The matrix M this leaves satisfies inv(A)[q][r_k] = M[r_q][k], so the
+// block is written out through the permutation, to X and, when X2 is given, to
+// X2 as well (X2 may be the input: it is read before the first barrier).  Two
+// __syncthreads per step: after the pivot column is published, and after the
+// pivot row is.
+// Bound by the latency of the chain of 64 steps (one CTA).  Each warp finds the
+// pivot with one integer reduction over the 64 candidates' moduli; a scan of
+// the column by every thread took most of a step (160 us per block of 64 in a
+// sweep, PIVFLOAT us now).
+__global__ void __launch_bounds__(256) k_block_inv(const float2* A, int64_t lda, int w, float2* X, int64_t ldx,
+                                                   float2* X2, int64_t ldx2, int* status) {
+  __shared__ float2 prow[2][64], pcol[2][64];
   __shared__ int prow_of[64], pos_of[64];
-  __shared__ unsigned char used[64];
-  __shared__ double red[8];
-  const int t = threadIdx.x, tx = t & 15, ty = t >> 4;
-  Cx a[4][4];
-  double amax = 0.0;
+  __shared__ float red[2][8];
+  const int t = threadIdx.x, tx = t & 15, ty = t >> 4, lane = t & 31;
+  float2 a[4][4];
+  float amax = 0.f;
 #pragma unroll
   for (int i = 0; i < 4; ++i)
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const int r = ty + 16 * i, c = tx + 16 * j;
-      a[i][j] = (r < w && c < w) ? A[r * lda + c] : mk<R>(r == c ? 1 : 0, 0);
-      if (r < w && c < w) amax = fmax(amax, sqrt(cabs2(a[i][j])));
+      a[i][j] = (r < w && c < w) ? A[r * lda + c] : make_float2(r == c ? 1.f : 0.f, 0.f);
+      if (r < w && c < w) amax = fmaxf(amax, sqrtf(a[i][j].x * a[i][j].x + a[i][j].y * a[i][j].y));
     }
-  if (t < 64) used[t] = 0;
+  // rows still free, lane and lane + 32 (the same in every warp)
+  bool free0 = lane < w, free1 = lane + 32 < w;
   for (int p = 0; p < w; ++p) {
     const int buf = p & 1;
     // 1. publish column p
 #pragma unroll
-    for (int i = 0; i < 4; ++i)
+    for (int j = 0; j < 4; ++j)
+      if (tx + 16 * j == p) {
 #pragma unroll
-      for (int j = 0; j < 4; ++j)
-        if (tx + 16 * j == p) pcol[buf][ty + 16 * i] = a[i][j];
+        for (int i = 0; i < 4; ++i) pcol[buf][ty + 16 * i] = a[i][j];
+      }
     __syncthreads();
-    // 2. pivot row: largest modulus among the unused rows (first one on ties)
-    int rp = -1;
-    R best = -1;
-    for (int r = 0; r < w; ++r) {
-      if (used[r]) continue;
-      const Cx v = pcol[buf][r];
-      const R m2 = v.x * v.x + v.y * v.y;
-      if (rp < 0 || m2 > best) { best = m2; rp = r; }
-    }
+    // 2. pivot row: largest modulus among the free rows (first one on ties);
+    //    the bits of a non-negative float order as integers, + 1 keeps a free
+    //    row with a zero entry above the used ones
+    const float2 v0 = pcol[buf][lane], v1 = pcol[buf][lane + 32];
+    const unsigned k0 = free0 ? __float_as_uint(v0.x * v0.x + v0.y * v0.y) + 1u : 0u;
+    const unsigned k1 = free1 ? __float_as_uint(v1.x * v1.x + v1.y * v1.y) + 1u : 0u;
+    const int rp = argmax64(k0, k1);
+    free0 = free0 && rp != lane;
+    free1 = free1 && rp != lane + 32;
     // 3. publish the pivot row
 #pragma unroll
     for (int i = 0; i < 4; ++i)
+      if (ty + 16 * i == rp) {
 #pragma unroll
-      for (int j = 0; j < 4; ++j)
-        if (ty + 16 * i == rp) prow[buf][tx + 16 * j] = a[i][j];
-    __syncthreads();
+        for (int j = 0; j < 4; ++j) prow[buf][tx + 16 * j] = a[i][j];
+      }
+    const float2 piv = pcol[buf][rp];
+    const float n2 = piv.x * piv.x + piv.y * piv.y;
+    const float rn2 = 1.f / n2;
+    const float2 inv = make_float2(piv.x * rn2, -piv.y * rn2);
     if (t == 0) {
-      used[rp] = 1;
+      if (!(n2 > 1e-30f && n2 < 1e30f)) atomicOr(status, 1);
       prow_of[p] = rp;
       pos_of[rp] = p;
     }
-    const Cx piv = prow[buf][p];
-    const R n2 = piv.x * piv.x + piv.y * piv.y;
-    if (t == 0 && !(n2 > (R)1e-30 && n2 < (R)1e30)) atomicOr(status, 1);
-    const R rn2 = (R)1 / n2;
-    const Cx inv = mk<R>(piv.x * rn2, -piv.y * rn2);
-    // One update a - pc_r pr_c serves every entry when the pivot column of pr
-    // holds 1 + 1/a_pp and the pivot row of pc holds a_pp - 1:
-    //   pivot row:    a_rc - (a_pp - 1) a_rc / a_pp = a_rc / a_pp
-    //   column p:     a_ip - a_ip (1 + 1/a_pp)      = -a_ip / a_pp
-    // (the pivot itself is set to 1/a_pp directly).
-    Cx pr[4], pc[4];
+    __syncthreads();
+    // a_rc <- a_rc - pc_r pr_c with pr_c = a_(rp)c / a_pp.  The pivot row keeps
+    // pr itself (0 + 1 * pr), the pivot column takes -pc / a_pp (0 - pc / a_pp).
+    float2 pr[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const int c = tx + 16 * j;
-      pr[j] = (c == p) ? mk<R>(1 + inv.x, inv.y) : cmul(prow[buf][c], inv);
+      pr[j] = (c == p) ? inv : cmul(prow[buf][c], inv);
     }
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
       const int r = ty + 16 * i;
-      pc[i] = (r == rp) ? mk<R>(piv.x - 1, piv.y) : pcol[buf][r];
-    }
-#pragma unroll
-    for (int i = 0; i < 4; ++i)
+      const bool isrow = r == rp;
+      const float2 m = isrow ? make_float2(-1.f, 0.f) : pcol[buf][r];
 #pragma unroll
       for (int j = 0; j < 4; ++j) {
-        const Cx v = csub(a[i][j], cmul(pc[i], pr[j]));
-        a[i][j] = (ty + 16 * i == rp && tx + 16 * j == p) ? inv : v;
+        const float2 base = (isrow || tx + 16 * j == p) ? make_float2(0.f, 0.f) : a[i][j];
+        a[i][j] = csub(base, cmul(m, pr[j]));
       }
+    }
   }
   __syncthreads();
-  double xmax = 0.0;
+  float xmax = 0.f;
 #pragma unroll
   for (int i = 0; i < 4; ++i)
 #pragma unroll
@@ -886,82 +895,236 @@ __global__ void __launch_bounds__(256) k_block_inv(const cplx<R>* __restrict__ A
       const int r = ty + 16 * i, c = tx + 16 * j;
       if (r < w && c < w) {
         X[(int64_t)pos_of[r] * ldx + prow_of[c]] = a[i][j];
-        xmax = fmax(xmax, sqrt(cabs2(a[i][j])));
+        if (X2) X2[(int64_t)pos_of[r] * ldx2 + prow_of[c]] = a[i][j];
+        xmax = fmaxf(xmax, sqrtf(a[i][j].x * a[i][j].x + a[i][j].y * a[i][j].y));
       }
     }
   // block maxima of |A| and |X| for the condition proxy
   for (int o = 16; o; o >>= 1) {
+    amax = fmaxf(amax, __shfl_xor_sync(0xffffffffu, amax, o));
+    xmax = fmaxf(xmax, __shfl_xor_sync(0xffffffffu, xmax, o));
+  }
+  if (lane == 0) { red[0][t >> 5] = amax; red[1][t >> 5] = xmax; }
+  __syncthreads();
+  if (t == 0) {
+    float am = 0.f, xm = 0.f;
+    for (int k = 0; k < 8; ++k) { am = fmaxf(am, red[0][k]); xm = fmaxf(xm, red[1][k]); }
+    record_cond(status, am, xm);
+  }
+}
+
+// The same elimination for a complex128 block (w <= 64) on a cluster of eight
+// CTAs: CTA q keeps columns 8 q .. 8 q + 7 (thread = row, two columns each), so
+// that the FP64 pipes of eight SMs share the rank-1 updates (FP64 runs at two
+// FMA per clock per SM: 64^3 complex multiply-adds are 270 us on one SM).
+// Step p: the owner of column p writes it, with an integer key of |re| + |im|
+// (the pivot measure of LAPACK's izamax), into every CTA's shared memory;
+// cluster barrier; every warp picks the pivot row from the keys; the row's
+// eight local columns are scaled by the reciprocal pivot, and each thread
+// updates its two entries.  The column buffer alternates, so one cluster
+// barrier per step suffices: a CTA that writes column p + 2 into a buffer has
+// passed barrier p + 1, which every CTA reaches after reading column p.
+// One CTA with the pivot scan in every thread took 1059 us per block of 64;
+// this takes PIVDOUBLE us.
+constexpr int BD_CL = 8, BD_THREADS = 256;
+__global__ void __cluster_dims__(BD_CL, 1, 1) __launch_bounds__(BD_THREADS)
+    k_block_inv_c128(const double2* A, int64_t lda, int w, double2* X, int64_t ldx, double2* X2, int64_t ldx2,
+                     int* status) {
+  namespace cg = cooperative_groups;
+  cg::cluster_group cluster = cg::this_cluster();
+  __shared__ double2 pcol[2][64], prow[8], inv_s;
+  __shared__ unsigned pkey[2][64];
+  __shared__ int prow_of[64], pos_of[64];
+  __shared__ double red[2][BD_THREADS / 32], cond_loc[2];
+  const int rank = (int)cluster.block_rank();
+  const int t = threadIdx.x, lane = t & 31, r = t & 63, cg2 = t >> 6;
+  double2 a[2];
+  double amax = 0.0, xmax = 0.0;
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    const int c = 8 * rank + 2 * cg2 + j;
+    a[j] = (r < w && c < w) ? A[(int64_t)r * lda + c] : make_double2(r == c ? 1.0 : 0.0, 0.0);
+    if (r < w && c < w) amax = fmax(amax, sqrt(cabs2(a[j])));
+  }
+  bool free0 = lane < w, free1 = lane + 32 < w;
+  cluster.sync();   // every CTA runs before its shared memory is written
+  for (int p = 0; p < w; ++p) {
+    const int buf = p & 1, lc = p & 7;
+    const bool owner = rank == (p >> 3);
+    if (owner && cg2 == (lc >> 1)) {
+      const double2 v = (lc & 1) ? a[1] : a[0];
+      const unsigned key = (unsigned)__double2hiint(fabs(v.x) + fabs(v.y)) + 1u;
+#pragma unroll
+      for (int q = 0; q < BD_CL; ++q) {
+        cluster.map_shared_rank(&pcol[buf][0], q)[r] = v;
+        cluster.map_shared_rank(&pkey[buf][0], q)[r] = key;
+      }
+    }
+    cluster.sync();
+    const unsigned k0 = free0 ? pkey[buf][lane] : 0u, k1 = free1 ? pkey[buf][lane + 32] : 0u;
+    const int rp = argmax64(k0, k1);
+    free0 = free0 && rp != lane;
+    free1 = free1 && rp != lane + 32;
+    // unscaled pivot row, and the reciprocal pivot from one thread
+    if (r == rp) {
+      prow[2 * cg2] = a[0];
+      prow[2 * cg2 + 1] = a[1];
+    }
+    if (t == 0) {
+      const double2 piv = pcol[buf][rp];
+      const double n2 = piv.x * piv.x + piv.y * piv.y, rn2 = 1.0 / n2;
+      inv_s = make_double2(piv.x * rn2, -piv.y * rn2);
+      if (rank == 0 && !(n2 > 1e-30 && n2 < 1e30)) atomicOr(status, 1);
+      prow_of[p] = rp;
+      pos_of[rp] = p;
+    }
+    __syncthreads();
+    if (t < 8) prow[t] = (owner && t == lc) ? inv_s : cmul(prow[t], inv_s);
+    __syncthreads();
+    const bool isrow = r == rp;
+    const double2 m = isrow ? make_double2(-1.0, 0.0) : pcol[buf][r];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const double2 pr = prow[2 * cg2 + j];
+      const bool iscol = owner && 2 * cg2 + j == lc;
+      const double2 base = (isrow || iscol) ? make_double2(0.0, 0.0) : a[j];
+      a[j].x = fma(m.y, pr.y, fma(-m.x, pr.x, base.x));
+      a[j].y = fma(-m.y, pr.x, fma(-m.x, pr.y, base.y));
+    }
+  }
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    const int c = 8 * rank + 2 * cg2 + j;
+    if (r < w && c < w) {
+      X[(int64_t)pos_of[r] * ldx + prow_of[c]] = a[j];
+      if (X2) X2[(int64_t)pos_of[r] * ldx2 + prow_of[c]] = a[j];
+      xmax = fmax(xmax, sqrt(cabs2(a[j])));
+    }
+  }
+  for (int o = 16; o; o >>= 1) {
     amax = fmax(amax, __shfl_xor_sync(0xffffffffu, amax, o));
     xmax = fmax(xmax, __shfl_xor_sync(0xffffffffu, xmax, o));
   }
-  if ((t & 31) == 0) red[t >> 5] = amax;
+  if (lane == 0) { red[0][t >> 5] = amax; red[1][t >> 5] = xmax; }
   __syncthreads();
-  if (t == 0) {
-    double am = 0.0;
-    for (int k = 0; k < 8; ++k) am = fmax(am, red[k]);
-    red[0] = am;
+  if (t < 2) {
+    double mx = 0.0;
+    for (int k = 0; k < BD_THREADS / 32; ++k) mx = fmax(mx, red[t][k]);
+    cond_loc[t] = mx;
   }
-  __syncthreads();
-  amax = red[0];
-  __syncthreads();
-  if ((t & 31) == 0) red[t >> 5] = xmax;
-  __syncthreads();
-  if (t == 0) {
-    double xm = 0.0;
-    for (int k = 0; k < 8; ++k) xm = fmax(xm, red[k]);
-    record_cond(status, amax, xm);
+  cluster.sync();
+  if (rank == 0 && t == 0) {
+    double am = 0.0, xm = 0.0;
+    for (int q = 0; q < BD_CL; ++q) {
+      const double* cl = cluster.map_shared_rank(cond_loc, q);
+      am = fmax(am, cl[0]);
+      xm = fmax(xm, cl[1]);
+    }
+    record_cond(status, am, xm);
   }
+  cluster.sync();   // no CTA may exit while another can still read its shared memory
+}
+
+static mnpbem_status launch_block_inv(const float2* A, int64_t lda, int w, float2* X, int64_t ldx, float2* X2,
+                                      int64_t ldx2, int* status, cudaStream_t st) {
+  ProfScope ps(PH_BLOCKINV, st, 8.0 * w * w * w, 0.0);
+  k_block_inv<<<1, 256, 0, st>>>(A, lda, w, X, ldx, X2, ldx2, status);
+  MNP_CHECK_LAUNCH();
+  return MNPBEM_OK;
+}
+static mnpbem_status launch_block_inv(const double2* A, int64_t lda, int w, double2* X, int64_t ldx, double2* X2,
+                                      int64_t ldx2, int* status, cudaStream_t st) {
+  ProfScope ps(PH_BLOCKINV, st, 8.0 * w * w * w, 0.0);
+  k_block_inv_c128<<<BD_CL, BD_THREADS, 0, st>>>(A, lda, w, X, ldx, X2, ldx2, status);
+  MNP_CHECK_LAUNCH();
+  return MNPBEM_OK;
 }
 
 // ------------------------------------- 256-wide pivot block on a CTA cluster
 // In-place Gauss-Jordan of one w x w complex64 block (w <= 256) by a cluster
-// of PB_CL CTAs.  CTA r keeps rows [r*PB_RPC, (r+1)*PB_RPC) in registers:
-// PB_TPR threads per row, thread (row l, phase ph) holding the columns
-// ph + PB_TPR * j.  The pivots are taken in panels of 16:
-//   1. the CTA owning the panel rows stages them in shared memory, inverts
-//      the 16 x 16 pivot block X (Gauss-Jordan, one entry per thread) and
-//      forms the new panel rows R = X * P (pivot columns replaced by X);
-//   2. every CTA stages its own 16 panel-column entries C; cluster barrier;
-//      the other CTAs copy R out of the owner's shared memory (distributed
-//      shared memory reads, spread over the cluster);
-//   3. every row i outside the panel: a_ij <- [j not a pivot column] a_ij
-//      - sum_k C_ik R_kj; the panel rows take R.
-// One cluster barrier per panel (R is double-buffered: a CTA may still be
-// copying panel p's R when the owner of panel p + 1 writes the other buffer),
-// 16 panels for w = 256.
+// of PB_CL CTAs.  CTA r keeps rows [r*PB_RPC, (r+1)*PB_RPC) in registers: thread
+// (ty, tx) the 4 x 4 entries of rows 4 ty + i and columns tx + 64 j.  The pivots
+// are taken in panels of 16:
+//   1. the CTA that owns the panel rows writes them (16 x 256, raw) to a
+//      scratch in global memory; every CTA stages its own 16 panel-column
+//      entries C; cluster barrier;
+//   2. every CTA reads the panel rows P back (L2) into shared memory, with the
+//      panel's own columns replaced by the identity, while its first warp
+//      inverts the 16 x 16 pivot block in registers (X);
+//   3. D = C X for the CTA's rows (for the panel rows themselves D = -X), and
+//      a_ij <- [i, j not pivots] a_ij - sum_k D_ik P_kj.
+// The panel goes through L2 because a broadcast out of one SM's shared memory
+// (distributed shared memory, 7 x 32 KB from one source per panel) is limited
+// by that SM's port; inverting the pivot block in every CTA saves a second
+// exchange, and D = C X (32 x 16 x 16 per CTA) replaces R = X P on one CTA.
+// One cluster barrier per panel, 16 panels for w = 256: the panel scratch and
+// the staging alternate, and a CTA that writes panel p + 2 has passed barrier
+// p + 1, which every CTA reaches after reading panel p.
+// The rank-16 updates are 34 us of FP32 FMA on eight SMs; PIV256 us measured
+// for w = 256 (248 us with the pivot block and R on the owner and R read from
+// its shared memory).
 // Rows and columns beyond w are identity and stay identity.
-constexpr int PB_W = 256, PB_CL = 8, PB_RPC = PB_W / PB_CL, PB_THREADS = 512;
-constexpr int PB_TPR = PB_THREADS / PB_RPC, PB_CPT = PB_W / PB_TPR, PB_PAN = 16;
-constexpr int PB_SMEM = (3 * PB_PAN * PB_W + 2 * PB_RPC * PB_PAN + 2 * PB_PAN * PB_PAN) * (int)sizeof(float2);
-static_assert(PB_PAN % PB_TPR == 0 || PB_TPR % PB_PAN == 0, "panel / thread layout");
+constexpr int PB_W = 256, PB_CL = 8, PB_RPC = PB_W / PB_CL, PB_THREADS = 512, PB_PAN = 16;
+constexpr int PB_LD = PB_RPC + 2;      // row stride of C and D: 16-byte aligned, spread over the banks
+constexpr int PB_SCRATCH = 2 * PB_PAN * PB_W * (int)sizeof(float2);
 static_assert(PB_RPC % PB_PAN == 0, "a panel lies inside one CTA");
+static_assert(PB_THREADS == 64 * (PB_RPC / 4), "4 x 4 entries per thread");
+
+// 16 x 16 Gauss-Jordan in one warp: lane (r, h) holds row r, columns 8 h .. 8 h + 7
+__device__ __forceinline__ bool warp_inv16(float2 (&v)[8], int lane) {
+  const int r = lane & 15, h = lane >> 4;
+  bool ok = true;
+#pragma unroll
+  for (int k = 0; k < PB_PAN; ++k) {
+    const int kh = k >> 3, kr = k & 7;
+    const float2 piv = make_float2(__shfl_sync(0xffffffffu, v[kr].x, k + 16 * kh),
+                                   __shfl_sync(0xffffffffu, v[kr].y, k + 16 * kh));
+    const float2 col = make_float2(__shfl_sync(0xffffffffu, v[kr].x, r + 16 * kh),
+                                   __shfl_sync(0xffffffffu, v[kr].y, r + 16 * kh));
+    const float n2 = piv.x * piv.x + piv.y * piv.y;
+    ok = ok && n2 > 1e-30f && n2 < 1e30f;
+    const float rn = 1.f / n2;
+    const float2 inv = make_float2(piv.x * rn, -piv.y * rn);
+#pragma unroll
+    for (int c = 0; c < 8; ++c) {
+      const float2 row = make_float2(__shfl_sync(0xffffffffu, v[c].x, k + 16 * h),
+                                     __shfl_sync(0xffffffffu, v[c].y, k + 16 * h));
+      const bool pc = c == kr && h == kh;              // the pivot column
+      const float2 rk = pc ? inv : cmul(row, inv);
+      const float2 base = pc ? make_float2(0.f, 0.f) : v[c];
+      v[c] = (r == k) ? rk : csub(base, cmul(col, rk));
+    }
+  }
+  return ok;
+}
 
 __global__ void __cluster_dims__(PB_CL, 1, 1) __launch_bounds__(PB_THREADS, 1)
     k_block_inv_cluster(const float2* A, int64_t lda, int w, float2* X, int64_t ldx, int* status,
-                        float2* __restrict__ Xr) {
+                        float2* __restrict__ Xr, float2* Pg) {
   namespace cg = cooperative_groups;
   cg::cluster_group cluster = cg::this_cluster();
-  extern __shared__ float2 pb_smem[];
-  float2* Rb = pb_smem;                              // [2][PAN][W]  new panel rows
-  float2* P = Rb + 2 * PB_PAN * PB_W;                // [PAN][W]     owner: raw panel rows
-  float2* Cb = P + PB_PAN * PB_W;                    // [2][RPC][PAN] own panel-column entries
-  float2* Xs = Cb + 2 * PB_RPC * PB_PAN;             // [2][PAN][PAN] pivot block, two copies (owner)
-  const int rank = (int)cluster.block_rank();
-  const int t = threadIdx.x, lr = t / PB_TPR, ph = t % PB_TPR;
-  const int grow = rank * PB_RPC + lr;
+  __shared__ __align__(16) float2 Ps[PB_PAN][PB_W];    // panel rows, panel columns = identity
+  __shared__ __align__(16) float2 Cs[PB_PAN][PB_LD];   // own panel-column entries, [k][row]
+  __shared__ __align__(16) float2 Ds[PB_PAN][PB_LD];   // D = C X, [k][row]
+  __shared__ float2 Xs[PB_PAN][PB_PAN];
   __shared__ float cond_red[PB_THREADS / 32], cond_loc[2];
-  float2 a[PB_CPT];
+  const int rank = (int)cluster.block_rank();
+  const int t = threadIdx.x, tx = t & 63, ty = t >> 6, warp = t >> 5, lane = t & 31;
+  const int row0 = rank * PB_RPC + 4 * ty;             // first of this thread's rows
+  float2 a[4][4];
   float amax = 0.f;
 #pragma unroll
-  for (int j = 0; j < PB_CPT; ++j) {
-    const int c = ph + PB_TPR * j;
-    a[j] = (grow < w && c < w) ? A[(int64_t)grow * lda + c] : make_float2(grow == c ? 1.f : 0.f, 0.f);
-    if (grow < w && c < w) amax = fmaxf(amax, sqrtf(a[j].x * a[j].x + a[j].y * a[j].y));
-  }
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int gr = row0 + i, c = tx + 64 * j;
+      a[i][j] = (gr < w && c < w) ? A[(int64_t)gr * lda + c] : make_float2(gr == c ? 1.f : 0.f, 0.f);
+      if (gr < w && c < w) amax = fmaxf(amax, sqrtf(a[i][j].x * a[i][j].x + a[i][j].y * a[i][j].y));
+    }
   // CTA maximum of a per-thread value into cond_loc[slot]
   const auto cta_max = [&](float v, int slot) {
     for (int o = 16; o; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-    if ((t & 31) == 0) cond_red[t >> 5] = v;
+    if (lane == 0) cond_red[warp] = v;
     __syncthreads();
     if (t == 0) {
       float mx = 0.f;
@@ -973,107 +1136,105 @@ __global__ void __cluster_dims__(PB_CL, 1, 1) __launch_bounds__(PB_THREADS, 1)
   cta_max(amax, 0);
   const int npan = (w + PB_PAN - 1) / PB_PAN;
   for (int pp = 0; pp < npan; ++pp) {
-    const int p0 = pp * PB_PAN, owner = p0 / PB_RPC, lp0 = p0 % PB_RPC, buf = pp & 1;
-    float2* R = Rb + buf * PB_PAN * PB_W;
-    float2* C = Cb + buf * PB_RPC * PB_PAN;
-    __syncthreads();                                  // the previous panel's reads of P / C are done
-    // own panel-column entries (every CTA)
-#pragma unroll
-    for (int j = 0; j < PB_CPT; ++j) {
-      const int c = ph + PB_TPR * j;
-      if (c >= p0 && c < p0 + PB_PAN) C[lr * PB_PAN + (c - p0)] = a[j];
-    }
-    if (rank == owner) {
-      if (lr >= lp0 && lr < lp0 + PB_PAN) {
-#pragma unroll
-        for (int j = 0; j < PB_CPT; ++j) P[(lr - lp0) * PB_W + ph + PB_TPR * j] = a[j];
-      }
-      __syncthreads();
-      // 16 x 16 Gauss-Jordan of the pivot block, one entry per thread; the
-      // pivot steps alternate between two copies of the block, so that one
-      // block barrier per step suffices
-      const int bi = t / PB_PAN, bj = t % PB_PAN;
-      const bool act = t < PB_PAN * PB_PAN;
-      if (act) Xs[bi * PB_PAN + bj] = P[bi * PB_W + p0 + bj];
-      __syncthreads();
-      for (int k = 0; k < PB_PAN; ++k) {
-        const float2* Xc = Xs + (k & 1) * PB_PAN * PB_PAN;
-        float2* Xn = Xs + ((k & 1) ^ 1) * PB_PAN * PB_PAN;
-        if (act) {
-          const float2 piv = Xc[k * PB_PAN + k];
-          const float n2 = piv.x * piv.x + piv.y * piv.y;
-          if (t == 0 && !(n2 > 1e-30f && n2 < 1e30f)) atomicOr(status, 1);
-          const float rn = 1.f / n2;
-          const float2 inv = make_float2(piv.x * rn, -piv.y * rn);
-          const float2 aik = Xc[bi * PB_PAN + k], akj = Xc[k * PB_PAN + bj], aij = Xc[bi * PB_PAN + bj];
-          float2 v;
-          if (bi == k && bj == k) v = inv;
-          else if (bi == k) v = cmul(akj, inv);
-          else if (bj == k) v = make_float2(-(aik.x * inv.x - aik.y * inv.y), -(aik.x * inv.y + aik.y * inv.x));
-          else v = csub(aij, cmul(aik, cmul(akj, inv)));
-          Xn[bi * PB_PAN + bj] = v;
-        }
-        __syncthreads();
-      }
-      // PB_PAN is even: the result is back in the first copy
-      static_assert(PB_PAN % 2 == 0, "the pivot block's Gauss-Jordan ends in its first copy");
-      // R = X * P with the pivot columns replaced by X
-      for (int e = t; e < PB_PAN * PB_W; e += PB_THREADS) {
-        const int i = e / PB_W, c = e % PB_W;
-        float2 r;
-        if (c >= p0 && c < p0 + PB_PAN) {
-          r = Xs[i * PB_PAN + (c - p0)];
-        } else {
-          r = make_float2(0.f, 0.f);
-#pragma unroll
-          for (int k = 0; k < PB_PAN; ++k) cfma(r, Xs[i * PB_PAN + k], P[k * PB_W + c]);
-        }
-        R[e] = r;
-      }
-    }
-    cluster.sync();
-    if (rank != owner) {
-      const float4* src = reinterpret_cast<const float4*>(cluster.map_shared_rank(R, owner));
-      float4* dst = reinterpret_cast<float4*>(R);
-#pragma unroll 4
-      for (int e = t; e < PB_PAN * PB_W / 2; e += PB_THREADS) dst[e] = src[e];
-      __syncthreads();
-    }
-    // update of this CTA's rows
-    const bool prow = (rank == owner) && lr >= lp0 && lr < lp0 + PB_PAN;
+    const int p0 = pp * PB_PAN, owner = p0 / PB_RPC, lp0 = p0 % PB_RPC;
+    float2* Pb = Pg + (pp & 1) * PB_PAN * PB_W;
+    const int jp = p0 >> 6, cp = tx - (p0 & 63);       // this thread's panel column, if 0 <= cp < 16
+    const bool inpan = cp >= 0 && cp < PB_PAN;
+    const bool prow = rank == owner && 4 * ty >= lp0 && 4 * ty < lp0 + PB_PAN;
     if (prow) {
 #pragma unroll
-      for (int j = 0; j < PB_CPT; ++j) a[j] = R[(lr - lp0) * PB_W + ph + PB_TPR * j];
-    } else {
-      float2 cr[PB_PAN];
+      for (int i = 0; i < 4; ++i)
 #pragma unroll
-      for (int k = 0; k < PB_PAN; ++k) cr[k] = C[lr * PB_PAN + k];
+        for (int j = 0; j < 4; ++j) Pb[(4 * ty + i - lp0) * PB_W + tx + 64 * j] = a[i][j];
+    }
+    if (inpan) {
 #pragma unroll
-      for (int j = 0; j < PB_CPT; ++j) {
-        const int c = ph + PB_TPR * j;
-        float2 acc = (c >= p0 && c < p0 + PB_PAN) ? make_float2(0.f, 0.f) : a[j];
+      for (int j = 0; j < 4; ++j)
+        if (j == jp) {
 #pragma unroll
-        for (int k = 0; k < PB_PAN; ++k) {
-          const float2 rv = R[k * PB_W + c];
-          acc.x = fmaf(-cr[k].x, rv.x, acc.x);
-          acc.x = fmaf(cr[k].y, rv.y, acc.x);
-          acc.y = fmaf(-cr[k].x, rv.y, acc.y);
-          acc.y = fmaf(-cr[k].y, rv.x, acc.y);
+          for (int i = 0; i < 4; ++i) Cs[cp][4 * ty + i] = a[i][j];
         }
-        a[j] = acc;
+    }
+    cluster.sync();
+    if (warp == 0) {
+      const int r = lane & 15, h = lane >> 4;
+      float2 v[8];
+#pragma unroll
+      for (int c = 0; c < 8; c += 2) {
+        const float4 q = __ldcg(reinterpret_cast<const float4*>(Pb + r * PB_W + p0 + 8 * h + c));
+        v[c] = make_float2(q.x, q.y);
+        v[c + 1] = make_float2(q.z, q.w);
+      }
+      const bool ok = warp_inv16(v, lane);
+      if (!ok && lane == 0 && rank == owner) atomicOr(status, 1);
+#pragma unroll
+      for (int c = 0; c < 8; ++c) Xs[r][8 * h + c] = v[c];
+    } else {
+      constexpr int NL = PB_PAN * PB_W / 2;            // float4 loads by the other warps
+#pragma unroll 3
+      for (int e = t - 32; e < NL; e += PB_THREADS - 32) {
+        const int k = e / (PB_W / 2), c = 2 * (e % (PB_W / 2));
+        float4 q = __ldcg(reinterpret_cast<const float4*>(Pb + k * PB_W + c));
+        if (c >= p0 && c < p0 + PB_PAN)
+          q = make_float4(c - p0 == k ? 1.f : 0.f, 0.f, c + 1 - p0 == k ? 1.f : 0.f, 0.f);
+        *reinterpret_cast<float4*>(&Ps[k][c]) = q;
+      }
+    }
+    __syncthreads();
+    {
+      // warp = pivot k, lane = row
+      const int lr = lane, k = warp;
+      float2 d = make_float2(0.f, 0.f);
+      if (rank == owner && lr >= lp0 && lr < lp0 + PB_PAN) {
+        d = make_float2(-Xs[lr - lp0][k].x, -Xs[lr - lp0][k].y);
+      } else {
+#pragma unroll
+        for (int l = 0; l < PB_PAN; ++l) cfma(d, Cs[l][lr], Xs[l][k]);
+      }
+      Ds[k][lr] = d;
+    }
+    if (prow) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+#pragma unroll
+        for (int j = 0; j < 4; ++j) a[i][j] = make_float2(0.f, 0.f);
+    }
+    if (inpan) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j)
+        if (j == jp) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) a[i][j] = make_float2(0.f, 0.f);
+        }
+    }
+    __syncthreads();
+#pragma unroll 4
+    for (int k = 0; k < PB_PAN; ++k) {
+      const float4 d01 = *reinterpret_cast<const float4*>(&Ds[k][4 * ty]);
+      const float4 d23 = *reinterpret_cast<const float4*>(&Ds[k][4 * ty + 2]);
+      const float2 d[4] = {make_float2(d01.x, d01.y), make_float2(d01.z, d01.w), make_float2(d23.x, d23.y),
+                           make_float2(d23.z, d23.w)};
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float2 rv = Ps[k][tx + 64 * j];
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          a[i][j].x = fmaf(-d[i].x, rv.x, a[i][j].x);
+          a[i][j].x = fmaf(d[i].y, rv.y, a[i][j].x);
+          a[i][j].y = fmaf(-d[i].x, rv.y, a[i][j].y);
+          a[i][j].y = fmaf(-d[i].y, rv.x, a[i][j].y);
+        }
       }
     }
   }
   float xmax = 0.f;
-  if (grow < w) {
 #pragma unroll
-    for (int j = 0; j < PB_CPT; ++j) {
-      const int c = ph + PB_TPR * j;
-      if (c < w) xmax = fmaxf(xmax, sqrtf(a[j].x * a[j].x + a[j].y * a[j].y));
-    }
-  }
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j)
+      if (row0 + i < w && tx + 64 * j < w)
+        xmax = fmaxf(xmax, sqrtf(a[i][j].x * a[i][j].x + a[i][j].y * a[i][j].y));
   cta_max(xmax, 1);
-  // no CTA may exit while another can still write into (or read) its shared memory
   cluster.sync();
   if (rank == 0 && t == 0) {
     float am = 0.f, xm = 0.f;
@@ -1085,33 +1246,32 @@ __global__ void __cluster_dims__(PB_CL, 1, 1) __launch_bounds__(PB_THREADS, 1)
     record_cond(status, am, xm);
   }
   // X may be the input block itself: every CTA read its rows at the start
-  if (grow < w) {
 #pragma unroll
-    for (int j = 0; j < PB_CPT; ++j) {
-      const int c = ph + PB_TPR * j;
+  for (int i = 0; i < 4; ++i) {
+    const int gr = row0 + i;
+    if (gr >= w) continue;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const int c = tx + 64 * j;
       if (c < w) {
-        X[(int64_t)grow * ldx + c] = a[j];
+        X[(int64_t)gr * ldx + c] = a[i][j];
         if (Xr) {   // copy rounded to TF32 (nearest): the A operand of tensor-core products
           uint32_t x, y;
-          asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(x) : "f"(a[j].x));
-          asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(y) : "f"(a[j].y));
-          Xr[(int64_t)grow * w + c] = make_float2(__uint_as_float(x), __uint_as_float(y));
+          asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(x) : "f"(a[i][j].x));
+          asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(y) : "f"(a[i][j].y));
+          Xr[(int64_t)gr * w + c] = make_float2(__uint_as_float(x), __uint_as_float(y));
         }
       }
     }
   }
-  cluster.sync();
+  cluster.sync();   // no CTA may exit while another can still read its shared memory
 }
 
 static mnpbem_status launch_block_inv_cluster(const float2* A, int64_t lda, int w, float2* X, int64_t ldx,
-                                              int* status, cudaStream_t st, float2* Xr = nullptr) {
-  static bool attr_set = false;
-  if (!attr_set) {
-    MNP_CUDA(cudaFuncSetAttribute(k_block_inv_cluster, cudaFuncAttributeMaxDynamicSharedMemorySize, PB_SMEM));
-    attr_set = true;
-  }
+                                              int* status, DevBuf& pan, cudaStream_t st, float2* Xr = nullptr) {
+  MNP_TRY(pan.ensure(PB_SCRATCH));
   ProfScope ps(PH_BLOCKINV, st, 8.0 * w * w * w, 0.0);
-  k_block_inv_cluster<<<PB_CL, PB_THREADS, PB_SMEM, st>>>(A, lda, w, X, ldx, status, Xr);
+  k_block_inv_cluster<<<PB_CL, PB_THREADS, 0, st>>>(A, lda, w, X, ldx, status, Xr, pan.as<float2>());
   MNP_CHECK_LAUNCH();
   return MNPBEM_OK;
 }
@@ -1216,11 +1376,9 @@ mnpbem_status gj_invert(cplx<R>* A, int64_t n, int64_t lda, GJWork<R>& w, GemmFn
           tc_gemm_eligible(*tc, n, bw, bw, Cf, bw, Af + k0, lda, b0) &&
           tc_gemm_eligible(*tc, n, n, bw, Cf, bw, Af, lda, b1)) {
         if (bw <= 64) {
-          ProfScope ps(PH_BLOCKINV, st, 8.0 * bw * bw * bw, 0.0);
-          k_block_inv<R><<<1, 256, 0, st>>>(A + k0 * lda + k0, lda, bw, X, bw, w.status.template as<int>());
-          MNP_CHECK_LAUNCH();
+          MNP_TRY(launch_block_inv(Af + k0 * lda + k0, lda, bw, Xf, bw, nullptr, 0, w.status.template as<int>(), st));
         } else if (bw <= PB_W) {
-          MNP_TRY(launch_block_inv_cluster(Af + k0 * lda + k0, lda, bw, Xf, bw, w.status.template as<int>(), st));
+          MNP_TRY(launch_block_inv_cluster(Af + k0 * lda + k0, lda, bw, Xf, bw, w.status.template as<int>(), w.pan, st));
         } else {
           // wider pivot blocks: inner Gauss-Jordan (256-wide steps) on a copy
           MNP_CUDA(cudaMemcpy2DAsync(X, cs * bw, A + k0 * lda + k0, cs * lda, cs * bw, bw, cudaMemcpyDeviceToDevice,
@@ -1246,12 +1404,10 @@ mnpbem_status gj_invert(cplx<R>* A, int64_t n, int64_t lda, GJWork<R>& w, GemmFn
     // 2. X <- inv(A_kk): one shared-memory kernel for blocks up to 64, else
     //    an inner Gauss-Jordan with 64-wide steps on a copy of the block
     if (bw <= 64) {
-      ProfScope ps(PH_BLOCKINV, st, 8.0 * bw * bw * bw, 0.0);
-      k_block_inv<R><<<1, 256, 0, st>>>(Ccol + k0 * bw, bw, bw, X, bw, w.status.template as<int>());
-      MNP_CHECK_LAUNCH();
+      MNP_TRY(launch_block_inv(Ccol + k0 * bw, bw, bw, X, bw, nullptr, 0, w.status.template as<int>(), st));
     } else if (sizeof(R) == 4 && bw <= PB_W) {
       MNP_TRY(launch_block_inv_cluster(reinterpret_cast<const float2*>(Ccol + k0 * bw), bw, bw,
-                                       reinterpret_cast<float2*>(X), bw, w.status.template as<int>(), st));
+                                       reinterpret_cast<float2*>(X), bw, w.status.template as<int>(), w.pan, st));
     } else {
       MNP_CUDA(cudaMemcpyAsync(X, Ccol + k0 * bw, cs * bw * bw, cudaMemcpyDeviceToDevice, st));
       MNP_TRY(gj_invert<R>(X, bw, bw, *w.inner, big_gemm, ctx, st));
@@ -1327,25 +1483,22 @@ static void copy_panel(const cplx<R>* src, int64_t lds, int64_t rows, int cols, 
 }
 
 // A_kk <- inv(A_kk) in place, with a copy in X (ld bw): 64-wide blocks with
-// partial pivoting on one CTA, 256-wide complex64 blocks on a CTA cluster,
-// whose copy in X is rounded to TF32 (nearest) for the tensor-core products
-// (the tensor cores would otherwise truncate it)
+// partial pivoting, 256-wide complex64 blocks on a CTA cluster, whose copy in X
+// is rounded to TF32 (nearest) for the tensor-core products (the tensor cores
+// would otherwise truncate it)
 template <typename R>
-static mnpbem_status block_inverse(cplx<R>* Akk, int64_t lda, int bw, cplx<R>* X, int* status, cudaStream_t st) {
-  if (bw <= 64) {
-    ProfScope ps(PH_BLOCKINV, st, 8.0 * bw * bw * bw, 0.0);
-    k_block_inv<R><<<1, 256, 0, st>>>(Akk, lda, bw, X, bw, status);
-    MNP_CHECK_LAUNCH();
-    MNP_CUDA(cudaMemcpy2DAsync(Akk, sizeof(cplx<R>) * lda, X, sizeof(cplx<R>) * bw, sizeof(cplx<R>) * bw, bw,
-                               cudaMemcpyDeviceToDevice, st));
-    return MNPBEM_OK;
-  }
+mnpbem_status block_inverse(cplx<R>* Akk, int64_t lda, int bw, cplx<R>* X, int* status, DevBuf& pan,
+                            cudaStream_t st) {
+  if (bw <= 64) return launch_block_inv(Akk, lda, bw, X, bw, Akk, lda, status, st);
   if (sizeof(R) == 4 && bw <= PB_W)
     return launch_block_inv_cluster(reinterpret_cast<const float2*>(Akk), lda, bw, reinterpret_cast<float2*>(Akk), lda,
-                                    status, st, reinterpret_cast<float2*>(X));
+                                    status, pan, st, reinterpret_cast<float2*>(X));
   set_error("block LDU: diagonal blocks of %d rows are not supported in this precision", bw);
   return MNPBEM_ERR_UNSUPPORTED;
 }
+
+template mnpbem_status block_inverse<float>(float2*, int64_t, int, float2*, int*, DevBuf&, cudaStream_t);
+template mnpbem_status block_inverse<double>(double2*, int64_t, int, double2*, int*, DevBuf&, cudaStream_t);
 
 template <typename R>
 mnpbem_status ldu_factor(cplx<R>* A, int64_t n, int64_t lda, LDUWork<R>& w, int* status, GemmFn<R> gemm,
@@ -1368,7 +1521,7 @@ mnpbem_status ldu_factor(cplx<R>* A, int64_t n, int64_t lda, LDUWork<R>& w, int*
       const int64_t ks = k0 + s;
       const int bs = (int)std::min<int64_t>(b, e - ks);
       const int64_t kb = ks + bs, below = n - kb;
-      MNP_TRY(block_inverse<R>(A + ks * lda + ks, lda, bs, X, status, st));
+      MNP_TRY(block_inverse<R>(A + ks * lda + ks, lda, bs, X, status, w.pan, st));
       if (below > 0) {
         Cx* Cs = Cc + (kb - k0) * B + s;
         // unscaled column panel (the A operand of every update of this step)

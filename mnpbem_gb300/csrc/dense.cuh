@@ -33,6 +33,7 @@ void round_tf32(float* x, int64_t count, cudaStream_t st);
 template <typename R>
 struct GJWork {
   DevBuf ccol, rrow, ncol, xblk, status;
+  DevBuf pan;                        // panel scratch of the 256-wide block inverse
   int nb = 64;
   bool round_a = true;               // round the A operand of the tensor-core updates to TF32 (nearest)
   bool fused = true;                 // tensor-core path: products written in place (no panel copies)
@@ -69,10 +70,16 @@ mnpbem_status gj_status_copy(GJWork<R>& w, int* host2, cudaStream_t st);
 template <typename R>
 struct LDUWork {
   DevBuf ccol, rrow, xblk, tmp;
+  DevBuf pan;            // panel scratch of the 256-wide block inverse
   int b = 64;
   int m = 1;
   bool round_a = true;   // tensor-core path: A operands rounded to nearest TF32
 };
+// A_kk <- inv(A_kk) in place (bw <= 64, or 256 in complex64), with a copy in X
+// (row stride bw; rounded to TF32 for bw > 64)
+template <typename R>
+mnpbem_status block_inverse(cplx<R>* Akk, int64_t lda, int bw, cplx<R>* X, int* status, DevBuf& pan,
+                            cudaStream_t st);
 // status: int[2] in device memory (see above)
 template <typename R>
 mnpbem_status ldu_factor(cplx<R>* A, int64_t n, int64_t lda, LDUWork<R>& w, int* status, GemmFn<R> gemm,
