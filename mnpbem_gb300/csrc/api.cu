@@ -1010,7 +1010,7 @@ void* tc_ctx(mnpbem_geom* G, Lane& L) { return G->tc_enabled ? (void*)&L.tc : nu
 // (cluster block inverse), else 64 (single-CTA block inverse with pivoting)
 template <typename R>
 int lu_block(const mnpbem_geom* G, void* ctx) {
-  return (sizeof(R) == 4 && ctx && G->g.n >= 1024) ? 256 : 64;
+  return (sizeof(R) == 4 && ctx && G->g.n > 64) ? 256 : 64;
 }
 
 // Lane matrices after initmat: mat[0] LDU(G1), mat[1] LDU(G2), mat[2] Sigma1,
@@ -1085,7 +1085,7 @@ mnpbem_status stage_initmat(mnpbem_geom* G, Lane& L, bool direct) {
   // 512-wide Gauss-Jordan steps 1.365 against 1.265 wavelength-solves/s for
   // rank-512 / 256-wide; at 4000 faces the 256-wide steps were faster)
   const bool large = n >= 12000;
-  gjw<R>(L).nb = (ctx && n >= 1024) ? (G->gj_nb ? G->gj_nb : (large ? 512 : 256)) : 64;
+  gjw<R>(L).nb = (ctx && n > 64) ? (G->gj_nb ? G->gj_nb : (large ? 512 : 256)) : 64;
   gjw<R>(L).round_a = G->tf32_rna;
   gjw<R>(L).fused = G->gj_fused;
   LDUWork<R>& lw = luw<R>(L);

@@ -790,6 +790,15 @@ __device__ __forceinline__ void record_cond(int* status, double amax, double xma
   atomicMax(status + 1, __float_as_int((float)c));
 }
 
+// 1 / x in FP32: the hardware's approximate reciprocal and one Newton step
+// (x in 1e-30 .. 1e30; within 1 ulp of the rounded quotient, and without the
+// division's range handling on the serial chain of the pivot steps)
+__device__ __forceinline__ float rcp_newton(float x) {
+  float r;
+  asm("rcp.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
+  return fmaf(r, fmaf(-x, r, 1.f), r);
+}
+
 // Row of the largest key among 64 candidates, keys of rows lane and lane + 32 in
 // k0 and k1 (0 = not a candidate); the lowest row on ties.  Every lane gets it.
 __device__ __forceinline__ int argmax64(unsigned k0, unsigned k1) {
@@ -858,31 +867,41 @@ __global__ void __launch_bounds__(256) k_block_inv(const float2* A, int64_t lda,
       }
     const float2 piv = pcol[buf][rp];
     const float n2 = piv.x * piv.x + piv.y * piv.y;
-    const float rn2 = 1.f / n2;
+    const float rn2 = rcp_newton(n2);
     const float2 inv = make_float2(piv.x * rn2, -piv.y * rn2);
     if (t == 0) {
       if (!(n2 > 1e-30f && n2 < 1e30f)) atomicOr(status, 1);
       prow_of[p] = rp;
       pos_of[rp] = p;
     }
-    __syncthreads();
-    // a_rc <- a_rc - pc_r pr_c with pr_c = a_(rp)c / a_pp.  The pivot row keeps
-    // pr itself (0 + 1 * pr), the pivot column takes -pc / a_pp (0 - pc / a_pp).
-    float2 pr[4];
-#pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int c = tx + 16 * j;
-      pr[j] = (c == p) ? inv : cmul(prow[buf][c], inv);
-    }
+    // a_rc <- a_rc - m_r row_c with m_r = a_rp / a_pp; the pivot row keeps
+    // row_c / a_pp (from 0 with m = -1 / a_pp), the pivot column -m_r (from 0
+    // with row_p = 1)
+    float2 m[4];
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      const int r = ty + 16 * i;
-      const bool isrow = r == rp;
-      const float2 m = isrow ? make_float2(-1.f, 0.f) : pcol[buf][r];
+      m[i] = cmul(pcol[buf][ty + 16 * i], inv);
+      if (ty + 16 * i == rp) {
+        m[i] = make_float2(-inv.x, -inv.y);
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float2 base = (isrow || tx + 16 * j == p) ? make_float2(0.f, 0.f) : a[i][j];
-        a[i][j] = csub(base, cmul(m, pr[j]));
+        for (int j = 0; j < 4; ++j) a[i][j] = make_float2(0.f, 0.f);
+      }
+    }
+    __syncthreads();
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      float2 row = prow[buf][tx + 16 * j];
+      if (tx + 16 * j == p) {
+        row = make_float2(1.f, 0.f);
+#pragma unroll
+        for (int i = 0; i < 4; ++i) a[i][j] = make_float2(0.f, 0.f);
+      }
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        a[i][j].x = fmaf(-m[i].x, row.x, a[i][j].x);
+        a[i][j].y = fmaf(-m[i].x, row.y, a[i][j].y);
+        a[i][j].x = fmaf(m[i].y, row.y, a[i][j].x);
+        a[i][j].y = fmaf(-m[i].y, row.x, a[i][j].y);
       }
     }
   }
@@ -917,13 +936,15 @@ __global__ void __launch_bounds__(256) k_block_inv(const float2* A, int64_t lda,
 // CTAs: CTA q keeps columns 8 q .. 8 q + 7 (thread = row, two columns each), so
 // that the FP64 pipes of eight SMs share the rank-1 updates (FP64 runs at two
 // FMA per clock per SM: 64^3 complex multiply-adds are 270 us on one SM).
-// Step p: the owner of column p writes it, with an integer key of |re| + |im|
-// (the pivot measure of LAPACK's izamax), into every CTA's shared memory;
-// cluster barrier; every warp picks the pivot row from the keys; the row's
-// eight local columns are scaled by the reciprocal pivot, and each thread
-// updates its two entries.  The column buffer alternates, so one cluster
-// barrier per step suffices: a CTA that writes column p + 2 into a buffer has
-// passed barrier p + 1, which every CTA reaches after reading column p.
+// Step p: every warp picks the pivot row from integer keys of |re| + |im| (the
+// pivot measure of LAPACK's izamax); the row's eight local columns go to shared
+// memory, and each thread updates its two entries.  The owner of column p + 1
+// updates it first and writes it, with its keys, into every CTA's shared memory
+// before it arrives at the cluster barrier of step p + 1, so that the exchange
+// overlaps the other updates.  The buffers alternate: a CTA that writes column
+// p + 2 has passed barrier p + 1, at which every CTA arrives after reading
+// column p, and one that writes its pivot row p + 2 has passed barrier p + 2,
+// at which its threads arrive after update p.
 // One CTA with the pivot scan in every thread took 1059 us per block of 64;
 // this takes PIVDOUBLE us.
 constexpr int BD_CL = 8, BD_THREADS = 256;
@@ -932,7 +953,7 @@ __global__ void __cluster_dims__(BD_CL, 1, 1) __launch_bounds__(BD_THREADS)
                      int* status) {
   namespace cg = cooperative_groups;
   cg::cluster_group cluster = cg::this_cluster();
-  __shared__ double2 pcol[2][64], prow[8], inv_s;
+  __shared__ double2 pcol[2][64], prow[2][8];
   __shared__ unsigned pkey[2][64];
   __shared__ int prow_of[64], pos_of[64];
   __shared__ double red[2][BD_THREADS / 32], cond_loc[2];
@@ -947,51 +968,67 @@ __global__ void __cluster_dims__(BD_CL, 1, 1) __launch_bounds__(BD_THREADS)
     if (r < w && c < w) amax = fmax(amax, sqrt(cabs2(a[j])));
   }
   bool free0 = lane < w, free1 = lane + 32 < w;
-  cluster.sync();   // every CTA runs before its shared memory is written
-  for (int p = 0; p < w; ++p) {
-    const int buf = p & 1, lc = p & 7;
-    const bool owner = rank == (p >> 3);
-    if (owner && cg2 == (lc >> 1)) {
-      const double2 v = (lc & 1) ? a[1] : a[0];
-      const unsigned key = (unsigned)__double2hiint(fabs(v.x) + fabs(v.y)) + 1u;
+  // column p (value v of this thread's row) and its keys into every CTA
+  const auto publish = [&](int p, double2 v) {
+    const unsigned key = (unsigned)__double2hiint(fabs(v.x) + fabs(v.y)) + 1u;
 #pragma unroll
-      for (int q = 0; q < BD_CL; ++q) {
-        cluster.map_shared_rank(&pcol[buf][0], q)[r] = v;
-        cluster.map_shared_rank(&pkey[buf][0], q)[r] = key;
-      }
+    for (int q = 0; q < BD_CL; ++q) {
+      cluster.map_shared_rank(&pcol[p & 1][0], q)[r] = v;
+      cluster.map_shared_rank(&pkey[p & 1][0], q)[r] = key;
     }
-    cluster.sync();
+  };
+  cluster.sync();   // every CTA runs before its shared memory is written
+  if (rank == 0 && cg2 == 0) publish(0, a[0]);
+  cluster.barrier_arrive();
+  for (int p = 0; p < w; ++p) {
+    const int buf = p & 1, lc = p - 8 * rank;      // local column of the pivot, if 0 <= lc < 8
+    cluster.barrier_wait();
     const unsigned k0 = free0 ? pkey[buf][lane] : 0u, k1 = free1 ? pkey[buf][lane + 32] : 0u;
     const int rp = argmax64(k0, k1);
     free0 = free0 && rp != lane;
     free1 = free1 && rp != lane + 32;
-    // unscaled pivot row, and the reciprocal pivot from one thread
-    if (r == rp) {
-      prow[2 * cg2] = a[0];
-      prow[2 * cg2 + 1] = a[1];
+    const bool isrow = r == rp;
+    // the pivot row's local entries, scaled by the reciprocal pivot in one warp
+    // (1 in the pivot column): a_rc <- a_rc - m_r row_c with m_r = a_rp, the
+    // pivot row (m = -1) and the pivot column starting from 0
+    if (isrow) {
+      prow[buf][2 * cg2] = lc == 2 * cg2 ? make_double2(1.0, 0.0) : a[0];
+      prow[buf][2 * cg2 + 1] = lc == 2 * cg2 + 1 ? make_double2(1.0, 0.0) : a[1];
+      a[0] = a[1] = make_double2(0.0, 0.0);
     }
-    if (t == 0) {
+    double2 inv = make_double2(0.0, 0.0);
+    if (t < 32) {
       const double2 piv = pcol[buf][rp];
       const double n2 = piv.x * piv.x + piv.y * piv.y, rn2 = 1.0 / n2;
-      inv_s = make_double2(piv.x * rn2, -piv.y * rn2);
-      if (rank == 0 && !(n2 > 1e-30 && n2 < 1e30)) atomicOr(status, 1);
-      prow_of[p] = rp;
-      pos_of[rp] = p;
+      inv = make_double2(piv.x * rn2, -piv.y * rn2);
+      if (t == 0) {
+        if (rank == 0 && !(n2 > 1e-30 && n2 < 1e30)) atomicOr(status, 1);
+        prow_of[p] = rp;
+        pos_of[rp] = p;
+      }
     }
-    __syncthreads();
-    if (t < 8) prow[t] = (owner && t == lc) ? inv_s : cmul(prow[t], inv_s);
-    __syncthreads();
-    const bool isrow = r == rp;
     const double2 m = isrow ? make_double2(-1.0, 0.0) : pcol[buf][r];
-#pragma unroll
-    for (int j = 0; j < 2; ++j) {
-      const double2 pr = prow[2 * cg2 + j];
-      const bool iscol = owner && 2 * cg2 + j == lc;
-      const double2 base = (isrow || iscol) ? make_double2(0.0, 0.0) : a[j];
-      a[j].x = fma(m.y, pr.y, fma(-m.x, pr.x, base.x));
-      a[j].y = fma(-m.y, pr.x, fma(-m.x, pr.y, base.y));
+    __syncthreads();
+    if (t < 8) prow[buf][t] = cmul(prow[buf][t], inv);
+    __syncthreads();
+    const auto update = [&](int j) {
+      const double2 row = prow[buf][2 * cg2 + j];
+      const double2 base = lc == 2 * cg2 + j ? make_double2(0.0, 0.0) : a[j];
+      a[j].x = fma(m.y, row.y, fma(-m.x, row.x, base.x));
+      a[j].y = fma(-m.y, row.x, fma(-m.x, row.y, base.y));
+    };
+    // the next pivot column first: its exchange overlaps the other updates
+    const int nx = lc + 1 - 2 * cg2;               // local index of column p + 1 in this thread, if 0 or 1
+    const bool next = p + 1 < w && lc + 1 >= 0 && lc + 1 < 8 && (nx == 0 || nx == 1);
+    if (next) {
+      if (nx == 0) { update(0); publish(p + 1, a[0]); }
+      else { update(1); publish(p + 1, a[1]); }
     }
+    cluster.barrier_arrive();
+    if (!next || nx != 0) update(0);
+    if (!next || nx != 1) update(1);
   }
+  cluster.barrier_wait();
 #pragma unroll
   for (int j = 0; j < 2; ++j) {
     const int c = 8 * rank + 2 * cg2 + j;
@@ -1045,86 +1082,120 @@ static mnpbem_status launch_block_inv(const double2* A, int64_t lda, int w, doub
 // of PB_CL CTAs.  CTA r keeps rows [r*PB_RPC, (r+1)*PB_RPC) in registers: thread
 // (ty, tx) the 4 x 4 entries of rows 4 ty + i and columns tx + 64 j.  The pivots
 // are taken in panels of 16:
-//   1. the CTA that owns the panel rows writes them (16 x 256, raw) to a
-//      scratch in global memory; every CTA stages its own 16 panel-column
-//      entries C; cluster barrier;
-//   2. every CTA reads the panel rows P back (L2) into shared memory, with the
-//      panel's own columns replaced by the identity, while its first warp
-//      inverts the 16 x 16 pivot block in registers (X);
-//   3. D = C X for the CTA's rows (for the panel rows themselves D = -X), and
-//      a_ij <- [i, j not pivots] a_ij - sum_k D_ik P_kj.
+//   1. the CTA that owns the panel rows has written them (P, 16 x 256, raw) and
+//      the inverse X of their pivot block to a scratch in global memory; every
+//      CTA stages its own 16 panel-column entries C; cluster barrier;
+//   2. every CTA reads X and P back (L2); four warps form D = C X for the CTA's
+//      rows (for the panel rows themselves D = -X) while the others stage P in
+//      shared memory, with the panel's own columns replaced by the identity;
+//   3. a_ij <- [i, j not pivots] a_ij - sum_k D_ik P_kj.  Meanwhile four more
+//      warps of the CTA that owns the next panel apply the same update to the
+//      next 16 x 16 pivot block and invert it (one warp alone, competing with
+//      the update for its scheduler, took longer than the update).
 // The panel goes through L2 because a broadcast out of one SM's shared memory
 // (distributed shared memory, 7 x 32 KB from one source per panel) is limited
-// by that SM's port; inverting the pivot block in every CTA saves a second
-// exchange, and D = C X (32 x 16 x 16 per CTA) replaces R = X P on one CTA.
-// One cluster barrier per panel, 16 panels for w = 256: the panel scratch and
-// the staging alternate, and a CTA that writes panel p + 2 has passed barrier
-// p + 1, which every CTA reaches after reading panel p.
+// by that SM's port, and D = C X (32 x 16 x 16 per CTA) replaces R = X P on one
+// CTA.  One cluster barrier per panel, 16 panels for w = 256: the scratch and
+// the next pivot block alternate between two buffers, and a CTA that writes
+// panel p + 2 has passed barrier p + 1, which every CTA reaches after reading
+// panel p.
 // The rank-16 updates are 34 us of FP32 FMA on eight SMs; PIV256 us measured
 // for w = 256 (248 us with the pivot block and R on the owner and R read from
 // its shared memory).
 // Rows and columns beyond w are identity and stay identity.
 constexpr int PB_W = 256, PB_CL = 8, PB_RPC = PB_W / PB_CL, PB_THREADS = 512, PB_PAN = 16;
 constexpr int PB_LD = PB_RPC + 2;      // row stride of C and D: 16-byte aligned, spread over the banks
-constexpr int PB_SCRATCH = 2 * PB_PAN * PB_W * (int)sizeof(float2);
+constexpr int PB_BUF = PB_PAN * (PB_W + PB_PAN);   // one panel and the inverse of its pivot block
+constexpr int PB_SCRATCH = 2 * PB_BUF * (int)sizeof(float2);
+constexpr int PB_ALL = PB_THREADS + 128;           // and the pivot warps
 static_assert(PB_RPC % PB_PAN == 0, "a panel lies inside one CTA");
 static_assert(PB_THREADS == 64 * (PB_RPC / 4), "4 x 4 entries per thread");
 
-// 16 x 16 Gauss-Jordan in one warp: lane (r, h) holds row r, columns 8 h .. 8 h + 7
-__device__ __forceinline__ bool warp_inv16(float2 (&v)[8], int lane) {
-  const int r = lane & 15, h = lane >> 4;
+__device__ __forceinline__ void named_sync(int id, int threads) {
+  asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
+}
+
+// (c.x, c.y) += a (b.x, b.y), lane by lane: two FP32 multiply-adds in one instruction
+__device__ __forceinline__ void fma2(float2& c, float2 a, float2 b) {
+  unsigned long long cc, aa, bb;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(cc) : "f"(c.x), "f"(c.y));
+  asm("mov.b64 %0, {%1, %2};" : "=l"(aa) : "f"(a.x), "f"(a.y));
+  asm("mov.b64 %0, {%1, %2};" : "=l"(bb) : "f"(b.x), "f"(b.y));
+  asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(cc) : "l"(aa), "l"(bb));
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(c.x), "=f"(c.y) : "l"(cc));
+}
+
+// 16 x 16 Gauss-Jordan by four warps (threads u = 0 .. 127): warp q holds
+// columns 4 q .. 4 q + 3, lane (r, h) row r and columns 4 q + 2 h, + 1 in v.
+// The pivot column passes through shared memory (one named barrier per step),
+// the pivot row through shuffles.  col: [2][16].
+__device__ __forceinline__ bool quad_inv16(float2 (&v)[2], int u, float2 (*col)[PB_PAN]) {
+  const int r = u & 15, h = (u >> 4) & 1, q = u >> 5;
   bool ok = true;
 #pragma unroll
   for (int k = 0; k < PB_PAN; ++k) {
-    const int kh = k >> 3, kr = k & 7;
-    const float2 piv = make_float2(__shfl_sync(0xffffffffu, v[kr].x, k + 16 * kh),
-                                   __shfl_sync(0xffffffffu, v[kr].y, k + 16 * kh));
-    const float2 col = make_float2(__shfl_sync(0xffffffffu, v[kr].x, r + 16 * kh),
-                                   __shfl_sync(0xffffffffu, v[kr].y, r + 16 * kh));
+    const int kq = k >> 2, kh = (k >> 1) & 1, kr = k & 1;
+    if (q == kq && h == kh) {
+      col[k & 1][r] = v[kr];
+      v[kr] = make_float2(r == k ? 1.f : 0.f, 0.f);    // the pivot column starts from the identity
+    }
+    float2 row[2];
+#pragma unroll
+    for (int c = 0; c < 2; ++c)
+      row[c] = make_float2(__shfl_sync(0xffffffffu, v[c].x, k + 16 * h), __shfl_sync(0xffffffffu, v[c].y, k + 16 * h));
+    named_sync(2, 128);
+    const float2 piv = col[k & 1][k], ck = col[k & 1][r];
     const float n2 = piv.x * piv.x + piv.y * piv.y;
     ok = ok && n2 > 1e-30f && n2 < 1e30f;
-    const float rn = 1.f / n2;
+    const float rn = rcp_newton(n2);
     const float2 inv = make_float2(piv.x * rn, -piv.y * rn);
+    // a_rc - (a_rk / a_kk) row_c; row k itself: 0 + row_c / a_kk
+    const bool isrow = r == k;
+    const float2 m = isrow ? make_float2(-inv.x, -inv.y) : cmul(ck, inv);
 #pragma unroll
-    for (int c = 0; c < 8; ++c) {
-      const float2 row = make_float2(__shfl_sync(0xffffffffu, v[c].x, k + 16 * h),
-                                     __shfl_sync(0xffffffffu, v[c].y, k + 16 * h));
-      const bool pc = c == kr && h == kh;              // the pivot column
-      const float2 rk = pc ? inv : cmul(row, inv);
-      const float2 base = pc ? make_float2(0.f, 0.f) : v[c];
-      v[c] = (r == k) ? rk : csub(base, cmul(col, rk));
+    for (int c = 0; c < 2; ++c) {
+      const float2 b = isrow ? make_float2(0.f, 0.f) : v[c];
+      v[c].x = fmaf(m.y, row[c].y, fmaf(-m.x, row[c].x, b.x));
+      v[c].y = fmaf(-m.y, row[c].x, fmaf(-m.x, row[c].y, b.y));
     }
   }
   return ok;
 }
 
-__global__ void __cluster_dims__(PB_CL, 1, 1) __launch_bounds__(PB_THREADS, 1)
+__global__ void __cluster_dims__(PB_CL, 1, 1) __launch_bounds__(PB_ALL, 1)
     k_block_inv_cluster(const float2* A, int64_t lda, int w, float2* X, int64_t ldx, int* status,
                         float2* __restrict__ Xr, float2* Pg) {
   namespace cg = cooperative_groups;
   cg::cluster_group cluster = cg::this_cluster();
   __shared__ __align__(16) float2 Ps[PB_PAN][PB_W];    // panel rows, panel columns = identity
   __shared__ __align__(16) float2 Cs[PB_PAN][PB_LD];   // own panel-column entries, [k][row]
-  __shared__ __align__(16) float2 Ds[PB_PAN][PB_LD];   // D = C X, [k][row]
-  __shared__ float2 Xs[PB_PAN][PB_PAN];
+  __shared__ __align__(16) float4 Ds[PB_PAN][PB_RPC];  // D = C X as (-re, -re, im, -im), [k][row]
+  __shared__ float2 colb[2][PB_PAN];
+  __shared__ __align__(16) float2 Xs[PB_PAN][PB_PAN];
+  __shared__ __align__(16) float2 Nb[2][PB_PAN][PB_PAN + 1];   // next pivot block before this panel's update
   __shared__ float cond_red[PB_THREADS / 32], cond_loc[2];
   const int rank = (int)cluster.block_rank();
   const int t = threadIdx.x, tx = t & 63, ty = t >> 6, warp = t >> 5, lane = t & 31;
+  const bool main = t < PB_THREADS;                    // the last four warps invert pivot blocks
   const int row0 = rank * PB_RPC + 4 * ty;             // first of this thread's rows
+  const int pr = lane & 15, pc = 4 * ((t >> 5) & 3) + 2 * (lane >> 4);   // pivot warps: row and first column
+  const int npan = (w + PB_PAN - 1) / PB_PAN;
   float2 a[4][4];
   float amax = 0.f;
+  if (main) {
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < 4; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const int gr = row0 + i, c = tx + 64 * j;
-      a[i][j] = (gr < w && c < w) ? A[(int64_t)gr * lda + c] : make_float2(gr == c ? 1.f : 0.f, 0.f);
-      if (gr < w && c < w) amax = fmaxf(amax, sqrtf(a[i][j].x * a[i][j].x + a[i][j].y * a[i][j].y));
-    }
+      for (int j = 0; j < 4; ++j) {
+        const int gr = row0 + i, c = tx + 64 * j;
+        a[i][j] = (gr < w && c < w) ? A[(int64_t)gr * lda + c] : make_float2(gr == c ? 1.f : 0.f, 0.f);
+        if (gr < w && c < w) amax = fmaxf(amax, sqrtf(a[i][j].x * a[i][j].x + a[i][j].y * a[i][j].y));
+      }
+  }
   // CTA maximum of a per-thread value into cond_loc[slot]
   const auto cta_max = [&](float v, int slot) {
     for (int o = 16; o; o >>= 1) v = fmaxf(v, __shfl_xor_sync(0xffffffffu, v, o));
-    if (lane == 0) cond_red[warp] = v;
+    if (main && lane == 0) cond_red[warp] = v;
     __syncthreads();
     if (t == 0) {
       float mx = 0.f;
@@ -1134,106 +1205,153 @@ __global__ void __cluster_dims__(PB_CL, 1, 1) __launch_bounds__(PB_THREADS, 1)
     __syncthreads();
   };
   cta_max(amax, 0);
-  const int npan = (w + PB_PAN - 1) / PB_PAN;
-  for (int pp = 0; pp < npan; ++pp) {
-    const int p0 = pp * PB_PAN, owner = p0 / PB_RPC, lp0 = p0 % PB_RPC;
-    float2* Pb = Pg + (pp & 1) * PB_PAN * PB_W;
-    const int jp = p0 >> 6, cp = tx - (p0 & 63);       // this thread's panel column, if 0 <= cp < 16
-    const bool inpan = cp >= 0 && cp < PB_PAN;
-    const bool prow = rank == owner && 4 * ty >= lp0 && 4 * ty < lp0 + PB_PAN;
-    if (prow) {
+  // panel pp (raw rows, pivot block inverted) into its scratch buffer, by the owner
+  const auto put_panel = [&](int pp) {
+    const int lp0 = pp * PB_PAN % PB_RPC;
+    if (rank == pp * PB_PAN / PB_RPC && 4 * ty >= lp0 && 4 * ty < lp0 + PB_PAN) {
+      float2* Pb = Pg + (pp & 1) * PB_BUF;
 #pragma unroll
       for (int i = 0; i < 4; ++i)
 #pragma unroll
         for (int j = 0; j < 4; ++j) Pb[(4 * ty + i - lp0) * PB_W + tx + 64 * j] = a[i][j];
     }
-    if (inpan) {
+  };
+  const auto put_inverse = [&](int pp, float2 (&v)[2]) {
+    const bool ok = quad_inv16(v, t - PB_THREADS, colb);
+    if (!ok && lane == 0) atomicOr(status, 1);
+    *reinterpret_cast<float4*>(Pg + (pp & 1) * PB_BUF + PB_PAN * PB_W + pr * PB_PAN + pc) =
+        make_float4(v[0].x, v[0].y, v[1].x, v[1].y);
+  };
+  if (main) {
+    put_panel(0);
+  } else if (rank == 0) {
+    float2 v[2];
 #pragma unroll
-      for (int j = 0; j < 4; ++j)
-        if (j == jp) {
+    for (int c = 0; c < 2; ++c)
+      v[c] = (pr < w && pc + c < w) ? A[(int64_t)pr * lda + pc + c] : make_float2(pr == pc + c ? 1.f : 0.f, 0.f);
+    put_inverse(0, v);
+  }
+  for (int pp = 0; pp < npan; ++pp) {
+    const int p0 = pp * PB_PAN, owner = p0 / PB_RPC, lp0 = p0 % PB_RPC;
+    const int p1 = p0 + PB_PAN, lp1 = p1 % PB_RPC;             // the next panel
+    const bool nown = pp + 1 < npan && rank == p1 / PB_RPC;
+    const float2* Pb = Pg + (pp & 1) * PB_BUF;
+    const int jp = p0 >> 6, cp = tx - (p0 & 63);       // this thread's panel column, if 0 <= cp < 16
+    const bool inpan = cp >= 0 && cp < PB_PAN;
+    const bool prow = rank == owner && 4 * ty >= lp0 && 4 * ty < lp0 + PB_PAN;
+    if (main) {
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        if (inpan && j == jp) {
 #pragma unroll
           for (int i = 0; i < 4; ++i) Cs[cp][4 * ty + i] = a[i][j];
         }
+        const int cn = tx + 64 * j - p1;
+        if (nown && 4 * ty >= lp1 && 4 * ty < lp1 + PB_PAN && cn >= 0 && cn < PB_PAN) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) Nb[pp & 1][4 * ty + i - lp1][cn] = a[i][j];
+        }
+      }
     }
     cluster.sync();
-    if (warp == 0) {
-      const int r = lane & 15, h = lane >> 4;
-      float2 v[8];
+    if (warp < 4) {
+      // D = C X: X through shared memory, warp = four pivots, lane = row
+      const float4 q = __ldcg(reinterpret_cast<const float4*>(Pb + PB_PAN * PB_W) + t);
+      reinterpret_cast<float4*>(&Xs[0][0])[t] = q;
+      named_sync(1, 128);
+      const int k0 = 4 * warp;
+      float2 d[4];
 #pragma unroll
-      for (int c = 0; c < 8; c += 2) {
-        const float4 q = __ldcg(reinterpret_cast<const float4*>(Pb + r * PB_W + p0 + 8 * h + c));
-        v[c] = make_float2(q.x, q.y);
-        v[c + 1] = make_float2(q.z, q.w);
-      }
-      const bool ok = warp_inv16(v, lane);
-      if (!ok && lane == 0 && rank == owner) atomicOr(status, 1);
+      for (int q2 = 0; q2 < 4; ++q2) d[q2] = make_float2(0.f, 0.f);
+      if (rank == owner && lane >= lp0 && lane < lp0 + PB_PAN) {
 #pragma unroll
-      for (int c = 0; c < 8; ++c) Xs[r][8 * h + c] = v[c];
-    } else {
-      constexpr int NL = PB_PAN * PB_W / 2;            // float4 loads by the other warps
-#pragma unroll 3
-      for (int e = t - 32; e < NL; e += PB_THREADS - 32) {
-        const int k = e / (PB_W / 2), c = 2 * (e % (PB_W / 2));
-        float4 q = __ldcg(reinterpret_cast<const float4*>(Pb + k * PB_W + c));
-        if (c >= p0 && c < p0 + PB_PAN)
-          q = make_float4(c - p0 == k ? 1.f : 0.f, 0.f, c + 1 - p0 == k ? 1.f : 0.f, 0.f);
-        *reinterpret_cast<float4*>(&Ps[k][c]) = q;
-      }
-    }
-    __syncthreads();
-    {
-      // warp = pivot k, lane = row
-      const int lr = lane, k = warp;
-      float2 d = make_float2(0.f, 0.f);
-      if (rank == owner && lr >= lp0 && lr < lp0 + PB_PAN) {
-        d = make_float2(-Xs[lr - lp0][k].x, -Xs[lr - lp0][k].y);
+        for (int q2 = 0; q2 < 4; ++q2) d[q2] = make_float2(-Xs[lane - lp0][k0 + q2].x, -Xs[lane - lp0][k0 + q2].y);
       } else {
 #pragma unroll
-        for (int l = 0; l < PB_PAN; ++l) cfma(d, Cs[l][lr], Xs[l][k]);
-      }
-      Ds[k][lr] = d;
-    }
-    if (prow) {
-#pragma unroll
-      for (int i = 0; i < 4; ++i)
-#pragma unroll
-        for (int j = 0; j < 4; ++j) a[i][j] = make_float2(0.f, 0.f);
-    }
-    if (inpan) {
-#pragma unroll
-      for (int j = 0; j < 4; ++j)
-        if (j == jp) {
-#pragma unroll
-          for (int i = 0; i < 4; ++i) a[i][j] = make_float2(0.f, 0.f);
+        for (int l = 0; l < PB_PAN; ++l) {
+          const float2 cv = Cs[l][lane];
+          const float4 x01 = *reinterpret_cast<const float4*>(&Xs[l][k0]);
+          const float4 x23 = *reinterpret_cast<const float4*>(&Xs[l][k0 + 2]);
+          cfma(d[0], cv, make_float2(x01.x, x01.y));
+          cfma(d[1], cv, make_float2(x01.z, x01.w));
+          cfma(d[2], cv, make_float2(x23.x, x23.y));
+          cfma(d[3], cv, make_float2(x23.z, x23.w));
         }
+      }
+#pragma unroll
+      for (int q2 = 0; q2 < 4; ++q2) Ds[k0 + q2][lane] = make_float4(-d[q2].x, -d[q2].x, d[q2].y, -d[q2].y);
+    } else if (main) {
+      constexpr int NL = PB_PAN * PB_W / 2, NT = PB_THREADS - 128, NQ = (NL + NT - 1) / NT;
+      float4 q[NQ];
+#pragma unroll
+      for (int u = 0; u < NQ; ++u) {
+        const int e = t - 128 + u * NT;
+        if (e < NL) q[u] = __ldcg(reinterpret_cast<const float4*>(Pb) + e);
+      }
+#pragma unroll
+      for (int u = 0; u < NQ; ++u) {
+        const int e = t - 128 + u * NT, k = e / (PB_W / 2), c = 2 * (e % (PB_W / 2));
+        if (c >= p0 && c < p1)
+          q[u] = make_float4(c - p0 == k ? 1.f : 0.f, 0.f, c + 1 - p0 == k ? 1.f : 0.f, 0.f);
+        if (e < NL) *reinterpret_cast<float4*>(&Ps[k][c]) = q[u];
+      }
     }
     __syncthreads();
+    if (main) {
+      if (prow) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) a[i][j] = make_float2(0.f, 0.f);
+      }
+      if (inpan) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j)
+          if (j == jp) {
+#pragma unroll
+            for (int i = 0; i < 4; ++i) a[i][j] = make_float2(0.f, 0.f);
+          }
+      }
 #pragma unroll 4
-    for (int k = 0; k < PB_PAN; ++k) {
-      const float4 d01 = *reinterpret_cast<const float4*>(&Ds[k][4 * ty]);
-      const float4 d23 = *reinterpret_cast<const float4*>(&Ds[k][4 * ty + 2]);
-      const float2 d[4] = {make_float2(d01.x, d01.y), make_float2(d01.z, d01.w), make_float2(d23.x, d23.y),
-                           make_float2(d23.z, d23.w)};
+      for (int k = 0; k < PB_PAN; ++k) {
+        float4 d[4];
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
-        const float2 rv = Ps[k][tx + 64 * j];
+        for (int i = 0; i < 4; ++i) d[i] = Ds[k][4 * ty + i];
 #pragma unroll
-        for (int i = 0; i < 4; ++i) {
-          a[i][j].x = fmaf(-d[i].x, rv.x, a[i][j].x);
-          a[i][j].x = fmaf(d[i].y, rv.y, a[i][j].x);
-          a[i][j].y = fmaf(-d[i].x, rv.y, a[i][j].y);
-          a[i][j].y = fmaf(-d[i].y, rv.x, a[i][j].y);
+        for (int j = 0; j < 4; ++j) {
+          const float2 rv = Ps[k][tx + 64 * j], rs = make_float2(rv.y, rv.x);
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            fma2(a[i][j], make_float2(d[i].x, d[i].y), rv);
+            fma2(a[i][j], make_float2(d[i].z, d[i].w), rs);
+          }
         }
       }
+      if (nown) put_panel(pp + 1);
+    } else if (nown) {
+      float2 v[2] = {Nb[pp & 1][pr][pc], Nb[pp & 1][pr][pc + 1]};
+#pragma unroll 4
+      for (int k = 0; k < PB_PAN; ++k) {
+        const float4 d = Ds[k][lp1 + pr];
+        const float4 q = *reinterpret_cast<const float4*>(&Ps[k][p1 + pc]);
+        const float2 d0 = make_float2(d.x, d.y), d1 = make_float2(d.z, d.w);
+        fma2(v[0], d0, make_float2(q.x, q.y));
+        fma2(v[0], d1, make_float2(q.y, q.x));
+        fma2(v[1], d0, make_float2(q.z, q.w));
+        fma2(v[1], d1, make_float2(q.w, q.z));
+      }
+      put_inverse(pp + 1, v);
     }
   }
   float xmax = 0.f;
+  if (main) {
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+    for (int i = 0; i < 4; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j)
-      if (row0 + i < w && tx + 64 * j < w)
-        xmax = fmaxf(xmax, sqrtf(a[i][j].x * a[i][j].x + a[i][j].y * a[i][j].y));
+      for (int j = 0; j < 4; ++j)
+        if (row0 + i < w && tx + 64 * j < w)
+          xmax = fmaxf(xmax, sqrtf(a[i][j].x * a[i][j].x + a[i][j].y * a[i][j].y));
+  }
   cta_max(xmax, 1);
   cluster.sync();
   if (rank == 0 && t == 0) {
@@ -1245,6 +1363,7 @@ __global__ void __cluster_dims__(PB_CL, 1, 1) __launch_bounds__(PB_THREADS, 1)
     }
     record_cond(status, am, xm);
   }
+  if (main) {
   // X may be the input block itself: every CTA read its rows at the start
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
@@ -1264,6 +1383,7 @@ __global__ void __cluster_dims__(PB_CL, 1, 1) __launch_bounds__(PB_THREADS, 1)
       }
     }
   }
+  }
   cluster.sync();   // no CTA may exit while another can still read its shared memory
 }
 
@@ -1271,7 +1391,7 @@ static mnpbem_status launch_block_inv_cluster(const float2* A, int64_t lda, int 
                                               int* status, DevBuf& pan, cudaStream_t st, float2* Xr = nullptr) {
   MNP_TRY(pan.ensure(PB_SCRATCH));
   ProfScope ps(PH_BLOCKINV, st, 8.0 * w * w * w, 0.0);
-  k_block_inv_cluster<<<PB_CL, PB_THREADS, 0, st>>>(A, lda, w, X, ldx, status, Xr, pan.as<float2>());
+  k_block_inv_cluster<<<PB_CL, PB_ALL, 0, st>>>(A, lda, w, X, ldx, status, Xr, pan.as<float2>());
   MNP_CHECK_LAUNCH();
   return MNPBEM_OK;
 }
