@@ -108,7 +108,7 @@ struct Lane {
   LDUWork<float> lu32;   // block LDU factors of G1, G2, Sigma
   LDUWork<double> lu64;
   DevBuf lu_status;      // LDU status words (see dense.cuh)
-  DevBuf lu_bar;         // grid-barrier words of the one-launch triangular sweeps
+  DevBuf lu_ctl, lu_tmp; // control words and intermediate vectors of the triangular sweeps
   TcGemmCtx tc;
   int* status_host = nullptr;     // pinned: Gauss-Jordan (4), LDU (2), tensor-core error word (1), spare
   double* norms_host = nullptr;   // pinned: refinement norms (4)
@@ -241,7 +241,7 @@ mnpbem_status add_lane(mnpbem_geom* G) {
   }
   if (s == MNPBEM_OK) s = L->lp_dev.ensure(sizeof(LamParams));
   if (s == MNPBEM_OK) s = L->lu_status.ensure(2 * sizeof(int));
-  if (s == MNPBEM_OK) s = L->lu_bar.ensure(2 * sizeof(unsigned));
+  if (s == MNPBEM_OK) s = L->lu_ctl.ensure(SWEEP_CTL * sizeof(unsigned));
   if (s != MNPBEM_OK) {
     lane_release(*L);
     return s;
@@ -894,6 +894,7 @@ mnpbem_status ensure_workspace(mnpbem_geom* G, Lane& L, int precision, int P, in
   MNP_TRY(L.vec64.ensure(sizeof(double2) * n * P * (8 + 8 + 8 + 16 + 32 + 8)));
   // working-precision vectors for MIXED: in (8nP) out (8nP) work (32nP)
   MNP_TRY(L.vecw.ensure(sizeof(float2) * n * P * (8 + 8 + 32)));
+  MNP_TRY(L.lu_tmp.ensure(es * 2 * n * 4 * P));   // G1 and G2 solved together, 4 P columns
   MNP_TRY(L.norms.ensure(sizeof(double) * 4));
   MNP_TRY(L.bsplit.ensure(sizeof(float2) * 2 * n * 4 * P));
   MNP_TRY(L.facebuf.ensure(sizeof(double2) * 2 * n + sizeof(float2) * 3 * n + sizeof(float) * 3 * n + 2 * n + 256));
@@ -933,7 +934,7 @@ uint64_t lane_sig(const mnpbem_geom* G, const Lane& L) {
   lu(L.lu32);
   lu(L.lu64);
   mixbuf(L.lu_status);
-  mixbuf(L.lu_bar);
+  mixbuf(L.lu_ctl); mixbuf(L.lu_tmp);
   mix(nullptr, (size_t)G->lu_steps);
   mix(nullptr, (size_t)G->gj_nb);
   mix(L.status_host, 0);
@@ -1026,7 +1027,9 @@ ChainMats<R> chain_mats(mnpbem_geom* G, Lane& L) {
   m.Deltai = L.mat[4].as<Cx>();
   m.ld = G->ld;
   m.b = lu_block<R>(G, sizeof(R) == 4 ? tc_ctx(G, L) : nullptr);
-  m.bar = L.lu_bar.as<unsigned>();
+  m.sw.ctl = L.lu_ctl.as<unsigned>();
+  m.sw.tmp = L.lu_tmp.ptr;
+  m.sw.tmp_bytes = L.lu_tmp.bytes;
   m.ng1 = (int)G->g1_off.size();
   for (int q = 0; q < m.ng1; ++q) {
     m.g1_off[q] = G->g1_off[q];
@@ -2458,16 +2461,22 @@ mnpbem_status chain_transpose(const AdjParams& p, const ChainMats<R>& m, const c
   Cx *lphi = lam, *la = lam + n, *lDe = lam + 4 * n, *lal = lam + 5 * n;
   Cx *gS2 = work, *gH2p = work + n, *v3 = work + 4 * n, *tS1 = work + 7 * n, *ga0 = work + 8 * n;
   auto g1solve = [&](Cx* x, int N) -> mnpbem_status {
-    for (int q = 0; q < m.ng1; ++q)
-      MNP_TRY(ldu_solve<R>(m.G1 + m.g1_off[q] * ld + m.g1_off[q], m.g1_n[q], ld, m.b, x + m.g1_off[q] * N, N, N,
-                           nullptr, gemm, ctx, st, m.bar));
-    return MNPBEM_OK;
+    LduProblem<R> g[CHAIN_MAXBLK];
+    for (int q = 0; q < m.ng1; ++q) {
+      const int64_t o = m.g1_off[q];
+      g[q] = {m.G1 + o * ld + o, ld, m.g1_n[q], x + o * N, N};
+    }
+    return ldu_solve_few<R>(g, m.ng1, m.b, N, m.sw, st);
+  };
+  auto solve1 = [&](const Cx* F, Cx* x, int N) {
+    const LduProblem<R> q = {F, ld, n, x, N};
+    return ldu_solve_few<R>(&q, 1, m.b, N, m.sw, st);
   };
   // G2^-T w_sig2, G2^-T w_h2
   MNP_CUDA(cudaMemcpyAsync(gS2, gs2, cs * n, cudaMemcpyDeviceToDevice, st));
   MNP_CUDA(cudaMemcpyAsync(gH2p, gh2, cs * 3 * n, cudaMemcpyDeviceToDevice, st));
-  MNP_TRY(ldu_solve<R>(m.G2, n, ld, m.b, gS2, 1, 1, nullptr, gemm, ctx, st, m.bar));
-  MNP_TRY(ldu_solve<R>(m.G2, n, ld, m.b, gH2p, 3, 3, nullptr, gemm, ctx, st, m.bar));
+  MNP_TRY(solve1(m.G2, gS2, 1));
+  MNP_TRY(solve1(m.G2, gH2p, 3));
   if (gs1) {
     MNP_CUDA(cudaMemcpyAsync(lphi, gs1, cs * n, cudaMemcpyDeviceToDevice, st));
     MNP_TRY(g1solve(lphi, 1));                                                     // G1^-T w_sig1
@@ -2483,7 +2492,7 @@ mnpbem_status chain_transpose(const AdjParams& p, const ChainMats<R>& m, const c
   MNP_TRY(gemm(n, 3, n, one, m.Deltai, ld, gH2p, 3, zero, lal, 3, st, ctx));        // Deltai^T
   adj_chainT<Cx>(p, 0, lal, nullptr, gS2, nullptr, nullptr, nullptr, st);
   MNP_CUDA(cudaMemcpyAsync(lDe, gS2, cs * n, cudaMemcpyDeviceToDevice, st));
-  MNP_TRY(ldu_solve<R>(m.Sigma, n, ld, m.b, lDe, 1, 1, nullptr, gemm, ctx, st, m.bar));   // Sigma^-T
+  MNP_TRY(solve1(m.Sigma, lDe, 1));   // Sigma^-T
   adj_chainT<Cx>(p, 1, lDe, nullptr, v3, nullptr, nullptr, nullptr, st);
   MNP_TRY(gemm(n, 3, n, one, m.Deltai, ld, v3, 3, one, lal, 3, st, ctx));           // += Deltai^T v
   MNP_TRY(gemm(n, 1, n, one, m.Sigma1, ld, lDe, 1, zero, tS1, 1, st, ctx));         // Sigma1^T

@@ -246,7 +246,8 @@ mnpbem_status apply_mldivide(const FaceData& f, int P, const LamParams* lp, cons
   k_chain_u<R><<<nb, 128, 0, st>>>(f, P, lp, Dp, t3, u);
   MNP_CHECK_LAUNCH();
   // sig2 = Sigma \ u (in place)
-  MNP_TRY(ldu_solve<R>(m.Sigma, n, m.ld, m.b, u, P, P, nullptr, gemm, ctx, st, m.bar));
+  const LduProblem<R> sys = {m.Sigma, m.ld, n, u, P};
+  MNP_TRY(ldu_solve_few<R>(&sys, 1, m.b, P, m.sw, st));
   s2 = u;
   k_chain_v<R><<<nb, 128, 0, st>>>(f, P, lp, s2, al, v3);
   MNP_CHECK_LAUNCH();
@@ -254,11 +255,13 @@ mnpbem_status apply_mldivide(const FaceData& f, int P, const LamParams* lp, cons
   // x1 = G1 \ [sig2 + phi | h2 + a], x2 = G2 \ [sig2 | h2]
   k_chain_y<R><<<nb, 128, 0, st>>>(n, P, s2, h2, phi, a, x1, x2);
   MNP_CHECK_LAUNCH();
-  for (int q = 0; q < m.ng1; ++q)
-    MNP_TRY(ldu_solve<R>(m.G1 + m.g1_off[q] * m.ld + m.g1_off[q], m.g1_n[q], m.ld, m.b, x1 + m.g1_off[q] * 4 * P,
-                         4 * P, 4 * P, nullptr, gemm, ctx, st, m.bar));
-  MNP_TRY(ldu_solve<R>(m.G2, n, m.ld, m.b, x2, 4 * P, 4 * P, nullptr, gemm, ctx, st, m.bar));
-  return MNPBEM_OK;
+  LduProblem<R> g[CHAIN_MAXBLK + 1];
+  for (int q = 0; q < m.ng1; ++q) {
+    const int64_t o = m.g1_off[q];
+    g[q] = {m.G1 + o * m.ld + o, m.ld, m.g1_n[q], x1 + o * 4 * P, 4 * P};
+  }
+  g[m.ng1] = {m.G2, m.ld, n, x2, 4 * P};
+  return ldu_solve_few<R>(g, m.ng1 + 1, m.b, 4 * P, m.sw, st);
 }
 template mnpbem_status apply_mldivide<float>(const FaceData&, int, const LamParams*, const ChainMats<float>&,
                                              const float2*, const float2*, const float2*,

@@ -820,7 +820,7 @@ __device__ __forceinline__ int argmax64(unsigned k0, unsigned k1) {
 // Bound by the latency of the chain of 64 steps (one CTA).  Each warp finds the
 // pivot with one integer reduction over the 64 candidates' moduli; a scan of
 // the column by every thread took most of a step (160 us per block of 64 in a
-// sweep, PIVFLOAT us now).
+// sweep, 41 us now).
 __global__ void __launch_bounds__(256) k_block_inv(const float2* A, int64_t lda, int w, float2* X, int64_t ldx,
                                                    float2* X2, int64_t ldx2, int* status) {
   __shared__ float2 prow[2][64], pcol[2][64];
@@ -946,7 +946,7 @@ __global__ void __launch_bounds__(256) k_block_inv(const float2* A, int64_t lda,
 // column p, and one that writes its pivot row p + 2 has passed barrier p + 2,
 // at which its threads arrive after update p.
 // One CTA with the pivot scan in every thread took 1059 us per block of 64;
-// this takes PIVDOUBLE us.
+// this takes 105 us.
 constexpr int BD_CL = 8, BD_THREADS = 256;
 __global__ void __cluster_dims__(BD_CL, 1, 1) __launch_bounds__(BD_THREADS)
     k_block_inv_c128(const double2* A, int64_t lda, int w, double2* X, int64_t ldx, double2* X2, int64_t ldx2,
@@ -1099,7 +1099,7 @@ static mnpbem_status launch_block_inv(const double2* A, int64_t lda, int w, doub
 // the next pivot block alternate between two buffers, and a CTA that writes
 // panel p + 2 has passed barrier p + 1, which every CTA reaches after reading
 // panel p.
-// The rank-16 updates are 34 us of FP32 FMA on eight SMs; PIV256 us measured
+// The rank-16 updates are 34 us of FP32 FMA on eight SMs; 95 us measured
 // for w = 256 (248 us with the pivot block and R on the owner and R read from
 // its shared memory).
 // Rows and columns beyond w are identity and stay identity.
@@ -1728,258 +1728,251 @@ mnpbem_status ldu_rsolve(cplx<R>* H, int64_t n, int64_t ldh, const cplx<R>* F, i
   return MNPBEM_OK;
 }
 
-// X[blk] <- X_k X[blk] for every diagonal block k (one CTA per block; a warp
-// per row, lanes over the block's columns, N <= 16 right-hand sides)
-template <typename R, int NB>
-__global__ void __launch_bounds__(256) k_ldu_diag(const cplx<R>* __restrict__ F, int64_t ldf, int64_t n, int b,
-                                                  cplx<R>* __restrict__ X, int64_t ldx, int N) {
+// ------------------------------------------------- triangular sweeps
+// The solves L y = x and U x = D^-1 y of the LDU factors for a few right-hand
+// sides, each sweep one launch over up to SWEEP_MAXPROB systems of one block
+// size (the diagonal blocks of G1 and G2 are solved together).  A work item is
+// a slice of RS = 8 RW rows of one block row; the CTAs take the items in the
+// order of their block rows from a counter, keep the slice's sums in registers
+// while they walk the block row, and wait for block k only when they need its
+// solution.  An item waits for items with smaller numbers alone, and these have
+// been taken by CTAs that run: no co-residency is needed, so the sweep neither
+// waits for a whole free GPU nor keeps other streams' kernels out while it
+// waits.  Forward: y_i = x_i - sum_{k<i} L_ik y_k into T.  Backward:
+// x_i = X_i y_i - sum_{k>i} U_ik x_k (X_i the stored inverse of D_i) into X.
+// Blocks complete in order, so one counter of finished slices per system says
+// how many are ready.  A thread's entries of the next block are loaded as those
+// of this one are used; they do not depend on the wait.
+// The waits are bounded by wall clock: on expiry the error word of the streamed
+// thin products is set, an abort word releases the other CTAs, and all return.
+// Bound by the chain of block rows (about 3 us each) at a few thousand rows and by
+// HBM at 24 000 (800 us for 2.3 GB).  Against the cooperative sweep before it (a
+// grid barrier per block row), with eight wavelengths of 4000 faces in flight:
+// 72 us against 131 to 150 us per sweep, 12 sweeps instead of 18 per direction and
+// wavelength, and no separate product with D^-1 (90 us on one CTA per block).
+constexpr int SWEEP_THREADS = 256;
+
+template <typename R> struct SweepArgs {
+  LduProblem<R> p[SWEEP_MAXPROB];
+  int nprob, b, N, items;
+  unsigned* ctl;            // [0], [1] item counters, [2] abort, [4 + 2 q + direction] finished slices
+};
+
+template <typename R, int NB, int RW, int CPL, bool LOWER>
+__global__ void __launch_bounds__(SWEEP_THREADS, 2) k_ldu_sweep(const __grid_constant__ SweepArgs<R> a) {
   using Cx = cplx<R>;
-  extern __shared__ unsigned char ldu_smem[];
-  Cx* xs = reinterpret_cast<Cx*>(ldu_smem);   // [b][NB], columns N .. NB - 1 zero
-  const int64_t k0 = (int64_t)blockIdx.x * b;
-  const int bs = (int)min((int64_t)b, n - k0);
-  for (int e = threadIdx.x; e < bs * NB; e += blockDim.x) {
-    const int r = e / NB, c = e % NB;
-    xs[e] = c < N ? X[(k0 + r) * ldx + c] : mk<R>(0, 0);
-  }
-  __syncthreads();
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  for (int r = warp; r < bs; r += 8) {
-    const Cx* frow = F + (k0 + r) * ldf + k0;
-    Cx acc[NB];
-#pragma unroll
-    for (int c = 0; c < NB; ++c) acc[c] = mk<R>(0, 0);
-    for (int l = lane; l < bs; l += 32) {
-      const Cx f = frow[l];
-#pragma unroll
-      for (int c = 0; c < NB; ++c) cfma(acc[c], f, xs[l * NB + c]);
-    }
-#pragma unroll
-    for (int c = 0; c < NB; ++c) {
-      Cx v = acc[c];
-      for (int o = 16; o; o >>= 1) {
-        v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
-        v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
-      }
-      if (lane == 0 && c < N) X[(k0 + r) * ldx + c] = v;
-    }
-  }
-}
-
-// ------------------------------------------- triangular sweeps, one launch
-// The forward (unit lower L) and backward (unit upper U) sweeps of the LDU
-// solve for a few right-hand sides as one cooperative launch each.  Step s
-// takes block k (k = s forward, nblk - 1 - s backward): every CTA stages x_k
-// (b x N) in shared memory and subtracts F[i, k block] x_k from its rows i of
-// the trailing (forward) or leading (backward) part; then the CTAs meet at a
-// grid barrier before the next block is read.  One CTA of 16 warps per SM;
-// rows go to the CTAs in groups (16 warps x 2 rows, by absolute index: group g
-// to CTA g mod G); a warp takes two rows at a time (lanes along the rows,
-// coalesced, both rows' loads in flight together) and reduces with shuffles.
-// X is read with ld.global.cg (L2), since other CTAs updated it.  The grid
-// barrier is a monotonic arrival counter (zeroed before the launch) with a
-// bounded wait; on expiry the error word of the streamed thin products is
-// set, an abort flag releases the other CTAs and every CTA returns.
-constexpr int TRSV_THREADS = 512, TRSV_WARPS = TRSV_THREADS / 32;
-
-__device__ __forceinline__ bool coop_barrier(unsigned* ctr, unsigned target, int* abortf) {
-  __shared__ int ok_s;
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    int ok = 1;
-    __threadfence();
-    atomicAdd(ctr, 1u);
-    const unsigned long long t0 = gtimer();
-    while (*(volatile unsigned*)ctr < target) {
-      if (*(volatile int*)abortf) { ok = 0; break; }
-      if (gtimer() - t0 > MBAR_WAIT_NS) {
-        atomicOr(&g_thin_stream_err, 64);
-        atomicExch(abortf, 1);
-        ok = 0;
-        break;
-      }
-    }
-    __threadfence();
-    ok_s = ok;
-  }
-  __syncthreads();
-  return ok_s != 0;
-}
-
-// one warp subtracts F[i, k block] x_k from RW rows i0, i0 + 1, ... at once
-// (independent accumulators keep the RW rows' loads in flight together)
-template <typename R, int NB, int RW>
-__device__ __forceinline__ void trsv_rows(const cplx<R>* __restrict__ F, int64_t ldf, int64_t k0, int bs,
-                                          const cplx<R>* xs, cplx<R>* X, int64_t ldx, int N, int64_t i0,
-                                          int64_t r0, int64_t r1, int lane) {
-  using Cx = cplx<R>;
-  Cx acc[RW][NB];
-#pragma unroll
-  for (int q = 0; q < RW; ++q)
-#pragma unroll
-    for (int c = 0; c < NB; ++c) acc[q][c] = mk<R>(0, 0);
-  const Cx* frow[RW];
-  bool act[RW];
-#pragma unroll
-  for (int q = 0; q < RW; ++q) {
-    act[q] = i0 + q >= r0 && i0 + q < r1;
-    frow[q] = F + (act[q] ? i0 + q : r0) * ldf + k0;
-  }
-  // two of a lane's entries per row in flight at a time: the full unroll (a
-  // row's entries all loaded first) raises the register count to 96-104 and
-  // keeps these CTAs from sharing SMs with the other lanes' kernels
-#pragma unroll 2
-  for (int l = lane; l < bs; l += 32) {
-    Cx f[RW];
-#pragma unroll
-    for (int q = 0; q < RW; ++q) f[q] = __ldg(frow[q] + l);
-#pragma unroll
-    for (int c = 0; c < NB; ++c) {
-      const Cx xv = xs[l * NB + c];
-#pragma unroll
-      for (int q = 0; q < RW; ++q) cfma(acc[q][c], f[q], xv);
-    }
-  }
-#pragma unroll
-  for (int q = 0; q < RW; ++q)
-#pragma unroll
-    for (int c = 0; c < NB; ++c) {
-      Cx v = acc[q][c];
-      for (int o = 16; o; o >>= 1) {
-        v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
-        v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
-      }
-      if (act[q] && lane == c && c < N) {
-        Cx* xp = X + (i0 + q) * ldx + c;
-        *xp = csub(__ldcg(xp), v);
-      }
-    }
-}
-
-template <typename R, int NB, bool LOWER>
-__global__ void __launch_bounds__(TRSV_THREADS) k_trsv_unit(const cplx<R>* __restrict__ F, int64_t ldf, int64_t n,
-                                                            int b, cplx<R>* X, int64_t ldx, int N, unsigned* bar) {
-  using Cx = cplx<R>;
-  constexpr int RW = NB <= 8 ? 2 : 1;          // rows per warp at a time
-  constexpr int GRP = TRSV_WARPS * RW;         // rows per group: one pass of the CTA's warps
-  extern __shared__ unsigned char trsv_smem[];
-  Cx* xs = reinterpret_cast<Cx*>(trsv_smem);   // [b][NB], columns N .. NB - 1 zero
-  const int nblk = (int)((n + b - 1) / b);
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t G = gridDim.x;
-  int* abortf = reinterpret_cast<int*>(bar + 1);
-  for (int s = 0; s + 1 < nblk; ++s) {
-    const int k = LOWER ? s : nblk - 1 - s;
-    const int64_t k0 = (int64_t)k * b;
-    const int bs = (int)min((int64_t)b, n - k0);
-    for (int e = threadIdx.x; e < bs * NB; e += TRSV_THREADS) {
-      const int r = e / NB, c = e % NB;
-      xs[e] = c < N ? __ldcg(X + (k0 + r) * ldx + c) : mk<R>(0, 0);
-    }
+  constexpr int RS = 8 * RW;
+  extern __shared__ __align__(16) unsigned char sweep_smem[];
+  Cx* xs = reinterpret_cast<Cx*>(sweep_smem);        // [2][NB][b + 4]
+  __shared__ int item_s, known_s;
+  const int b = a.b, N = a.N, xld = b + 4;
+  const int S = (b + RS - 1) / RS;
+  const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+  volatile unsigned* abortw = a.ctl + 2;
+  for (;;) {
     __syncthreads();
-    const int64_t r0 = LOWER ? k0 + bs : 0, r1 = LOWER ? n : k0;
-    // groups of GRP rows by absolute index, group g to CTA g mod G
-    int64_t g = r0 / GRP;
-    g += (blockIdx.x - g % G + G) % G;
-    for (; g * GRP < r1; g += G)
-      trsv_rows<R, NB, RW>(F, ldf, k0, bs, xs, X, ldx, N, g * GRP + warp * RW, r0, r1, lane);
-    if (!coop_barrier(bar, (unsigned)((s + 1) * G), abortf)) return;
-  }
-}
-
-static int trsv_sms() {
-  static int sms = 0;
-  if (!sms) {
-    int dev = 0;
-    cudaGetDevice(&dev);
-    if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) {
-      cudaGetLastError();
-      sms = 148;
+    if (t == 0) item_s = (int)atomicAdd(a.ctl + (LOWER ? 0 : 1), 1u);
+    __syncthreads();
+    const int item = item_s;
+    if (item >= a.items) return;
+    const int q = item % a.nprob, lv = item / a.nprob, i = lv / S, s = lv - i * S;
+    const LduProblem<R>& p = a.p[q];
+    const int nblk = (int)((p.n + b - 1) / b);
+    if (i >= nblk) continue;
+    const int blk = LOWER ? i : nblk - 1 - i;
+    unsigned* arrived = a.ctl + 4 + 2 * q + (LOWER ? 0 : 1);
+    const int64_t row0 = (int64_t)blk * b + s * RS + warp * RW;
+    const int64_t rend = min(p.n, (int64_t)(blk + 1) * b);
+    const Cx* frow[RW];
+    bool act[RW];
+#pragma unroll
+    for (int r = 0; r < RW; ++r) {
+      act[r] = row0 + r < rend;
+      frow[r] = p.F + (act[r] ? row0 + r : (int64_t)blk * b) * p.ldf;
+    }
+    Cx acc[RW][NB], f[RW][CPL];
+#pragma unroll
+    for (int r = 0; r < RW; ++r)
+#pragma unroll
+      for (int c = 0; c < NB; ++c) acc[r][c] = mk<R>(0, 0);
+    // step c of the walk: forward block c; backward the diagonal block, then nblk - c
+    const int nstep = LOWER ? i : i + 1;
+    const auto col_block = [&](int c) { return LOWER ? c : (c == 0 ? blk : nblk - c); };
+    const auto load_f = [&](int c, int r, int u) {
+      const int k = col_block(c), l = lane + 32 * u;
+      const int64_t k0 = (int64_t)k * b;
+      if (k0 + l < p.n && l < b) f[r][u] = __ldg(frow[r] + k0 + l);
+      else f[r][u] = mk<R>(0, 0);
+    };
+    if (nstep > 0) {
+#pragma unroll
+      for (int r = 0; r < RW; ++r)
+#pragma unroll
+        for (int u = 0; u < CPL; ++u) load_f(0, r, u);
+    }
+    int known = 0;                                     // slices known to have finished
+    for (int c = 0; c < nstep; ++c) {
+      const int need = LOWER ? (c + 1) * S : c * S;
+      if (need > known) {
+        if (t == 0) {
+          unsigned v;
+          const unsigned long long t0 = gtimer();
+          for (;;) {
+            asm volatile("ld.acquire.gpu.global.u32 %0, [%1];" : "=r"(v) : "l"(arrived) : "memory");
+            if (v >= (unsigned)need) break;
+            if (*abortw) { v = 0; break; }
+            if (gtimer() - t0 > MBAR_WAIT_NS) {
+              atomicOr(&g_thin_stream_err, 64);
+              *abortw = 1u;
+              v = 0;
+              break;
+            }
+          }
+          known_s = (int)v;
+        }
+        __syncthreads();
+        known = known_s;
+        if (known < need) return;
+      }
+      const int64_t k0 = (int64_t)col_block(c) * b;
+      const int bs = (int)min((int64_t)b, p.n - k0);
+      const bool from_t = LOWER || c == 0;
+      const Cx* src = from_t ? p.T + k0 * N : p.X + k0 * p.ldx;
+      const int64_t lds = from_t ? N : p.ldx;
+      Cx* xb = xs + (c & 1) * NB * xld;
+      for (int e = t; e < b * NB; e += SWEEP_THREADS) {
+        const int r = e / NB, cc = e % NB;
+        xb[cc * xld + r] = (r < bs && cc < N) ? __ldcg(src + r * lds + cc) : mk<R>(0, 0);
+      }
+      __syncthreads();
+      const bool more = c + 1 < nstep;
+#pragma unroll
+      for (int u = 0; u < CPL; ++u) {
+        const int l = min(lane + 32 * u, b - 1);       // beyond b: f is zero
+        Cx xv[NB];
+#pragma unroll
+        for (int cc = 0; cc < NB; ++cc) xv[cc] = xb[cc * xld + l];
+#pragma unroll
+        for (int r = 0; r < RW; ++r) {
+#pragma unroll
+          for (int cc = 0; cc < NB; ++cc) cfma(acc[r][cc], f[r][u], xv[cc]);
+          if (more) load_f(c + 1, r, u);
+        }
+      }
+      if (!LOWER && c == 0) {
+#pragma unroll
+        for (int r = 0; r < RW; ++r)
+#pragma unroll
+          for (int cc = 0; cc < NB; ++cc) acc[r][cc] = mk<R>(-acc[r][cc].x, -acc[r][cc].y);
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < RW; ++r)
+#pragma unroll
+      for (int cc = 0; cc < NB; ++cc) {
+        Cx v = acc[r][cc];
+#pragma unroll
+        for (int o = 16; o; o >>= 1) {
+          v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
+          v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
+        }
+        if (act[r] && lane == cc && cc < N) {
+          Cx* xp = p.X + (row0 + r) * p.ldx + cc;
+          if (LOWER) p.T[(row0 + r) * N + cc] = csub(*xp, v);
+          else *xp = mk<R>(-v.x, -v.y);
+        }
+      }
+    __syncthreads();
+    if (t == 0) {
+      __threadfence();
+      atomicAdd(arrived, 1u);
     }
   }
-  return sms;
 }
 
-template <typename R, int NB, bool LOWER>
-static mnpbem_status launch_trsv(const cplx<R>* F, int64_t n, int64_t ldf, int b, cplx<R>* X, int64_t ldx, int N,
-                                 unsigned* bar, cudaStream_t st) {
-  using Cx = cplx<R>;
-  const size_t smem = sizeof(Cx) * b * NB;
+template <typename R, int NB, int RW, bool LOWER>
+static mnpbem_status launch_sweep(SweepArgs<R> a, int maxblk, cudaStream_t st) {
+  constexpr int CPL = sizeof(R) == 4 ? 8 : 2;          // entries per lane and block row: b <= 32 CPL
+  auto kern = k_ldu_sweep<R, NB, RW, CPL, LOWER>;
+  const int smem = (int)sizeof(cplx<R>) * 2 * NB * (a.b + 4);
+  constexpr int SMEM_MAX = (int)sizeof(cplx<R>) * 2 * NB * (32 * CPL + 4);
   static int per_sm = -1;
   if (per_sm < 0) {
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_trsv_unit<R, NB, LOWER>, TRSV_THREADS,
-                                                      sizeof(Cx) * 256 * NB) != cudaSuccess) {
-      cudaGetLastError();
-      per_sm = 1;
-    }
-    per_sm = std::max(1, std::min(per_sm, 1));
+    MNP_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX));
+    int occ = 0;
+    MNP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, SWEEP_THREADS, SMEM_MAX));
+    per_sm = std::max(1, occ);
   }
-  const unsigned grid = (unsigned)(per_sm * trsv_sms());
-  MNP_CUDA(cudaMemsetAsync(bar, 0, 2 * sizeof(unsigned), st));
-  ProfScope ps(PH_GEMM_SMALL, st, 4.0 * n * n * N, (double)sizeof(Cx) * 0.5 * n * n);
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid);
-  cfg.blockDim = dim3(TRSV_THREADS);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeCooperative;
-  attr[0].val.cooperative = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  MNP_CUDA(cudaLaunchKernelEx(&cfg, k_trsv_unit<R, NB, LOWER>, F, ldf, n, b, X, ldx, N, bar));
+  const int S = (a.b + 8 * RW - 1) / (8 * RW);
+  a.items = maxblk * S * a.nprob;
+  double half = 0.0;
+  for (int q = 0; q < a.nprob; ++q) half += 0.5 * (double)a.p[q].n * a.p[q].n;
+  ProfScope ps(PH_GEMM_SMALL, st, 8.0 * half * a.N, (double)sizeof(cplx<R>) * half);
+  kern<<<(unsigned)std::min(a.items, per_sm * stream_sms()), SWEEP_THREADS, smem, st>>>(a);
+  MNP_CHECK_LAUNCH();
   return MNPBEM_OK;
 }
 
-template <typename R, bool LOWER>
-static mnpbem_status trsv_sweep(const cplx<R>* F, int64_t n, int64_t ldf, int b, cplx<R>* X, int64_t ldx, int N,
-                                unsigned* bar, cudaStream_t st) {
-  if (N <= 4) return launch_trsv<R, 4, LOWER>(F, n, ldf, b, X, ldx, N, bar, st);
-  if (N <= 8) return launch_trsv<R, 8, LOWER>(F, n, ldf, b, X, ldx, N, bar, st);
-  return launch_trsv<R, 16, LOWER>(F, n, ldf, b, X, ldx, N, bar, st);
+template <typename R>
+mnpbem_status ldu_solve_few(const LduProblem<R>* probs, int nprob, int b, int64_t N, const LduSweepWs& ws,
+                            cudaStream_t st) {
+  if (nprob < 1 || nprob > SWEEP_MAXPROB || N < 1 || N > 16 || b < 1 || b > (sizeof(R) == 4 ? 256 : 64) || !ws.ctl) {
+    set_error("ldu_solve_few: invalid arguments");
+    return MNPBEM_ERR_INVALID_ARG;
+  }
+  SweepArgs<R> a;
+  a.nprob = 0;
+  a.b = b;
+  a.N = (int)N;
+  a.ctl = ws.ctl;
+  int64_t rows = 0, maxn = 0;
+  for (int q = 0; q < nprob; ++q) {
+    if (probs[q].n <= 0) continue;
+    a.p[a.nprob] = probs[q];
+    a.p[a.nprob].T = reinterpret_cast<cplx<R>*>(ws.tmp) + rows * N;
+    rows += probs[q].n;
+    maxn = std::max(maxn, probs[q].n);
+    ++a.nprob;
+  }
+  if (a.nprob == 0) return MNPBEM_OK;
+  if (sizeof(cplx<R>) * rows * N > ws.tmp_bytes) { set_error("ldu_solve_few: workspace too small"); return MNPBEM_ERR_INVALID_ARG; }
+  MNP_CUDA(cudaMemsetAsync(ws.ctl, 0, SWEEP_CTL * sizeof(unsigned), st));
+  const int mb = (int)cdiv_up(maxn, (int64_t)b);
+  // rows per warp: two, one where 16 sums per row fill the registers
+  if (N <= 4) {
+    MNP_TRY((launch_sweep<R, 4, 2, true>(a, mb, st)));
+    return launch_sweep<R, 4, 2, false>(a, mb, st);
+  }
+  if (N <= 8) {
+    MNP_TRY((launch_sweep<R, 8, 2, true>(a, mb, st)));
+    return launch_sweep<R, 8, 2, false>(a, mb, st);
+  }
+  MNP_TRY((launch_sweep<R, 16, 1, true>(a, mb, st)));
+  return launch_sweep<R, 16, 1, false>(a, mb, st);
 }
 
 template <typename R>
 mnpbem_status ldu_solve(const cplx<R>* F, int64_t n, int64_t ldf, int b, cplx<R>* X, int64_t ldx, int64_t N,
-                        cplx<R>* tmp, GemmFn<R> gemm, void* ctx, cudaStream_t st, unsigned* bar) {
+                        cplx<R>* tmp, GemmFn<R> gemm, void* ctx, cudaStream_t st) {
   using Cx = cplx<R>;
   if (n <= 0 || N <= 0) return MNPBEM_OK;
+  if (!tmp) { set_error("ldu_solve: workspace required"); return MNPBEM_ERR_INVALID_ARG; }
   const Cx one = mk<R>(1, 0), zero = mk<R>(0, 0), mone = mk<R>(-1, 0);
   const int64_t nblk = cdiv_up(n, (int64_t)b);
-  const bool sweep = bar && N <= 16 && b <= 256;
   // forward: L unit lower
-  if (sweep) {
-    if (nblk > 1) MNP_TRY((trsv_sweep<R, true>(F, n, ldf, b, X, ldx, (int)N, bar, st)));
-  } else {
-    for (int64_t k = 0; k + 1 < nblk; ++k) {
-      const int64_t k0 = k * b, kb = k0 + b;
-      MNP_TRY(gemm(n - kb, N, b, mone, F + kb * ldf + k0, ldf, X + k0 * ldx, ldx, one, X + kb * ldx, ldx, st, ctx));
-    }
+  for (int64_t k = 0; k + 1 < nblk; ++k) {
+    const int64_t k0 = k * b, kb = k0 + b;
+    MNP_TRY(gemm(n - kb, N, b, mone, F + kb * ldf + k0, ldf, X + k0 * ldx, ldx, one, X + kb * ldx, ldx, st, ctx));
   }
   // block diagonal
-  if (N <= 16) {
-    const size_t smem = sizeof(Cx) * b * (N <= 4 ? 4 : N <= 8 ? 8 : 16);
-    ProfScope ps(PH_GEMM_SMALL, st, 8.0 * n * b * N, (double)sizeof(Cx) * ((double)n * b + 2.0 * n * N));
-    const int Ni = (int)N;
-    if (N <= 4) k_ldu_diag<R, 4><<<(unsigned)nblk, 256, smem, st>>>(F, ldf, n, b, X, ldx, Ni);
-    else if (N <= 8) k_ldu_diag<R, 8><<<(unsigned)nblk, 256, smem, st>>>(F, ldf, n, b, X, ldx, Ni);
-    else k_ldu_diag<R, 16><<<(unsigned)nblk, 256, smem, st>>>(F, ldf, n, b, X, ldx, Ni);
-    MNP_CHECK_LAUNCH();
-  } else {
-    if (!tmp) { set_error("ldu_solve: workspace required for more than 16 right-hand sides"); return MNPBEM_ERR_INVALID_ARG; }
-    for (int64_t k = 0; k < nblk; ++k) {
-      const int64_t k0 = k * b;
-      const int bs = (int)std::min<int64_t>(b, n - k0);
-      MNP_CUDA(cudaMemcpy2DAsync(tmp, sizeof(Cx) * N, X + k0 * ldx, sizeof(Cx) * ldx, sizeof(Cx) * N, bs,
-                                 cudaMemcpyDeviceToDevice, st));
-      MNP_TRY(gemm(bs, N, bs, one, F + k0 * ldf + k0, ldf, tmp, N, zero, X + k0 * ldx, ldx, st, ctx));
-    }
+  for (int64_t k = 0; k < nblk; ++k) {
+    const int64_t k0 = k * b;
+    const int bs = (int)std::min<int64_t>(b, n - k0);
+    MNP_CUDA(cudaMemcpy2DAsync(tmp, sizeof(Cx) * N, X + k0 * ldx, sizeof(Cx) * ldx, sizeof(Cx) * N, bs,
+                               cudaMemcpyDeviceToDevice, st));
+    MNP_TRY(gemm(bs, N, bs, one, F + k0 * ldf + k0, ldf, tmp, N, zero, X + k0 * ldx, ldx, st, ctx));
   }
   // backward: U unit upper
-  if (sweep) {
-    if (nblk > 1) MNP_TRY((trsv_sweep<R, false>(F, n, ldf, b, X, ldx, (int)N, bar, st)));
-    return MNPBEM_OK;
-  }
   for (int64_t k = nblk - 1; k >= 1; --k) {
     const int64_t k0 = k * b;
     const int bs = (int)std::min<int64_t>(b, n - k0);
@@ -1997,8 +1990,12 @@ template mnpbem_status ldu_rsolve<float>(float2*, int64_t, int64_t, const float2
 template mnpbem_status ldu_rsolve<double>(double2*, int64_t, int64_t, const double2*, int64_t, LDUWork<double>&,
                                           GemmFn<double>, void*, cudaStream_t);
 template mnpbem_status ldu_solve<float>(const float2*, int64_t, int64_t, int, float2*, int64_t, int64_t, float2*,
-                                        GemmFn<float>, void*, cudaStream_t, unsigned*);
+                                        GemmFn<float>, void*, cudaStream_t);
 template mnpbem_status ldu_solve<double>(const double2*, int64_t, int64_t, int, double2*, int64_t, int64_t, double2*,
-                                         GemmFn<double>, void*, cudaStream_t, unsigned*);
+                                         GemmFn<double>, void*, cudaStream_t);
+template mnpbem_status ldu_solve_few<float>(const LduProblem<float>*, int, int, int64_t, const LduSweepWs&,
+                                            cudaStream_t);
+template mnpbem_status ldu_solve_few<double>(const LduProblem<double>*, int, int, int64_t, const LduSweepWs&,
+                                             cudaStream_t);
 
 }  // namespace mnpbem

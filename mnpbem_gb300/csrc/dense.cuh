@@ -88,13 +88,29 @@ mnpbem_status ldu_factor(cplx<R>* A, int64_t n, int64_t lda, LDUWork<R>& w, int*
 template <typename R>
 mnpbem_status ldu_rsolve(cplx<R>* H, int64_t n, int64_t ldh, const cplx<R>* F, int64_t ldf, LDUWork<R>& w,
                          GemmFn<R> gemm, void* ctx, cudaStream_t st);
-// X [n x N] <- F^-1 X in place (F block LDU factors with blocks of b rows).
+// X [n x N] <- F^-1 X in place (F block LDU factors with blocks of b rows), one
+// product per block.  tmp: workspace of b * N values.
 // The transposed solve F^-T X is the same call on the in-place transpose of F.
-// tmp: workspace of b * N values, used only for N > 16 (may be null otherwise).
-// bar: two device words for the grid barrier of the one-launch triangular
-// sweeps (N <= 16; one pair per stream); null: one product per block instead.
 template <typename R>
 mnpbem_status ldu_solve(const cplx<R>* F, int64_t n, int64_t ldf, int b, cplx<R>* X, int64_t ldx, int64_t N,
-                        cplx<R>* tmp, GemmFn<R> gemm, void* ctx, cudaStream_t st, unsigned* bar = nullptr);
+                        cplx<R>* tmp, GemmFn<R> gemm, void* ctx, cudaStream_t st);
+
+// The same for N <= 16 right-hand sides of several systems at once (b <= 256 in
+// complex64, <= 64 in complex128), two launches: a forward and a backward sweep.
+template <typename R> struct LduProblem {
+  const cplx<R>* F; int64_t ldf, n;
+  cplx<R>* X; int64_t ldx;
+  cplx<R>* T = nullptr;             // set by ldu_solve_few
+};
+constexpr int SWEEP_MAXPROB = 17;   // the diagonal blocks of G1 (at most 16) and G2
+constexpr int SWEEP_CTL = 4 + 2 * SWEEP_MAXPROB;
+struct LduSweepWs {                 // one per stream
+  unsigned* ctl = nullptr;          // SWEEP_CTL words
+  void* tmp = nullptr;              // N values per row of every system
+  size_t tmp_bytes = 0;
+};
+template <typename R>
+mnpbem_status ldu_solve_few(const LduProblem<R>* probs, int nprob, int b, int64_t N, const LduSweepWs& ws,
+                            cudaStream_t st);
 
 }  // namespace mnpbem
