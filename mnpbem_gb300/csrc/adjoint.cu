@@ -20,6 +20,7 @@
 // J and the chain rule of norm_flat.m (centroids, normals, areas -> vertices).
 // Every accumulation is FP64 (atomicAdd on per-face / per-vertex arrays).
 #include "adjoint.cuh"
+#include "cis.cuh"
 #include "profile.cuh"
 
 namespace mnpbem {
@@ -68,13 +69,12 @@ struct FarGrad {
   double2 gk;    // d(lam^T A x) / dk   (medium 1 only)
 };
 
-// far-pair contribution -Re(WG dG + WF dF) of one medium (eval1.m:24-40, 110-124)
-__device__ __forceinline__ void far_grad(double2 k, double2 WG, double2 WF, double3 R, double d, double3 ni,
-                                         double Aj, FarGrad& g, bool want_k) {
-  const double inv = 1.0 / d;
+// far-pair contribution -Re(WG dG + WF dF) of one medium (eval1.m:24-40, 110-124);
+// inv = 1 / d, E = exp(i k d)
+__device__ __forceinline__ void far_grad(double2 k, double2 E, double2 WG, double2 WF, double3 R, double d, double inv,
+                                         double3 ni, double Aj, FarGrad& g, bool want_k) {
   const double3 Rh = vscale(R, inv);
   const double nR = vdot(ni, R);
-  const double2 E = cexpi(k, d);
   const double2 ikm = cx(-k.y - inv, k.x);                      // ik - 1/d
   const double2 G = cscl(E, Aj * inv);
   const double2 phi = cscl(cmul(ikm, E), inv * inv);            // (ik - 1/d) e / d^2
@@ -100,12 +100,11 @@ __device__ __forceinline__ void far_grad(double2 k, double2 WG, double2 WF, doub
 }
 
 // closed-surface term Re(c_b dT_ab), T_ab = -A_a (n_a . R) / d^3, R = r_a - r_b
-__device__ __forceinline__ void closed_far_grad(double cb, double3 R, double d, double3 na, double Aa,
+__device__ __forceinline__ void closed_far_grad(double cb, double3 R, double inv, double3 na, double Aa,
                                                 double3& gra, double3& grb, double3& gna, double& gaa) {
-  const double inv = 1.0 / d, inv3 = inv * inv * inv;
+  const double inv3 = inv * inv * inv;
   const double nR = vdot(na, R);
-  const double T = -Aa * nR * inv3;
-  gaa += cb * T / Aa;
+  gaa -= cb * nR * inv3;
   gna = vadd(gna, vscale(R, -cb * Aa * inv3));
   const double3 gR = vscale(vsub(vscale(na, inv3), vscale(R, 3.0 * nR * inv3 * inv * inv)), -cb * Aa);
   gra = vadd(gra, gR);
@@ -115,7 +114,9 @@ __device__ __forceinline__ void closed_far_grad(double cb, double3 R, double d, 
 constexpr int PG_COLS = 128, PG_ROWS = 16;
 
 // all pairs i != j: far-field derivatives of both media + closed-surface term
-__global__ void __launch_bounds__(PG_COLS) k_adj_pairs(AdjParams p) {
+__global__ void __launch_bounds__(PG_COLS) k_adj_pairs(AdjParams p, const CisTable* table) {
+  __shared__ CisTable T;
+  cis_load(T, table);
   const int64_t j = (int64_t)blockIdx.x * PG_COLS + threadIdx.x;
   const int64_t i0 = (int64_t)blockIdx.y * PG_ROWS;
   const bool jok = j < p.n;
@@ -143,11 +144,11 @@ __global__ void __launch_bounds__(PG_COLS) k_adj_pairs(AdjParams p) {
     double cga = 0.0;
     if (jok && i != j) {
       const double3 R = vsub(ri, rj);
-      const double d = sqrt(vdot(R, R));
+      const double dd = vdot(R, R), inv = rsqrt(dd), d = dd * inv;
       const double2* U = p.U + i * 16;
-      far_grad(p.k1, wdot(U, X1), wdot(U + 4, X1), R, d, ni, Aj, g, true);
-      far_grad(p.k2, wdot(U + 8, X2), wdot(U + 12, X2), R, d, ni, Aj, g, false);
-      closed_far_grad(cb, R, d, ni, Ai, cgi, cgj, cgn, cga);
+      far_grad(p.k1, cis_exp(T, p.k1, d), wdot(U, X1), wdot(U + 4, X1), R, d, inv, ni, Aj, g, true);
+      far_grad(p.k2, cis_exp(T, p.k2, d), wdot(U + 8, X2), wdot(U + 12, X2), R, d, inv, ni, Aj, g, false);
+      closed_far_grad(cb, R, inv, ni, Ai, cgi, cgj, cgn, cga);
     }
     grj = vadd(grj, vadd(g.grj, cgj));
     gaj += g.gaj;
@@ -207,221 +208,245 @@ __device__ __forceinline__ void tri_area_grad(double* gv, int a, int b, int c, d
 }
 
 // refined off-diagonal pairs: the near derivative replaces the far one
-// (greenret/private/init.m:98-177 coefficients, eval1.m:36-39 / 119-123)
-__global__ void k_adj_near(AdjParams p) {
+// (greenret/private/init.m:98-177 coefficients, eval1.m:36-39 / 119-123).
+// With D_o = (r - d)^o / o! the integrands of a quadrature point are
+//   G: (ik)^o D_o / r,   F: (ik)^o n.rho (-D_o / r^3 + D_(o-1) / r^2),
+// real factors times powers of ik.  What multiplies the weights W E is needed
+// as a real part only, so the powers of both media are folded beforehand into
+// real coefficients cg_o, cf_o = sum_m Re(W_m E_m (ik_m)^o), and what is needed
+// as a complex number (derivatives by d and k) is a sum over the points of
+// ww D_o / r, ww n.rho D_o / r^2 and ww n.rho D_o / r^3: three real moments per
+// order, combined with (ik)^o once per pair.  About 130 FP64 operations per
+// point (FP64 is the bound: two per clock and SM); evaluating every order's
+// derivatives per medium, with divisions by the factorials, took about 2600.
+// For the 2016-face rod this pass and the next took 26 ms together; this one
+// takes 1.04 ms now.
+// MO: highest order held in registers (the coefficients above p.order are 0).
+template <int MO>
+__global__ void __launch_bounds__(64) k_adj_near(AdjParams p) {
   const int t = blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= p.noff) return;
   const int e = p.off_idx[t];
   const int i = p.ref_row[e], j = p.ref_col[e];
-  const int O = p.order;
   const double3 ri = vld(p.pos, i), rj = vld(p.pos, j), ni = vld(p.nvec, i);
   const double Ai = p.area[i], Aj = p.area[j];
   const double3 R = vsub(ri, rj);
-  const double d = sqrt(vdot(R, R));
-  const double3 Rh = vscale(R, 1.0 / d);
+  const double d = sqrt(vdot(R, R)), inv = 1.0 / d;
+  const double3 Rh = vscale(R, inv);
   const double2* U = p.U + (int64_t)i * 16;
   double2 X1[4], X2[4];
 #pragma unroll
   for (int r = 0; r < 4; ++r) { X1[r] = p.X[(int64_t)j * 8 + r]; X2[r] = p.X[(int64_t)j * 8 + 4 + r]; }
-  const double2 W[4] = {wdot(U, X1), wdot(U + 4, X1), wdot(U + 8, X2), wdot(U + 12, X2)};
-  const double2 ks[2] = {p.k1, p.k2};
+  double2 W[4] = {wdot(U, X1), wdot(U + 4, X1), wdot(U + 8, X2), wdot(U + 12, X2)};
   // remove the far derivative that the pair pass applied
   FarGrad g;
   g.gri = g.grj = g.gni = v3(0, 0, 0);
   g.gaj = 0.0;
   g.gk = make_double2(0, 0);
-  far_grad(p.k1, W[0], W[1], R, d, ni, Aj, g, true);
-  far_grad(p.k2, W[2], W[3], R, d, ni, Aj, g, false);
+  const double2 Em[2] = {cexpi(p.k1, d), cexpi(p.k2, d)};
+  far_grad(p.k1, Em[0], W[0], W[1], R, d, inv, ni, Aj, g, true);
+  far_grad(p.k2, Em[1], W[2], W[3], R, d, inv, ni, Aj, g, false);
   double3 gri = vscale(g.gri, -1.0), grj = vscale(g.grj, -1.0), gni = vscale(g.gni, -1.0);
-  double gaj = -g.gaj;
+  double gaj = -g.gaj, gai = 0.0;
   double2 gk = cscl(g.gk, -1.0);
   const double cb = p.cb[j];
   {
     double3 ca = v3(0, 0, 0), cbv = v3(0, 0, 0), cn = v3(0, 0, 0);
     double cga = 0.0;
-    closed_far_grad(cb, R, d, ni, Ai, ca, cbv, cn, cga);
+    closed_far_grad(cb, R, inv, ni, Ai, ca, cbv, cn, cga);
     gri = vsub(gri, ca);
     grj = vsub(grj, cbv);
     gni = vsub(gni, cn);
-    atomicAdd(p.garea + i, -cga);
+    gai -= cga;
   }
-  // near derivative, per medium and per quadrature point of face j
-  double2 E[2], c[2][MAX_ORDER_ADJ + 1];
+  // weights times phase, and the real coefficients of the orders
+  double cg[MO + 1], cf[MO + 1];
+#pragma unroll
+  for (int o = 0; o <= MO; ++o) cg[o] = cf[o] = 0.0;
+#pragma unroll
   for (int m = 0; m < 2; ++m) {
-    E[m] = cexpi(ks[m], d);
-    double2 ik = cx(-ks[m].y, ks[m].x), pw = cx(1.0, 0.0);
-    double fo = 1.0;
-    for (int o = 0; o <= O; ++o) {
-      if (o) fo *= o;
-      c[m][o] = cscl(pw, 1.0 / fo);      // (ik)^o / o!
+    const double2 k = m ? p.k2 : p.k1;
+    const double2 ik = cx(-k.y, k.x);
+    W[2 * m] = cmul(W[2 * m], Em[m]);
+    W[2 * m + 1] = cmul(W[2 * m + 1], Em[m]);
+    double2 pw = cx(1.0, 0.0);
+#pragma unroll
+    for (int o = 0; o <= MO; ++o) {
+      if (o <= p.order) {
+        cg[o] += remul(W[2 * m], pw);
+        cf[o] += remul(W[2 * m + 1], pw);
+      }
       pw = cmul(pw, ik);
     }
   }
-  double2 gam[2] = {cx(0, 0), cx(0, 0)}, phn[2] = {cx(0, 0), cx(0, 0)};
-  double2 sGd[2] = {cx(0, 0), cx(0, 0)}, sPd[2] = {cx(0, 0), cx(0, 0)};
-  double2 sGk = cx(0, 0), sPk = cx(0, 0);
-  double3 grho_sum = v3(0, 0, 0);
-  double3 gni_sum = v3(0, 0, 0);
-  double ccl_area_a = 0.0, ccl_area_b = 0.0;   // closed-surface area terms
-  double3 ccl_na = v3(0, 0, 0), ccl_ra = v3(0, 0, 0);
-  const double fac = -Ai / Aj;
+  double T1[MO + 1], V2[MO + 1], V3[MO + 1];
+#pragma unroll
+  for (int o = 0; o <= MO; ++o) T1[o] = V2[o] = V3[o] = 0.0;
+  const double cbf = -cb * Ai / Aj;                // closed-surface near term: cbf sum_w ww nrho / r^3
   const int* f = p.faces + 4 * j;
   const int ntri = f[3] < 0 ? 1 : 2;
-  // first pass: sums over the points (gam, phn, d-derivatives) per medium
-  // and the per-point gradients, which need gam-independent factors only
+  double3 grho_sum = v3(0, 0, 0);
   for (int tr = 0; tr < ntri; ++tr) {
     int a, b, cc;
     tri_ids(f, tr, a, b, cc);
     const double3 va = vld(p.verts, a), vb = vld(p.verts, b), vc = vld(p.verts, cc);
     const double3 N = vcross(vsub(vb, va), vsub(vc, va));
     const double atri = 0.5 * sqrt(vdot(N, N));
-    double3 gva = v3(0, 0, 0), gvb = v3(0, 0, 0), gvc = v3(0, 0, 0);
-    double gatri = 0.0;
+    const double3 rc = vsub(ri, vc), ea = vsub(va, vc), eb = vsub(vb, vc);
+    // dJ / d rho = al rho + be n_i per point: sums with weights 1, x and y
+    double3 S = v3(0, 0, 0), Sx = v3(0, 0, 0), Sy = v3(0, 0, 0);
+    double B = 0.0, Bx = 0.0, By = 0.0, gatri = 0.0;
     for (int q = 0; q < p.ntri; ++q) {
-      const double x = p.xt[q], y = p.yt[q], z = 1 - x - y;
-      const double3 pt = v3(x * va.x + y * vb.x + z * vc.x, x * va.y + y * vb.y + z * vc.y,
-                            x * va.z + y * vb.z + z * vc.z);
-      const double qw = p.wt[q];
+      const double x = p.xt[q], y = p.yt[q], qw = p.wt[q];
       const double ww = qw * atri;
-      const double3 rho = vsub(ri, pt);
-      const double r = sqrt(vdot(rho, rho));
-      const double ir = 1.0 / r;
-      const double3 rh = vscale(rho, ir);
+      const double3 rho = v3(rc.x - x * ea.x - y * eb.x, rc.y - x * ea.y - y * eb.y, rc.z - x * ea.z - y * eb.z);
+      const double r2 = vdot(rho, rho);
+      const double ir = rsqrt(r2), ir2 = ir * ir, ir3 = ir2 * ir;
       const double nrho = vdot(ni, rho);
-      const double dr = r - d;
-      double3 gpt = v3(0, 0, 0);   // dJ / d rho (this point)
-      double gw = 0.0;             // dJ / d ww
-      for (int m = 0; m < 2; ++m) {
-        double2 Gam = cx(0, 0), Gr = cx(0, 0), Gd = cx(0, 0), Psi = cx(0, 0), Pr = cx(0, 0), Pd = cx(0, 0);
-        double2 Gk = cx(0, 0), Pk = cx(0, 0);
-        double drp = 1.0, drm = 0.0, drmm = 0.0;   // dr^o, dr^(o-1), dr^(o-2)
-        double fo = 1.0, fo1 = 1.0;                // o!, (o-1)!
-        const double2 ik = cx(-ks[m].y, ks[m].x);
-        double2 ikm1 = cx(1.0, 0.0);               // (ik)^(o-1) for o >= 1
-        for (int o = 0; o <= O; ++o) {
-          if (o) { fo1 = fo; fo *= o; }
-          const double2 co = cscl(c[m][o], fo);    // (ik)^o
-          const double gam_o = drp * ir / fo;
-          const double gr_o = ((o ? o * drm * ir : 0.0) - drp * ir * ir) / fo;
-          const double gd_o = -(o ? o * drm * ir : 0.0) / fo;
-          double ps, psr, psd;
-          if (o == 0) {
-            ps = -ir * ir * ir;
-            psr = 3.0 * ir * ir * ir * ir;
-            psd = 0.0;
-          } else {
-            ps = -drp * ir * ir * ir / fo + drm * ir * ir / fo1;
-            psr = -(o * drm * ir * ir * ir - 3.0 * drp * ir * ir * ir * ir) / fo +
-                  ((o > 1 ? (o - 1) * drmm : 0.0) * ir * ir - 2.0 * drm * ir * ir * ir) / fo1;
-            psd = o * drm * ir * ir * ir / fo - (o > 1 ? (o - 1) * drmm : 0.0) * ir * ir / fo1;
-          }
-          Gam = cadd(Gam, cscl(co, gam_o));
-          Gr = cadd(Gr, cscl(co, gr_o));
-          Gd = cadd(Gd, cscl(co, gd_o));
-          Psi = cadd(Psi, cscl(co, ps));
-          Pr = cadd(Pr, cscl(co, psr));
-          Pd = cadd(Pd, cscl(co, psd));
-          if (o && m == 0) {
-            // d/dk (ik)^o = o i (ik)^(o-1)
-            const double2 dko = cscl(imul(ikm1), (double)o);
-            Gk = cadd(Gk, cscl(dko, gam_o));
-            Pk = cadd(Pk, cscl(dko, ps));
-          }
-          if (o) ikm1 = cmul(ikm1, ik);
-          drmm = drm;
-          drm = drp;
-          drp *= dr;
-        }
-        const double2 WgE = cmul(W[2 * m], E[m]), WfE = cmul(W[2 * m + 1], E[m]);
-        gam[m] = cadd(gam[m], cscl(Gam, ww));
-        phn[m] = cadd(phn[m], cscl(Psi, ww * nrho));
-        sGd[m] = cadd(sGd[m], cscl(Gd, ww));
-        sPd[m] = cadd(sPd[m], cscl(Pd, ww * nrho));
-        if (m == 0) {
-          sGk = cadd(sGk, cscl(Gk, ww));
-          sPk = cadd(sPk, cscl(Pk, ww * nrho));
-        }
-        // crho = WgE ww Gr rh + WfE ww (n Psi + nrho Pr rh); dJ/drho = -Re(crho)
-        const double2 a1 = cscl(cmul(WgE, Gr), ww);
-        const double2 a2 = cscl(cmul(WfE, Psi), ww);
-        const double2 a3 = cscl(cmul(WfE, Pr), ww * nrho);
-        gpt = vsub(gpt, vadd(vscale(rh, a1.x + a3.x), vscale(ni, a2.x)));
-        gw -= remul(WgE, Gam) + remul(WfE, cscl(Psi, nrho));
-        gni_sum = vsub(gni_sum, vscale(rho, remul(WfE, cscl(Psi, ww))));
+      const double dr = r2 * ir - d;
+      double D[MO + 1];
+      D[0] = 1.0;
+#pragma unroll
+      for (int o = 1; o <= MO; ++o) D[o] = D[o - 1] * (dr * (1.0 / o));
+      double P0 = cg[0], P1 = 0.0, Q0 = cf[0], Q1 = 0.0, Q2 = 0.0;
+#pragma unroll
+      for (int o = 1; o <= MO; ++o) {
+        P0 += cg[o] * D[o];
+        P1 += cg[o] * D[o - 1];
+        Q0 += cf[o] * D[o];
+        Q1 += cf[o] * D[o - 1];
+        if (o > 1) Q2 += cf[o] * D[o - 2];
       }
-      // closed-surface near term T = fac sum_w ww nrho / r^3 (order 0, k = 0)
-      {
-        const double ir3 = ir * ir * ir;
-        const double Tq = fac * ww * nrho * ir3;
-        ccl_area_a += cb * Tq / Ai;
-        ccl_area_b -= cb * Tq / Aj;
-        ccl_na = vadd(ccl_na, vscale(rho, cb * fac * ww * ir3));
-        const double3 gq = vscale(vsub(vscale(ni, ir3), vscale(rho, 3.0 * nrho * ir3 * ir * ir)), cb * fac * ww);
-        gpt = vadd(gpt, gq);
-        gw += cb * fac * nrho * ir3;
+      const double w1 = ww * ir, w2 = ww * nrho * ir2, w3 = w2 * ir;
+#pragma unroll
+      for (int o = 0; o <= MO; ++o) {
+        T1[o] += w1 * D[o];
+        V2[o] += w2 * D[o];
+        V3[o] += w3 * D[o];
       }
-      grho_sum = vadd(grho_sum, gpt);
-      // rho = r_i - x_w, x_w = x va + y vb + z vc
-      gva = vsub(gva, vscale(gpt, x));
-      gvb = vsub(gvb, vscale(gpt, y));
-      gvc = vsub(gvc, vscale(gpt, z));
-      gatri += gw * qw;
+      const double ps = ir2 * (Q1 - ir * Q0);                                      // sum cf_o psi_o
+      const double pr = ir2 * (Q2 - 3.0 * ir * (Q1 - ir * Q0));                    // its derivative by r
+      const double gr = ir * (P1 - ir * P0);                                       // sum cg_o d(D_o / r)/dr
+      const double bw = cbf * ir3 - ps;
+      const double be = ww * bw;
+      const double al = -ww * ir * (gr + nrho * (pr + 3.0 * cbf * ir3 * ir));
+      gatri += qw * (nrho * bw - ir * P0);
+      const double3 ar = vscale(rho, al);
+      S = vadd(S, ar);
+      Sx = v3(Sx.x + x * ar.x, Sx.y + x * ar.y, Sx.z + x * ar.z);
+      Sy = v3(Sy.x + y * ar.x, Sy.y + y * ar.y, Sy.z + y * ar.z);
+      B += be;
+      Bx += x * be;
+      By += y * be;
+      gni = v3(gni.x + be * rho.x, gni.y + be * rho.y, gni.z + be * rho.z);
     }
-    vatomic(p.gv, a, gva);
-    vatomic(p.gv, b, gvb);
-    vatomic(p.gv, cc, gvc);
+    S = vadd(S, vscale(ni, B));
+    Sx = vadd(Sx, vscale(ni, Bx));
+    Sy = vadd(Sy, vscale(ni, By));
+    grho_sum = vadd(grho_sum, S);
+    // rho = r_i - x_w, x_w = x va + y vb + (1 - x - y) vc
+    vatomic(p.gv, a, vscale(Sx, -1.0));
+    vatomic(p.gv, b, vscale(Sy, -1.0));
+    vatomic(p.gv, cc, vsub(vadd(Sx, Sy), S));
     tri_area_grad(p.gv, a, b, cc, va, vb, vc, gatri);
   }
   gri = vadd(gri, grho_sum);
-  gni = vadd(gni, gni_sum);
-  gni = vadd(gni, ccl_na);
-  // explicit d-dependence (incl. the phase): -Re(W E (sum d-derivatives + (gam or phn) ik))
+  gai += cbf * V3[0] / Ai;
+  gaj -= cbf * V3[0] / Aj;
+  // explicit d-dependence (incl. the phase): -Re(W E (sum d-derivatives + (gam or phn) ik)),
+  // and d/dk1: E (sum dk-terms + (gam or phn) i d)
+#pragma unroll
   for (int m = 0; m < 2; ++m) {
-    const double2 ik = cx(-ks[m].y, ks[m].x);
-    const double2 cd = cadd(cmul(cmul(W[2 * m], E[m]), cadd(sGd[m], cmul(gam[m], ik))),
-                            cmul(cmul(W[2 * m + 1], E[m]), cadd(sPd[m], cmul(phn[m], ik))));
+    const double2 k = m ? p.k2 : p.k1;
+    const double2 ik = cx(-k.y, k.x);
+    double2 gam = cx(0, 0), phn = cx(0, 0), gd = cx(0, 0), pd = cx(0, 0), Gk = cx(0, 0), Pk = cx(0, 0);
+    double2 pw = cx(1.0, 0.0), pm = cx(0.0, 0.0);      // (ik)^o, (ik)^(o-1)
+#pragma unroll
+    for (int o = 0; o <= MO; ++o) {
+      if (o <= p.order) {
+        const double po = (o ? V2[o - 1] : 0.0) - V3[o];
+        gam = cadd(gam, cscl(pw, T1[o]));
+        phn = cadd(phn, cscl(pw, po));
+        if (o) {
+          gd = csub(gd, cscl(pw, T1[o - 1]));
+          pd = cadd(pd, cscl(pw, V3[o - 1] - (o > 1 ? V2[o - 2] : 0.0)));
+          const double2 dk = cscl(imul(pm), (double)o);     // d/dk (ik)^o = o i (ik)^(o-1)
+          Gk = cadd(Gk, cscl(dk, T1[o]));
+          Pk = cadd(Pk, cscl(dk, po));
+        }
+      }
+      pm = pw;
+      pw = cmul(pw, ik);
+    }
+    const double2 cd = cadd(cmul(W[2 * m], cadd(gd, cmul(gam, ik))), cmul(W[2 * m + 1], cadd(pd, cmul(phn, ik))));
     gri = vsub(gri, vscale(Rh, cd.x));
     grj = vadd(grj, vscale(Rh, cd.x));
+    if (m == 0)
+      gk = cadd(gk, cadd(cmul(W[0], cadd(Gk, imul(cscl(gam, d)))), cmul(W[1], cadd(Pk, imul(cscl(phn, d))))));
   }
-  // d/dk1 of the refined entries: E (sum dk-terms + (gam or phn) i d)
-  gk = cadd(gk, cadd(cmul(cmul(W[0], E[0]), cadd(sGk, imul(cscl(gam[0], d)))),
-                     cmul(cmul(W[1], E[0]), cadd(sPk, imul(cscl(phn[0], d))))));
   vatomic(p.gpos, i, gri);
   vatomic(p.gpos, j, grj);
   vatomic(p.gnv, i, gni);
   atomicAdd(p.garea + j, gaj);
-  atomicAdd(p.garea + i, ccl_area_a);
-  atomicAdd(p.garea + j, ccl_area_b);
+  atomicAdd(p.garea + i, gai);
   atomicAdd(p.gk1, gk.x);
   atomicAdd(p.gk1 + 1, gk.y);
 }
 
+__device__ __forceinline__ double warp_sum(double v) {
+#pragma unroll
+  for (int o = 16; o; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  return v;
+}
+
 // self elements: G_ii = sum_w ww sum_o (ik)^o r^(o-1) / o! over the polar
 // points of face i (greenret/private/init.m:42-95); weights ww = w3 A_i for
-// triangles, w4 |dx/du x dx/dv| for quadrilaterals (quadpol_flat.m:33-77)
-__global__ void k_adj_self(AdjParams p) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
+// triangles, w4 |dx/du x dx/dv| for quadrilaterals (quadpol_flat.m:33-77).
+// One warp per face, lanes over its points; both media's weights are folded
+// into real coefficients of the powers of r (as above), so a point costs two
+// Horner sums and a few moments.  One thread per face with a pow() per order,
+// medium and point ran 144 points serially on a quarter of the SMs.
+constexpr int SELF_WARPS = 4;
+template <int MO>
+__global__ void __launch_bounds__(32 * SELF_WARPS) k_adj_self(AdjParams p) {
+  const int i = blockIdx.x * SELF_WARPS + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (i >= p.n) return;
-  const int O = p.order;
   const int* f = p.faces + 4 * i;
   const bool quad = f[3] >= 0;
   const int nv = quad ? 4 : 3;
   double3 vv[4];
-  for (int a = 0; a < nv; ++a) vv[a] = vld(p.verts, f[a]);
+#pragma unroll
+  for (int a = 0; a < 4; ++a) vv[a] = a < nv ? vld(p.verts, f[a]) : v3(0, 0, 0);
   double3 cen = v3(0, 0, 0);
-  for (int a = 0; a < nv; ++a) cen = vadd(cen, vv[a]);
+#pragma unroll
+  for (int a = 0; a < 4; ++a) cen = vadd(cen, vv[a]);
   cen = vscale(cen, 1.0 / nv);
   const double2* U = p.U + (int64_t)i * 16;
   double2 X1[4], X2[4];
 #pragma unroll
   for (int r = 0; r < 4; ++r) { X1[r] = p.X[(int64_t)i * 8 + r]; X2[r] = p.X[(int64_t)i * 8 + 4 + r]; }
-  const double2 WG[2] = {wdot(U, X1), wdot(U + 8, X2)};
-  const double2 ks[2] = {p.k1, p.k2};
+  const double2 WG0 = wdot(U, X1);
+  double A[MO + 1];                                 // sum_m Re(WG_m (ik_m)^o / o!)
+#pragma unroll
+  for (int o = 0; o <= MO; ++o) A[o] = 0.0;
+#pragma unroll
+  for (int m = 0; m < 2; ++m) {
+    const double2 k = m ? p.k2 : p.k1;
+    const double2 ik = cx(-k.y, k.x), w = m ? wdot(U + 8, X2) : WG0;
+    double2 pw = cx(1.0, 0.0);
+#pragma unroll
+    for (int o = 0; o <= MO; ++o) {
+      if (o <= p.order) A[o] += remul(w, pw);
+      pw = cscl(cmul(pw, ik), 1.0 / (o + 1));
+    }
+  }
   double3 gv[4] = {v3(0, 0, 0), v3(0, 0, 0), v3(0, 0, 0), v3(0, 0, 0)};
   double garea = 0.0;
-  double2 gk = cx(0, 0);
+  double M[MO + 1];                                 // sum_w ww r^(o-1), o >= 1
+#pragma unroll
+  for (int o = 0; o <= MO; ++o) M[o] = 0.0;
   const int npts = quad ? p.n4 : p.n3;
-  for (int q = 0; q < npts; ++q) {
+  for (int q = lane; q < npts; q += 32) {
     double s[4], sx[4], sy[4];
     double w0;
     if (!quad) {
@@ -437,56 +462,69 @@ __global__ void k_adj_self(AdjParams p) {
       w0 = p.w4[q];
     }
     double3 pt = v3(0, 0, 0);
-    for (int a = 0; a < nv; ++a) pt = vadd(pt, vscale(vv[a], s[a]));
+#pragma unroll
+    for (int a = 0; a < 4; ++a) pt = vadd(pt, vscale(vv[a], s[a]));
     const double3 rho = vsub(cen, pt);
-    const double r = sqrt(vdot(rho, rho));
-    const double3 rh = vscale(rho, 1.0 / r);
+    const double r = sqrt(vdot(rho, rho)), ir = 1.0 / r;
     double ww, jn = 0.0;
     double3 jac = v3(0, 0, 0), px = v3(0, 0, 0), py = v3(0, 0, 0);
     if (!quad) {
       ww = w0 * p.area[i];
     } else {
+#pragma unroll
       for (int a = 0; a < 4; ++a) { px = vadd(px, vscale(vv[a], sx[a])); py = vadd(py, vscale(vv[a], sy[a])); }
       jac = vcross(px, py);
       jn = sqrt(vdot(jac, jac));
       ww = w0 * jn;
     }
-    double3 grho = v3(0, 0, 0);
-    double gw = 0.0;
-    for (int m = 0; m < 2; ++m) {
-      const double2 ik = cx(-ks[m].y, ks[m].x);
-      double2 pw = cx(1.0, 0.0), ikm1 = cx(1.0, 0.0);
-      double2 Gam = cx(0, 0), Gr = cx(0, 0), Gk = cx(0, 0);
-      double fo = 1.0;
-      for (int o = 0; o <= O; ++o) {
-        if (o) fo *= o;
-        const double ro1 = pow(r, (double)(o - 1));
-        Gam = cadd(Gam, cscl(pw, ro1 / fo));
-        Gr = cadd(Gr, cscl(pw, (o - 1) * pow(r, (double)(o - 2)) / fo));
-        if (o && m == 0) {
-          Gk = cadd(Gk, cscl(imul(ikm1), (double)o * ro1 / fo));
-          ikm1 = cmul(ikm1, ik);
-        }
-        pw = cmul(pw, ik);
-      }
-      grho = vsub(grho, vscale(rh, remul(WG[m], cscl(Gr, ww))));
-      gw -= remul(WG[m], Gam);
-      if (m == 0) gk = cadd(gk, cmul(WG[0], cscl(Gk, ww)));
+    double h0 = A[MO], h1 = (MO - 1) * A[MO], pw = ww;
+#pragma unroll
+    for (int o = MO - 1; o >= 0; --o) {
+      h0 = h0 * r + A[o];
+      h1 = h1 * r + (o - 1) * A[o];
     }
+#pragma unroll
+    for (int o = 1; o <= MO; ++o) {
+      M[o] += pw;
+      pw *= r;
+    }
+    const double gw = -ir * h0;                     // -sum A_o r^(o-1)
+    const double3 grho = vscale(rho, -ww * h1 * ir * ir * ir);
     // rho = cen - pt = sum_a (1/nv - s_a) v_a
-    for (int a = 0; a < nv; ++a) gv[a] = vadd(gv[a], vscale(grho, 1.0 / nv - s[a]));
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+      if (a < nv) gv[a] = vadd(gv[a], vscale(grho, 1.0 / nv - s[a]));
     if (!quad) {
       garea += gw * w0;
     } else {
       const double3 gj = vscale(jac, gw * w0 / jn);
       const double3 gpx = vcross(py, gj), gpy = vcross(gj, px);
+#pragma unroll
       for (int a = 0; a < 4; ++a) gv[a] = vadd(gv[a], vadd(vscale(gpx, sx[a]), vscale(gpy, sy[a])));
     }
   }
-  for (int a = 0; a < nv; ++a) vatomic(p.gv, f[a], gv[a]);
-  atomicAdd(p.garea + i, garea);
-  atomicAdd(p.gk1, gk.x);
-  atomicAdd(p.gk1 + 1, gk.y);
+#pragma unroll
+  for (int a = 0; a < 4; ++a) gv[a] = v3(warp_sum(gv[a].x), warp_sum(gv[a].y), warp_sum(gv[a].z));
+  garea = warp_sum(garea);
+#pragma unroll
+  for (int o = 1; o <= MO; ++o) M[o] = warp_sum(M[o]);
+  if (lane == 0) {
+#pragma unroll
+    for (int a = 0; a < 4; ++a)
+      if (a < nv) vatomic(p.gv, f[a], gv[a]);
+    atomicAdd(p.garea + i, garea);
+    // dG/dk1: sum_o i (ik)^(o-1) / (o-1)! M_o
+    const double2 ik = cx(-p.k1.y, p.k1.x);
+    double2 pw = cx(0.0, 1.0), sk = cx(0, 0);
+#pragma unroll
+    for (int o = 1; o <= MO; ++o) {
+      if (o <= p.order) sk = cadd(sk, cscl(pw, M[o]));
+      pw = cscl(cmul(pw, ik), 1.0 / o);
+    }
+    const double2 gk = cmul(WG0, sk);
+    atomicAdd(p.gk1, gk.x);
+    atomicAdd(p.gk1 + 1, gk.y);
+  }
 }
 
 // per face: weights U, X and the closed-surface factor c_i = WH1_ii + WH2_ii
@@ -950,17 +988,24 @@ void adj_weights(const AdjParams& p, const double2* lphi, const double2* la, con
   k_adj_weights<<<(unsigned)cdiv_up(p.n, 128), 128, 0, st>>>(p, lphi, la, lDe, lal, x1, x2, P, ip);
 }
 
-void adj_geometry(const AdjParams& p, int which, const double* pol, const double* dir, const double2* lphi,
-                  const double2* la, const double2* lDe, const double2* lal, const double2* GX1,
-                  const double2* GX2, const double2* HX1, double* geps, cudaStream_t st) {
+mnpbem_status adj_geometry(const AdjParams& p, int which, const double* pol, const double* dir, const double2* lphi,
+                           const double2* la, const double2* lDe, const double2* lal, const double2* GX1,
+                           const double2* GX2, const double2* HX1, double* geps, cudaStream_t st) {
+  const CisTable* table = nullptr;
+  MNP_TRY(cis_table(&table, st));
   ProfScope ps(PH_ASSEMBLE, st, 0.0, 0.0, 5);
   dim3 g((unsigned)cdiv_up(p.n, PG_COLS), (unsigned)cdiv_up(p.n, PG_ROWS));
-  k_adj_pairs<<<g, PG_COLS, 0, st>>>(p);
-  if (p.noff > 0) k_adj_near<<<(unsigned)cdiv_up(p.noff, 64), 64, 0, st>>>(p);
-  k_adj_self<<<(unsigned)cdiv_up(p.n, 64), 64, 0, st>>>(p);
+  k_adj_pairs<<<g, PG_COLS, 0, st>>>(p, table);
+  // orders up to 5 (the default) in registers, else up to the limit
+  const auto near = p.order <= 5 ? k_adj_near<5> : k_adj_near<MAX_ORDER_ADJ>;
+  const auto self = p.order <= 5 ? k_adj_self<5> : k_adj_self<MAX_ORDER_ADJ>;
+  if (p.noff > 0) near<<<(unsigned)cdiv_up(p.noff, 64), 64, 0, st>>>(p);
+  self<<<(unsigned)cdiv_up(p.n, (int64_t)SELF_WARPS), 32 * SELF_WARPS, 0, st>>>(p);
   k_adj_faces<<<(unsigned)cdiv_up(p.n, 128), 128, 0, st>>>(p, which, pol, dir, lphi, la, lDe, lal, GX1, GX2, HX1,
                                                            geps);
   k_adj_norm_flat<<<(unsigned)cdiv_up(p.n, 128), 128, 0, st>>>(p);
+  MNP_CHECK_LAUNCH();
+  return MNPBEM_OK;
 }
 
 }  // namespace mnpbem

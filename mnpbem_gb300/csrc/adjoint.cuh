@@ -67,8 +67,8 @@ void adj_chain_step(const AdjParams& p, int mode, const double2* a, const double
 void adj_weights(const AdjParams& p, const double2* lphi, const double2* la, const double2* lDe,
                  const double2* lal, const double2* x1, const double2* x2, int P, int ip, cudaStream_t st);
 // all geometric contractions and the chain rule to the vertices (which: 0 ext, 1 sca)
-void adj_geometry(const AdjParams& p, int which, const double* pol, const double* dir, const double2* lphi,
-                  const double2* la, const double2* lDe, const double2* lal, const double2* GX1,
-                  const double2* GX2, const double2* HX1, double* geps, cudaStream_t st);
+mnpbem_status adj_geometry(const AdjParams& p, int which, const double* pol, const double* dir, const double2* lphi,
+                           const double2* la, const double2* lDe, const double2* lal, const double2* GX1,
+                           const double2* GX2, const double2* HX1, double* geps, cudaStream_t st);
 
 }  // namespace mnpbem

@@ -1288,8 +1288,7 @@ mnpbem_status stage_spectra(mnpbem_geom* G, Lane& L, const SolveCtx& c) {
   const double* inf_area = inf_nvec + 3 * ninf;
   double2* fields = L.fields.as<double2>();
   const LamParams* lp = L.lp_dev.as<LamParams>();
-  launch_farfield(face_data(G, L), P, v.x1, v.x2, dirs, P + ninf, lp, fields, L.st);
-  MNP_CHECK_LAUNCH();
+  MNP_TRY(launch_farfield(face_data(G, L), P, v.x1, v.x2, dirs, P + ninf, lp, fields, L.st));
   double* slot = L.outbuf.as<double>();
   launch_cross_sections_lp(P, pol, inf_nvec, inf_area, ninf, fields, lp, slot, slot + P, L.st);
   MNP_CHECK_LAUNCH();
@@ -2720,8 +2719,7 @@ mnpbem_status mnpbem_cross_section_gradient(mnpbem_geom* G, const mnpbem_planewa
     MNP_TRY(gemm_simt<double>(n, 1, n, one, ap.H1, ld, Xb, 8, zero, HX1, 1, st));
   }
   // ---- geometric contractions and the chain rule to the vertices
-  adj_geometry(p, which, pol_d, dir_d, gphi, ga, gDe, gAl, GX1, GX2, HX1, geps, st);
-  MNP_CHECK_LAUNCH();
+  MNP_TRY(adj_geometry(p, which, pol_d, dir_d, gphi, ga, gDe, gAl, GX1, GX2, HX1, geps, st));
   MNP_CUDA(cudaMemcpyAsync(verts_grad, p.gv, sizeof(double) * 3 * nv, cudaMemcpyDeviceToHost, st));
   double hk[4];
   MNP_CUDA(cudaMemcpyAsync(hk, p.gk1, sizeof(double) * 4, cudaMemcpyDeviceToHost, st));

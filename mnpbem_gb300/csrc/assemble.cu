@@ -8,34 +8,16 @@
 //
 // One pass writes G1, H1, G2, H2 as complex128 and/or complex64 (row-major, ld).
 #include "assemble.cuh"
+#include "cis.cuh"
 #include "profile.cuh"
+
+#include <atomic>
 
 namespace mnpbem {
 
 struct PairVal { double2 G, F; };
 
-// ------------------------------------------------------- exp(i k d), FP64
-// Table-driven evaluation (Cody-Waite argument reduction + short Taylor
-// polynomials), a few FP64 FMAs per call instead of a library sincos and exp:
-//   phase  th = Re(k) d = j (2 pi / 256) + t,  |t| <= pi / 256:
-//          cis(th) = cis(2 pi j / 256) * (cos t + i sin t), Taylor to t^8;
-//   decay  x = Im(k) d = y (ln 2 / 64) + u,   |u| <= ln 2 / 128:
-//          exp(-x) = 2^(-floor(y/64)) * 2^(-(y mod 64)/64) * exp(-u), Taylor to u^7.
-// The reduction constants are split in a 32-bit head (exact products with
-// |j| < 2^20) and a tail; the tables come from the device's sincospi / exp2
-// once per device.  Accuracy: a few ulp of the FP64 result.
-constexpr int CIS_N = 256;
-constexpr double CIS_INV = 40.74366543152521;        // 256 / (2 pi)
-constexpr double CIS_C1 = 0.024543692605220713;      // 2 pi / 256, head
-constexpr double CIS_C2 = 9.495469541415925e-13;     // 2 pi / 256, tail
-constexpr double EXP_INV = 92.33248261689366;        // 64 / ln 2
-constexpr double EXP_L1 = 0.01083042469326756;       // ln 2 / 64, head
-constexpr double EXP_L2 = 2.9815858269852933e-12;    // ln 2 / 64, tail
-
-struct CisTable {
-  double2 cs[CIS_N];   // (cos, sin)(2 pi j / 256)
-  double e2[64];       // 2^(-m / 64)
-};
+// ------------------------------------------------- table of exp(i k d), FP64
 __device__ CisTable g_cis;
 
 __global__ void k_cis_init() {
@@ -46,52 +28,7 @@ __global__ void k_cis_init() {
   if (j < 64) g_cis.e2[j] = exp2(-j / 64.0);
 }
 
-struct CisShared {
-  double2 cs[CIS_N];
-  double e2[64];
-};
-
-__device__ __forceinline__ void cis_load(CisShared& t) {
-  for (int q = threadIdx.x; q < CIS_N; q += blockDim.x) t.cs[q] = g_cis.cs[q];
-  for (int q = threadIdx.x; q < 64; q += blockDim.x) t.e2[q] = g_cis.e2[q];
-  __syncthreads();
-}
-
-// exp(i k d) for complex k (Im k >= 0 for passive media; any sign works)
-__device__ __forceinline__ double2 cis_exp(const CisShared& T, double2 k, double d) {
-  const double th = k.x * d;
-  const double jf = rint(th * CIS_INV);
-  const double t = fma(-jf, CIS_C2, fma(-jf, CIS_C1, th));
-  const double t2 = t * t;
-  const double sn = t * fma(t2, fma(t2, fma(t2, -1.0 / 5040.0, 1.0 / 120.0), -1.0 / 6.0), 1.0);
-  const double cn = fma(t2, fma(t2, fma(t2, fma(t2, 1.0 / 40320.0, -1.0 / 720.0), 1.0 / 24.0), -0.5), 1.0);
-  const double2 tb = T.cs[((long long)jf) & (CIS_N - 1)];
-  double cr = tb.x * cn - tb.y * sn;
-  double sr = fma(tb.y, cn, tb.x * sn);
-  if (k.y != 0.0) {
-    const double x = k.y * d;
-    double e;
-    if (x > 700.0) {
-      e = 0.0;
-    } else {
-      const double yf = rint(x * EXP_INV);
-      const double u = fma(-yf, EXP_L2, fma(-yf, EXP_L1, x));
-      const double v = -u;
-      const double ev = fma(v, fma(v, fma(v, fma(v, fma(v, fma(v, fma(v, 1.0 / 5040.0, 1.0 / 720.0), 1.0 / 120.0),
-                                                          1.0 / 24.0), 1.0 / 6.0), 0.5), 1.0), 1.0);
-      const long long yi = (long long)yf;
-      const long long nn = yi >> 6;                 // floor(y / 64)
-      const int m = (int)(yi - (nn << 6));
-      const double scale = __longlong_as_double((unsigned long long)(1023 - nn) << 52);   // 2^(-nn)
-      e = ev * T.e2[m] * scale;
-    }
-    cr *= e;
-    sr *= e;
-  }
-  return make_double2(cr, sr);
-}
-
-static bool g_cis_ready[64];
+static std::atomic<bool> g_cis_ready[64];
 static mnpbem_status ensure_cis(cudaStream_t st) {
   int dev = 0;
   MNP_CUDA(cudaGetDevice(&dev));
@@ -99,13 +36,23 @@ static mnpbem_status ensure_cis(cudaStream_t st) {
   if (!g_cis_ready[dev]) {
     k_cis_init<<<1, CIS_N, 0, st>>>();
     MNP_CHECK_LAUNCH();
-    if (!capturing_now()) g_cis_ready[dev] = true;
+    if (!capturing_now()) {
+      MNP_CUDA(cudaStreamSynchronize(st));   // other streams may read it from now on
+      g_cis_ready[dev] = true;
+    }
   }
+  return MNPBEM_OK;
+}
+mnpbem_status cis_table(const CisTable** table, cudaStream_t st) {
+  MNP_TRY(ensure_cis(st));
+  void* p = nullptr;
+  MNP_CUDA(cudaGetSymbolAddress(&p, g_cis));
+  *table = static_cast<const CisTable*>(p);
   return MNPBEM_OK;
 }
 
 // G and F of one pair for wavenumber k (far-field formula); inv = 1 / d
-__device__ __forceinline__ PairVal far_pair(const CisShared& T, double2 k, double dd, double inv, double in,
+__device__ __forceinline__ PairVal far_pair(const CisTable& T, double2 k, double dd, double inv, double in,
                                             double area) {
   const double2 ph = cis_exp(T, k, dd);
   const double ga = area * inv;
@@ -161,7 +108,7 @@ constexpr int ASM_DS_ROWS = 8;
 struct Val4 { double2 g1, h1, g2, h2; };
 
 // G1, H1, G2, H2 of the pair (i, j) by the far-field formula
-__device__ __forceinline__ Val4 far4(const AsmParams& p, const CisShared& T, int64_t i, const double4_32a& sj,
+__device__ __forceinline__ Val4 far4(const AsmParams& p, const CisTable& T, int64_t i, const double4_32a& sj,
                                      int pj) {
   const double4_32a si = p.src[i];
   const double4_32a ni = p.nrm[i];
@@ -184,8 +131,8 @@ __device__ __forceinline__ Val4 far4(const AsmParams& p, const CisShared& T, int
 
 template <bool W64, bool W32>
 __global__ void __launch_bounds__(ASM_COLS) k_asm_far(AsmParams p) {
-  __shared__ CisShared T;
-  cis_load(T);
+  __shared__ CisTable T;
+  cis_load(T, &g_cis);
   int64_t j = (int64_t)blockIdx.x * ASM_COLS + threadIdx.x;
   int64_t i0 = (int64_t)blockIdx.y * ASM_ROWS;
   if (j >= p.n) return;
@@ -204,8 +151,8 @@ __global__ void __launch_bounds__(ASM_COLS) k_asm_far(AsmParams p) {
 // function on leaf pairs of the cluster tree, FP64, block b row-major at
 // val[q] + foff[b] (Greenfun/@hmatrix/fillval.m with compgreenret's eval)
 __global__ void __launch_bounds__(256) k_asm_leaf(AsmParams p, LeafAsm la) {
-  __shared__ CisShared T;
-  cis_load(T);
+  __shared__ CisTable T;
+  cis_load(T, &g_cis);
   const int b = blockIdx.x;
   const int4 blk = la.fblk[b];   // (r0, m, c0, nb)
   const int64_t cnt = (int64_t)blk.y * blk.w;

@@ -1,6 +1,7 @@
 // Excitation, the bemret solution chain, the FP64 residual of the full BEM
 // operator, and the far-field cross sections.
 #include "bem.cuh"
+#include "cis.cuh"
 #include "farfield.cuh"
 #include "dense.cuh"
 #include "profile.cuh"
@@ -448,17 +449,24 @@ struct PackedSrc {
 
 __global__ void __launch_bounds__(256) k_farfield(FaceData f, int P, const double2* x1,
                                                   const double2* x2, const double* dirs,
-                                                  const LamParams* lp, double2* fields) {
+                                                  const LamParams* lp, double2* fields, const CisTable* table) {
+  __shared__ CisTable T;
+  cis_load(T, table);
   const int d = blockIdx.x;
-  farfield_dir<MAXPOL>(f.n, P, f.pos, f.area, f.exc_in, f.exc_out, PackedSrc{x1, x2, P}, dirs[3 * d],
+  const auto cis = [](double2 k, double s) { return cis_exp(T, k, s); };
+  farfield_dir<MAXPOL>(f.n, P, f.pos, f.area, f.exc_in, f.exc_out, PackedSrc{x1, x2, P}, cis, dirs[3 * d],
                        dirs[3 * d + 1], dirs[3 * d + 2], lp->kexc, lp->k0, d, fields);
 }
 
-void launch_farfield(const FaceData& f, int P, const double2* x1, const double2* x2,
-                     const double* dirs, int ndir, const LamParams* lp, double2* fields,
-                     cudaStream_t st) {
+mnpbem_status launch_farfield(const FaceData& f, int P, const double2* x1, const double2* x2,
+                              const double* dirs, int ndir, const LamParams* lp, double2* fields,
+                              cudaStream_t st) {
+  const CisTable* table = nullptr;
+  MNP_TRY(cis_table(&table, st));
   ProfScope ps_(PH_SPECTRA, st, 0.0, 0.0, 1);
-  k_farfield<<<ndir, 256, 0, st>>>(f, P, x1, x2, dirs, lp, fields);
+  k_farfield<<<ndir, 256, 0, st>>>(f, P, x1, x2, dirs, lp, fields, table);
+  MNP_CHECK_LAUNCH();
+  return MNPBEM_OK;
 }
 
 __device__ __forceinline__ void cross_sections_body(int P, const double* pol, const double* inf_nvec,

@@ -103,9 +103,9 @@ void launch_sigma_add(int64_t n, cplx<R>* S, const cplx<R>* Di, int64_t ld, cons
 // dirs [ndir][3]: first P rows are the excitation directions (extinction),
 // the remaining ninf rows the sphere at infinity with weights inf_area.
 // fields: scratch of ndir * 6 * P complex values.
-void launch_farfield(const FaceData& f, int P, const double2* x1, const double2* x2,
-                     const double* dirs, int ndir, const LamParams* lp, double2* fields,
-                     cudaStream_t st);
+mnpbem_status launch_farfield(const FaceData& f, int P, const double2* x1, const double2* x2,
+                              const double* dirs, int ndir, const LamParams* lp, double2* fields,
+                              cudaStream_t st);
 void launch_cross_sections(int P, const double* pol, const double* inf_nvec, const double* inf_area,
                            int ninf, const double2* fields, double2 k_med, double2 nb1,
                            double* ext, double* sca, cudaStream_t st);

@@ -5,18 +5,19 @@
 // every face whose inside (sig1, h1) or outside (sig2, h2) medium is the
 // excitation medium, summed over the faces for each polarisation, then
 //   e = i k0 Ph - i k (d Ps),   h = i k d x Ph      (@spectrumret/farfield.m)
-// into fields [d][6][P].  Src gives sig(side, j, p) and h(side, j, c, p).
+// into fields [d][6][P].  Src gives sig(side, j, p) and h(side, j, c, p), and
+// Cis gives exp(i k s).
 #pragma once
 #include "common.cuh"
 
 namespace mnpbem {
 
-template <int MAXP, typename Src>
+template <int MAXP, typename Src, typename Cis>
 __device__ __forceinline__ void farfield_dir(int64_t n, int P, const double* __restrict__ pos,
                                              const double* __restrict__ area,
                                              const unsigned char* __restrict__ exc_in,
                                              const unsigned char* __restrict__ exc_out, const Src& src,
-                                             double dx, double dy, double dz, double2 k, double k0, int d,
+                                             const Cis& cis, double dx, double dy, double dz, double2 k, double k0, int d,
                                              double2* fields) {
   double2 Ps[MAXP], Ph[3][MAXP];
   for (int p = 0; p < MAXP; ++p) {
@@ -27,11 +28,7 @@ __device__ __forceinline__ void farfield_dir(int64_t n, int P, const double* __r
     const bool in1 = exc_in[j] != 0, in2 = exc_out[j] != 0;
     if (!in1 && !in2) continue;
     const double s = dx * pos[3 * j] + dy * pos[3 * j + 1] + dz * pos[3 * j + 2];
-    // exp(-i k s) * area
-    double sn, cs;
-    sincos(k.x * s, &sn, &cs);
-    const double ee = exp(k.y * s) * area[j];
-    const double2 ph = make_double2(ee * cs, -ee * sn);
+    const double2 ph = cscale(cis(make_double2(-k.x, -k.y), s), area[j]);   // exp(-i k s) * area
     for (int p = 0; p < P; ++p) {
       double2 sv = make_double2(0, 0);
       double2 hv[3] = {make_double2(0, 0), make_double2(0, 0), make_double2(0, 0)};

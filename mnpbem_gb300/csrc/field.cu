@@ -7,6 +7,7 @@
 // closer than RelCutoff element radii to a face (refinematrix.m:27-67 with the
 // face's radius) take the refined Taylor coefficients of the (point, face)
 // pair (Greenfun/@greenret/private/init.m:98-177), as the face pairs do.
+#include "cis.cuh"
 #include "field.cuh"
 #include "geom_dev.cuh"
 #include "profile.cuh"
@@ -17,8 +18,13 @@ constexpr int FLD_MAXPOL = 4;
 
 __device__ __forceinline__ int pt_flag(double3 p, const GeomDev& g, int j, double rel_cut, double abs_cut) {
   const double3 v = sub3(p, ld3(g.pos, j));
-  const double d2 = sqrt(dot3(v, v)) - g.rad[j];
-  return (d2 < abs_cut || d2 / g.rad[j] < rel_cut) ? 1 : 0;
+  const double rad = g.rad[j], vv = dot3(v, v);
+  // beyond both cutoffs by more than any rounding: no square root, no division
+  // (most pairs; FP64 is the bound of these passes)
+  const double far = (rad + fmax(abs_cut, rel_cut * rad)) * (1 + 1e-9);
+  if (far > 0.0 && vv > far * far) return 0;
+  const double d2 = sqrt(vv) - rad;
+  return (d2 < abs_cut || d2 / rad < rel_cut) ? 1 : 0;
 }
 
 // one warp per point: number of refined faces
@@ -81,34 +87,42 @@ struct FieldArgs {
   double2 *e, *h;
 };
 
-// one block per point
-__global__ void __launch_bounds__(128) k_pt_field(FieldArgs a) {
-  const int64_t i = blockIdx.x;
+// One warp per point, lanes over the faces; the points of a CTA share the table
+// of exp(i k d).  Bound by FP64: about 65 operations per pair and 48 per
+// polarisation (five complex-times-real and nine complex products).  Against one
+// CTA per point with the library's sincos and exp, a binary search for the
+// refined faces and sums indexed by a run-time polarisation (local memory):
+// 3.6 ms instead of 5.2 ms for 9797 points, 1176 faces and two polarisations.
+constexpr int PTF_WARPS = 8;
+template <int P>
+__global__ void __launch_bounds__(32 * PTF_WARPS) k_pt_field(FieldArgs a, int64_t npts, const CisTable* table) {
+  __shared__ CisTable T;
+  cis_load(T, table);
+  const int lane = threadIdx.x & 31;
+  const int64_t i = (int64_t)blockIdx.x * PTF_WARPS + (threadIdx.x >> 5);
+  if (i >= npts) return;
   const GeomDev& g = a.g;
-  const int n = g.n, O = g.order, P = a.npol;
+  const int n = g.n, O = g.order;
   const int med = a.pt_med[i];
   const double2 k = a.kmed[med];
   const double2 ik = make_double2(-k.y, k.x);
   const double3 p = ld3(a.pts, i);
-  const int64_t r0 = a.offs[i], r1 = a.offs[i + 1];
-  double2 E[3][FLD_MAXPOL], H[3][FLD_MAXPOL];
-  for (int c = 0; c < 3; ++c)
-    for (int q = 0; q < FLD_MAXPOL; ++q) E[c][q] = H[c][q] = make_double2(0, 0);
-  for (int j = threadIdx.x; j < n; j += blockDim.x) {
+  int64_t lo = a.offs[i];
+  const int64_t r1 = a.offs[i + 1];
+  double2 S[6][P];                     // E, H
+#pragma unroll
+  for (int c = 0; c < 6; ++c)
+#pragma unroll
+    for (int q = 0; q < P; ++q) S[c][q] = make_double2(0, 0);
+  for (int j = lane; j < n; j += 32) {
     const bool s1 = a.face_med[j] == med, s2 = a.face_med[n + j] == med;
     if (!s1 && !s2) continue;
     const double3 v = sub3(p, ld3(g.pos, j));
-    const double d = fmax(sqrt(dot3(v, v)), DBL_EPS);
-    double sn, cs;
-    sincos(k.x * d, &sn, &cs);
-    const double ee = exp(-k.y * d);
-    const double2 ph = make_double2(ee * cs, ee * sn);
-    // refined pair?  (faces of row i are sorted ascending)
-    int64_t lo = r0, hi = r1;
-    while (lo < hi) {
-      const int64_t mid = (lo + hi) >> 1;
-      if (a.pcol[mid] < j) lo = mid + 1; else hi = mid;
-    }
+    const double vv = dot3(v, v);
+    const double d = fmax(sqrt(vv), DBL_EPS), inv = 1.0 / d;
+    const double2 ph = cis_exp(T, k, d);
+    // refined pair?  (the faces of row i ascend, and so do this lane's)
+    while (lo < r1 && a.pcol[lo] < j) ++lo;
     double2 G, Gp[3];
     if (lo < r1 && a.pcol[lo] == j) {
       const double* cg = a.cg + lo * (O + 1);
@@ -116,56 +130,62 @@ __global__ void __launch_bounds__(128) k_pt_field(FieldArgs a) {
       double2 pw = make_double2(1, 0), gs = make_double2(0, 0), fs[3] = {gs, gs, gs};
       for (int o = 0; o <= O; ++o) {
         gs.x += cg[o] * pw.x; gs.y += cg[o] * pw.y;
+#pragma unroll
         for (int c = 0; c < 3; ++c) { fs[c].x += cf[c * (O + 1) + o] * pw.x; fs[c].y += cf[c * (O + 1) + o] * pw.y; }
         pw = cmul(pw, ik);
       }
       G = cmul(gs, ph);
+#pragma unroll
       for (int c = 0; c < 3; ++c) Gp[c] = cmul(fs[c], ph);
     } else {
-      const double A = g.area[j], inv = 1.0 / d;
-      G = make_double2(A * inv * ph.x, A * inv * ph.y);
+      const double ai = g.area[j] * inv;
+      G = make_double2(ai * ph.x, ai * ph.y);
       // (ik - 1/d) / d^2 * A * (p - pos_j)
-      const double2 t = cmul(make_double2(-k.y - inv, k.x), ph);
-      const double s = A * inv * inv;
-      const double vc[3] = {v.x, v.y, v.z};
-      for (int c = 0; c < 3; ++c) Gp[c] = make_double2(t.x * s * vc[c], t.y * s * vc[c]);
+      const double2 t = cscale(cmul(make_double2(-k.y - inv, k.x), ph), ai * inv);
+      Gp[0] = cscale(t, v.x);
+      Gp[1] = cscale(t, v.y);
+      Gp[2] = cscale(t, v.z);
     }
     const double2 ik0G = make_double2(-a.k0 * G.y, a.k0 * G.x);
+    const double2 mGp[3] = {make_double2(-Gp[0].x, -Gp[0].y), make_double2(-Gp[1].x, -Gp[1].y),
+                            make_double2(-Gp[2].x, -Gp[2].y)};
+#pragma unroll
     for (int side = 0; side < 2; ++side) {
       if (!(side == 0 ? s1 : s2)) continue;
       const double2* sg = side == 0 ? a.sig1 : a.sig2;
       const double2* hh = side == 0 ? a.h1 : a.h2;
+#pragma unroll
       for (int q = 0; q < P; ++q) {
-        const double2 sv = sg[(int64_t)j * P + q];
+        const double2 sv = __ldg(sg + (int64_t)j * P + q);
         double2 hv[3];
-        for (int c = 0; c < 3; ++c) hv[c] = hh[((int64_t)j * 3 + c) * P + q];
-        for (int c = 0; c < 3; ++c) E[c][q] = csub(cadd(E[c][q], cmul(ik0G, hv[c])), cmul(Gp[c], sv));
-        H[0][q] = cadd(H[0][q], csub(cmul(Gp[1], hv[2]), cmul(Gp[2], hv[1])));
-        H[1][q] = cadd(H[1][q], csub(cmul(Gp[2], hv[0]), cmul(Gp[0], hv[2])));
-        H[2][q] = cadd(H[2][q], csub(cmul(Gp[0], hv[1]), cmul(Gp[1], hv[0])));
+#pragma unroll
+        for (int c = 0; c < 3; ++c) hv[c] = __ldg(hh + ((int64_t)j * 3 + c) * P + q);
+#pragma unroll
+        for (int c = 0; c < 3; ++c) {
+          cfma(S[c][q], ik0G, hv[c]);
+          cfma(S[c][q], mGp[c], sv);
+        }
+        cfma(S[3][q], Gp[1], hv[2]);
+        cfma(S[3][q], mGp[2], hv[1]);
+        cfma(S[4][q], Gp[2], hv[0]);
+        cfma(S[4][q], mGp[0], hv[2]);
+        cfma(S[5][q], Gp[0], hv[1]);
+        cfma(S[5][q], mGp[1], hv[0]);
       }
     }
   }
-  // block reduction (fixed order): warp shuffles, then the four warps in order
-  __shared__ double2 red[4][6 * FLD_MAXPOL];
-  const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+#pragma unroll
   for (int c = 0; c < 6; ++c)
+#pragma unroll
     for (int q = 0; q < P; ++q) {
-      double2 v = c < 3 ? E[c][q] : H[c - 3][q];
+      double2 v = S[c][q];
+#pragma unroll
       for (int o = 16; o; o >>= 1) {
         v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
         v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
       }
-      if (lane == 0) red[wid][c * FLD_MAXPOL + q] = v;
+      if (lane == 0) (c < 3 ? a.e : a.h)[(i * 3 + (c % 3)) * P + q] = v;
     }
-  __syncthreads();
-  for (int t = threadIdx.x; t < 6 * P; t += blockDim.x) {
-    const int c = t / P, q = t % P;
-    double2 s = make_double2(0, 0);
-    for (int w = 0; w < 4; ++w) s = cadd(s, red[w][c * FLD_MAXPOL + q]);
-    double2* out = c < 3 ? a.e : a.h;
-    out[(i * 3 + (c % 3)) * P + q] = s;
-  }
 }
 
 mnpbem_status point_fields(const GeomDev& g, const int* face_med, int64_t npts, const double* pts,
@@ -218,7 +238,10 @@ mnpbem_status point_fields(const GeomDev& g, const int* face_med, int64_t npts, 
   a.kmed = d_k.as<double2>(); a.k0 = k0; a.npol = npol;
   a.sig1 = sig1; a.sig2 = sig2; a.h1 = h1; a.h2 = h2;
   a.offs = offs.as<int64_t>(); a.pcol = pcol; a.cg = cg; a.cf = cf; a.e = e; a.h = h;
-  k_pt_field<<<(unsigned)npts, 128, 0, st>>>(a);
+  const CisTable* table = nullptr;
+  MNP_TRY(cis_table(&table, st));
+  const auto kern = npol == 1 ? k_pt_field<1> : npol == 2 ? k_pt_field<2> : npol == 3 ? k_pt_field<3> : k_pt_field<4>;
+  kern<<<(unsigned)cdiv_up(npts, (int64_t)PTF_WARPS), 32 * PTF_WARPS, 0, st>>>(a, npts, table);
   MNP_CHECK_LAUNCH();
   MNP_CUDA(cudaStreamSynchronize(st));   // the temporary buffers are released on return
   return MNPBEM_OK;
@@ -413,7 +436,9 @@ struct FarArgs {
 };
 
 // one block (4 warps) per direction
-__global__ void __launch_bounds__(128) k_far_dirs(FarArgs a) {
+__global__ void __launch_bounds__(128) k_far_dirs(FarArgs a, const CisTable* table) {
+  __shared__ CisTable T;
+  cis_load(T, table);
   const int d = blockIdx.x;
   const GeomDev& g = a.g;
   const int n = g.n, P = a.npol;
@@ -425,10 +450,7 @@ __global__ void __launch_bounds__(128) k_far_dirs(FarArgs a) {
     const bool s1 = a.face_med[j] == a.med, s2 = a.face_med[n + j] == a.med;
     if (!s1 && !s2) continue;
     const double s = dot3(dv, ld3(g.pos, j));
-    double sn, cs;
-    sincos(a.k.x * s, &sn, &cs);
-    const double ee = exp(a.k.y * s) * g.area[j];
-    const double2 ph = make_double2(ee * cs, -ee * sn);
+    const double2 ph = cscale(cis_exp(T, make_double2(-a.k.x, -a.k.y), s), g.area[j]);   // exp(-i k s) A
     for (int sd = 0; sd < 2; ++sd) {
       if (!(sd == 0 ? s1 : s2)) continue;
       const double2* sg = sd == 0 ? a.sig1 : a.sig2;
@@ -488,7 +510,9 @@ mnpbem_status far_fields(const GeomDev& g, const int* face_med, int med, double2
   FarArgs a;
   a.g = g; a.face_med = face_med; a.med = med; a.k = k; a.k0 = k0; a.npol = npol; a.dirs = dirs;
   a.sig1 = sig1; a.sig2 = sig2; a.h1 = h1; a.h2 = h2; a.e = e; a.h = h;
-  k_far_dirs<<<(unsigned)ndir, 128, 0, st>>>(a);
+  const CisTable* table = nullptr;
+  MNP_TRY(cis_table(&table, st));
+  k_far_dirs<<<(unsigned)ndir, 128, 0, st>>>(a, table);
   MNP_CHECK_LAUNCH();
   return MNPBEM_OK;
 }

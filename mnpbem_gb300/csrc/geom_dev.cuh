@@ -73,12 +73,10 @@ __device__ __forceinline__ void near_coefficients(const GeomDev& g, double3 pi, 
   double3 v0 = sub3(pj, pi);
   double r0 = sqrt(dot3(v0, v0));
   double ag[MAX_ORDER + 1], ax[MAX_ORDER + 1], ay[MAX_ORDER + 1], az[MAX_ORDER + 1];
-  for (int o = 0; o <= O; ++o) ag[o] = ax[o] = ay[o] = az[o] = 0.0;
+#pragma unroll
+  for (int o = 0; o <= MAX_ORDER; ++o) ag[o] = ax[o] = ay[o] = az[o] = 0.0;
   const int* f = g.faces + 4 * j;
   int ntri = f[3] < 0 ? 1 : 2;
-  double invfact[MAX_ORDER + 2];
-  invfact[0] = 1.0;
-  for (int o = 1; o <= O; ++o) invfact[o] = invfact[o - 1] / o;
   for (int tr = 0; tr < ntri; ++tr) {
     int a = tr == 0 ? f[0] : f[2], b = tr == 0 ? f[1] : f[3], c = tr == 0 ? f[2] : f[0];
     double3 va = ld3(g.verts, a), vb = ld3(g.verts, b), vc = ld3(g.verts, c);
@@ -100,18 +98,22 @@ __device__ __forceinline__ void near_coefficients(const GeomDev& g, double3 pi, 
       double3 v = sub3(pi, pt);
       double r = sqrt(v.x * v.x + v.y * v.y + v.z * v.z);
       double dr = r - r0;
-      double ir = 1.0 / r, ir2 = ir * ir, ir3 = ir2 * ir;
-      double drp = 1.0;   // dr^o
-      double drm = 0.0;   // dr^(o-1)
-      for (int o = 0; o <= O; ++o) {
-        ag[o] += (drp * ir * invfact[o]) * w;
-        double ff = (o == 0) ? -ir3 : (-drp * ir3 * invfact[o] + drm * ir2 * invfact[o - 1]);
-        ax[o] += v.x * ff * w; ay[o] += v.y * ff * w; az[o] += v.z * ff * w;
-        drm = drp; drp *= dr;
+      double ir = 1.0 / r, wi = w * ir, w2 = wi * ir, w3 = w2 * ir;
+      double drp = 1.0;   // dr^o / o!
+      double drm = 0.0;   // dr^(o-1) / (o-1)!
+#pragma unroll
+      for (int o = 0; o <= MAX_ORDER; ++o) {
+        if (o > O) break;
+        ag[o] += wi * drp;
+        const double ff = w2 * drm - w3 * drp;
+        ax[o] += v.x * ff; ay[o] += v.y * ff; az[o] += v.z * ff;
+        drm = drp; drp *= dr * (1.0 / (o + 1));
       }
     }
   }
-  for (int o = 0; o <= O; ++o) {
+#pragma unroll
+  for (int o = 0; o <= MAX_ORDER; ++o) {
+    if (o > O) break;
     go[o] = ag[o];
     fo[0 * (O + 1) + o] = ax[o];
     fo[1 * (O + 1) + o] = ay[o];

@@ -42,6 +42,16 @@ static __device__ __align__(256) double2 g_noalloc_fields[NOALLOC_MAX_DIRS * 6 *
 // (sig [n][P], h [n][3][P] per side); direction d < P is dir[d], else
 // inf_nvec[d - P].  The far-field routine of the solve (farfield.cuh) with
 // this layout.
+// exp(i k s) from the device's library: no table that a device reset would lose
+struct LibCis {
+  __device__ double2 operator()(double2 k, double s) const {
+    double sn, cs;
+    sincos(k.x * s, &sn, &cs);
+    const double e = exp(-k.y * s);
+    return make_double2(e * cs, e * sn);
+  }
+};
+
 struct SplitSrc {
   const double2 *s1, *h1, *s2, *h2;
   int P;
@@ -57,8 +67,8 @@ __global__ void __launch_bounds__(256) k_farfield_noalloc(
     double2 k, double k0, double2* fields) {
   const int d = blockIdx.x;
   const double* dv = d < P ? dir + 3 * d : inf_nvec + 3 * (d - P);
-  farfield_dir<NOALLOC_MAX_POL>(n, P, pos, area, exc_in, exc_out, SplitSrc{sig1, h1, sig2, h2, P}, dv[0], dv[1],
-                                dv[2], k, k0, d, fields);
+  farfield_dir<NOALLOC_MAX_POL>(n, P, pos, area, exc_in, exc_out, SplitSrc{sig1, h1, sig2, h2, P},
+                                LibCis{}, dv[0], dv[1], dv[2], k, k0, d, fields);
 }
 
 // device address of the scratch array in the current context, looked up on
