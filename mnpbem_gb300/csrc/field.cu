@@ -69,7 +69,7 @@ __global__ void k_pt_coef(int64_t npair, const double* __restrict__ pts, GeomDev
   const int64_t t = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
   if (t >= npair) return;
   const int O = g.order;
-  near_coefficients(g, ld3(pts, prow[t]), pcol[t], cg + t * (O + 1), cf + t * 3 * (O + 1));
+  near_coefficients<true>(g, ld3(pts, prow[t]), pcol[t], cg + t * (O + 1), cf + t * 3 * (O + 1));
 }
 
 struct FieldArgs {

