@@ -14,7 +14,7 @@ HERE = os.path.dirname(os.path.abspath(__file__))
 CSRC = os.path.join(HERE, "csrc")
 BUILD = os.path.join(HERE, "_build")
 LIB = os.path.join(HERE, "libmnpbem_gpu.so")
-SOURCES = ["geometry.cu", "assemble.cu", "dense.cu", "bem.cu", "tc_gemm.cu", "noalloc.cu", "adjoint.cu", "field.cu", "hmat.cu",
+SOURCES = ["geometry.cu", "assemble.cu", "dense.cu", "bem.cu", "tc_gemm.cu", "tc_gemm64.cu", "noalloc.cu", "adjoint.cu", "field.cu", "hmat.cu",
            "hlu.cu", "api.cu"]
 ARCH = ["-gencode", "arch=compute_103a,code=sm_103a"]
 FLAGS = ["-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden",

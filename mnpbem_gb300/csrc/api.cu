@@ -73,7 +73,10 @@ struct ProfBind {
 // GEMM adapters
 static mnpbem_status gemm64(int64_t M, int64_t N, int64_t K, double2 al, const double2* A,
                             int64_t lda, const double2* B, int64_t ldb, double2 be, double2* C,
-                            int64_t ldc, cudaStream_t st, void*) {
+                            int64_t ldc, cudaStream_t st, void* ctx) {
+  TcGemmCtx* tc = reinterpret_cast<TcGemmCtx*>(ctx);
+  if (tc && tc_gemm64_eligible(*tc, M, N, K, al, be))
+    return tc_gemm_c128(*tc, M, N, K, al.x, A, lda, B, ldb, be.x != 0.0, C, ldc, st);
   return gemm_simt<double>(M, N, K, al, A, lda, B, ldb, be, C, ldc, st);
 }
 static mnpbem_status gemm32(int64_t M, int64_t N, int64_t K, float2 al, const float2* A, int64_t lda,
@@ -809,6 +812,39 @@ mnpbem_status mnpbem_gemm_c64(int32_t device, int32_t path, int64_t M, int64_t N
   return MNPBEM_OK;
 }
 
+mnpbem_status mnpbem_gemm_c128(int32_t device, int32_t path, int64_t M, int64_t N, int64_t K, double alpha,
+                               const double* A, int64_t lda, const double* B, int64_t ldb, double beta, double* C,
+                               int64_t ldc) {
+  if (M <= 0 || N <= 0 || K <= 0 || !A || !B || !C || lda < K || ldb < N || ldc < N || path < 0 || path > 1) {
+    set_error("mnpbem_gemm_c128: invalid arguments");
+    return MNPBEM_ERR_INVALID_ARG;
+  }
+  MNP_CUDA(cudaSetDevice(device));
+  TcGemmCtx tc;
+  DevBuf dA, dB, dC;
+  MNP_TRY(dA.ensure(sizeof(double2) * M * lda));
+  MNP_TRY(dB.ensure(sizeof(double2) * K * ldb));
+  MNP_TRY(dC.ensure(sizeof(double2) * M * ldc));
+  MNP_CUDA(cudaMemcpy(dA.ptr, A, sizeof(double2) * M * lda, cudaMemcpyHostToDevice));
+  MNP_CUDA(cudaMemcpy(dB.ptr, B, sizeof(double2) * K * ldb, cudaMemcpyHostToDevice));
+  MNP_CUDA(cudaMemcpy(dC.ptr, C, sizeof(double2) * M * ldc, cudaMemcpyHostToDevice));
+  const double2 al = make_double2(alpha, 0.0), be = make_double2(beta, 0.0);
+  mnpbem_status s = MNPBEM_OK;
+  if (path == 1) {
+    if (!tc_gemm64_eligible(tc, M, N, K, al, be)) {
+      set_error("complex128 tensor-core GEMM not available for this device or shape");
+      return MNPBEM_ERR_UNSUPPORTED;
+    }
+    s = tc_gemm_c128(tc, M, N, K, alpha, dA.as<double2>(), lda, dB.as<double2>(), ldb, beta != 0.0, dC.as<double2>(),
+                     ldc, nullptr);
+    if (s == MNPBEM_OK) s = tc_check_error(tc, nullptr);
+  } else {
+    s = gemm_simt<double>(M, N, K, al, dA.as<double2>(), lda, dB.as<double2>(), ldb, be, dC.as<double2>(), ldc, nullptr);
+  }
+  if (s == MNPBEM_OK) MNP_CUDA(cudaMemcpy(C, dC.ptr, sizeof(double2) * M * ldc, cudaMemcpyDeviceToHost));
+  return s;
+}
+
 mnpbem_status mnpbem_block_inverse(int32_t device, int32_t precision, int32_t w, void* A, int32_t lda,
                                    double* cond) {
   const bool fp64 = precision == MNPBEM_FP64;
@@ -879,6 +915,7 @@ size_t lane_bytes_estimate(const mnpbem_geom* G, int precision, int P, int ninf)
   size_t b = 5 * es * n * ld;
   // hi / lo planes, B' of the rank-1024 products and the LDU panels
   if (precision == MNPBEM_MIXED) b += 4 * 2 * sizeof(float2) * n * ld + 3 * 8 * 1024 * n;
+  else b += 3 * 2048 * n;   // digit slices of the complex128 products
   b += sizeof(double2) * n * P * 80 + sizeof(float2) * n * P * 56;
   b += 3 * es * n * 256 + sizeof(double2) * (size_t)(P + ninf) * 6 * P + 64 * n;
   return b;
@@ -915,7 +952,8 @@ uint64_t lane_sig(const mnpbem_geom* G, const Lane& L) {
   for (int q = 0; q < 4; ++q) mixbuf(L.mat64[q]);
   mixbuf(L.vec64); mixbuf(L.vecw); mixbuf(L.facebuf); mixbuf(L.fields); mixbuf(L.norms);
   mixbuf(L.outbuf); mixbuf(L.bsplit); mixbuf(L.lp_dev); mixbuf(G->exbuf);
-  mixbuf(L.tc.bexp); mixbuf(L.tc.err);
+  mixbuf(L.tc.bexp); mixbuf(L.tc.err); mixbuf(L.tc.a16); mixbuf(L.tc.scales); mixbuf(L.tc.ctr);
+  mixbuf(L.tc.a8); mixbuf(L.tc.b8); mixbuf(L.tc.exps);
   auto gj = [&](const auto& w) {
     mixbuf(w.ccol); mixbuf(w.rrow); mixbuf(w.ncol); mixbuf(w.xblk); mixbuf(w.status); mixbuf(w.pan);
     mix(nullptr, (size_t)w.nb);
@@ -1081,14 +1119,14 @@ mnpbem_status stage_initmat(mnpbem_geom* G, Lane& L, bool direct) {
   const int64_t n = G->g.n, ld = G->ld;
   Cx* M[5];
   for (int q = 0; q < 5; ++q) M[q] = L.mat[q].as<Cx>();
-  void* ctx = sizeof(R) == 4 ? tc_ctx(G, L) : nullptr;
+  void* ctx = tc_ctx(G, L);
   // wider Gauss-Jordan steps when the rank-nb updates run on tensor cores:
   // fewer passes over the n x n matrix (each step reads and writes it once)
   // By size (measured on GB300, 24 000-face dimer: rank-1024 LDU updates and
   // 512-wide Gauss-Jordan steps 1.365 against 1.265 wavelength-solves/s for
   // rank-512 / 256-wide; at 4000 faces the 256-wide steps were faster)
   const bool large = n >= 12000;
-  gjw<R>(L).nb = (ctx && n > 64) ? (G->gj_nb ? G->gj_nb : (large ? 512 : 256)) : 64;
+  gjw<R>(L).nb = (sizeof(R) == 4 && ctx && n > 64) ? (G->gj_nb ? G->gj_nb : (large ? 512 : 256)) : 64;
   gjw<R>(L).round_a = G->tf32_rna;
   gjw<R>(L).fused = G->gj_fused;
   LDUWork<R>& lw = luw<R>(L);

@@ -1649,14 +1649,16 @@ mnpbem_status ldu_factor(cplx<R>* A, int64_t n, int64_t lda, LDUWork<R>& w, int*
         MNP_CHECK_LAUNCH();
         // L panel: A[kb:, ks:kb] = C X
         MNP_TRY(gemm(below, bs, bs, one, Cs, B, X, bs, zero, A + kb * lda + ks, lda, st, ctx));
-        // U row: A[ks:kb, kb:] = X A[ks:kb, kb:] (the tensor-core product copies its
-        // B operand before it runs, so it may write in place; the CUDA-core
+        // U row: A[ks:kb, kb:] = X A[ks:kb, kb:] (the tensor-core products copy their
+        // B operand before they run, so they may write in place; the CUDA-core
         // products may not)
         bool inplace = false;
-        if constexpr (sizeof(R) == 4) {
-          if (tc)
-            inplace = tc_gemm_eligible(*reinterpret_cast<TcGemmCtx*>(ctx), bs, below, bs, X, bs, A + ks * lda + kb,
-                                       lda, make_float2(0.f, 0.f));
+        if (ctx) {
+          TcGemmCtx& tcc = *reinterpret_cast<TcGemmCtx*>(ctx);
+          if constexpr (sizeof(R) == 4)
+            inplace = tc_gemm_eligible(tcc, bs, below, bs, X, bs, A + ks * lda + kb, lda, make_float2(0.f, 0.f));
+          else
+            inplace = tc_gemm64_eligible(tcc, bs, below, bs, one, zero);
         }
         if (inplace) {
           MNP_TRY(gemm(bs, below, bs, one, X, bs, A + ks * lda + kb, lda, zero, A + ks * lda + kb, lda, st, ctx));

@@ -25,6 +25,7 @@
 #include "mbarrier.cuh"
 #include "profile.cuh"
 #include "tc_gemm.cuh"
+#include "tc_prims.cuh"
 
 #include <algorithm>
 
@@ -44,12 +45,6 @@ constexpr uint32_t TC_IDESC_F16 = (1u << 4) | (0u << 7) | (0u << 10) | ((uint32_
 constexpr uint32_t TC_IDESC = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(TC_BN >> 3) << 17) |
                               ((uint32_t)(TC_BM >> 4) << 24);
 
-__device__ __forceinline__ void tma_load_2d(uint32_t dst, const CUtensorMap* map, uint32_t bar, int x, int y) {
-  asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1, {%3, %4}], [%2];"
-      ::"r"(dst), "l"((unsigned long long)map), "r"(bar), "r"(x), "r"(y)
-      : "memory");
-}
 // L2 prefetch of one C tile (128 rows x 256 floats, unswizzled map) so that the
 // epilogue's reduce-add finds C in L2 instead of waiting for HBM
 __device__ __forceinline__ void tma_prefetch_2d(const CUtensorMap* map, int x, int y) {
@@ -74,37 +69,6 @@ __device__ __forceinline__ void mma_tf32(uint32_t dtmem, uint64_t a, uint64_t b,
       ::"r"(dtmem), "l"(a), "l"(b), "r"(idesc), "r"(acc)
       : "memory");
 }
-__device__ __forceinline__ void mma_f16(uint32_t dtmem, uint64_t a, uint64_t b, uint32_t idesc, uint32_t acc) {
-  asm volatile(
-      "{\n .reg .pred p;\n setp.ne.b32 p, %4, 0;\n"
-      " tcgen05.mma.cta_group::1.kind::f16 [%0], %1, %2, %3, p;\n}\n"
-      ::"r"(dtmem), "l"(a), "l"(b), "r"(idesc), "r"(acc)
-      : "memory");
-}
-__device__ __forceinline__ void mma_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar)
-               : "memory");
-}
-// Tile order of the persistent kernels: groups of TC_GROUP_M row tiles, and
-// within a group the column tiles one after another (the group's row tiles
-// fastest).  The CTAs in flight then share a few A row panels (TC_GROUP_M x
-// 128 rows) and a few B' tiles, which stay in L2; with the plain row-fastest
-// order every column of tiles sweeps the whole A panel, which at n = 24 000
-// and K = 512 (98 MB) does not stay in L2 next to the streamed C tiles and is
-// read again from HBM for every column.
-constexpr int TC_GROUP_M = 32;
-__device__ __forceinline__ void tile_coords(int t, int MT, int NT, int& mt, int& nt) {
-  const int per_group = TC_GROUP_M * NT;
-  const int g = t / per_group;
-  const int m_first = g * TC_GROUP_M;
-  const int gm = min(TC_GROUP_M, MT - m_first);
-  const int r = t - g * per_group;
-  mt = m_first + r % gm;
-  nt = r / gm;
-}
-__device__ __forceinline__ void tc_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tc_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-
 __device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&r)[32]) {
   asm volatile(
       "tcgen05.ld.sync.aligned.32x32b.x32.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
@@ -890,6 +854,24 @@ static bool make_map(PFN_cuTensorMapEncodeTiled_v12000 enc, CUtensorMap* map, co
   return r == CUDA_SUCCESS;
 }
 
+bool tc_device_ready(TcGemmCtx& c) {
+  const float2 b0 = make_float2(0.f, 0.f);
+  tc_gemm_eligible(c, 128, 64, 16, nullptr, 2, nullptr, 2, b0);   // probes the device once
+  return c.usable && c.enabled;
+}
+
+bool tc_f16_map(TcGemmCtx& c, void* map, const void* ptr, uint64_t inner, uint64_t rows, uint32_t box_inner,
+                uint32_t box_rows) {
+  auto enc = get_encode(c);
+  if (!enc) return false;
+  cuuint64_t dims[2] = {inner, rows}, strides[1] = {inner * 2};
+  cuuint32_t box[2] = {box_inner, box_rows}, es[2] = {1, 1};
+  return enc(reinterpret_cast<CUtensorMap*>(map), CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, const_cast<void*>(ptr), dims,
+             strides, box, es, CU_TENSOR_MAP_INTERLEAVE_NONE,
+             box_inner == 32 ? CU_TENSOR_MAP_SWIZZLE_64B : CU_TENSOR_MAP_SWIZZLE_128B,
+             CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE) == CUDA_SUCCESS;
+}
+
 bool tc_gemm_eligible(TcGemmCtx& c, int64_t M, int64_t N, int64_t K, const void* A, int64_t lda,
                       const void* C, int64_t ldc, float2 beta) {
   if (!c.checked) {
@@ -1106,6 +1088,9 @@ void tc_release(TcGemmCtx& c) {
   c.bexp.release();
   c.a16.release();
   c.scales.release();
+  c.a8.release();
+  c.b8.release();
+  c.exps.release();
   c.err.release();
   c.ctr.release();
 }

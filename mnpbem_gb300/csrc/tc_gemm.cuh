@@ -14,6 +14,7 @@ struct TcGemmCtx {
   bool f16 = false;       // FP16 operands with power-of-two row / column scaling (kind::f16)
   int f16_min_k = 512;    // ... for products with K >= f16_min_k
   int f16_min_mn = 512;   //     and M, N >= f16_min_mn
+  DevBuf a8, b8, exps;    // complex128 products: digit slices of A and B', row / column exponents
   DevBuf err;             // device error word of the bounded waits
   DevBuf ctr;             // tile counter of the persistent kernel (zeroed before each launch)
   int num_sms = 0;
@@ -36,6 +37,19 @@ bool tc_gemm_eligible(TcGemmCtx& c, int64_t M, int64_t N, int64_t K, const void*
 mnpbem_status tc_gemm_c64(TcGemmCtx& c, int64_t M, int64_t N, int64_t K, float2 alpha,
                           const float2* A, int64_t lda, const float2* B, int64_t ldb, float2 beta,
                           float2* C, int64_t ldc, cudaStream_t st, int64_t bz0 = 0, int64_t bz1 = 0);
+// C = alpha A B + beta C in complex128 on the tensor cores (tc_gemm64.cu):
+// operands cut into eight 8-bit digits per row of A and column of B, exact
+// products, FP64-class results.  alpha = +-1, beta 0 or 1, K <= TC64_K; A and B are
+// copied before C is written, so C may overlap them.
+constexpr int TC64_K = 64;
+bool tc_gemm64_eligible(TcGemmCtx& c, int64_t M, int64_t N, int64_t K, double2 alpha, double2 beta);
+mnpbem_status tc_gemm_c128(TcGemmCtx& c, int64_t M, int64_t N, int64_t K, double alpha, const double2* A, int64_t lda,
+                           const double2* B, int64_t ldb, bool accumulate, double2* C, int64_t ldc, cudaStream_t st);
+// device probed and the tensor-core path usable
+bool tc_device_ready(TcGemmCtx& c);
+// CUtensorMap of a row-major fp16 matrix [rows][inner] (box_inner 32: 64-byte swizzle, 64: 128-byte)
+bool tc_f16_map(TcGemmCtx& c, void* map, const void* ptr, uint64_t inner, uint64_t rows, uint32_t box_inner,
+                uint32_t box_rows);
 // reads (and clears) the device error word; MNPBEM_ERR_TIMEOUT if a wait expired
 mnpbem_status tc_check_error(TcGemmCtx& c, cudaStream_t st);
 void tc_release(TcGemmCtx& c);
