@@ -27,7 +27,8 @@
 // Tile: 128 rows x 64 real columns, eight accumulators of 64 columns (all 512
 // tensor-memory columns), K chunks of 32 halves (64-byte swizzle rows) of all
 // sixteen slices (96 KB), two of them in flight.  Roles as in tc_gemm.cu: TMA
-// producer, MMA issuer, four epilogue warps; persistent with a tile counter.
+// producer, MMA issuer, eight epilogue warps (two per scheduler, so that one
+// converts while the other waits for FP64); persistent with a tile counter.
 #include <cuda.h>
 #include <cuda_fp16.h>
 #include <cudaTypedefs.h>
@@ -46,8 +47,8 @@ constexpr int Z_BM = 128, Z_BN = 64, Z_BK = 32, Z_KT = Z_KR / Z_BK;
 constexpr int Z_A_BYTES = Z_BM * Z_BK * 2, Z_B_BYTES = Z_BN * Z_BK * 2;
 constexpr int Z_STAGE = Z_S * (Z_A_BYTES + Z_B_BYTES);  // 96 KB
 constexpr int Z_ST = 2;
-constexpr int Z_EPI = 4;                                // epilogue warps
-constexpr int Z_CH = 16;                                // columns per epilogue step
+constexpr int Z_EPI = 8;                                // epilogue warps: two per 32 rows, half of the columns each
+constexpr int Z_CH = 8;                                 // columns per epilogue step
 constexpr int Z_THREADS = 32 * (2 + Z_EPI);
 constexpr int Z_SMEM = Z_ST * Z_STAGE + Z_EPI * 32 * Z_CH * 8 + 1024;
 constexpr uint32_t Z_IDESC = (1u << 4) | ((uint32_t)(Z_BN >> 3) << 17) | ((uint32_t)(Z_BM >> 4) << 24);
@@ -166,54 +167,27 @@ __global__ void __launch_bounds__(256) k_slice_b(const double2* __restrict__ B, 
 }
 
 // ----------------------------------------------------------------- epilogue
-// (hi 2^32 + lo) 2^ex as a double, rounded once to nearest even; |hi| < 2^62
-__device__ __forceinline__ double fixed_to_double(long long hi, unsigned lo, int ex) {
-  const bool neg = hi < 0;
-  unsigned long long h = (unsigned long long)hi;
-  if (neg) {                                            // negate the 96-bit value
-    lo = 0u - lo;
-    h = ~h + (lo == 0u ? 1ull : 0ull);
-  }
-  unsigned long long u;                                 // value u 2^sh, sticky bit in u's bit 0
-  int sh = 0;
-  if (h >> 31) {
-    // more than 63 bits: drop 32 bits into the sticky bit
-    u = h | (lo != 0u ? 1ull : 0ull);
-    sh = 32;
-    const int lz = __clzll((long long)h);               // keep 62 bits: bring bits of lo back in
-    const int up = min(lz - 2, 32);
-    if (up > 0) {
-      u = (h << up) | (lo >> (32 - up)) | ((lo << up) != 0u && up < 32 ? 1ull : 0ull);
-      sh = 32 - up;
-    }
-  } else {
-    u = (h << 32) | lo;
-    if (u == 0) return 0.0;
-  }
-  const int top = 63 - __clzll((long long)u);           // u in [2^top, 2^(top + 1))
-  unsigned long long m;                                 // 53 bits
-  int e = top - 52;
-  if (e > 0) {
-    const unsigned long long rem = u & ((1ull << e) - 1), half = 1ull << (e - 1);
-    m = u >> e;
-    if (rem > half || (rem == half && (m & 1))) ++m;
-  } else {
-    m = u << -e;
-  }
-  e += sh + ex + 1075;                                  // biased exponent of a 53-bit m
-  double v;
-  if (e > 0 && e < 2046) v = __longlong_as_double((long long)(((unsigned long long)e << 52) + (m - (1ull << 52))));
-  else v = scalbn((double)m, max(min(e - 1075, 4000), -4000));
-  return neg ? -v : v;
+// hi + lo 2^-32 as a double, rounded once to nearest even; |hi| < 2^50.  Two FP64
+// operations: hi enters through the bits of 1.5 2^52 + hi, lo through those of
+// 2^52 + lo, and the constants cancel in exact steps.
+__device__ __forceinline__ double fixed_to_double(long long hi, unsigned lo) {
+  const double xh = __longlong_as_double(hi + 0x4338000000000000ll) - (6755399441055744.0 + 1048576.0);   // hi - 2^20
+  const double xl = __longlong_as_double(0x4330000000000000ll | (long long)lo);                           // 2^52 + lo
+  return fma(xl, 0x1p-32, xh);
+}
+// v 2^ex for v = 0 or 2^-32 <= |v| < 2^51 and |ex| <= Z_EXMAX: the exponent field stays
+// in range, no branch and no FP64 operation (a branch per value serialised the FP64
+// latencies: 8400 cycles per 16 columns instead of 4800)
+constexpr int Z_EXMAX = 960;
+__device__ __forceinline__ double shift_exp(double v, int ex) {
+  const long long b = __double_as_longlong(v);
+  return __longlong_as_double((b << 1) == 0 ? b : b + ((long long)ex << 52));
 }
 
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, uint32_t (&r)[16]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, "
-      "%14, %15}, [%16];"
-      : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]),
-        "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
-      : "r"(taddr));
+__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr));
 }
 // shared-memory matrix descriptor: K-major, 64-byte swizzle, 8-row groups 512 B apart
 __device__ __forceinline__ uint64_t desc_sw64(uint32_t addr) {
@@ -338,8 +312,9 @@ __global__ void __launch_bounds__(Z_THREADS, 1)
       }
     }
   } else {
-    // ---------------- epilogue warps: TMEM lane quarter (warp % 4) = 32 rows of the tile
-    const int quarter = warp & 3;
+    // ---------------- epilogue warps: TMEM lane quarter (warp % 4) = 32 rows of the
+    // tile, columns 32 half .. 32 half + 31
+    const int quarter = warp & 3, half = (warp - 2) >> 2;
     double* stage = reinterpret_cast<double*>(smem_raw + (base - smem_u32(smem_raw)) + Z_ST * Z_STAGE) +
                     (warp - 2) * 32 * Z_CH;
     for (int j = 0;; ++j) {
@@ -357,33 +332,40 @@ __global__ void __launch_bounds__(Z_THREADS, 1)
       tile_coords(t, MT, NT, mt, nt);
       const int row0 = mt * Z_BM + quarter * 32, c0 = nt * (Z_BN / 2);     // c0: complex column
       const int er = row0 + lane < M ? __ldg(ea + row0 + lane) : 0;
-      for (int ch = 0; ch < Z_BN / Z_CH; ++ch) {
+      constexpr int NCH = Z_BN / 2 / Z_CH;
+      for (int ch = half * NCH; ch < (half + 1) * NCH; ++ch) {
         const int cc0 = c0 + ch * (Z_CH / 2);
-        // this lane's part of C for the coalesced pass below: eight lanes per row
+        // this lane's part of C for the coalesced pass below: four lanes per row
         double2 old[Z_CH / 2];
         if (accumulate) {
 #pragma unroll
           for (int i = 0; i < Z_CH / 2; ++i) {
-            const int row = row0 + 4 * i + (lane >> 3), cc = cc0 + (lane & 7);
+            const int row = row0 + 8 * i + (lane >> 2), cc = cc0 + (lane & 3);
             old[i] = (row < M && cc < N) ? C[(long long)row * ldc + cc] : make_double2(0, 0);
           }
         }
         uint32_t a[Z_S][Z_CH];
 #pragma unroll
         for (int l = 0; l < Z_S; ++l)
-          tmem_ld16(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(l * Z_BN + ch * Z_CH), a[l]);
+          tmem_ld8(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(l * Z_BN + ch * Z_CH), a[l]);
         asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-        if (ch == Z_BN / Z_CH - 1) {
+        if (ch == (half + 1) * NCH - 1) {
           // the accumulators have been read: the MMA warp may overwrite them
           tc_fence_before();
           __syncwarp();
           if (lane == 0) mbar_arrive(acce);
         }
         if (row0 < M && cc0 < N) {
+          int ex[Z_CH / 2];                              // exponents of (row = lane, complex column)
+          bool far = false;
+#pragma unroll
+          for (int c = 0; c < Z_CH / 2; ++c) {
+            ex[c] = er + (cc0 + c < N ? __ldg(eb + cc0 + c) : 0) - 36;
+            far = far || ex[c] > Z_EXMAX || ex[c] < -Z_EXMAX;
+          }
+          double val[Z_CH];
 #pragma unroll
           for (int c = 0; c < Z_CH; ++c) {
-            const int cc = cc0 + (c >> 1);
-            const int ec = cc < N ? __ldg(eb + cc) : 0;
             long long h = 0, w = 0;
 #pragma unroll
             for (int l = 0; l < 4; ++l) {
@@ -391,16 +373,30 @@ __global__ void __launch_bounds__(Z_THREADS, 1)
               w = (w << 8) + (long long)__float2int_rn(__uint_as_float(a[l + 4][c]));
             }
             // sum of the levels = (h 2^32 + w) 2^56 units of 2^-124
-            double v = fixed_to_double(h + (w >> 32), (unsigned)w, er + ec - 68);
-            if (er == Z_NAN || ec == Z_NAN) v = __longlong_as_double(0x7ff8000000000000ll);
-            // row = lane; 16-byte units (re, im) spread over the banks by the row
-            stage[lane * Z_CH + 2 * ((c >> 1) ^ (lane & 7)) + (c & 1)] = negate ? -v : v;
+            val[c] = fixed_to_double(h + (w >> 32), (unsigned)w);
           }
+          if (!__any_sync(0xffffffffu, far)) {
+#pragma unroll
+            for (int c = 0; c < Z_CH; ++c) val[c] = shift_exp(val[c], ex[c >> 1]);
+          } else {                                       // results near the ends of the range, or non-finite operands
+#pragma unroll
+            for (int c = 0; c < Z_CH; ++c) {
+              const int e = ex[c >> 1], e1 = max(min(e / 2, Z_EXMAX), -Z_EXMAX), e2 = max(min(e - e1, Z_EXMAX), -Z_EXMAX);
+              const double f1 = __longlong_as_double(e > Z_NAN / 2 ? 0x7ff8000000000000ll : (long long)(1023 + e1) << 52);
+              val[c] = val[c] * f1 * __longlong_as_double((long long)(1023 + e2) << 52);
+            }
+          }
+          // row = lane; 16-byte units (re, im) spread over the banks by the row
+          double2* st2 = reinterpret_cast<double2*>(stage);
+#pragma unroll
+          for (int c = 0; c < Z_CH / 2; ++c)
+            st2[lane * (Z_CH / 2) + (c ^ ((lane >> 1) & 3))] =
+                negate ? make_double2(-val[2 * c], -val[2 * c + 1]) : make_double2(val[2 * c], val[2 * c + 1]);
           __syncwarp();
 #pragma unroll
           for (int i = 0; i < Z_CH / 2; ++i) {
-            const int rr = 4 * i + (lane >> 3), row = row0 + rr, cc = cc0 + (lane & 7);
-            double2 v = reinterpret_cast<const double2*>(stage)[rr * (Z_CH / 2) + ((lane & 7) ^ (rr & 7))];
+            const int rr = 8 * i + (lane >> 2), row = row0 + rr, cc = cc0 + (lane & 3);
+            double2 v = st2[rr * (Z_CH / 2) + ((lane & 3) ^ ((rr >> 1) & 3))];
             if (accumulate) v = cadd(v, old[i]);
             if (row < M && cc < N) C[(long long)row * ldc + cc] = v;
           }
