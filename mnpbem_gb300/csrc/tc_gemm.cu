@@ -39,9 +39,6 @@ constexpr uint32_t TC_TMEM_COLS = 256;
 constexpr unsigned long long TC_WAIT_NS = MBAR_WAIT_NS;
 
 // instruction descriptor: D f32, A/B tf32, K-major A and B, N = 256, M = 128
-// kind::f16 with FP16 A and B (the same type for both), FP32 accumulator
-constexpr uint32_t TC_IDESC_F16 = (1u << 4) | (0u << 7) | (0u << 10) | ((uint32_t)(TC_BN >> 3) << 17) |
-                                  ((uint32_t)(TC_BM >> 4) << 24);
 constexpr uint32_t TC_IDESC = (1u << 4) | (2u << 7) | (2u << 10) | ((uint32_t)(TC_BN >> 3) << 17) |
                               ((uint32_t)(TC_BM >> 4) << 24);
 
@@ -143,18 +140,12 @@ __device__ __forceinline__ void epi_chunk_lsu(const uint32_t (&r)[32], float* st
   __syncwarp();
 }
 
-// F16: A and B' are FP16 (kind::f16), scaled per row of A and per complex
-// column of B' into FP16's range; the epilogue multiplies each accumulator by
-// inv_r[row] * inv_c[column / 2] before storing.  K2 counts elements of the
-// operand type (TF32 floats or halves); a K chunk is one 128-byte swizzle row
-// either way (32 floats or 64 halves).
-template <int ST, int EPI, bool F16>
+template <int ST, int EPI>
 __global__ void __launch_bounds__(TC_THREADS, 1)
     k_tc_gemm(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
               const __grid_constant__ CUtensorMap mapC, const __grid_constant__ CUtensorMap mapP,
-              float* __restrict__ Cp, long long ldcf, int M, int N2, int K2, int accumulate, int* tile_ctr, int* err,
-              const float* __restrict__ inv_r, const float* __restrict__ inv_c) {
-  constexpr int BK = F16 ? 64 : TC_BK;
+              float* __restrict__ Cp, long long ldcf, int M, int N2, int K2, int accumulate, int* tile_ctr, int* err) {
+  constexpr int BK = TC_BK;
   extern __shared__ unsigned char smem_raw[];
   __shared__ __align__(8) unsigned long long bars[2 * ST + 4 + 2 * TC_TQ];
   __shared__ int tq[TC_TQ];
@@ -261,11 +252,8 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
           const uint64_t da = desc_sw128(sa), db = desc_sw128(sb);
 #pragma unroll
           for (int kk = 0; kk < 4; ++kk) {
-            // advance 8 tf32 or 16 halves = 32 bytes along K inside the swizzle row
-            if constexpr (F16)
-              mma_f16(dt, da + 2 * kk, db + 2 * kk, TC_IDESC_F16, (kt > 0 || kk > 0) ? 1u : 0u);
-            else
-              mma_tf32(dt, da + 2 * kk, db + 2 * kk, TC_IDESC, (kt > 0 || kk > 0) ? 1u : 0u);
+            // advance 8 tf32 = 32 bytes along K inside the swizzle row
+            mma_tf32(dt, da + 2 * kk, db + 2 * kk, TC_IDESC, (kt > 0 || kk > 0) ? 1u : 0u);
           }
           mma_commit(empty0 + 8 * s);
         }
@@ -301,18 +289,6 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
         uint32_t r[32];
         tmem_ld32(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(b * TC_TMEM_COLS + c * 32), r);
         if (col0 >= N2 || row0 >= M) continue;            // warp-uniform
-        if constexpr (F16) {
-          // undo the operand scaling: row scale of this lane's row, column
-          // scale of each complex column (two floats)
-          const float rs = (row0 + lane < M) ? __ldg(inv_r + row0 + lane) : 0.f;
-#pragma unroll
-          for (int q = 0; q < 16; ++q) {
-            const int cc = (col0 >> 1) + q;
-            const float sc = rs * ((2 * cc < N2) ? __ldg(inv_c + cc) : 0.f);
-            r[2 * q] = __float_as_uint(__uint_as_float(r[2 * q]) * sc);
-            r[2 * q + 1] = __float_as_uint(__uint_as_float(r[2 * q + 1]) * sc);
-          }
-        }
         if constexpr (EPI == 1) {
           epi_chunk_lsu(r, stage_gen, lane, Cp, ldcf, row0, col0, M, N2, accumulate);
           continue;
@@ -322,6 +298,256 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
         __syncwarp();
         // row = lane of a 32 x 32 tile in the 128-byte swizzled layout of the
         // C tensor map: 16-byte chunk c of row l sits at chunk c ^ (l & 7)
+        float4* st = reinterpret_cast<float4*>(stage_gen + buf * 1024) + lane * 8;
+#pragma unroll
+        for (int c4 = 0; c4 < 8; ++c4)
+          st[c4 ^ (lane & 7)] = make_float4(__uint_as_float(r[4 * c4]), __uint_as_float(r[4 * c4 + 1]),
+                                            __uint_as_float(r[4 * c4 + 2]), __uint_as_float(r[4 * c4 + 3]));
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        __syncwarp();
+        if (lane == 0) {
+          const uint32_t src = stage0 + (uint32_t)buf * 4096u;
+          if (accumulate)
+            asm volatile(
+                "cp.reduce.async.bulk.tensor.2d.global.shared::cta.add.bulk_group [%0, {%1, %2}], [%3];"
+                ::"l"((unsigned long long)&mapC), "r"(col0), "r"(row0), "r"(src)
+                : "memory");
+          else
+            asm volatile("cp.async.bulk.tensor.2d.global.shared::cta.bulk_group [%0, {%1, %2}], [%3];"
+                         ::"l"((unsigned long long)&mapC), "r"(col0), "r"(row0), "r"(src)
+                         : "memory");
+          asm volatile("cp.async.bulk.commit_group;" ::: "memory");
+        }
+        ++nstores;
+      }
+      // this accumulator has been read: the MMA warp may overwrite it
+      tc_fence_before();
+      __syncwarp();
+      if (lane == 0) mbar_arrive(acce0 + 8 * b);
+    }
+    if (lane == 0) asm volatile("cp.async.bulk.wait_group 0;" ::: "memory");
+    __syncwarp();
+  }
+  // ---------------- drain loads still in flight after an error, free TMEM
+  if (warp == 0 && lane == 0 && *(volatile int*)err) {
+    for (int i = issued - ST > 0 ? issued - ST : 0; i < issued; ++i) {
+      const int s = i % ST;
+      mbar_wait(full0 + 8 * s, (i / ST) & 1, err, 8);
+    }
+  }
+  tc_fence_before();
+  __syncthreads();
+  if (warp == 0) {
+    tc_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(2 * TC_TMEM_COLS) : "memory");
+  }
+}
+
+// ------------------------------------------------ FP16 operands, planes
+// C = A B (+ C) from FP16 planes Ar, Ai [M][Kp] and Br, Bi [N][Kp] (B transposed),
+// scaled per row of A and per column of B into FP16's range (k_a_planes,
+// k_b_planes).  A tile is 128 rows x 128 complex columns, its accumulator
+// [Cr | Ci] (256 tensor-memory columns); per 16 k
+//     [Cr | Ci] += Ar [Br; Bi]  (N = 256),   Cr -= Ai Bi,   Ci += Ai Br  (N = 128),
+// the sign through the instruction descriptor.  A K chunk of 64 (one 128-byte
+// swizzle row per plane) is 64 KB for the tensor work that needs 96 KB with the
+// interleaved operands of the TF32 kernel, whose B' holds every entry twice: the
+// FP16 product was bound by L2 reads (96 bytes per clock and SM at full rate,
+// 55 delivered), not by the tensor cores.  The epilogue interleaves Cr and Ci,
+// undoes the scales and stores as the TF32 kernel does.
+// Measured with the operand passes: 23 000 x 23 000 x 1024 1458 TFLOP/s (1305 before),
+// 4000 x 4000 x 512 745 TFLOP/s (639 before).
+constexpr int PF_BK = 64;
+constexpr int PF_PLANE = 128 * PF_BK * 2;               // 16 KB: one plane of A or B
+constexpr int PF_STAGE = 4 * PF_PLANE;
+constexpr int pf_psmem(int stages) { return stages * PF_STAGE + TC_STAGE_SMEM + 1024; }
+constexpr uint32_t PF_IDESC_256 = (1u << 4) | ((uint32_t)(256 >> 3) << 17) | ((uint32_t)(TC_BM >> 4) << 24);
+constexpr uint32_t PF_IDESC_128 = (1u << 4) | ((uint32_t)(128 >> 3) << 17) | ((uint32_t)(TC_BM >> 4) << 24);
+constexpr uint32_t PF_NEG_A = 1u << 13;                 // D = -A B + D
+
+// 16 columns of Cr and of Ci, interleaved into r (one asm statement: nothing may
+// touch the registers between the loads and the wait)
+__device__ __forceinline__ void tmem_ld_complex16(uint32_t tr, uint32_t ti, uint32_t (&r)[32]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%32];\n"
+      " tcgen05.ld.sync.aligned.32x32b.x16.b32 {%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%33];\n"
+      " tcgen05.wait::ld.sync.aligned;"
+      : "=r"(r[0]), "=r"(r[2]), "=r"(r[4]), "=r"(r[6]), "=r"(r[8]), "=r"(r[10]), "=r"(r[12]), "=r"(r[14]), "=r"(r[16]), "=r"(r[18]), "=r"(r[20]), "=r"(r[22]), "=r"(r[24]), "=r"(r[26]), "=r"(r[28]), "=r"(r[30]),
+        "=r"(r[1]), "=r"(r[3]), "=r"(r[5]), "=r"(r[7]), "=r"(r[9]), "=r"(r[11]), "=r"(r[13]), "=r"(r[15]), "=r"(r[17]), "=r"(r[19]), "=r"(r[21]), "=r"(r[23]), "=r"(r[25]), "=r"(r[27]), "=r"(r[29]), "=r"(r[31])
+      : "r"(tr), "r"(ti)
+      : "memory");
+}
+
+template <int ST, int EPI>
+__global__ void __launch_bounds__(TC_THREADS, 1)
+    k_tc_gemm_f16(const __grid_constant__ CUtensorMap mapA, const __grid_constant__ CUtensorMap mapB,
+                  const __grid_constant__ CUtensorMap mapC, const __grid_constant__ CUtensorMap mapP,
+                  float* __restrict__ Cp, long long ldcf, int M, int N, int Kp, int accumulate, int* tile_ctr, int* err,
+                  const float* __restrict__ inv_r, const float* __restrict__ inv_c) {
+  extern __shared__ unsigned char smem_raw[];
+  __shared__ __align__(8) unsigned long long bars[2 * ST + 4 + 2 * TC_TQ];
+  __shared__ int tq[TC_TQ];
+  __shared__ uint32_t tmem_slot;
+  const uint32_t base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int N2 = 2 * N;
+  const int KT = Kp / PF_BK;
+  const int MT = (M + TC_BM - 1) / TC_BM, NT = (N2 + TC_BN - 1) / TC_BN;
+  const int ntiles = MT * NT;
+  const uint32_t full0 = smem_u32(&bars[0]), empty0 = smem_u32(&bars[ST]);
+  const uint32_t accf0 = smem_u32(&bars[2 * ST]), acce0 = smem_u32(&bars[2 * ST + 2]);
+  const uint32_t tqf0 = smem_u32(&bars[2 * ST + 4]), tqe0 = smem_u32(&bars[2 * ST + 4 + TC_TQ]);
+  const uint32_t stage_base = base + ST * PF_STAGE;
+
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < ST; ++s) {
+      mbar_init(full0 + 8 * s, 1);
+      mbar_init(empty0 + 8 * s, 1);
+    }
+    for (int b = 0; b < 2; ++b) {
+      mbar_init(accf0 + 8 * b, 1);
+      mbar_init(acce0 + 8 * b, TC_EPI_WARPS);
+    }
+    for (int q = 0; q < TC_TQ; ++q) {
+      mbar_init(tqf0 + 8 * q, 1);
+      mbar_init(tqe0 + 8 * q, 1 + TC_EPI_WARPS);
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+  }
+  __syncwarp();
+  if (warp == 0) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(&tmem_slot)),
+                 "r"(2 * TC_TMEM_COLS)
+                 : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tc_fence_before();
+  __syncthreads();
+  tc_fence_after();
+  const uint32_t tmem = tmem_slot;
+
+  int issued = 0;   // producer: K chunks issued (for the drain after an error)
+  if (warp == 0) {
+    if (lane == 0) {
+      // ---------------- tile scheduler + TMA producer (counter read one tile ahead)
+      int it = 0;
+      int t_next = atomicAdd(tile_ctr, 1);
+      for (int j = 0;; ++j) {
+        const int q = j % TC_TQ;
+        if (j >= TC_TQ && !mbar_wait(tqe0 + 8 * q, ((j / TC_TQ) - 1) & 1, err, 16)) break;
+        int t = *(volatile int*)err ? -1 : t_next;
+        if (t >= ntiles) t = -1;
+        if (t >= 0) t_next = atomicAdd(tile_ctr, 1);
+        tq[q] = t;
+        mbar_arrive(tqf0 + 8 * q);
+        if (t < 0) break;
+        int mt, nt;
+        tile_coords(t, MT, NT, mt, nt);
+        const int m0 = mt * TC_BM, n0 = nt * (TC_BN / 2);       // n0: complex column
+        if (accumulate) tma_prefetch_2d(&mapP, 2 * n0, m0);
+        bool ok = true;
+        for (int kt = 0; kt < KT; ++kt, ++it) {
+          const int s = it % ST;
+          if (it >= ST && !mbar_wait(empty0 + 8 * s, ((it / ST) - 1) & 1, err, 1)) { ok = false; break; }
+          const uint32_t sa = base + s * PF_STAGE;
+          mbar_expect_tx(full0 + 8 * s, PF_STAGE);
+          tma_load_2d(sa, &mapA, full0 + 8 * s, kt * PF_BK, m0);
+          tma_load_2d(sa + 2 * PF_PLANE, &mapB, full0 + 8 * s, kt * PF_BK, n0);
+          tma_load_2d(sa + 3 * PF_PLANE, &mapB, full0 + 8 * s, kt * PF_BK, N + n0);
+          tma_load_2d(sa + PF_PLANE, &mapA, full0 + 8 * s, kt * PF_BK, M + m0);
+          issued = it + 1;
+        }
+        if (!ok) {
+          // hand out an end marker in the next slot so that the other roles stop
+          const int q2 = (j + 1) % TC_TQ;
+          if (j + 1 < TC_TQ || mbar_wait(tqe0 + 8 * q2, (((j + 1) / TC_TQ) - 1) & 1, err, 16)) {
+            tq[q2] = -1;
+            mbar_arrive(tqf0 + 8 * q2);
+          }
+          break;
+        }
+      }
+    }
+  } else if (warp == 1) {
+    if (lane == 0) {
+      // ---------------- MMA issuer
+      int it = 0;
+      for (int j = 0;; ++j) {
+        const int q = j % TC_TQ;
+        if (!mbar_wait(tqf0 + 8 * q, (j / TC_TQ) & 1, err, 32)) break;
+        const int t = *(volatile int*)&tq[q];
+        mbar_arrive(tqe0 + 8 * q);
+        if (t < 0) break;
+        const int b = j & 1;
+        if (j >= 2 && !mbar_wait(acce0 + 8 * b, ((j >> 1) - 1) & 1, err, 64)) break;
+        tc_fence_after();
+        const uint32_t dt = tmem + (uint32_t)(b * TC_TMEM_COLS);
+        bool ok = true;
+        for (int kt = 0; kt < KT; ++kt, ++it) {
+          const int s = it % ST;
+          if (!mbar_wait(full0 + 8 * s, (it / ST) & 1, err, 2)) { ok = false; break; }
+          tc_fence_after();
+          const uint32_t sa = base + s * PF_STAGE;
+          const uint64_t ar = desc_sw128(sa), ai = desc_sw128(sa + PF_PLANE);
+          const uint64_t br = desc_sw128(sa + 2 * PF_PLANE), bi = desc_sw128(sa + 3 * PF_PLANE);
+#pragma unroll
+          for (int kk = 0; kk < 4; ++kk) {             // 16 halves = 32 bytes along K
+            mma_f16(dt, ar + 2 * kk, br + 2 * kk, PF_IDESC_256, (kt > 0 || kk > 0) ? 1u : 0u);
+            mma_f16(dt, ai + 2 * kk, bi + 2 * kk, PF_IDESC_128 | PF_NEG_A, 1u);
+            mma_f16(dt + 128, ai + 2 * kk, br + 2 * kk, PF_IDESC_128, 1u);
+          }
+          mma_commit(empty0 + 8 * s);
+        }
+        if (!ok) break;
+        mma_commit(accf0 + 8 * b);
+      }
+    }
+  } else {
+    // ---------------- epilogue warps: TMEM lane quarter (warp % 4) = 32 rows of the tile
+    const int ew = warp - 2;                 // staging slot
+    const int quarter = warp & 3;
+    const uint32_t stage0 = stage_base + (uint32_t)ew * 2u * 4096u;
+    float* stage_gen = reinterpret_cast<float*>(smem_raw + (stage_base - smem_u32(smem_raw))) + ew * 2 * 1024;
+    int nstores = 0;
+    for (int j = 0;; ++j) {
+      const int q = j % TC_TQ;
+      int t = -1;
+      const bool okq = __all_sync(0xffffffffu, mbar_wait(tqf0 + 8 * q, (j / TC_TQ) & 1, err, 128) ? 1 : 0) != 0;
+      if (okq) t = *(volatile int*)&tq[q];
+      __syncwarp();
+      if (lane == 0 && okq) mbar_arrive(tqe0 + 8 * q);
+      if (!okq || t < 0) break;
+      const int b = j & 1;
+      int mt, nt;
+      tile_coords(t, MT, NT, mt, nt);
+      const int row0 = mt * TC_BM + quarter * 32, n0 = nt * TC_BN;   // n0: real column
+      const float rs = (row0 + lane < M) ? __ldg(inv_r + row0 + lane) : 0.f;
+      const bool ok = __all_sync(0xffffffffu, mbar_wait(accf0 + 8 * b, (j >> 1) & 1, err, 4) ? 1 : 0) != 0;
+      if (!ok) break;
+      tc_fence_after();
+      for (int c = 0; c < TC_BN / 32; ++c) {
+        const int col0 = n0 + c * 32;
+        uint32_t r[32];
+        const uint32_t ta = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(b * TC_TMEM_COLS + c * 16);
+        tmem_ld_complex16(ta, ta + 128, r);
+        if (col0 >= N2 || row0 >= M) continue;            // warp-uniform
+        // undo the operand scaling: row scale of this lane's row, column scale
+        // of each complex column
+        const int cj = (col0 >> 1) + (lane & 15);
+        const float sl = cj < N ? __ldg(inv_c + cj) : 0.f;
+#pragma unroll
+        for (int qq = 0; qq < 16; ++qq) {
+          const float sc = rs * __shfl_sync(0xffffffffu, sl, qq);
+          r[2 * qq] = __float_as_uint(__uint_as_float(r[2 * qq]) * sc);
+          r[2 * qq + 1] = __float_as_uint(__uint_as_float(r[2 * qq + 1]) * sc);
+        }
+        if constexpr (EPI == 1) {
+          epi_chunk_lsu(r, stage_gen, lane, Cp, ldcf, row0, col0, M, N2, accumulate);
+          continue;
+        }
+        const int buf = nstores & 1;
+        if (lane == 0) asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory");
+        __syncwarp();
         float4* st = reinterpret_cast<float4*>(stage_gen + buf * 1024) + lane * 8;
 #pragma unroll
         for (int c4 = 0; c4 < 8; ++c4)
@@ -701,8 +927,9 @@ __device__ __forceinline__ float to_tf32(float x) {
   return __uint_as_float(r);
 }
 __global__ void k_expand_b(int K, int N, float2 alpha, const float2* __restrict__ B, int64_t ldb, float* __restrict__ Bp,
-                           int K2p, int bz0, int bz1) {
+                           int K2p, int bz0, int bz1, int* tile_ctr) {
   __shared__ float2 tile[32][33];
+  if (blockIdx.x == 0 && blockIdx.y == 0 && threadIdx.x == 0 && threadIdx.y == 0) *tile_ctr = 0;   // of the product that follows
   const int l0 = blockIdx.y * 32, j0 = blockIdx.x * 32;
   const int tx = threadIdx.x, ty = threadIdx.y;   // 32 x 8
   for (int r = ty; r < 32; r += 8) {
@@ -744,21 +971,35 @@ __device__ __forceinline__ float pow2_scale(float mx) {
   return ldexpf(1.f, 14 - ilogbf(mx));
 }
 
-// A16[i][0 .. K2p) = fp16(s_i A_r[i][k]) for k < 2K (A_r: the complex64 row read as
-// floats), zero beyond; inv_r[i] = 1 / s_i with s_i from the row's largest entry.
-// One warp per row.
-__global__ void k_a_to_f16(const float2* __restrict__ A, int64_t lda, int M, int K, __half* __restrict__ A16,
-                           int K2p, float* __restrict__ inv_r) {
+// Planes Ar, Ai [M][Kp] of fp16(s_i A[i][k]) for k < K, zero beyond; inv_r[i] =
+// 1 / s_i with s_i from the row's largest entry.  One warp per row, two
+// neighbouring k per lane (A 16-byte aligned, lda even).  The first CTAs also
+// clear the tile counter and the column maxima of the passes that follow.
+__global__ void k_a_planes(const float2* __restrict__ A, int64_t lda, int M, int K, __half* __restrict__ Ar,
+                           __half* __restrict__ Ai, int Kp, float* __restrict__ inv_r, int* tile_ctr,
+                           unsigned* __restrict__ colmax, int N) {
+  for (int j = blockIdx.x * 256 + threadIdx.x; j < N; j += gridDim.x * 256) colmax[j] = 0u;
+  if (blockIdx.x == 0 && threadIdx.x == 0) *tile_ctr = 0;
   const int row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (row >= M) return;
-  const float* a = reinterpret_cast<const float*>(A + (int64_t)row * lda);
+  const float2* a = A + (int64_t)row * lda;
   float mx = 0.f;
-  for (int k = lane; k < 2 * K; k += 32) mx = fmaxf(mx, fabsf(a[k]));
+  for (int k = 2 * lane; k < K; k += 64) {
+    const float4 v = k + 1 < K ? *reinterpret_cast<const float4*>(a + k) : make_float4(a[k].x, a[k].y, 0.f, 0.f);
+    mx = fmaxf(mx, fmaxf(fmaxf(fabsf(v.x), fabsf(v.y)), fmaxf(fabsf(v.z), fabsf(v.w))));
+  }
   for (int o = 16; o; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
   const float sc = pow2_scale(mx);
   if (lane == 0) inv_r[row] = 1.f / sc;
-  __half* dst = A16 + (int64_t)row * K2p;
-  for (int k = lane; k < K2p; k += 32) dst[k] = __float2half_rn(k < 2 * K ? a[k] * sc : 0.f);
+  __half2* dr = reinterpret_cast<__half2*>(Ar + (int64_t)row * Kp);
+  __half2* di = reinterpret_cast<__half2*>(Ai + (int64_t)row * Kp);
+  for (int k = 2 * lane; k < Kp; k += 64) {
+    float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (k + 1 < K) v = *reinterpret_cast<const float4*>(a + k);
+    else if (k < K) v = make_float4(a[k].x, a[k].y, 0.f, 0.f);
+    dr[k >> 1] = __floats2half2_rn(v.x * sc, v.z * sc);
+    di[k >> 1] = __floats2half2_rn(v.y * sc, v.w * sc);
+  }
 }
 
 // per complex column j of alpha * B (K x N, row stride ldb): the largest real
@@ -786,42 +1027,37 @@ __global__ void k_b_colmax(const float2* __restrict__ B, int64_t ldb, int K, int
   }
 }
 
-// B'[2N][K2p] in FP16 from c_j alpha B (c_j from colmax), the same real layout
-// as k_expand_b; the CTAs of the first row of tiles write inv_c
-__global__ void k_expand_b16(int K, int N, float2 alpha, const float2* __restrict__ B, int64_t ldb,
-                             __half* __restrict__ Bp, int K2p, int bz0, int bz1, const unsigned* __restrict__ colmax,
-                             float* __restrict__ inv_c) {
-  __shared__ float2 tile[32][33];
-  const int l0 = blockIdx.y * 32, j0 = blockIdx.x * 32;
+// Planes Br, Bi [N][Kp] of fp16(c_j alpha B[k][j]), transposed, zero for k >= K (c_j
+// from colmax); the CTAs of the first row of tiles write inv_c.  CTA (32 x 8
+// threads): a tile of 64 k x 32 columns, two k per thread on the way out.
+__global__ void k_b_planes(int K, int N, float2 alpha, const float2* __restrict__ B, int64_t ldb,
+                           __half* __restrict__ Br, __half* __restrict__ Bi, int Kp, int bz0, int bz1,
+                           const unsigned* __restrict__ colmax, float* __restrict__ inv_c) {
+  __shared__ float2 tile[64][33];
+  const int l0 = blockIdx.y * 64, j0 = blockIdx.x * 32;
   const int tx = threadIdx.x, ty = threadIdx.y;   // 32 x 8
   {
     const int j = j0 + tx;
-    if (blockIdx.y == 0 && ty == 0 && j < N) inv_c[j] = 1.f / pow2_scale(__uint_as_float(colmax[j]));
-  }
-  for (int r = ty; r < 32; r += 8) {
-    const int l = l0 + r, j = j0 + tx;
-    float2 v = make_float2(0.f, 0.f);
-    if (l < K && j < N && (j < bz0 || j >= bz1)) {
-      const float2 b = B[(int64_t)l * ldb + j];
-      const float s = pow2_scale(__uint_as_float(colmax[j]));
-      v = make_float2((alpha.x * b.x - alpha.y * b.y) * s, (alpha.x * b.y + alpha.y * b.x) * s);
+    const bool in = j < N && (j < bz0 || j >= bz1);
+    const float s = j < N ? pow2_scale(__uint_as_float(colmax[j])) : 1.f;
+    if (blockIdx.y == 0 && ty == 0 && j < N) inv_c[j] = 1.f / s;
+    for (int r = ty; r < 64; r += 8) {
+      const int l = l0 + r;
+      float2 v = make_float2(0.f, 0.f);
+      if (l < K && in) {
+        const float2 b = B[(int64_t)l * ldb + j];
+        v = make_float2((alpha.x * b.x - alpha.y * b.y) * s, (alpha.x * b.y + alpha.y * b.x) * s);
+      }
+      tile[r][tx] = v;
     }
-    tile[r][tx] = v;
   }
   __syncthreads();
   for (int r = ty; r < 32; r += 8) {
-    const int j = j0 + r, l = l0 + tx;
-    if (j >= N || 2 * l >= K2p) continue;
-    const float2 v = tile[tx][r];
-    __half2* r0 = reinterpret_cast<__half2*>(Bp + (int64_t)(2 * j) * K2p) + l;
-    __half2* r1 = reinterpret_cast<__half2*>(Bp + (int64_t)(2 * j + 1) * K2p) + l;
-    if (l < K) {
-      *r0 = __floats2half2_rn(v.x, -v.y);
-      *r1 = __floats2half2_rn(v.y, v.x);
-    } else {
-      *r0 = __floats2half2_rn(0.f, 0.f);
-      *r1 = __floats2half2_rn(0.f, 0.f);
-    }
+    const int j = j0 + r;
+    if (j >= N) continue;
+    const float2 v0 = tile[2 * tx][r], v1 = tile[2 * tx + 1][r];
+    reinterpret_cast<__half2*>(Br + (int64_t)j * Kp + l0)[tx] = __floats2half2_rn(v0.x, v1.x);
+    reinterpret_cast<__half2*>(Bi + (int64_t)j * Kp + l0)[tx] = __floats2half2_rn(v0.y, v1.y);
   }
 }
 
@@ -881,14 +1117,14 @@ bool tc_gemm_eligible(TcGemmCtx& c, int64_t M, int64_t N, int64_t K, const void*
     cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, dev);
     cudaDeviceGetAttribute(&minor, cudaDevAttrComputeCapabilityMinor, dev);
     c.usable = (major == 10 && minor == 3) && get_encode(c) != nullptr &&
-               cudaFuncSetAttribute(k_tc_gemm<3, 0, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, tc_psmem(3)) == cudaSuccess &&
-               cudaFuncSetAttribute(k_tc_gemm<4, 0, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, tc_psmem(4)) == cudaSuccess &&
-               cudaFuncSetAttribute(k_tc_gemm<3, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, tc_psmem(3)) == cudaSuccess &&
-               cudaFuncSetAttribute(k_tc_gemm<4, 1, false>, cudaFuncAttributeMaxDynamicSharedMemorySize, tc_psmem(4)) == cudaSuccess &&
-               cudaFuncSetAttribute(k_tc_gemm<3, 0, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, tc_psmem(3)) == cudaSuccess &&
-               cudaFuncSetAttribute(k_tc_gemm<4, 0, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, tc_psmem(4)) == cudaSuccess &&
-               cudaFuncSetAttribute(k_tc_gemm<3, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, tc_psmem(3)) == cudaSuccess &&
-               cudaFuncSetAttribute(k_tc_gemm<4, 1, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, tc_psmem(4)) == cudaSuccess &&
+               cudaFuncSetAttribute(k_tc_gemm<3, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, tc_psmem(3)) == cudaSuccess &&
+               cudaFuncSetAttribute(k_tc_gemm<4, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, tc_psmem(4)) == cudaSuccess &&
+               cudaFuncSetAttribute(k_tc_gemm<3, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, tc_psmem(3)) == cudaSuccess &&
+               cudaFuncSetAttribute(k_tc_gemm<4, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, tc_psmem(4)) == cudaSuccess &&
+               cudaFuncSetAttribute(k_tc_gemm_f16<2, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, pf_psmem(2)) == cudaSuccess &&
+               cudaFuncSetAttribute(k_tc_gemm_f16<3, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, pf_psmem(3)) == cudaSuccess &&
+               cudaFuncSetAttribute(k_tc_gemm_f16<2, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, pf_psmem(2)) == cudaSuccess &&
+               cudaFuncSetAttribute(k_tc_gemm_f16<3, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, pf_psmem(3)) == cudaSuccess &&
                cudaFuncSetAttribute(k_tc_gemm_pair<5, 4, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, tp_psmem(5, 4)) == cudaSuccess &&
                cudaFuncSetAttribute(k_tc_gemm_pair<6, 2, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, tp_psmem(6, 2)) == cudaSuccess &&
                cudaFuncSetAttribute(k_tc_gemm_pair<6, 2, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, tp_psmem(6, 2)) == cudaSuccess &&
@@ -907,40 +1143,40 @@ bool tc_gemm_eligible(TcGemmCtx& c, int64_t M, int64_t N, int64_t K, const void*
   return M >= 128 && N >= 64 && K >= 16 && M < (1 << 30) && 2 * N < (1 << 30) && 2 * K < (1 << 30);
 }
 
-// The product with FP16 operands: A converted row by row and B' column by
-// column into FP16 with power-of-two scales (k_a_to_f16, k_b_colscale,
-// k_expand_b16), kind::f16 MMAs with FP32 accumulation, the scales undone in
-// the epilogue.  FP16 keeps TF32's 10-bit significand and issues at twice the
-// TF32 rate with half the operand bytes per multiply-add.
+// The product with FP16 operands: the planes of A scaled row by row and of B
+// column by column by powers of two (k_a_planes, k_b_colmax, k_b_planes),
+// kind::f16 MMAs with FP32 accumulation, the scales undone in the epilogue.
+// FP16 keeps TF32's 10-bit significand and issues at twice the TF32 rate with
+// half the operand bytes per multiply-add.
 static mnpbem_status tc_gemm_f16(TcGemmCtx& c, int64_t M, int64_t N, int64_t K, float2 alpha, const float2* A,
                                  int64_t lda, const float2* B, int64_t ldb, float2 beta, float2* C, int64_t ldc,
                                  cudaStream_t st, int64_t bz0, int64_t bz1) {
-  constexpr int BK = 64;
-  const int64_t K2 = 2 * K, N2 = 2 * N, K2p = round_up(K2, BK);
-  MNP_TRY(c.bexp.ensure(sizeof(__half) * N2 * K2p));
-  MNP_TRY(c.a16.ensure(sizeof(__half) * M * K2p));
+  const int64_t N2 = 2 * N, Kp = round_up(K, (int64_t)PF_BK);
+  MNP_TRY(c.bexp.ensure(sizeof(__half) * N2 * Kp));
+  MNP_TRY(c.a16.ensure(sizeof(__half) * 2 * M * Kp));
   MNP_TRY(c.scales.ensure(sizeof(float) * (M + 2 * N)));
   MNP_TRY(c.err.ensure(sizeof(int)));
+  MNP_TRY(c.ctr.ensure(sizeof(int)));
   __half* Bp = c.bexp.as<__half>();
   __half* A16 = c.a16.as<__half>();
   float* inv_r = c.scales.as<float>();
   unsigned* colmax = reinterpret_cast<unsigned*>(inv_r + M);
   float* inv_c = inv_r + M + N;
   {
-    ProfScope ps(PH_ELEMWISE, st, 0.0, 16.0 * K * N + 8.0 * M * K + 4.0 * M * K + 8.0 * N * K);
-    MNP_CUDA(cudaMemsetAsync(colmax, 0, sizeof(unsigned) * N, st));
-    k_a_to_f16<<<(unsigned)cdiv_up(M, (int64_t)8), 256, 0, st>>>(A, lda, (int)M, (int)K, A16, (int)K2p, inv_r);
+    ProfScope ps(PH_ELEMWISE, st, 0.0, 16.0 * K * N + 8.0 * M * K + 4.0 * M * K + 4.0 * N * K);
+    k_a_planes<<<(unsigned)cdiv_up(M, (int64_t)8), 256, 0, st>>>(A, lda, (int)M, (int)K, A16, A16 + M * Kp, (int)Kp,
+                                                                 inv_r, c.ctr.as<int>(), colmax, (int)N);
     k_b_colmax<<<dim3((unsigned)cdiv_up(N, 32), (unsigned)cdiv_up(K, 128)), dim3(32, 8), 0, st>>>(
         B, ldb, (int)K, (int)N, alpha, (int)bz0, (int)bz1, colmax);
-    dim3 g((unsigned)cdiv_up(N, 32), (unsigned)cdiv_up(K2p / 2, 32));
-    k_expand_b16<<<g, dim3(32, 8), 0, st>>>((int)K, (int)N, alpha, B, ldb, Bp, (int)K2p, (int)bz0, (int)bz1, colmax,
-                                            inv_c);
+    dim3 g((unsigned)cdiv_up(N, 32), (unsigned)(Kp / 64));
+    k_b_planes<<<g, dim3(32, 8), 0, st>>>((int)K, (int)N, alpha, B, ldb, Bp, Bp + N * Kp, (int)Kp, (int)bz0, (int)bz1,
+                                          colmax, inv_c);
     MNP_CHECK_LAUNCH();
   }
   auto enc = get_encode(c);
   CUtensorMap ma, mb, mc, mp;
-  if (!make_map(enc, &ma, A16, (uint64_t)K2p, (uint64_t)M, (uint64_t)K2p * 2, TC_BM, true, BK, true) ||
-      !make_map(enc, &mb, Bp, (uint64_t)K2p, (uint64_t)N2, (uint64_t)K2p * 2, TC_BN, true, BK, true) ||
+  if (!make_map(enc, &ma, A16, (uint64_t)Kp, (uint64_t)(2 * M), (uint64_t)Kp * 2, TC_BM, true, PF_BK, true) ||
+      !make_map(enc, &mb, Bp, (uint64_t)Kp, (uint64_t)N2, (uint64_t)Kp * 2, TC_BN / 2, true, PF_BK, true) ||
       !make_map(enc, &mc, C, (uint64_t)N2, (uint64_t)M, (uint64_t)ldc * 8, 32, true) ||
       !make_map(enc, &mp, C, (uint64_t)N2, (uint64_t)M, (uint64_t)ldc * 8, TC_BM, false, TC_BN)) {
     set_error("cuTensorMapEncodeTiled failed");
@@ -952,8 +1188,6 @@ static mnpbem_status tc_gemm_f16(TcGemmCtx& c, int64_t M, int64_t N, int64_t K, 
   }
   const int64_t MT = cdiv_up(M, TC_BM), NT = cdiv_up(N2, TC_BN);
   if (MT * NT >= (1ll << 31)) { set_error("tc_gemm_c64: too many tiles"); return MNPBEM_ERR_INVALID_ARG; }
-  MNP_TRY(c.ctr.ensure(sizeof(int)));
-  MNP_CUDA(cudaMemsetAsync(c.ctr.ptr, 0, sizeof(int), st));
   const bool lsu = c.pair_epi == 1 || (N2 & 3) != 0;
   float* Cf = reinterpret_cast<float*>(C);
   const long long ldcf = 2ll * ldc;
@@ -963,9 +1197,10 @@ static mnpbem_status tc_gemm_f16(TcGemmCtx& c, int64_t M, int64_t N, int64_t K, 
   ProfScope ps(M >= 128 && N >= 128 ? PH_GEMM_BIG : PH_GEMM_SMALL, st, 8.0 * M * N * K,
                8.0 * ((double)M * K + (double)K * N + 2.0 * M * N));
   const unsigned grid = (unsigned)std::min<int64_t>(MT * NT, ctas);
-  auto kern = c.stages == 3 ? (lsu ? k_tc_gemm<3, 1, true> : k_tc_gemm<3, 0, true>)
-                            : (lsu ? k_tc_gemm<4, 1, true> : k_tc_gemm<4, 0, true>);
-  kern<<<grid, TC_THREADS, tc_psmem(c.stages == 3 ? 3 : 4), st>>>(ma, mb, mc, mp, Cf, ldcf, (int)M, (int)N2, (int)K2p,
+  // a stage holds 64 KB here, 48 KB in the TF32 kernel: one stage fewer
+  auto kern = c.stages == 3 ? (lsu ? k_tc_gemm_f16<2, 1> : k_tc_gemm_f16<2, 0>)
+                            : (lsu ? k_tc_gemm_f16<3, 1> : k_tc_gemm_f16<3, 0>);
+  kern<<<grid, TC_THREADS, pf_psmem(c.stages == 3 ? 2 : 3), st>>>(ma, mb, mc, mp, Cf, ldcf, (int)M, (int)N, (int)Kp,
                                                                   acc, c.ctr.as<int>(), c.err.as<int>(), inv_r, inv_c);
   MNP_CHECK_LAUNCH();
   return MNPBEM_OK;
@@ -988,11 +1223,13 @@ mnpbem_status tc_gemm_c64(TcGemmCtx& c, int64_t M, int64_t N, int64_t K, float2 
   const int64_t K2p = round_up(K2, TC_BK);
   MNP_TRY(c.bexp.ensure(sizeof(float) * N2 * K2p));
   MNP_TRY(c.err.ensure(sizeof(int)));
+  MNP_TRY(c.ctr.ensure(sizeof(int)));
   float* Bp = c.bexp.as<float>();
   {
     ProfScope ps(PH_ELEMWISE, st, 0.0, 8.0 * K * N + 16.0 * K * N);
     dim3 g((unsigned)cdiv_up(N, 32), (unsigned)cdiv_up(K2p / 2, 32));
-    k_expand_b<<<g, dim3(32, 8), 0, st>>>((int)K, (int)N, alpha, B, ldb, Bp, (int)K2p, (int)bz0, (int)bz1);
+    k_expand_b<<<g, dim3(32, 8), 0, st>>>((int)K, (int)N, alpha, B, ldb, Bp, (int)K2p, (int)bz0, (int)bz1,
+                                          c.ctr.as<int>());
     MNP_CHECK_LAUNCH();
   }
   auto enc = get_encode(c);
@@ -1015,8 +1252,6 @@ mnpbem_status tc_gemm_c64(TcGemmCtx& c, int64_t M, int64_t N, int64_t K, float2 
   }
   const int64_t MT = cdiv_up(M, pair ? TP_TILE : TC_BM), NT = cdiv_up(N2, pair ? TP_TILE : TC_BN);
   if (MT * NT >= (1ll << 31)) { set_error("tc_gemm_c64: too many tiles"); return MNPBEM_ERR_INVALID_ARG; }
-  MNP_TRY(c.ctr.ensure(sizeof(int)));
-  MNP_CUDA(cudaMemsetAsync(c.ctr.ptr, 0, sizeof(int), st));
   // 2N floats per row that are not a multiple of 16 bytes: vector stores, not TMA
   const bool lsu = c.pair_epi == 1 || (N2 & 3) != 0;
   float* Cf = reinterpret_cast<float*>(C);
@@ -1043,11 +1278,9 @@ mnpbem_status tc_gemm_c64(TcGemmCtx& c, int64_t M, int64_t N, int64_t K, float2 
       return MNPBEM_OK;
     }
     const unsigned grid = (unsigned)std::min<int64_t>(MT * NT, ctas);
-    auto kern = c.stages == 3 ? (lsu ? k_tc_gemm<3, 1, false> : k_tc_gemm<3, 0, false>)
-                              : (lsu ? k_tc_gemm<4, 1, false> : k_tc_gemm<4, 0, false>);
+    auto kern = c.stages == 3 ? (lsu ? k_tc_gemm<3, 1> : k_tc_gemm<3, 0>) : (lsu ? k_tc_gemm<4, 1> : k_tc_gemm<4, 0>);
     kern<<<grid, TC_THREADS, tc_psmem(c.stages == 3 ? 3 : 4), st>>>(ma, mb, mc, mp, Cf, ldcf, (int)M, (int)N2, (int)K2,
-                                                                    acc, c.ctr.as<int>(), c.err.as<int>(), nullptr,
-                                                                    nullptr);
+                                                                    acc, c.ctr.as<int>(), c.err.as<int>());
     MNP_CHECK_LAUNCH();
   }
   return MNPBEM_OK;

@@ -49,6 +49,7 @@ constexpr int Z_STAGE = Z_S * (Z_A_BYTES + Z_B_BYTES);  // 96 KB
 constexpr int Z_ST = 2;
 constexpr int Z_EPI = 8;                                // epilogue warps: two per 32 rows, half of the columns each
 constexpr int Z_CH = 8;                                 // columns per epilogue step
+static_assert(Z_CH == 8 && Z_S == 8, "tmem_ld_levels");
 constexpr int Z_THREADS = 32 * (2 + Z_EPI);
 constexpr int Z_SMEM = Z_ST * Z_STAGE + Z_EPI * 32 * Z_CH * 8 + 1024;
 constexpr uint32_t Z_IDESC = (1u << 4) | ((uint32_t)(Z_BN >> 3) << 17) | ((uint32_t)(Z_BM >> 4) << 24);
@@ -93,7 +94,8 @@ __device__ __forceinline__ void digits(long long v, int (&q)[Z_S]) {
 // A [M][K] -> a8 [S][M][Z_KR] (slice s of row i: digit s of its 2K reals, zero
 // beyond), ea [M].  One warp per row.
 __global__ void __launch_bounds__(256) k_slice_a(const double2* __restrict__ A, int64_t lda, int M, int K,
-                                                 __half* __restrict__ a8, int* __restrict__ ea) {
+                                                 __half* __restrict__ a8, int* __restrict__ ea, int* tile_ctr) {
+  if (blockIdx.x == 0 && threadIdx.x == 0) *tile_ctr = 0;   // of the product that follows
   const int row = blockIdx.x * 8 + (threadIdx.x >> 5), lane = threadIdx.x & 31;
   if (row >= M) return;
   double2 v[2];
@@ -184,10 +186,21 @@ __device__ __forceinline__ double shift_exp(double v, int ex) {
   return __longlong_as_double((b << 1) == 0 ? b : b + ((long long)ex << 52));
 }
 
-__device__ __forceinline__ void tmem_ld8(uint32_t taddr, uint32_t (&r)[8]) {
-  asm volatile("tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
-               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
-               : "r"(taddr));
+// eight columns of four consecutive levels (one asm statement: nothing may touch
+// the registers between the loads and the wait)
+__device__ __forceinline__ void tmem_ld_levels(uint32_t taddr, uint32_t (&a)[4][8]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x8.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%32];\n"
+      " tcgen05.ld.sync.aligned.32x32b.x8.b32 {%8, %9, %10, %11, %12, %13, %14, %15}, [%33];\n"
+      " tcgen05.ld.sync.aligned.32x32b.x8.b32 {%16, %17, %18, %19, %20, %21, %22, %23}, [%34];\n"
+      " tcgen05.ld.sync.aligned.32x32b.x8.b32 {%24, %25, %26, %27, %28, %29, %30, %31}, [%35];\n"
+      " tcgen05.wait::ld.sync.aligned;"
+      : "=r"(a[0][0]), "=r"(a[0][1]), "=r"(a[0][2]), "=r"(a[0][3]), "=r"(a[0][4]), "=r"(a[0][5]), "=r"(a[0][6]), "=r"(a[0][7]),
+        "=r"(a[1][0]), "=r"(a[1][1]), "=r"(a[1][2]), "=r"(a[1][3]), "=r"(a[1][4]), "=r"(a[1][5]), "=r"(a[1][6]), "=r"(a[1][7]),
+        "=r"(a[2][0]), "=r"(a[2][1]), "=r"(a[2][2]), "=r"(a[2][3]), "=r"(a[2][4]), "=r"(a[2][5]), "=r"(a[2][6]), "=r"(a[2][7]),
+        "=r"(a[3][0]), "=r"(a[3][1]), "=r"(a[3][2]), "=r"(a[3][3]), "=r"(a[3][4]), "=r"(a[3][5]), "=r"(a[3][6]), "=r"(a[3][7])
+      : "r"(taddr), "r"(taddr + Z_BN), "r"(taddr + 2 * Z_BN), "r"(taddr + 3 * Z_BN)
+      : "memory");
 }
 // shared-memory matrix descriptor: K-major, 64-byte swizzle, 8-row groups 512 B apart
 __device__ __forceinline__ uint64_t desc_sw64(uint32_t addr) {
@@ -344,11 +357,10 @@ __global__ void __launch_bounds__(Z_THREADS, 1)
             old[i] = (row < M && cc < N) ? C[(long long)row * ldc + cc] : make_double2(0, 0);
           }
         }
-        uint32_t a[Z_S][Z_CH];
-#pragma unroll
-        for (int l = 0; l < Z_S; ++l)
-          tmem_ld8(tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(l * Z_BN + ch * Z_CH), a[l]);
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+        uint32_t ah[4][Z_CH], aw[4][Z_CH];              // levels 0 .. 3 and 4 .. 7
+        const uint32_t ta = tmem + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(ch * Z_CH);
+        tmem_ld_levels(ta, ah);
+        tmem_ld_levels(ta + 4 * Z_BN, aw);
         if (ch == (half + 1) * NCH - 1) {
           // the accumulators have been read: the MMA warp may overwrite them
           tc_fence_before();
@@ -369,8 +381,8 @@ __global__ void __launch_bounds__(Z_THREADS, 1)
             long long h = 0, w = 0;
 #pragma unroll
             for (int l = 0; l < 4; ++l) {
-              h = (h << 8) + (long long)__float2int_rn(__uint_as_float(a[l][c]));
-              w = (w << 8) + (long long)__float2int_rn(__uint_as_float(a[l + 4][c]));
+              h = (h << 8) + (long long)__float2int_rn(__uint_as_float(ah[l][c]));
+              w = (w << 8) + (long long)__float2int_rn(__uint_as_float(aw[l][c]));
             }
             // sum of the levels = (h 2^32 + w) 2^56 units of 2^-124
             val[c] = fixed_to_double(h + (w >> 32), (unsigned)w);
@@ -444,10 +456,9 @@ mnpbem_status tc_gemm_c128(TcGemmCtx& c, int64_t M, int64_t N, int64_t K, double
     MNP_CUDA(cudaMemsetAsync(c.err.ptr, 0, sizeof(int), st));
     c.err_cleared = true;
   }
-  MNP_CUDA(cudaMemsetAsync(c.ctr.ptr, 0, sizeof(int), st));
   {
     ProfScope ps(PH_ELEMWISE, st, 0.0, 16.0 * K * (M + N) + 2.0 * Z_S * Z_KR * (M + 2.0 * N));
-    k_slice_a<<<(unsigned)cdiv_up(M, (int64_t)8), 256, 0, st>>>(A, lda, (int)M, (int)K, a8, ea);
+    k_slice_a<<<(unsigned)cdiv_up(M, (int64_t)8), 256, 0, st>>>(A, lda, (int)M, (int)K, a8, ea, c.ctr.as<int>());
     k_slice_b<<<(unsigned)cdiv_up(N, (int64_t)ZB_COLS), 256, 0, st>>>(B, ldb, (int)K, (int)N, b8, eb);
     MNP_CHECK_LAUNCH();
   }
