@@ -23,7 +23,7 @@ import numpy as np
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 TUNED = os.path.join(_HERE, "data", "tuned.json")
-GRID = {"tc_stages": (3, 4), "gj_block": (256, 512), "lu_steps": (1, 2, 4), "lanes": (2, 4, 6, 8)}
+GRID = {"tc_stages": (3, 4), "gj_block": (256, 512), "lu_steps": (1, 2, 4), "lanes": (2, 4, 6, 8, 12, 16)}
 
 
 def load():

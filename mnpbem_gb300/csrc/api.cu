@@ -21,6 +21,7 @@
 #include <complex>
 #include <functional>
 #include <algorithm>
+#include <atomic>
 #include <memory>
 #include <thread>
 #include <vector>
@@ -121,6 +122,7 @@ struct Lane {
     int precision = -1, P = 0, ninf = 0;
     bool prof = false;
     uint64_t sig = 0;             // addresses of every buffer the graphs captured
+    uint64_t uid = 0;             // of this set of captures, never used again in the process
     cudaGraphExec_t exec[NSTAGES] = {};
     cudaGraph_t graph[NSTAGES] = {};   // the captured stages (child graphs of a sweep graph)
     Profiler::GraphRec rec[NSTAGES];
@@ -191,6 +193,8 @@ struct mnpbem_geom {
   int sweep_err = 0;        // CUDA error that turned them off
   cudaGraphExec_t sweep_exec = nullptr;
   uint64_t sweep_key = 0;
+  cudaGraphExec_t batch_exec = nullptr;   // the last batch whose first handle this is
+  uint64_t batch_key = 0;
   DevBuf sweep_lp, sweep_ctl, sweep_res;   // parameters [nenei], job control, per-wavelength results
 };
 
@@ -527,6 +531,8 @@ mnpbem_status mnpbem_geom_destroy(mnpbem_geom* g) {
   g->prof.flush();
   if (g->sweep_exec) cudaGraphExecDestroy(g->sweep_exec);
   g->sweep_exec = nullptr;
+  if (g->batch_exec) cudaGraphExecDestroy(g->batch_exec);
+  g->batch_exec = nullptr;
   for (auto& L : g->lanes) lane_release(*L);
   g->lanes.clear();
   if (g->lp_ring) cudaFreeHost(g->lp_ring);
@@ -1368,14 +1374,10 @@ mnpbem_status capture_stage(mnpbem_geom* G, Lane& L, const SolveCtx& c, int stag
     return s;
   }
   MNP_CUDA(e);
-  cudaGraphExec_t exec = nullptr;
-  e = cudaGraphInstantiate(&exec, graph, 0);
-  if (e != cudaSuccess) cudaGraphDestroy(graph);
-  MNP_CUDA(e);
   if (gr.exec[stage]) cudaGraphExecDestroy(gr.exec[stage]);
   if (gr.graph[stage]) cudaGraphDestroy(gr.graph[stage]);
   Profiler::release(gr.rec[stage]);
-  gr.exec[stage] = exec;
+  gr.exec[stage] = nullptr;     // instantiated when a host-scheduled sweep launches it
   gr.graph[stage] = graph;
   cap.move_to(gr.rec[stage]);
   return MNPBEM_OK;
@@ -1404,6 +1406,7 @@ bool graphs_match(const mnpbem_geom* G, const Lane& L, const SolveCtx& c) {
 
 mnpbem_status launch_stage(mnpbem_geom* G, Lane& L, const SolveCtx& c, int stage, bool graphs) {
   if (!graphs) return run_stage(G, L, c, stage, true);
+  if (!L.graphs.exec[stage]) MNP_CUDA(cudaGraphInstantiate(&L.graphs.exec[stage], L.graphs.graph[stage], 0));
   MNP_CUDA(cudaGraphLaunch(L.graphs.exec[stage], L.st));
   G->prof.replayed.push_back(&L.graphs.rec[stage]);
   return MNPBEM_OK;
@@ -1787,9 +1790,51 @@ mnpbem_status job_setup(Job& j, const mnpbem_planewave* exc, int32_t nenei, cons
   return MNPBEM_OK;
 }
 
-// lanes without graphs for this configuration run one wavelength directly
-// (sizing every buffer), then capture the stages; without graphs every
-// wavelength runs directly on lane 0
+// the buffers that a lane's stages size as they first run, sized as those of a
+// lane that has run them, so that the stages can be captured without a run
+template <typename R>
+mnpbem_status size_gj(GJWork<R>& d, const GJWork<R>& s) {
+  MNP_TRY(d.ccol.ensure(s.ccol.bytes));
+  MNP_TRY(d.rrow.ensure(s.rrow.bytes));
+  MNP_TRY(d.ncol.ensure(s.ncol.bytes));
+  MNP_TRY(d.xblk.ensure(s.xblk.bytes));
+  MNP_TRY(d.status.ensure(s.status.bytes));
+  MNP_TRY(d.pan.ensure(s.pan.bytes));
+  if (!s.inner) return MNPBEM_OK;
+  if (!d.inner) d.inner.reset(new GJWork<R>());
+  return size_gj(*d.inner, *s.inner);
+}
+template <typename R>
+mnpbem_status size_lu(LDUWork<R>& d, const LDUWork<R>& s) {
+  MNP_TRY(d.ccol.ensure(s.ccol.bytes));
+  MNP_TRY(d.rrow.ensure(s.rrow.bytes));
+  MNP_TRY(d.xblk.ensure(s.xblk.bytes));
+  MNP_TRY(d.tmp.ensure(s.tmp.bytes));
+  return d.pan.ensure(s.pan.bytes);
+}
+mnpbem_status size_like(Lane& d, const Lane& s) {
+  MNP_TRY(size_gj(d.gj32, s.gj32));
+  MNP_TRY(size_gj(d.gj64, s.gj64));
+  MNP_TRY(size_lu(d.lu32, s.lu32));
+  MNP_TRY(size_lu(d.lu64, s.lu64));
+  MNP_TRY(d.tc.bexp.ensure(s.tc.bexp.bytes));
+  MNP_TRY(d.tc.a16.ensure(s.tc.a16.bytes));
+  MNP_TRY(d.tc.scales.ensure(s.tc.scales.bytes));
+  MNP_TRY(d.tc.a8.ensure(s.tc.a8.bytes));
+  MNP_TRY(d.tc.b8.ensure(s.tc.b8.bytes));
+  MNP_TRY(d.tc.exps.ensure(s.tc.exps.bytes));
+  MNP_TRY(d.tc.err.ensure(s.tc.err.bytes));
+  MNP_TRY(d.tc.ctr.ensure(s.tc.ctr.bytes));
+  // the host reads the error word at the end of a call even if the lane ran nothing
+  if (d.tc.err.ptr) MNP_CUDA(cudaMemsetAsync(d.tc.err.ptr, 0, sizeof(int), d.st));
+  tc_device_ready(d.tc);
+  return MNPBEM_OK;
+}
+
+// without graphs for this configuration on any lane, one lane runs a wavelength
+// directly (sizing every buffer); the other lanes take its buffer sizes, and
+// every lane captures the stages; without graphs every wavelength runs directly
+// on lane 0
 mnpbem_status job_prepare(Job& j) {
   mnpbem_geom* G = j.G;
   ProfBind pb_(&G->prof);
@@ -1807,17 +1852,25 @@ mnpbem_status job_prepare(Job& j) {
     return MNPBEM_OK;
   }
   std::vector<int> fresh;
+  const Lane* sized = nullptr;
+  for (int l = 0; l < j.nl && !sized; ++l)
+    if (graphs_match(G, *G->lanes[l], c)) sized = G->lanes[l].get();
   for (int l = 0; l < j.nl && j.next < s.nenei; ++l) {
     Lane& L = *G->lanes[l];
     if (graphs_match(G, L, c)) continue;
     if (L.graphs.valid) drop_graphs(G, L);
-    const int w = j.next++;
-    MNP_TRY(upload_lp(G, L, s, w));
-    L.w = w;
-    MNP_TRY(solve_one(G, L, c, s.ref, false, &L.iters, &L.res));
-    MNP_TRY(write_outputs(G, L, c, s, w));
-    MNP_CUDA(cudaStreamSynchronize(L.st));
-    if (!G->use_graphs) break;
+    if (!sized) {
+      const int w = j.next++;
+      MNP_TRY(upload_lp(G, L, s, w));
+      L.w = w;
+      MNP_TRY(solve_one(G, L, c, s.ref, false, &L.iters, &L.res));
+      MNP_TRY(write_outputs(G, L, c, s, w));
+      MNP_CUDA(cudaStreamSynchronize(L.st));
+      if (!G->use_graphs) break;
+      sized = &L;
+    } else {
+      MNP_TRY(size_like(L, *sized));
+    }
     fresh.push_back(l);
   }
   for (int l : fresh) {
@@ -1835,6 +1888,8 @@ mnpbem_status job_prepare(Job& j) {
       gr.ninf = c.exc->ninf;
       gr.prof = G->prof.enabled;
       gr.sig = lane_sig(G, L);
+      static std::atomic<uint64_t> next_uid{1};
+      gr.uid = next_uid++;
     } else {
       drop_graphs(G, L);
       G->use_graphs = false;   // run directly from now on
@@ -2319,7 +2374,7 @@ mnpbem_status jobs_graph(std::vector<Job*>& jobs) {
     MNP_CUDA(cudaMemsetAsync(G->sweep_res.ptr, 0, G->sweep_res.bytes, G->st));
     MNP_CUDA(cudaStreamSynchronize(G->st));   // jc lives on this stack frame
   }
-  // build (or reuse, for a single job on an unchanged handle) the graph
+  // build the graph, or reuse the kept one on unchanged handles
   Job& j0 = *jobs[0];
   mnpbem_geom* G0 = j0.G;
   uint64_t key = 1469598103934665603ull;
@@ -2338,13 +2393,15 @@ mnpbem_status jobs_graph(std::vector<Job*>& jobs) {
     for (const Lane* L : j.run) {
       mix((uint64_t)(uintptr_t)L);
       mix(L->graphs.sig);
-      for (int s = 0; s < NSTAGES; ++s) mix((uint64_t)(uintptr_t)L->graphs.graph[s]);
+      mix(L->graphs.uid);   // a graph of captures that are gone never matches, whatever reuses their addresses
     }
   }
+  // the first handle keeps the graph of its last single sweep and of its last batch
+  cudaGraphExec_t& kept = jobs.size() == 1 ? G0->sweep_exec : G0->batch_exec;
+  uint64_t& kept_key = jobs.size() == 1 ? G0->sweep_key : G0->batch_key;
   cudaGraphExec_t exec = nullptr;
-  const bool cache = jobs.size() == 1;
-  if (cache && G0->sweep_exec && G0->sweep_key == key) {
-    exec = G0->sweep_exec;
+  if (kept && kept_key == key) {
+    exec = kept;
   } else {
     GraphBuild gb;
     cudaError_t e = cudaGraphCreate(&gb.top, 0);
@@ -2362,11 +2419,9 @@ mnpbem_status jobs_graph(std::vector<Job*>& jobs) {
       }
       return MNPBEM_ERR_UNSUPPORTED;
     }
-    if (cache) {
-      if (G0->sweep_exec) cudaGraphExecDestroy(G0->sweep_exec);
-      G0->sweep_exec = exec;
-      G0->sweep_key = key;
-    }
+    if (kept) cudaGraphExecDestroy(kept);
+    kept = exec;
+    kept_key = key;
   }
   // every lane's stream has finished its earlier work; the graph runs on the
   // first handle's stream after all of them
@@ -2380,7 +2435,6 @@ mnpbem_status jobs_graph(std::vector<Job*>& jobs) {
     }
   const cudaError_t le = cudaGraphLaunch(exec, G0->st);
   const cudaError_t se = le == cudaSuccess ? cudaStreamSynchronize(G0->st) : le;
-  if (!cache) cudaGraphExecDestroy(exec);
   MNP_CUDA(se);
   for (size_t q = 0; q < jobs.size(); ++q) {
     jobs[q]->next = jobs[q]->s.nenei;

@@ -102,3 +102,29 @@ def test_sweep_graph_page_locked_outputs():
     assert bem.stat("sweep_graph_runs") > 0
     for k in ("ext", "sca", "sig2", "h2"):
         assert np.array_equal(np.asarray(got[k]).reshape(ref[k].shape), ref[k]), k
+
+
+@pytest.mark.parametrize("faces,precision,nw", [(116, "mixed", 3), (116, "fp64", 3), (232, "mixed", 5), (300, "mixed", 2)])
+def test_lanes_captured_without_a_run(gpu_lib, faces, precision, nw):
+    """A first sweep on more lanes than wavelengths are left for the graph (one
+    lane runs directly, the others are captured and some never run), a second
+    one, and a batch on the same handles twice: all as a one-lane solver's."""
+    def solver(lanes):
+        cp = m.comparticle([m.epsconst(1.77), drude()], [m.particle(*shapes.fibsphere(faces, 20.0))], [[2, 1]], 1)
+        return m.bemsolver(cp, m.bemoptions(precision=precision, lanes=lanes))
+    exc = m.planewave([[1, 0, 0]], [[0, 0, 1]])
+    enei = np.linspace(480.0, 620.0, nw)
+    want = solver(1).spectrum(exc, enei, fields=True)
+    a, b = solver(16), solver(16)
+    for _ in range(2):
+        got = a.spectrum(exc, enei, fields=True)
+        for k in ("ext", "sca", "sig1", "sig2", "h1", "h2"):
+            assert np.array_equal(got[k], want[k]), k
+    for _ in range(2):
+        for r in m.spectrum_batch([(a, exc, enei), (b, exc, enei)]):
+            assert np.array_equal(r["ext"], want["ext"]) and np.array_equal(r["sca"], want["sca"])
+    del b                                   # the first handle still keeps the batch's graph
+    assert np.array_equal(a.spectrum(exc, enei)["ext"], want["ext"])
+    c = solver(16)
+    for r in m.spectrum_batch([(a, exc, enei), (c, exc, enei)]):
+        assert np.array_equal(r["ext"], want["ext"])
