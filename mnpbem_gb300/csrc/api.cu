@@ -1170,7 +1170,7 @@ mnpbem_status stage_initmat(mnpbem_geom* G, Lane& L, bool direct) {
     }
   }
   if (direct && ctx) MNP_TRY(tc_check_error(L.tc, L.st));
-  if (direct) MNP_TRY(thin_stream_check(L.st));
+  if (direct) MNP_TRY(sweep_check(L.st));
   return MNPBEM_OK;
 }
 
@@ -2469,7 +2469,7 @@ mnpbem_status job_finish(Job& j, bool failed) {
     MNP_TRY(check_pivots(L, j.c.precision));
     if (j.c.precision == MNPBEM_MIXED && G->tc_enabled) MNP_TRY(tc_check_error(L.tc, L.st));
   }
-  MNP_TRY(thin_stream_check(G->st));
+  MNP_TRY(sweep_check(G->st));
   return MNPBEM_OK;
 }
 
@@ -2794,7 +2794,7 @@ mnpbem_status mnpbem_cross_section_gradient(mnpbem_geom* G, const mnpbem_planewa
       MNP_CHECK_LAUNCH();
     }
     MNP_TRY(tc_check_error(L.tc, st));
-    MNP_TRY(thin_stream_check(st));
+    MNP_TRY(sweep_check(st));
   }
   // ---- weights, then G1 [sig1 h1], G2 [sig2 h2], H1 sig1 from freshly assembled FP64 matrices
   adj_weights(p, gphi, ga, gDe, gAl, vv.x1, vv.x2, P, ipol, st);

@@ -143,81 +143,138 @@ __global__ void __launch_bounds__(32 * THIN_WARPS) k_gemm_thin(int64_t M, int64_
   }
 }
 
-// complex64 variant with 16-byte loads: each lane takes two consecutive k
-// (one float4 of A per row, two rows of B), halving the load instructions of
-// the matrix stream.  Needs lda even and A 16-byte aligned; an odd K leaves
-// one k that warp 0 adds at the end.
-template <int N, int TR>
-__global__ void __launch_bounds__(32 * THIN_WARPS) k_gemm_thin_c64(int64_t M, int64_t K, float2 alpha,
-                                                                 const float2* __restrict__ A, int64_t lda,
-                                                                 const float2* __restrict__ B, int64_t ldb,
-                                                                 float2 beta, float2* __restrict__ C,
-                                                                 int64_t ldc) {
-  __shared__ float2 red[THIN_WARPS][TR][N];
+// complex64 products with few columns (N <= 8): C (complex64) = alpha A B + beta C
+// (MODE 0), or C (complex128) = A B (MODE 1).  Bound by HBM on A (at 4000 rows and
+// more far larger than what the caches keep between products).  A CTA of eight
+// warps owns 8 RW rows over all of K; B comes in chunks of 512 or 256 rows through
+// shared memory (transposed, so that a lane reads its two neighbouring k as one
+// 16-byte word per column), the next chunk's entries being loaded while this one
+// is used; a lane keeps 4 x RW 16-byte loads of A in flight, two CTAs per SM.  The
+// order of every sum is fixed.  Needs an even lda and a 16-byte aligned A; an odd K
+// leaves one k to lane 0.  The kernels it replaces read B through L1 per element
+// (register tiles: 1.85 TB/s at 12 000 rows) or waited on it per chunk (rows
+// streamed by bulk copies: 3.2 TB/s at 24 000); this one reaches 6.1 TB/s at 24 000
+// rows, 5.1 at 12 000 and 3.3 at 4000.
+constexpr int TV_WARPS = 8;
+template <int N, int RW, int MODE>
+__global__ void __launch_bounds__(32 * TV_WARPS, 2) k_gemm_thin_c64(int64_t M, int64_t K, float2 alpha,
+                                                                  const float2* __restrict__ A, int64_t lda,
+                                                                  const float2* __restrict__ B, int64_t ldb,
+                                                                  float2 beta, void* __restrict__ Cv, int64_t ldc) {
+  constexpr int TV_KC = N <= 4 ? 512 : 256;            // k per chunk
+  __shared__ __align__(16) float2 xs[N][TV_KC + 4];
+  constexpr int NE = TV_KC * N / (32 * TV_WARPS);      // entries of a chunk of B per thread
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t row0 = (int64_t)blockIdx.x * TR;
-  const int64_t KP = K >> 1;   // pairs
-  const int64_t kw = (KP + THIN_WARPS - 1) / THIN_WARPS;
-  const int64_t pbeg = warp * kw, pend = min(KP, pbeg + kw);
-  const float2* arow[TR];
+  const int64_t row0 = ((int64_t)blockIdx.x * TV_WARPS + warp) * RW;
+  const float2* arow[RW];
 #pragma unroll
-  for (int r = 0; r < TR; ++r) arow[r] = A + min(row0 + r, M - 1) * lda;
-  float2 acc[TR][N];
+  for (int r = 0; r < RW; ++r) arow[r] = A + min(row0 + r, M - 1) * lda;
+  float2 acc[RW][N];
 #pragma unroll
-  for (int r = 0; r < TR; ++r)
+  for (int r = 0; r < RW; ++r)
 #pragma unroll
     for (int c = 0; c < N; ++c) acc[r][c] = make_float2(0.f, 0.f);
-#pragma unroll 2
-  for (int64_t kp = pbeg + lane; kp < pend; kp += 32) {
-    const int64_t k = 2 * kp;
-    float2 b0[N], b1[N];
+  const int64_t Ke = K & ~(int64_t)1;                  // even part
+  float2 nb[NE];
+  const auto fetch = [&](int64_t k0) {
 #pragma unroll
-    for (int c = 0; c < N; ++c) {
-      b0[c] = __ldg(B + k * ldb + c);
-      b1[c] = __ldg(B + (k + 1) * ldb + c);
+    for (int q = 0; q < NE; ++q) {
+      const int e = threadIdx.x + 32 * TV_WARPS * q;
+      const int64_t k = k0 + e / N;
+      nb[q] = k < Ke ? __ldg(B + k * ldb + e % N) : make_float2(0.f, 0.f);
     }
+  };
+  fetch(0);
+  for (int64_t k0 = 0; k0 < Ke; k0 += TV_KC) {
+    __syncthreads();
 #pragma unroll
-    for (int r = 0; r < TR; ++r) {
-      const float4 a = __ldg(reinterpret_cast<const float4*>(arow[r] + k));
-      const float2 a0 = make_float2(a.x, a.y), a1 = make_float2(a.z, a.w);
+    for (int q = 0; q < NE; ++q) {
+      const int e = threadIdx.x + 32 * TV_WARPS * q;
+      xs[e % N][e / N] = nb[q];
+    }
+    __syncthreads();
+    if (k0 + TV_KC < Ke) fetch(k0 + TV_KC);
 #pragma unroll
-      for (int c = 0; c < N; ++c) {
-        cfma(acc[r][c], a0, b0[c]);
-        cfma(acc[r][c], a1, b1[c]);
+    for (int h = 0; h < TV_KC / 256; ++h) {            // 256 k at a time: four 16-byte loads per row
+      float4 a[4][RW];
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int64_t k = k0 + 256 * h + 64 * u + 2 * lane;
+#pragma unroll
+        for (int r = 0; r < RW; ++r)
+          a[u][r] = k < Ke ? __ldg(reinterpret_cast<const float4*>(arow[r] + k)) : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u) {
+        const int kk = 256 * h + 64 * u + 2 * lane;
+#pragma unroll
+        for (int c = 0; c < N; ++c) {
+          const float4 b = *reinterpret_cast<const float4*>(&xs[c][kk]);
+#pragma unroll
+          for (int r = 0; r < RW; ++r) {
+            cfma(acc[r][c], make_float2(a[u][r].x, a[u][r].y), make_float2(b.x, b.y));
+            cfma(acc[r][c], make_float2(a[u][r].z, a[u][r].w), make_float2(b.z, b.w));
+          }
+        }
       }
     }
   }
-  if ((K & 1) && warp == 0 && lane == 0) {
-    const int64_t k = K - 1;
+  if ((K & 1) && lane == 0) {
 #pragma unroll
-    for (int r = 0; r < TR; ++r)
+    for (int r = 0; r < RW; ++r)
 #pragma unroll
-      for (int c = 0; c < N; ++c) cfma(acc[r][c], arow[r][k], B[k * ldb + c]);
+      for (int c = 0; c < N; ++c) cfma(acc[r][c], arow[r][K - 1], B[(K - 1) * ldb + c]);
   }
+  const bool zero_beta = (beta.x == 0 && beta.y == 0);
 #pragma unroll
-  for (int r = 0; r < TR; ++r)
+  for (int r = 0; r < RW; ++r)
 #pragma unroll
     for (int c = 0; c < N; ++c) {
       float2 v = acc[r][c];
+#pragma unroll
       for (int o = 16; o; o >>= 1) {
         v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
         v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
       }
-      if (lane == 0) red[warp][r][c] = v;
+      const int64_t row = row0 + r;
+      if (lane == (r * N + c) % 32 && row < M) {
+        if (MODE == 0) {
+          float2* C = reinterpret_cast<float2*>(Cv);
+          float2 out = cmul(alpha, v);
+          if (!zero_beta) out = cadd(out, cmul(beta, C[row * ldc + c]));
+          C[row * ldc + c] = out;
+        } else {
+          reinterpret_cast<double2*>(Cv)[row * ldc + c] = make_double2(v.x, v.y);
+        }
+      }
     }
-  __syncthreads();
-  const bool zero_beta = (beta.x == 0 && beta.y == 0);
-  for (int t = threadIdx.x; t < TR * N; t += blockDim.x) {
-    const int r = t / N, c = t % N;
-    const int64_t row = row0 + r;
-    if (row >= M) continue;
-    float2 v = make_float2(0.f, 0.f);
-#pragma unroll
-    for (int w = 0; w < THIN_WARPS; ++w) v = cadd(v, red[w][r][c]);
-    float2 out = cmul(alpha, v);
-    if (!zero_beta) out = cadd(out, cmul(beta, C[row * ldc + c]));
-    C[row * ldc + c] = out;
+}
+
+template <int MODE>
+static mnpbem_status launch_thin_c64(int64_t M, int64_t N, int64_t K, const float2* A, int64_t lda, const float2* B,
+                                     int64_t ldb, float2 alpha, float2 beta, void* C, int64_t ldc, cudaStream_t st) {
+  // rows per warp: four with up to three columns, two beyond (the sums and the
+  // loads in flight fill the registers: N = 4 at 24 000 rows 6.1 TB/s with two,
+  // 4.9 with four); fewer where the rows would not give every SM two CTAs
+#define TV_CASE(NN, RW)                                                                                              \
+  k_gemm_thin_c64<NN, RW, MODE><<<(unsigned)cdiv_up(M, (int64_t)(TV_WARPS * RW)), 32 * TV_WARPS, 0, st>>>(           \
+      M, K, alpha, A, lda, B, ldb, beta, C, ldc)
+#define TV_N(NN, RW)                                     \
+  case NN:                                               \
+    if (M >= 2 * 152 * TV_WARPS * RW) TV_CASE(NN, RW);   \
+    else if (M >= 152 * TV_WARPS * 2) TV_CASE(NN, 2);    \
+    else TV_CASE(NN, 1);                                 \
+    break;
+  switch (N) {
+    TV_N(1, 4) TV_N(2, 4) TV_N(3, 4) TV_N(4, 2) TV_N(5, 2) TV_N(6, 2) TV_N(7, 2) TV_N(8, 2)
+    default:
+      set_error("thin product: N must be 1..8");
+      return MNPBEM_ERR_INVALID_ARG;
   }
+#undef TV_N
+#undef TV_CASE
+  MNP_CHECK_LAUNCH();
+  return MNPBEM_OK;
 }
 
 // ------------------------------------------- double-single thin GEMM (N <= 16)
@@ -357,228 +414,9 @@ __global__ void __launch_bounds__(32 * DS_WARPS) k_gemm_thin_hi(int64_t M, int64
   }
 }
 
-// the same product with 16-byte loads of A (two k per lane and load): even K
-// and lda, 16-byte aligned A; the FP32 residual products of the refinement at
-// large n, where the 8-byte loads above leave HBM half used
-template <int N>
-__global__ void __launch_bounds__(32 * DS_WARPS) k_gemm_thin_hi4(int64_t M, int64_t K, const float2* __restrict__ Ahi,
-                                                               int64_t lda, const float2* __restrict__ Bh, int64_t ldb,
-                                                               double2* __restrict__ C, int64_t ldc) {
-  __shared__ float2 red[DS_WARPS][DS_TR][N];
-  const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  const int64_t row0 = (int64_t)blockIdx.x * DS_TR;
-  const int64_t KP = K >> 1;
-  const int64_t kw = (KP + DS_WARPS - 1) / DS_WARPS;
-  const int64_t pbeg = warp * kw, pend = min(KP, pbeg + kw);
-  const float4* arow[DS_TR];
-#pragma unroll
-  for (int r = 0; r < DS_TR; ++r) arow[r] = reinterpret_cast<const float4*>(Ahi + min(row0 + r, M - 1) * lda);
-  float2 acc[DS_TR][N];
-#pragma unroll
-  for (int r = 0; r < DS_TR; ++r)
-#pragma unroll
-    for (int c = 0; c < N; ++c) acc[r][c] = make_float2(0.f, 0.f);
-#pragma unroll 2
-  for (int64_t kp = pbeg + lane; kp < pend; kp += 32) {
-    const int64_t k = 2 * kp;
-    float2 x0[N], x1[N];
-#pragma unroll
-    for (int c = 0; c < N; ++c) {
-      x0[c] = __ldg(Bh + k * ldb + c);
-      x1[c] = __ldg(Bh + (k + 1) * ldb + c);
-    }
-    float4 a[DS_TR];
-#pragma unroll
-    for (int r = 0; r < DS_TR; ++r) a[r] = __ldg(arow[r] + kp);
-#pragma unroll
-    for (int r = 0; r < DS_TR; ++r) {
-      const float2 a0 = make_float2(a[r].x, a[r].y), a1 = make_float2(a[r].z, a[r].w);
-#pragma unroll
-      for (int c = 0; c < N; ++c) {
-        cfma(acc[r][c], a0, x0[c]);
-        cfma(acc[r][c], a1, x1[c]);
-      }
-    }
-  }
-#pragma unroll
-  for (int r = 0; r < DS_TR; ++r)
-#pragma unroll
-    for (int c = 0; c < N; ++c) {
-      float2 v = acc[r][c];
-      for (int o = 16; o; o >>= 1) {
-        v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
-        v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
-      }
-      if (lane == 0) red[warp][r][c] = v;
-    }
-  __syncthreads();
-  for (int t = threadIdx.x; t < DS_TR * N; t += blockDim.x) {
-    const int r = t / N, c = t % N;
-    const int64_t row = row0 + r;
-    if (row >= M) continue;
-    float2 v = make_float2(0.f, 0.f);
-#pragma unroll
-    for (int w = 0; w < DS_WARPS; ++w) v = cadd(v, red[w][r][c]);
-    C[row * ldc + c] = make_double2(v.x, v.y);
-  }
-}
+__device__ int g_sweep_err;   // a bounded wait of the triangular sweeps expired
 
-// ------------------------------------------- streamed thin GEMM (bulk copies)
-// C[M x N] = A[M x K] * B[K x N], N <= 4, for a complex64 A far larger than
-// L2 (the chain products and FP32 residuals of the refinement read a whole
-// n x n matrix for a few right-hand sides: pure HBM streaming).  One CTA per
-// SM owns a contiguous, balanced share of the rows.  A producer warp streams
-// row segments of TS_KC complex values with bulk copies (cp.async.bulk: long
-// sequential requests, TS_ST stages in flight) into shared memory; eight
-// consumer warps take the chunk's k range in parallel (lane = k), read B
-// through L1 and accumulate TS_TR rows x N in registers; at the end of a row
-// block the warps' partial sums are added in a fixed order (deterministic).
-// Sixteen consumer warps: TS_KG k groups x TS_RG row groups (TS_RPW rows each),
-// so that each warp keeps few accumulators and each scheduler has four warps
-// to hide the L1 / shared-memory latencies (eight warps with all rows each
-// were latency bound: 29 % issue, 32 % of HBM).
-// Waits are bounded; after a timeout every role skips the remaining waits
-// (the result is then garbage and the error word is set) so that no barrier
-// is left waiting.
-constexpr int TS_TR = 8, TS_KC = 512, TS_ST = 4, TS_RG = 2, TS_KG = 8, TS_CW = TS_RG * TS_KG, TS_RPW = TS_TR / TS_RG;
-constexpr int TS_THREADS = 32 * (TS_CW + 1);
-constexpr int TS_STAGE = TS_TR * TS_KC * 8;               // 32 KB
-constexpr int TS_SMEM = TS_ST * TS_STAGE;
-__device__ int g_thin_stream_err;
-
-__device__ __forceinline__ void bulk_copy_g2s(uint32_t dst, const void* src, uint32_t bytes, uint32_t bar) {
-  asm volatile("cp.async.bulk.shared::cluster.global.mbarrier::complete_tx::bytes [%0], [%1], %2, [%3];"
-               ::"r"(dst), "l"(src), "r"(bytes), "r"(bar)
-               : "memory");
-}
-__device__ __forceinline__ void consumer_sync() {
-  asm volatile("bar.sync 1, %0;" ::"n"(32 * TS_CW) : "memory");
-}
-
-// MODE 0: C (complex64) = alpha A B + beta C;  MODE 1: C (complex128) = A B
-template <int N, int MODE>
-__global__ void __launch_bounds__(TS_THREADS, 1)
-    k_gemm_thin_stream(int64_t M, int64_t K, const float2* __restrict__ A, int64_t lda, const float2* __restrict__ B,
-                       int64_t ldb, float2 alpha, float2 beta, void* __restrict__ Cv, int64_t ldc) {
-  extern __shared__ __align__(128) unsigned char ts_smem[];
-  __shared__ __align__(8) unsigned long long bars[2 * TS_ST];
-  __shared__ float2 red[TS_KG][TS_TR][N];
-  __shared__ int abort_flag;
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int64_t rb = M * blockIdx.x / gridDim.x, re = M * (blockIdx.x + 1) / gridDim.x;
-  const int64_t nchunk = (K + TS_KC - 1) / TS_KC;
-  const uint32_t full0 = smem_u32(&bars[0]), empty0 = smem_u32(&bars[TS_ST]);
-  const uint32_t sbase = smem_u32(ts_smem);
-  int* err = &g_thin_stream_err;
-  volatile int* abort_v = &abort_flag;
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < TS_ST; ++s) {
-      mbar_init(full0 + 8 * s, 1);
-      mbar_init(empty0 + 8 * s, TS_CW);
-    }
-    abort_flag = 0;
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-  }
-  __syncthreads();
-  if (warp == TS_CW) {
-    // ---------------- producer: row segments of the CTA's rows, block by block
-    if (lane == 0) {
-      int it = 0;
-      for (int64_t r0 = rb; r0 < re && !*abort_v; r0 += TS_TR) {
-        const int nr = (int)min((int64_t)TS_TR, re - r0);
-        for (int64_t ch = 0; ch < nchunk; ++ch, ++it) {
-          const int s = it % TS_ST;
-          if (it >= TS_ST && !*abort_v && !mbar_wait(empty0 + 8 * s, ((it / TS_ST) - 1) & 1, err, 1)) *abort_v = 1;
-          if (*abort_v) break;
-          const int64_t k0 = ch * TS_KC;
-          const uint32_t bytes = (uint32_t)min((int64_t)TS_KC, K - k0) * 8u;
-          mbar_expect_tx(full0 + 8 * s, bytes * (uint32_t)nr);
-          for (int r = 0; r < nr; ++r)
-            bulk_copy_g2s(sbase + (uint32_t)(s * TS_STAGE + r * TS_KC * 8), A + (r0 + r) * lda + k0, bytes,
-                          full0 + 8 * s);
-        }
-      }
-      if (*abort_v) {
-        // copies may still be landing: give them time before the CTA exits
-        const unsigned long long t0 = gtimer();
-        while (gtimer() - t0 < 200000ull) {
-        }
-      }
-    }
-  } else {
-    // ---------------- consumers
-    const float2* As = reinterpret_cast<const float2*>(ts_smem);
-    const int rg = warp / TS_KG, kg = warp % TS_KG;
-    int it = 0;
-    for (int64_t r0 = rb; r0 < re; r0 += TS_TR) {
-      const int nr = (int)min((int64_t)TS_TR, re - r0);
-      const int nrw = max(0, min(TS_RPW, nr - rg * TS_RPW));   // this warp's rows in the block
-      float2 acc[TS_RPW][N];
-#pragma unroll
-      for (int r = 0; r < TS_RPW; ++r)
-#pragma unroll
-        for (int c = 0; c < N; ++c) acc[r][c] = make_float2(0.f, 0.f);
-      for (int64_t ch = 0; ch < nchunk; ++ch, ++it) {
-        const int s = it % TS_ST;
-        if (!*abort_v && !mbar_wait(full0 + 8 * s, (it / TS_ST) & 1, err, 2)) *abort_v = 1;
-        const int64_t k0 = ch * TS_KC;
-        const int kl = (int)min((int64_t)TS_KC, K - k0);
-        const float2* Ast = As + s * (TS_TR * TS_KC) + rg * TS_RPW * TS_KC;
-#pragma unroll
-        for (int j = 0; j < TS_KC / (32 * TS_KG); ++j) {
-          const int kk = kg * (TS_KC / TS_KG) + 32 * j + lane;
-          if (kk < kl) {
-            float2 b[N];
-#pragma unroll
-            for (int c = 0; c < N; ++c) b[c] = __ldg(B + (k0 + kk) * ldb + c);
-#pragma unroll
-            for (int r = 0; r < TS_RPW; ++r) {
-              if (r < nrw) {
-                const float2 a = Ast[r * TS_KC + kk];
-#pragma unroll
-                for (int c = 0; c < N; ++c) cfma(acc[r][c], a, b[c]);
-              }
-            }
-          }
-        }
-        __syncwarp();
-        if (lane == 0) mbar_arrive(empty0 + 8 * s);
-      }
-#pragma unroll
-      for (int r = 0; r < TS_RPW; ++r)
-#pragma unroll
-        for (int c = 0; c < N; ++c) {
-          float2 v = acc[r][c];
-#pragma unroll
-          for (int o = 16; o; o >>= 1) {
-            v.x += __shfl_xor_sync(0xffffffffu, v.x, o);
-            v.y += __shfl_xor_sync(0xffffffffu, v.y, o);
-          }
-          if (lane == 0) red[kg][rg * TS_RPW + r][c] = v;
-        }
-      consumer_sync();
-      for (int t = threadIdx.x; t < nr * N; t += 32 * TS_CW) {
-        const int r = t / N, c = t % N;
-        float2 v = make_float2(0.f, 0.f);
-#pragma unroll
-        for (int w = 0; w < TS_KG; ++w) v = cadd(v, red[w][r][c]);
-        const int64_t row = r0 + r;
-        if (MODE == 0) {
-          float2* C = reinterpret_cast<float2*>(Cv);
-          float2 out = cmul(alpha, v);
-          if (beta.x != 0.f || beta.y != 0.f) out = cadd(out, cmul(beta, C[row * ldc + c]));
-          C[row * ldc + c] = out;
-        } else {
-          reinterpret_cast<double2*>(Cv)[row * ldc + c] = make_double2(v.x, v.y);
-        }
-      }
-      consumer_sync();
-    }
-  }
-  __syncthreads();
-}
-
-static int stream_sms() {
+static int num_sms() {
   static int sms = 0;
   if (!sms) {
     int dev = 0;
@@ -591,58 +429,15 @@ static int stream_sms() {
   return sms;
 }
 
-// the streamed kernel applies: N <= 4, even K and lda (16-byte row segments),
-// a 16-byte aligned A, and a matrix of at least 2^22 entries.  Measured on
-// GB300 (standalone, complex64): equal to the register-tiled kernel for N = 1,
-// faster for N = 3 at n = 4000 (44 against 61 us), slower for N = 4 at
-// n = 12000 (417 against 305 us); inside the multi-lane sweep at n = 4000 it
-// shortens the thin-product phase by 15 %.  N = 4 uses it up to 2^26 entries.
-static bool thin_stream_ok(int64_t M, int64_t N, int64_t K, const void* A, int64_t lda) {
-  static int enabled = -1;
-  if (enabled < 0) {
-    const char* e = getenv("MNPBEM_THIN_STREAM");
-    enabled = (e && e[0] == '0') ? 0 : 1;
-  }
-  const int64_t mk = M * K;
-  return enabled && N >= 1 && N <= 4 && !(K & 1) && !(lda & 1) && !(reinterpret_cast<uintptr_t>(A) & 15) &&
-         mk >= (int64_t(1) << 22) && (N <= 3 || mk <= (int64_t(1) << 26));
-}
-
-template <int MODE>
-static mnpbem_status launch_thin_stream(int64_t M, int64_t N, int64_t K, const float2* A, int64_t lda,
-                                        const float2* B, int64_t ldb, float2 alpha, float2 beta, void* C,
-                                        int64_t ldc, cudaStream_t st) {
-  static bool attr[2][5] = {};
-  const unsigned grid = (unsigned)std::min<int64_t>(M, stream_sms());
-#define TS_CASE(NN)                                                                                       \
-  case NN:                                                                                                \
-    if (!attr[MODE][NN]) {                                                                                \
-      MNP_CUDA(cudaFuncSetAttribute(k_gemm_thin_stream<NN, MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize, \
-                                    TS_SMEM));                                                            \
-      attr[MODE][NN] = true;                                                                              \
-    }                                                                                                     \
-    k_gemm_thin_stream<NN, MODE><<<grid, TS_THREADS, TS_SMEM, st>>>(M, K, A, lda, B, ldb, alpha, beta, C, ldc); \
-    break;
-  switch (N) {
-    TS_CASE(1) TS_CASE(2) TS_CASE(3) TS_CASE(4)
-    default:
-      set_error("thin stream GEMM: N must be 1..4");
-      return MNPBEM_ERR_INVALID_ARG;
-  }
-#undef TS_CASE
-  MNP_CHECK_LAUNCH();
-  return MNPBEM_OK;
-}
-
-mnpbem_status thin_stream_check(cudaStream_t st) {
+mnpbem_status sweep_check(cudaStream_t st) {
   int* p = nullptr;
-  MNP_CUDA(cudaGetSymbolAddress(reinterpret_cast<void**>(&p), g_thin_stream_err));
+  MNP_CUDA(cudaGetSymbolAddress(reinterpret_cast<void**>(&p), g_sweep_err));
   int h = 0;
   MNP_CUDA(cudaMemcpyAsync(&h, p, sizeof(int), cudaMemcpyDeviceToHost, st));
   MNP_CUDA(cudaStreamSynchronize(st));
   if (h) {
     MNP_CUDA(cudaMemsetAsync(p, 0, sizeof(int), st));
-    set_error("streamed thin GEMM: a bounded pipeline wait expired (code %d)", h);
+    set_error("triangular sweep: a bounded wait expired (code %d)", h);
     return MNPBEM_ERR_TIMEOUT;
   }
   return MNPBEM_OK;
@@ -676,13 +471,11 @@ static mnpbem_status gemm_thin_ds_block(int64_t M, int64_t N, int64_t K, const f
   const unsigned nblk = (unsigned)cdiv_up(M, (int64_t)DS_TR);
   if (!Alo) {
     ProfScope ps(PH_GEMM_SMALL, st, 8.0 * M * N * K, 8.0 * M * K + 8.0 * K * N + 16.0 * M * N);
-    if (thin_stream_ok(M, N, K, Ahi, lda))
-      return launch_thin_stream<1>(M, N, K, Ahi, lda, Bh, N, make_float2(1.f, 0.f), make_float2(0.f, 0.f), C, ldc, st);
-    const bool v4 = !(K & 1) && !(lda & 1) && !(reinterpret_cast<uintptr_t>(Ahi) & 15);
+    if (!(lda & 1) && !(reinterpret_cast<uintptr_t>(Ahi) & 15))
+      return launch_thin_c64<1>(M, N, K, Ahi, lda, Bh, N, make_float2(1.f, 0.f), make_float2(0.f, 0.f), C, ldc, st);
 #define HI_CASE(NN)                                                                                \
   case NN:                                                                                         \
-    if (v4) k_gemm_thin_hi4<NN><<<nblk, 32 * DS_WARPS, 0, st>>>(M, K, Ahi, lda, Bh, N, C, ldc);    \
-    else k_gemm_thin_hi<NN><<<nblk, 32 * DS_WARPS, 0, st>>>(M, K, Ahi, lda, Bh, N, C, ldc);        \
+    k_gemm_thin_hi<NN><<<nblk, 32 * DS_WARPS, 0, st>>>(M, K, Ahi, lda, Bh, N, C, ldc);        \
     break;
     switch (N) {
       HI_CASE(1) HI_CASE(2) HI_CASE(3) HI_CASE(4) HI_CASE(5) HI_CASE(6) HI_CASE(7) HI_CASE(8)
@@ -733,18 +526,7 @@ mnpbem_status gemm_simt(int64_t M, int64_t N, int64_t K, cplx<R> alpha, const cp
     const float2* Bf = reinterpret_cast<const float2*>(B);
     float2* Cf = reinterpret_cast<float2*>(C);
     const float2 al = make_float2((float)alpha.x, (float)alpha.y), be = make_float2((float)beta.x, (float)beta.y);
-    if (N <= 4 && thin_stream_ok(M, N, K, Af, lda))
-      return launch_thin_stream<0>(M, N, K, Af, lda, Bf, ldb, al, be, Cf, ldc, st);
-#define C64_CASE(NN)                                                                                    \
-  case NN:                                                                                              \
-    k_gemm_thin_c64<NN, 4><<<(unsigned)cdiv_up(M, 4), 32 * THIN_WARPS, 0, st>>>(M, K, al, Af, lda, Bf, ldb, be, Cf, ldc); \
-    break;
-    switch (N) {
-      C64_CASE(1) C64_CASE(2) C64_CASE(3) C64_CASE(4) C64_CASE(5) C64_CASE(6) C64_CASE(7) C64_CASE(8)
-    }
-#undef C64_CASE
-    MNP_CHECK_LAUNCH();
-    return MNPBEM_OK;
+    return launch_thin_c64<0>(M, N, K, Af, lda, Bf, ldb, al, be, Cf, ldc, st);
   }
   if (N <= THIN_NMAX && K > 0) {
     ProfScope ps(PH_GEMM_SMALL, st, 8.0 * M * N * K,
@@ -1745,8 +1527,8 @@ mnpbem_status ldu_rsolve(cplx<R>* H, int64_t n, int64_t ldh, const cplx<R>* F, i
 // Blocks complete in order, so one counter of finished slices per system says
 // how many are ready.  A thread's entries of the next block are loaded as those
 // of this one are used; they do not depend on the wait.
-// The waits are bounded by wall clock: on expiry the error word of the streamed
-// thin products is set, an abort word releases the other CTAs, and all return.
+// The waits are bounded by wall clock: on expiry an error word is set, an abort
+// word releases the other CTAs, and all return.
 // Bound by the chain of block rows (about 3 us each) at a few thousand rows and by
 // HBM at 24 000 (800 us for 2.3 GB).  Against the cooperative sweep before it (a
 // grid barrier per block row), with eight wavelengths of 4000 faces in flight:
@@ -1824,7 +1606,7 @@ __global__ void __launch_bounds__(SWEEP_THREADS, 2) k_ldu_sweep(const __grid_con
             if (v >= (unsigned)need) break;
             if (*abortw) { v = 0; break; }
             if (gtimer() - t0 > MBAR_WAIT_NS) {
-              atomicOr(&g_thin_stream_err, 64);
+              atomicOr(&g_sweep_err, 64);
               *abortw = 1u;
               v = 0;
               break;
@@ -1910,7 +1692,7 @@ static mnpbem_status launch_sweep(SweepArgs<R> a, int maxblk, cudaStream_t st) {
   double half = 0.0;
   for (int q = 0; q < a.nprob; ++q) half += 0.5 * (double)a.p[q].n * a.p[q].n;
   ProfScope ps(PH_GEMM_SMALL, st, 8.0 * half * a.N, (double)sizeof(cplx<R>) * half);
-  kern<<<(unsigned)std::min(a.items, per_sm * stream_sms()), SWEEP_THREADS, smem, st>>>(a);
+  kern<<<(unsigned)std::min(a.items, per_sm * num_sms()), SWEEP_THREADS, smem, st>>>(a);
   MNP_CHECK_LAUNCH();
   return MNPBEM_OK;
 }
