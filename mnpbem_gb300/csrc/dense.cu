@@ -150,11 +150,14 @@ __global__ void __launch_bounds__(32 * THIN_WARPS) k_gemm_thin(int64_t M, int64_
 // shared memory (transposed, so that a lane reads its two neighbouring k as one
 // 16-byte word per column), the next chunk's entries being loaded while this one
 // is used; a lane keeps 4 x RW 16-byte loads of A in flight, two CTAs per SM.  The
-// order of every sum is fixed.  Needs an even lda and a 16-byte aligned A; an odd K
+// order of every sum is fixed, and a lane adds up each chunk by itself first, so
+// that no chain of FP32 additions grows with K (one chain per lane costs 1 to 10 %
+// less time but its rounding error is 2.5 times that of a K range split over the
+// warps).  Needs an even lda and a 16-byte aligned A; an odd K
 // leaves one k to lane 0.  The kernels it replaces read B through L1 per element
 // (register tiles: 1.85 TB/s at 12 000 rows) or waited on it per chunk (rows
-// streamed by bulk copies: 3.2 TB/s at 24 000); this one reaches 6.1 TB/s at 24 000
-// rows, 5.1 at 12 000 and 3.3 at 4000.
+// streamed by bulk copies: 3.2 TB/s at 24 000); this one reaches 6.0 to
+// 6.5 TB/s at 24 000 rows, 5.2 at 12 000 and 3.3 at 4000.
 constexpr int TV_WARPS = 8;
 template <int N, int RW, int MODE>
 __global__ void __launch_bounds__(32 * TV_WARPS, 2) k_gemm_thin_c64(int64_t M, int64_t K, float2 alpha,
@@ -194,6 +197,11 @@ __global__ void __launch_bounds__(32 * TV_WARPS, 2) k_gemm_thin_c64(int64_t M, i
     }
     __syncthreads();
     if (k0 + TV_KC < Ke) fetch(k0 + TV_KC);
+    float2 part[RW][N];
+#pragma unroll
+    for (int r = 0; r < RW; ++r)
+#pragma unroll
+      for (int c = 0; c < N; ++c) part[r][c] = make_float2(0.f, 0.f);
 #pragma unroll
     for (int h = 0; h < TV_KC / 256; ++h) {            // 256 k at a time: four 16-byte loads per row
       float4 a[4][RW];
@@ -212,12 +220,16 @@ __global__ void __launch_bounds__(32 * TV_WARPS, 2) k_gemm_thin_c64(int64_t M, i
           const float4 b = *reinterpret_cast<const float4*>(&xs[c][kk]);
 #pragma unroll
           for (int r = 0; r < RW; ++r) {
-            cfma(acc[r][c], make_float2(a[u][r].x, a[u][r].y), make_float2(b.x, b.y));
-            cfma(acc[r][c], make_float2(a[u][r].z, a[u][r].w), make_float2(b.z, b.w));
+            cfma(part[r][c], make_float2(a[u][r].x, a[u][r].y), make_float2(b.x, b.y));
+            cfma(part[r][c], make_float2(a[u][r].z, a[u][r].w), make_float2(b.z, b.w));
           }
         }
       }
     }
+#pragma unroll
+    for (int r = 0; r < RW; ++r)
+#pragma unroll
+      for (int c = 0; c < N; ++c) acc[r][c] = cadd(acc[r][c], part[r][c]);
   }
   if ((K & 1) && lane == 0) {
 #pragma unroll
@@ -253,9 +265,10 @@ __global__ void __launch_bounds__(32 * TV_WARPS, 2) k_gemm_thin_c64(int64_t M, i
 template <int MODE>
 static mnpbem_status launch_thin_c64(int64_t M, int64_t N, int64_t K, const float2* A, int64_t lda, const float2* B,
                                      int64_t ldb, float2 alpha, float2 beta, void* C, int64_t ldc, cudaStream_t st) {
-  // rows per warp: four with up to three columns, two beyond (the sums and the
-  // loads in flight fill the registers: N = 4 at 24 000 rows 6.1 TB/s with two,
-  // 4.9 with four); fewer where the rows would not give every SM two CTAs
+  // rows per warp: four with up to two columns, two up to six, one beyond (the sums
+  // and the loads in flight fill the registers: at 24 000 rows N = 3 takes 707 us
+  // with two and 873 with four, N = 4 763 and 951; 2904 rows, N = 8: 50 us with
+  // one, 56 with two); fewer where the rows would not give every SM two CTAs
 #define TV_CASE(NN, RW)                                                                                              \
   k_gemm_thin_c64<NN, RW, MODE><<<(unsigned)cdiv_up(M, (int64_t)(TV_WARPS * RW)), 32 * TV_WARPS, 0, st>>>(           \
       M, K, alpha, A, lda, B, ldb, beta, C, ldc)
@@ -266,7 +279,7 @@ static mnpbem_status launch_thin_c64(int64_t M, int64_t N, int64_t K, const floa
     else TV_CASE(NN, 1);                                 \
     break;
   switch (N) {
-    TV_N(1, 4) TV_N(2, 4) TV_N(3, 4) TV_N(4, 2) TV_N(5, 2) TV_N(6, 2) TV_N(7, 2) TV_N(8, 2)
+    TV_N(1, 4) TV_N(2, 4) TV_N(3, 2) TV_N(4, 2) TV_N(5, 2) TV_N(6, 2) TV_N(7, 1) TV_N(8, 1)
     default:
       set_error("thin product: N must be 1..8");
       return MNPBEM_ERR_INVALID_ARG;

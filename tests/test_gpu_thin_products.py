@@ -5,7 +5,7 @@ sizes cover every N, the edges of a CTA's rows (8 warps), the row counts at whic
 the rows per warp change, k ranges below, at and beyond one staged chunk of B with
 odd remainders, a row pitch of C wider than N and alpha / beta other than 1 / 0.
 
-Tolerance: each lane of a warp adds ceil(K / 32) products in FP32 and five
+Tolerance: each lane of a warp adds at most ceil(K / 32) products in FP32 and five
 shuffles add the lanes, so a sum's relative error stays below
 (2 ceil(K / 32) + 7) 2^-24 of the sum of moduli; on random data, whose sums of
 moduli are about sqrt(K) times the largest result, rounding errors of both signs
