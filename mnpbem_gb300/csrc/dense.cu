@@ -77,6 +77,75 @@ __global__ void __launch_bounds__(256) k_gemm_nn(int64_t M, int64_t N, int64_t K
   }
 }
 
+// The same product for a few tiles (panel products of a last, narrow block): 16 x
+// 32 tiles and the k range of a step shared by four groups of 64 threads, whose
+// sums are added in a fixed order at the end.  Bound by latency: with 64 x 64
+// tiles such a product ran on one to eight SMs and K = 256 took 46 us whatever the
+// size, now 8 (64 x 64 x 64: 16 and 4; 512 x 512 x 64, 64 old tiles: 16 and 9).
+constexpr int SG_M = 16, SG_N = 32, SG_K = 64;
+__global__ void __launch_bounds__(256) k_gemm_small(int64_t M, int64_t N, int64_t K, float2 alpha,
+                                                    const float2* __restrict__ A, int64_t lda,
+                                                    const float2* __restrict__ B, int64_t ldb, float2 beta,
+                                                    float2* __restrict__ C, int64_t ldc) {
+  __shared__ float2 As[SG_K][SG_M + 1], Bs[SG_K][SG_N], red[4][SG_M * SG_N];
+  const int t = threadIdx.x, g = t >> 6, u = t & 63, tx = u & 15, ty = u >> 4;
+  const int64_t m0 = (int64_t)blockIdx.y * SG_M, n0 = (int64_t)blockIdx.x * SG_N;
+  float2 acc[4][2];
+#pragma unroll
+  for (int r = 0; r < 4; ++r) acc[r][0] = acc[r][1] = make_float2(0.f, 0.f);
+  float2 pa[4], pb[8];
+  const auto fetch = [&](int64_t k0) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+      const int e = t + 256 * q;
+      const int64_t r = m0 + (e >> 6), k = k0 + (e & 63);
+      pa[q] = (r < M && k < K) ? A[r * lda + k] : make_float2(0.f, 0.f);
+    }
+#pragma unroll
+    for (int q = 0; q < 8; ++q) {
+      const int e = t + 256 * q;
+      const int64_t k = k0 + (e >> 5), c = n0 + (e & 31);
+      pb[q] = (k < K && c < N) ? B[k * ldb + c] : make_float2(0.f, 0.f);
+    }
+  };
+  fetch(0);
+  for (int64_t k0 = 0; k0 < K; k0 += SG_K) {
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < 4; ++q) As[(t + 256 * q) & 63][(t + 256 * q) >> 6] = pa[q];
+#pragma unroll
+    for (int q = 0; q < 8; ++q) Bs[(t + 256 * q) >> 5][(t + 256 * q) & 31] = pb[q];
+    __syncthreads();
+    if (k0 + SG_K < K) fetch(k0 + SG_K);
+#pragma unroll
+    for (int q = 0; q < SG_K / 4; ++q) {
+      const int kk = g * (SG_K / 4) + q;
+      const float2 b0 = Bs[kk][tx], b1 = Bs[kk][tx + 16];
+#pragma unroll
+      for (int r = 0; r < 4; ++r) {
+        const float2 a = As[kk][ty + 4 * r];
+        cfma(acc[r][0], a, b0);
+        cfma(acc[r][1], a, b1);
+      }
+    }
+  }
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    red[g][(ty + 4 * r) * SG_N + tx] = acc[r][0];
+    red[g][(ty + 4 * r) * SG_N + tx + 16] = acc[r][1];
+  }
+  __syncthreads();
+  const bool zero_beta = (beta.x == 0 && beta.y == 0);
+  for (int e = t; e < SG_M * SG_N; e += 256) {
+    const int64_t r = m0 + e / SG_N, c = n0 + e % SG_N;
+    if (r >= M || c >= N) continue;
+    const float2 v = cadd(cadd(red[0][e], red[1][e]), cadd(red[2][e], red[3][e]));
+    float2 out = cmul(alpha, v);
+    if (!zero_beta) out = cadd(out, cmul(beta, C[r * ldc + c]));
+    C[r * ldc + c] = out;
+  }
+}
+
 // ------------------------------------------------------- thin GEMM (N <= 16)
 // Matrix times a few vectors, memory-bound on A.  A block of 8 warps owns
 // TR rows; warp w streams its own slice of K (no barriers in the main loop),
@@ -564,6 +633,18 @@ mnpbem_status gemm_simt(int64_t M, int64_t N, int64_t K, cplx<R> alpha, const cp
   if (grid.y > 65535) { set_error("gemm_simt: M too large"); return MNPBEM_ERR_INVALID_ARG; }
   constexpr int BK = sizeof(R) == 4 ? 16 : 8;
   const bool big = M >= 128 && N >= 128;
+  // complex64 products that would leave half of the SMs without a 64 x 64 tile
+  // (76 tiles and fewer: 512 x 512 x 64, 64 tiles, 9 us and 16 with the large tile);
+  // C may not overlap A or B in either
+  if constexpr (sizeof(R) == 4) {
+    if (K >= 16 && (int64_t)grid.x * grid.y <= 76) {
+      ProfScope ps(PH_GEMM_SMALL, st, 8.0 * M * N * K, 8.0 * ((double)M * K + (double)K * N + 2.0 * M * N));
+      k_gemm_small<<<dim3((unsigned)cdiv_up(N, (int64_t)SG_N), (unsigned)cdiv_up(M, (int64_t)SG_M)), 256, 0, st>>>(
+          M, N, K, alpha, A, lda, B, ldb, beta, C, ldc);
+      MNP_CHECK_LAUNCH();
+      return MNPBEM_OK;
+    }
+  }
   ProfScope ps(big ? PH_GEMM_BIG : PH_GEMM_SMALL, st, 8.0 * M * N * K,
                (double)sizeof(cplx<R>) * ((double)M * K + (double)K * N + 2.0 * M * N));
   k_gemm_nn<R, BK><<<grid, 256, 0, st>>>(M, N, K, alpha, A, lda, B, ldb, beta, C, ldc);
