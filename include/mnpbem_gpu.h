@@ -366,6 +366,13 @@ MNPBEM_API mnpbem_status mnpbem_solve_potentials(mnpbem_geom* g, const mnpbem_po
                                                  const double* eps_media, int32_t nmed, int32_t precision,
                                                  const mnpbem_refine* refine, mnpbem_solution* out);
 
+/* The same for ngroups sets of up to four columns (pots[q] -> outs[q]): the
+ * matrices of the wavelength are assembled and factored once.              */
+MNPBEM_API mnpbem_status mnpbem_solve_potentials_groups(mnpbem_geom* g, const mnpbem_potentials* pots,
+                                                        int32_t ngroups, double enei, const double* eps_media,
+                                                        int32_t nmed, int32_t precision,
+                                                        const mnpbem_refine* refine, mnpbem_solution* outs);
+
 /* Electric and magnetic fields at points off the particle boundary
  * (Greenfun/@compgreenret/field.m:17-38 on the Green function between a
  * compoint and the particle; Simulation/misc/@meshfield): for a point in

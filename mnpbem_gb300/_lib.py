@@ -99,6 +99,9 @@ SIGNATURES = {
     "mnpbem_solve_potentials": (ctypes.c_int, [ctypes.c_void_p, ctypes.POINTER(Potentials), ctypes.c_double,
                                                c_double_p, ctypes.c_int32, ctypes.c_int32,
                                                ctypes.POINTER(Refine), ctypes.POINTER(Solution)]),
+    "mnpbem_solve_potentials_groups": (ctypes.c_int, [ctypes.c_void_p, ctypes.POINTER(Potentials), ctypes.c_int32,
+                                                      ctypes.c_double, c_double_p, ctypes.c_int32, ctypes.c_int32,
+                                                      ctypes.POINTER(Refine), ctypes.POINTER(Solution)]),
     "mnpbem_solve_iter": (ctypes.c_int, [ctypes.c_void_p, ctypes.POINTER(ClusterTree), ctypes.POINTER(IterOptions),
                                          ctypes.POINTER(PlaneWave), ctypes.POINTER(Potentials), ctypes.c_double,
                                          c_double_p, ctypes.c_int32, ctypes.c_int32, ctypes.POINTER(Solution),

@@ -426,7 +426,7 @@ class bemret:
         ``exc`` from a plane wave (``planewave(...)(p, enei)``) or with
         external potentials ``phi1, phi1p, phi2, phi2p [n, P]``, ``a1, a1p, a2,
         a2p [n, 3, P]`` (e.g. ``dipoleret.potential``), solved in groups of at
-        most four columns by ``mnpbem_solve_potentials``."""
+        most four columns by ``mnpbem_solve_potentials_groups``."""
         if not hasattr(exc, "exc"):
             return self._solve_potentials(exc)
         pw = exc.exc
@@ -495,33 +495,33 @@ class bemret:
         em = np.ascontiguousarray(self.p.eps_media(enei)[0])
         out = {k: np.zeros((n, P), np.complex128) for k in ("sig1", "sig2")}
         out.update({k: np.zeros((n, 3, P), np.complex128) for k in ("h1", "h2")})
-        iters = []
-        for c0 in range(0, P, 4):
-            cols = slice(c0, min(P, c0 + 4))
+        ng = (P + 3) // 4
+        pots, sols = (_lib.Potentials * ng)(), (_lib.Solution * ng)()
+        keep, parts, iters = [], [], np.zeros(ng, np.int32)
+        for q in range(ng):              # up to four columns per group
+            cols = slice(4 * q, min(P, 4 * q + 4))
             w = cols.stop - cols.start
-            keep = []
-            pot = _lib.Potentials()
-            pot.npol = w
+            pots[q].npol = w
             for k in keys1 + keys3:
                 if hasattr(exc, k):
                     arr = np.ascontiguousarray(np.asarray(getattr(exc, k))[..., cols], dtype=np.complex128)
                     keep.append(arr)
-                    setattr(pot, k, arr.ctypes.data)
+                    setattr(pots[q], k, arr.ctypes.data)
             part = {k: np.zeros((n, w) if k.startswith("sig") else (n, 3, w), np.complex128)
                     for k in ("sig1", "sig2", "h1", "h2")}
-            it, res = np.zeros(1, np.int32), np.zeros(1)
-            sol = _lib.Solution()
-            sol.sig1, sol.sig2 = part["sig1"].ctypes.data, part["sig2"].ctypes.data
-            sol.h1, sol.h2 = part["h1"].ctypes.data, part["h2"].ctypes.data
-            sol.ir_iters, sol.ir_resid = it.ctypes.data, res.ctypes.data
+            sols[q].sig1, sols[q].sig2 = part["sig1"].ctypes.data, part["sig2"].ctypes.data
+            sols[q].h1, sols[q].h2 = part["h1"].ctypes.data, part["h2"].ctypes.data
+            sols[q].ir_iters = iters[q:].ctypes.data
+            parts.append((cols, part))
+        if ng:
             ref = _lib.Refine(self.refine_iters, self.refine_tol)
-            _lib.check(self._lib.mnpbem_solve_potentials(
-                self._h, ctypes.byref(pot), enei, em.view(np.float64).ctypes.data_as(_lib.c_double_p), em.size,
-                self.precision, ctypes.byref(ref), ctypes.byref(sol)))
+            _lib.check(self._lib.mnpbem_solve_potentials_groups(
+                self._h, pots, ng, enei, em.view(np.float64).ctypes.data_as(_lib.c_double_p), em.size,
+                self.precision, ctypes.byref(ref), sols))
+        for cols, part in parts:
             for k in part:
                 out[k][..., cols] = part[k]
-            iters.append(int(it[0]))
-        return compstruct(self.p, enei, ir_iters=max(iters), **out)
+        return compstruct(self.p, enei, ir_iters=int(max(iters)), **out)
 
 
 class dipoleret:

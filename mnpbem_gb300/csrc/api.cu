@@ -913,6 +913,7 @@ struct SolveCtx {
   const mnpbem_planewave* exc;
   const double2* ext_pot = nullptr;   // external potentials instead of the plane wave (device)
   bool spectra = true;                // far fields and cross sections of the plane wave
+  bool factored = false;              // the lane holds this wavelength's matrices and factors
 };
 
 size_t lane_bytes_estimate(const mnpbem_geom* G, int precision, int P, int ninf) {
@@ -1525,7 +1526,7 @@ void refine_reset(Lane& L) {
 mnpbem_status solve_one(mnpbem_geom* G, Lane& L, const SolveCtx& c, const Refine& ref, bool graphs,
                         int32_t* iters, double* resid) {
   cudaStream_t st = L.st;
-  for (int stage = 0; stage < 3; ++stage) MNP_TRY(launch_stage(G, L, c, stage, graphs));
+  for (int stage = c.factored ? 2 : 0; stage < 3; ++stage) MNP_TRY(launch_stage(G, L, c, stage, graphs));
   MNP_TRY(status_copy(L, c.precision));
   int used = 0;
   double final_res = -1.0;
@@ -1703,10 +1704,15 @@ int choose_lanes(mnpbem_geom* G, int precision, int P, int ninf, int nenei) {
 // One wavelength sweep on one handle.  A call of mnpbem_solve is one job; a
 // call of mnpbem_solve_batch runs several jobs (particles) through one
 // scheduler loop, so that the lanes of every handle stay busy together.
+struct PotGroup {
+  const mnpbem_potentials* pot;   // up to four columns
+  mnpbem_solution out;
+};
 struct Job {
   mnpbem_geom* G = nullptr;
   SolveCtx c;
   Sweep s;
+  std::vector<PotGroup> groups;  // external potentials (c.ext_pot): column groups of one wavelength
   int nl = 1;
   int next = 0;                 // next wavelength to hand out
   int active = 0;               // lanes with queued work
@@ -1841,14 +1847,34 @@ mnpbem_status job_prepare(Job& j) {
   const SolveCtx& c = j.c;
   const Sweep& s = j.s;
   if (c.ext_pot) {
-    // external potentials: direct solves on lane 0 (no captured graphs)
+    // external potentials: direct solves on lane 0 (no captured graphs), one column
+    // group after the other with the factors of the first
     Lane& L = *G->lanes[0];
-    for (; j.next < s.nenei; ++j.next) {
-      MNP_TRY(upload_lp(G, L, s, j.next));
-      L.w = j.next;
-      MNP_TRY(solve_one(G, L, c, s.ref, false, &L.iters, &L.res));
-      MNP_TRY(write_outputs(G, L, c, s, j.next));
+    const int64_t n = G->g.n;
+    double2* D = const_cast<double2*>(c.ext_pot);
+    MNP_TRY(upload_lp(G, L, s, 0));
+    L.w = 0;
+    for (PotGroup& gr : j.groups) {
+      const mnpbem_potentials& pot = *gr.pot;
+      const int P = pot.npol;
+      const double* src[8] = {pot.phi1, pot.phi1p, pot.phi2, pot.phi2p, pot.a1, pot.a1p, pot.a2, pot.a2p};
+      for (int q = 0; q < 8; ++q) {
+        const int64_t cnt = (q < 4 ? 1 : 3) * n * P;
+        double2* dst = D + (q < 4 ? q * n * P : 4 * n * P + (q - 4) * 3 * n * P);
+        if (src[q])
+          MNP_CUDA(cudaMemcpyAsync(dst, src[q], sizeof(double2) * cnt, cudaMemcpyHostToDevice, L.st));
+        else
+          MNP_CUDA(cudaMemsetAsync(dst, 0, sizeof(double2) * cnt, L.st));
+      }
+      SolveCtx cg = c;
+      cg.P = P;
+      cg.factored = &gr != &j.groups.front();
+      Sweep sg = s;
+      sg.out = &gr.out;
+      MNP_TRY(solve_one(G, L, cg, s.ref, false, &L.iters, &L.res));
+      MNP_TRY(write_outputs(G, L, cg, sg, 0));
     }
+    j.next = s.nenei;
     return MNPBEM_OK;
   }
   std::vector<int> fresh;
@@ -3008,44 +3034,47 @@ mnpbem_status mnpbem_farfield(mnpbem_geom* G, double enei, const double* eps_med
   return MNPBEM_OK;
 }
 
-mnpbem_status mnpbem_solve_potentials(mnpbem_geom* G, const mnpbem_potentials* pot, double enei,
-                                      const double* eps_media, int32_t nmed, int32_t precision,
-                                      const mnpbem_refine* refine, mnpbem_solution* out) {
+mnpbem_status mnpbem_solve_potentials_groups(mnpbem_geom* G, const mnpbem_potentials* pots, int32_t ngroups,
+                                             double enei, const double* eps_media, int32_t nmed, int32_t precision,
+                                             const mnpbem_refine* refine, mnpbem_solution* outs) {
   MNP_TRY(check_geom(G));
-  if (!pot || pot->npol < 1 || pot->npol > 4 || !out || !(enei > 0)) {
+  bool ok = pots && outs && ngroups >= 1 && enei > 0;
+  int P = 0;
+  for (int q = 0; ok && q < ngroups; ++q) {
+    ok = pots[q].npol >= 1 && pots[q].npol <= 4;
+    P = std::max(P, (int)pots[q].npol);
+  }
+  if (!ok) {
     set_error("mnpbem_solve_potentials: invalid arguments");
     return MNPBEM_ERR_INVALID_ARG;
   }
-  const int P = pot->npol;
-  const double* src[8] = {pot->phi1, pot->phi1p, pot->phi2, pot->phi2p, pot->a1, pot->a1p, pot->a2, pot->a2p};
   // a plane wave without directions stands in for the job's excitation; the
   // potentials replace its excitation and no spectra are computed
   std::vector<double> zero(3 * P, 0.0);
   mnpbem_planewave pw{P, zero.data(), zero.data(), 1, 0, nullptr, nullptr};
-  mnpbem_solution o = *out;
-  o.ext = o.sca = nullptr;
-  MNP_TRY(validate_job(G, &pw, 1, &enei, eps_media, nmed, precision, &o));
-  MNP_CUDA(cudaSetDevice(G->device));
-  const int64_t n = G->g.n;
-  DevBuf dpot;
-  MNP_TRY(dpot.ensure(sizeof(double2) * 16 * n * P));
-  double2* D = dpot.as<double2>();
-  for (int q = 0; q < 8; ++q) {
-    const int64_t cnt = (q < 4 ? 1 : 3) * n * P;
-    double2* dst = D + (q < 4 ? q * n * P : 4 * n * P + (q - 4) * 3 * n * P);
-    if (src[q])
-      MNP_CUDA(cudaMemcpyAsync(dst, src[q], sizeof(double2) * cnt, cudaMemcpyHostToDevice, G->st));
-    else
-      MNP_CUDA(cudaMemsetAsync(dst, 0, sizeof(double2) * cnt, G->st));
-  }
-  MNP_CUDA(cudaStreamSynchronize(G->st));
   std::vector<Job> jobs(1);
-  jobs[0].G = G;
-  MNP_TRY(job_setup(jobs[0], &pw, 1, &enei, eps_media, nmed, precision, refine, &o));
-  jobs[0].c.ext_pot = D;
-  jobs[0].c.spectra = false;
-  jobs[0].nl = 1;
+  Job& j = jobs[0];
+  for (int q = 0; q < ngroups; ++q) {
+    j.groups.push_back(PotGroup{pots + q, outs[q]});
+    mnpbem_solution& o = j.groups.back().out;
+    o.ext = o.sca = nullptr;
+    MNP_TRY(validate_job(G, &pw, 1, &enei, eps_media, nmed, precision, &o));
+  }
+  MNP_CUDA(cudaSetDevice(G->device));
+  DevBuf dpot;
+  MNP_TRY(dpot.ensure(sizeof(double2) * 16 * G->g.n * P));
+  j.G = G;
+  MNP_TRY(job_setup(j, &pw, 1, &enei, eps_media, nmed, precision, refine, &j.groups[0].out));
+  j.c.ext_pot = dpot.as<double2>();
+  j.c.spectra = false;
+  j.nl = 1;
   return run_jobs(jobs);
+}
+
+mnpbem_status mnpbem_solve_potentials(mnpbem_geom* G, const mnpbem_potentials* pot, double enei,
+                                      const double* eps_media, int32_t nmed, int32_t precision,
+                                      const mnpbem_refine* refine, mnpbem_solution* out) {
+  return mnpbem_solve_potentials_groups(G, pot, 1, enei, eps_media, nmed, precision, refine, out);
 }
 
 // ======================================================================
