@@ -212,30 +212,33 @@ __global__ void __launch_bounds__(32 * THIN_WARPS) k_gemm_thin(int64_t M, int64_
   }
 }
 
-// complex64 products with few columns (N <= 8): C (complex64) = alpha A B + beta C
-// (MODE 0), or C (complex128) = A B (MODE 1).  Bound by HBM on A (at 4000 rows and
+// complex64 products with few columns: C (complex64) = alpha A B + beta C (MODE 0, N
+// <= 16), or C (complex128) = A B (MODE 1, N <= 8).  Bound by HBM on A (at 4000 rows and
 // more far larger than what the caches keep between products).  A CTA of eight
-// warps owns 8 RW rows over all of K; B comes in chunks of 512 or 256 rows through
+// warps owns 8 RW rows over all of K; B comes in chunks of 512 to 128 rows through
 // shared memory (transposed, so that a lane reads its two neighbouring k as one
 // 16-byte word per column), the next chunk's entries being loaded while this one
-// is used; a lane keeps 4 x RW 16-byte loads of A in flight, two CTAs per SM.  The
-// order of every sum is fixed, and a lane adds up each chunk by itself first, so
-// that no chain of FP32 additions grows with K (one chain per lane costs 1 to 10 %
-// less time but its rounding error is 2.5 times that of a K range split over the
-// warps).  Needs an even lda and a 16-byte aligned A; an odd K
+// is used; a lane keeps 4 x RW 16-byte loads of A in flight (two beyond eight
+// columns), two CTAs per SM.  The order of every sum is fixed, and a lane adds up each
+// chunk by itself first, so that no long chain of FP32 additions builds up (one chain
+// per lane costs 1 to 10 % less time but its rounding error is 2.5 times that of a K
+// range split over the warps).  Needs an even lda and a 16-byte aligned A; an odd K
 // leaves one k to lane 0.  The kernels it replaces read B through L1 per element
 // (register tiles: 1.85 TB/s at 12 000 rows) or waited on it per chunk (rows
 // streamed by bulk copies: 3.2 TB/s at 24 000); this one reaches 6.0 to
-// 6.5 TB/s at 24 000 rows, 5.2 at 12 000 and 3.3 at 4000.
+// 6.5 TB/s at 24 000 rows, 5.2 at 12 000 and 3.3 at 4000 up to four columns.  Beyond
+// six columns the reads of B from shared memory bound it (12 000 rows: N = 8 452 us,
+// 12 700, 16 1081; the register tiles took 1126 and 3859 for the last two).
 constexpr int TV_WARPS = 8;
 template <int N, int RW, int MODE>
 __global__ void __launch_bounds__(32 * TV_WARPS, 2) k_gemm_thin_c64(int64_t M, int64_t K, float2 alpha,
                                                                   const float2* __restrict__ A, int64_t lda,
                                                                   const float2* __restrict__ B, int64_t ldb,
                                                                   float2 beta, void* __restrict__ Cv, int64_t ldc) {
-  constexpr int TV_KC = N <= 4 ? 512 : 256;            // k per chunk
+  constexpr int TV_KC = N <= 4 ? 512 : N <= 8 ? 256 : 128;   // k per chunk
+  constexpr int U = TV_KC >= 256 ? 4 : 2;              // loads per row in flight
   __shared__ __align__(16) float2 xs[N][TV_KC + 4];
-  constexpr int NE = TV_KC * N / (32 * TV_WARPS);      // entries of a chunk of B per thread
+  constexpr int NE = (TV_KC * N + 32 * TV_WARPS - 1) / (32 * TV_WARPS);   // entries of a chunk of B per thread
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t row0 = ((int64_t)blockIdx.x * TV_WARPS + warp) * RW;
   const float2* arow[RW];
@@ -253,7 +256,7 @@ __global__ void __launch_bounds__(32 * TV_WARPS, 2) k_gemm_thin_c64(int64_t M, i
     for (int q = 0; q < NE; ++q) {
       const int e = threadIdx.x + 32 * TV_WARPS * q;
       const int64_t k = k0 + e / N;
-      nb[q] = k < Ke ? __ldg(B + k * ldb + e % N) : make_float2(0.f, 0.f);
+      nb[q] = k < Ke && e < TV_KC * N ? __ldg(B + k * ldb + e % N) : make_float2(0.f, 0.f);
     }
   };
   fetch(0);
@@ -262,7 +265,7 @@ __global__ void __launch_bounds__(32 * TV_WARPS, 2) k_gemm_thin_c64(int64_t M, i
 #pragma unroll
     for (int q = 0; q < NE; ++q) {
       const int e = threadIdx.x + 32 * TV_WARPS * q;
-      xs[e % N][e / N] = nb[q];
+      if (e < TV_KC * N) xs[e % N][e / N] = nb[q];
     }
     __syncthreads();
     if (k0 + TV_KC < Ke) fetch(k0 + TV_KC);
@@ -272,18 +275,18 @@ __global__ void __launch_bounds__(32 * TV_WARPS, 2) k_gemm_thin_c64(int64_t M, i
 #pragma unroll
       for (int c = 0; c < N; ++c) part[r][c] = make_float2(0.f, 0.f);
 #pragma unroll
-    for (int h = 0; h < TV_KC / 256; ++h) {            // 256 k at a time: four 16-byte loads per row
-      float4 a[4][RW];
+    for (int h = 0; h < TV_KC / (64 * U); ++h) {       // 64 U k at a time: U 16-byte loads per row
+      float4 a[U][RW];
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int64_t k = k0 + 256 * h + 64 * u + 2 * lane;
+      for (int u = 0; u < U; ++u) {
+        const int64_t k = k0 + 64 * U * h + 64 * u + 2 * lane;
 #pragma unroll
         for (int r = 0; r < RW; ++r)
           a[u][r] = k < Ke ? __ldg(reinterpret_cast<const float4*>(arow[r] + k)) : make_float4(0.f, 0.f, 0.f, 0.f);
       }
 #pragma unroll
-      for (int u = 0; u < 4; ++u) {
-        const int kk = 256 * h + 64 * u + 2 * lane;
+      for (int u = 0; u < U; ++u) {
+        const int kk = 64 * U * h + 64 * u + 2 * lane;
 #pragma unroll
         for (int c = 0; c < N; ++c) {
           const float4 b = *reinterpret_cast<const float4*>(&xs[c][kk]);
@@ -337,7 +340,7 @@ static mnpbem_status launch_thin_c64(int64_t M, int64_t N, int64_t K, const floa
   // rows per warp: four with up to two columns, two up to six, one beyond (the sums
   // and the loads in flight fill the registers: at 24 000 rows N = 3 takes 707 us
   // with two and 873 with four, N = 4 763 and 951; 2904 rows, N = 8: 50 us with
-  // one, 56 with two); fewer where the rows would not give every SM two CTAs
+  // one, 56 with two); fewer where the rows would not give every SM a CTA
 #define TV_CASE(NN, RW)                                                                                              \
   k_gemm_thin_c64<NN, RW, MODE><<<(unsigned)cdiv_up(M, (int64_t)(TV_WARPS * RW)), 32 * TV_WARPS, 0, st>>>(           \
       M, K, alpha, A, lda, B, ldb, beta, C, ldc)
@@ -347,12 +350,22 @@ static mnpbem_status launch_thin_c64(int64_t M, int64_t N, int64_t K, const floa
     else if (M >= 152 * TV_WARPS * 2) TV_CASE(NN, 2);    \
     else TV_CASE(NN, 1);                                 \
     break;
+#define TV_1(NN) case NN: TV_CASE(NN, 1); break;
   switch (N) {
     TV_N(1, 4) TV_N(2, 4) TV_N(3, 2) TV_N(4, 2) TV_N(5, 2) TV_N(6, 2) TV_N(7, 1) TV_N(8, 1)
     default:
-      set_error("thin product: N must be 1..8");
-      return MNPBEM_ERR_INVALID_ARG;
+      if constexpr (MODE == 0) {
+        switch (N) {
+          TV_1(9) TV_1(10) TV_1(11) TV_1(12) TV_1(13) TV_1(14) TV_1(15) TV_1(16)
+          default: break;
+        }
+      }
+      if (MODE != 0 || N < 1 || N > THIN_NMAX) {
+        set_error("thin product: unsupported number of columns");
+        return MNPBEM_ERR_INVALID_ARG;
+      }
   }
+#undef TV_1
 #undef TV_N
 #undef TV_CASE
   MNP_CHECK_LAUNCH();
@@ -601,7 +614,7 @@ mnpbem_status gemm_simt(int64_t M, int64_t N, int64_t K, cplx<R> alpha, const cp
                         int64_t lda, const cplx<R>* B, int64_t ldb, cplx<R> beta, cplx<R>* C,
                         int64_t ldc, cudaStream_t st) {
   if (M <= 0 || N <= 0) return MNPBEM_OK;
-  if (sizeof(R) == 4 && N <= 8 && K > 1 && !(lda & 1) && !(reinterpret_cast<uintptr_t>(A) & 15)) {
+  if (sizeof(R) == 4 && N <= THIN_NMAX && K > 1 && !(lda & 1) && !(reinterpret_cast<uintptr_t>(A) & 15)) {
     ProfScope ps(PH_GEMM_SMALL, st, 8.0 * M * N * K,
                  (double)sizeof(cplx<R>) * ((double)M * K + (double)K * N + 2.0 * M * N));
     const float2* Af = reinterpret_cast<const float2*>(A);

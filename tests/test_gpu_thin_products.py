@@ -1,4 +1,4 @@
-"""Complex64 products with few columns (mnpbem_gemm_c64, path 0, N <= 8).
+"""Complex64 products with few columns (mnpbem_gemm_c64, path 0, N <= 16).
 
 One warp takes one to four rows of A by the number of columns and of rows: the
 sizes cover every N, the edges of a CTA's rows (8 warps), the row counts at which
@@ -19,7 +19,7 @@ from test_gpu_gemm import run
 pytestmark = pytest.mark.gpu
 
 
-@pytest.mark.parametrize("N", range(1, 9))
+@pytest.mark.parametrize("N", range(1, 17))
 def test_thin_products(gpu_lib, N):
     for M, K in [(1, 2), (7, 34), (33, 254), (65, 514), (1217, 258), (2433, 300), (4865, 66), (9729, 34),
                  (300, 1100)]:
