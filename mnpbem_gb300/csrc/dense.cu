@@ -417,13 +417,7 @@ __global__ void __launch_bounds__(32 * DS_WARPS) k_gemm_thin_ds(int64_t M, int64
       const float2 ah = __ldg(Ahi + roff[r] + k), al = __ldg(Alo + roff[r] + k);
 #pragma unroll
       for (int c = 0; c < N; ++c) {
-        ds_acc_prod(re[r][c], ah.x, xh[c].x);
-        ds_acc_prod(re[r][c], -ah.y, xh[c].y);
-        ds_acc_prod(im[r][c], ah.x, xh[c].y);
-        ds_acc_prod(im[r][c], ah.y, xh[c].x);
-        // first-order corrections from the low parts (relative size 2^-24)
-        re[r][c].lo += (ah.x * xl[c].x - ah.y * xl[c].y) + (al.x * xh[c].x - al.y * xh[c].y);
-        im[r][c].lo += (ah.x * xl[c].y + ah.y * xl[c].x) + (al.x * xh[c].y + al.y * xh[c].x);
+        ds_cfma(re[r][c], im[r][c], ah, al, xh[c], xl[c]);
       }
     }
   }

@@ -197,10 +197,10 @@ __global__ void __launch_bounds__(256) k_hmv_t(HmatDev h) {
     for (int c = 0; c < N; ++c) re[c] = im[c] = DS{0.f, 0.f};
     for (int j = lane; j < blk.w; j += 32) {
       const float4 bv = B[(int64_t)kk * blk.w + j];
-      const float4* xr = x + (int64_t)h.perm[blk.z + j] * N;
+      const float4* xr = x + blk.z + j;
 #pragma unroll
       for (int c = 0; c < N; ++c) {
-        const float4 xv = xr[c];
+        const float4 xv = xr[(int64_t)c * h.n];
         ds_cfma(re[c], im[c], f4hi(bv), f4lo(bv), f4hi(xv), f4lo(xv));
       }
     }
@@ -251,10 +251,10 @@ __global__ void __launch_bounds__(256) k_hmv_leaf(HmatDev h, YPtrs ys, int rs) {
           float4 v[R];
 #pragma unroll
           for (int r = 0; r < R; ++r) v[r] = V[r][j];
-          const float4* xr = x + (int64_t)h.perm[fb.z + j] * N;
+          const float4* xr = x + fb.z + j;
 #pragma unroll
           for (int c = 0; c < N; ++c) {
-            const float4 xv = xr[c];
+            const float4 xv = xr[(int64_t)c * h.n];
 #pragma unroll
             for (int r = 0; r < R; ++r) ds_cfma(re[r][c], im[r][c], f4hi(v[r]), f4lo(v[r]), f4hi(xv), f4lo(xv));
           }
@@ -345,11 +345,14 @@ __global__ void k_split_factors(HmatDev h) {
   for (int64_t e = threadIdx.x; e < (int64_t)rank * blk.w; e += blockDim.x) split_in_place(B, e);
 }
 
-__global__ void k_split_x(const double2* __restrict__ x1, const double2* __restrict__ x2, int64_t count,
-                          float4* xs) {
-  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < count; e += (int64_t)gridDim.x * blockDim.x) {
-    xs[e] = split4(x1[e]);
-    xs[count + e] = split4(x2[e]);
+// the product's vectors [n][N] in face order -> hi / lo pairs, one plane of n per
+// column in cluster order, which the products read as they stand
+__global__ void k_split_x(const double2* __restrict__ x1, const double2* __restrict__ x2, const int* __restrict__ perm,
+                          int64_t n, int N, float4* xs) {
+  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < n * N; e += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t c = e / n, i = e - c * n, src = (int64_t)perm[i] * N + c;
+    xs[e] = split4(x1[src]);
+    xs[n * N + e] = split4(x2[src]);
   }
 }
 
@@ -465,7 +468,7 @@ mnpbem_status hmat_mv(const HmatDev& h, int N, const double2* x1, const double2*
   const int64_t cnt = (int64_t)h.n * N;
   // CTAs per leaf: at least two waves of CTAs over the SMs, at least 8 rows per CTA
   const int rs = (int)std::max<int64_t>(1, std::min<int64_t>(cdiv_up(2 * 152, 4 * (int64_t)h.nleaf), 4));
-  k_split_x<<<(unsigned)std::min<int64_t>(cdiv_up(cnt, 256), 4096), 256, 0, st>>>(x1, x2, cnt, h.xs);
+  k_split_x<<<(unsigned)std::min<int64_t>(cdiv_up(cnt, 256), 4096), 256, 0, st>>>(x1, x2, h.perm, h.n, N, h.xs);
 #define HMV_CASE(NN)                                                                  \
   case NN:                                                                            \
     if (h.nlow > 0) k_hmv_t<NN><<<dim3((unsigned)h.nlow, 4), 256, 0, st>>>(h);        \
