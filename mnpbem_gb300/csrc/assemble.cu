@@ -9,6 +9,7 @@
 // One pass writes G1, H1, G2, H2 as complex128 and/or complex64 (row-major, ld).
 #include "assemble.cuh"
 #include "cis.cuh"
+#include "ds_math.cuh"
 #include "profile.cuh"
 
 #include <atomic>
@@ -150,19 +151,33 @@ __global__ void __launch_bounds__(ASM_COLS) k_asm_far(AsmParams p) {
 // full (near-field) blocks of the H-matrices: entries of the complete Green
 // function on leaf pairs of the cluster tree, FP64, block b row-major at
 // val[q] + foff[b] (Greenfun/@hmatrix/fillval.m with compgreenret's eval)
+// Bound by the FP64 pipe (24.8 million pairs at 6000 faces: 5.6 ms alone).  One CTA
+// per SM over slices of the blocks' rows keeps that pipe busy and leaves the rest
+// of the SM to the kernels of the dense preconditioner, which run beside it.
+// split: values stored as (hi, lo) float pairs, as the products read them; a pass
+// over the stored values took 1.4 ms.
+constexpr int LEAF_SLICES = 16;
+__device__ __forceinline__ void leaf_store(const LeafAsm& la, int64_t o, const Val4& v) {
+  const double2 w[4] = {v.g1, v.h1, v.g2, v.h2};
+#pragma unroll
+  for (int q = 0; q < 4; ++q) {
+    if (la.split) reinterpret_cast<float4*>(la.val[q])[o] = split4(w[q]);
+    else la.val[q][o] = w[q];
+  }
+}
 __global__ void __launch_bounds__(256) k_asm_leaf(AsmParams p, LeafAsm la) {
   __shared__ CisTable T;
   cis_load(T, &g_cis);
-  const int b = blockIdx.x;
-  const int4 blk = la.fblk[b];   // (r0, m, c0, nb)
-  const int64_t cnt = (int64_t)blk.y * blk.w;
-  const int64_t off = la.foff[b];
-  for (int64_t e = threadIdx.x; e < cnt; e += blockDim.x) {
-    const int r = (int)(e / blk.w), c = (int)(e - (int64_t)r * blk.w);
-    const int i = la.perm[blk.x + r], j = la.perm[blk.z + c];
-    const Val4 v = far4(p, T, i, p.src[j], p.part[j]);
-    la.val[0][off + e] = v.g1; la.val[1][off + e] = v.h1;
-    la.val[2][off + e] = v.g2; la.val[3][off + e] = v.h2;
+  for (int64_t it = blockIdx.x; it < (int64_t)la.nfull * LEAF_SLICES; it += gridDim.x) {
+    const int b = (int)(it / LEAF_SLICES), s = (int)(it % LEAF_SLICES);
+    const int4 blk = la.fblk[b];   // (r0, m, c0, nb)
+    const int64_t beg = (int64_t)blk.y * s / LEAF_SLICES * blk.w, end = (int64_t)blk.y * (s + 1) / LEAF_SLICES * blk.w;
+    const int64_t off = la.foff[b];
+    for (int64_t e = beg + threadIdx.x; e < end; e += blockDim.x) {
+      const int r = (int)(e / blk.w), c = (int)(e - (int64_t)r * blk.w);
+      const int i = la.perm[blk.x + r], j = la.perm[blk.z + c];
+      leaf_store(la, off + e, far4(p, T, i, p.src[j], p.part[j]));
+    }
   }
 }
 
@@ -457,15 +472,14 @@ __global__ void k_asm_leaf_near(AsmParams p, LeafAsm la) {
   if (b < 0) return;
   const int4 blk = la.fblk[b];
   const int64_t o = la.foff[b] + (int64_t)(ci - blk.x) * blk.w + (cj - blk.z);
-  const Val4 v = near4(p, e, i, j);
-  la.val[0][o] = v.g1; la.val[1][o] = v.h1; la.val[2][o] = v.g2; la.val[3][o] = v.h2;
+  leaf_store(la, o, near4(p, e, i, j));
 }
 
 mnpbem_status assemble_leaves(const AsmParams& p, const LeafAsm& la, cudaStream_t st) {
   MNP_TRY(ensure_cis(st));
   if (la.nfull > 0) {
     ProfScope ps(PH_HMAT_BUILD, st, 0.0, 64.0 * (double)la.nvals, p.nref > 0 ? 2 : 1);
-    k_asm_leaf<<<la.nfull, 256, 0, st>>>(p, la);
+    k_asm_leaf<<<(unsigned)std::min<int64_t>((int64_t)la.nfull * LEAF_SLICES, 152), 256, 0, st>>>(p, la);
     MNP_CHECK_LAUNCH();
     if (p.nref > 0) {
       k_asm_leaf_near<<<(unsigned)cdiv_up(p.nref, 128), 128, 0, st>>>(p, la);

@@ -47,6 +47,7 @@ struct LeafAsm {
   const int* leaf_of = nullptr;  // [n] leaf index of each cluster position
   const int* fidx = nullptr;     // [nleaf][nleaf] full block of a leaf pair, -1 if none
   double2* val[4] = {};          // G1, H1, G2, H2 block values, row-major per block
+  bool split = false;            // values as float4 (hi.re, hi.im, lo.re, lo.im) instead of complex128
 };
 mnpbem_status assemble_leaves(const AsmParams& p, const LeafAsm& la, cudaStream_t st);
 

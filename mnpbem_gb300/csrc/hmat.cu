@@ -325,9 +325,9 @@ __device__ __forceinline__ void split_in_place(double2* p, int64_t i) {
 
 __global__ void k_split_vals(double2* v0, double2* v1, double2* v2, double2* v3, int64_t count) {
   double2* v[4] = {v0, v1, v2, v3};
-  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < 4 * count;
-       e += (int64_t)gridDim.x * blockDim.x)
-    split_in_place(v[e / count], e % count);
+  for (int64_t e = (int64_t)blockIdx.x * blockDim.x + threadIdx.x; e < count; e += (int64_t)gridDim.x * blockDim.x)
+#pragma unroll
+    for (int q = 0; q < 4; ++q) split_in_place(v[q], e);
 }
 
 __global__ void k_split_factors(HmatDev h) {
@@ -447,10 +447,10 @@ mnpbem_status hmat_aca(const AsmParams& p, const HmatDev& h, cudaStream_t st) {
   return MNPBEM_OK;
 }
 
-mnpbem_status hmat_split(const HmatDev& h, cudaStream_t st) {
-  ProfScope ps(PH_HMAT_BUILD, st, 0.0, 0.0, h.nlow > 0 ? 2 : 1);
-  if (h.nvals > 0)
-    k_split_vals<<<(unsigned)std::min<int64_t>(cdiv_up(4 * h.nvals, 256), 8192), 256, 0, st>>>(
+mnpbem_status hmat_split(const HmatDev& h, bool values, cudaStream_t st) {
+  ProfScope ps(PH_HMAT_BUILD, st, 0.0, 0.0, (h.nlow > 0) + (values && h.nvals > 0));
+  if (values && h.nvals > 0)
+    k_split_vals<<<(unsigned)std::min<int64_t>(cdiv_up(h.nvals, 256), 8192), 256, 0, st>>>(
         h.val[0], h.val[1], h.val[2], h.val[3], h.nvals);
   if (h.nlow > 0) k_split_factors<<<dim3((unsigned)h.nlow, 4), 256, 0, st>>>(h);
   MNP_CHECK_LAUNCH();
@@ -466,8 +466,11 @@ mnpbem_status hmat_mv(const HmatDev& h, int N, const double2* x1, const double2*
   YPtrs ys{{y[0], y[1], y[2], y[3]}};
   ProfScope ps(PH_HMAT_MV, st, 0.0, bytes, h.nlow > 0 ? 3 : 2);
   const int64_t cnt = (int64_t)h.n * N;
-  // CTAs per leaf: at least two waves of CTAs over the SMs, at least 8 rows per CTA
-  const int rs = (int)std::max<int64_t>(1, std::min<int64_t>(cdiv_up(2 * 152, 4 * (int64_t)h.nleaf), 4));
+  // CTAs per leaf: one group of rows per warp at the mean leaf size, so that the CTAs
+  // are many and short (32 leaves of 188 rows, N = 4: 817 us, with three CTAs per
+  // leaf 1102; four rows per warp 918)
+  const int rows = N <= 8 ? 16 : 8;
+  const int rs = (int)std::max<int64_t>(1, std::min<int64_t>(cdiv_up(h.n, rows * (int64_t)std::max(1, h.nleaf)), 32));
   k_split_x<<<(unsigned)std::min<int64_t>(cdiv_up(cnt, 256), 4096), 256, 0, st>>>(x1, x2, h.perm, h.n, N, h.xs);
 #define HMV_CASE(NN)                                                                  \
   case NN:                                                                            \

@@ -45,9 +45,9 @@ struct HmatDev {
 // low-rank blocks of the four matrices by ACA (mex/hlib/aca.cpp restated,
 // kernel of mex/acagreen/acagreen.cpp greenret::getrow / getcol)
 mnpbem_status hmat_aca(const AsmParams& p, const HmatDev& h, cudaStream_t st);
-// values and right factors -> (hi, lo) float4 in place, left factors -> At
-// (row-major, split) (after hmat_aca)
-mnpbem_status hmat_split(const HmatDev& h, cudaStream_t st);
+// right factors (and, if asked for, values) -> (hi, lo) float4 in place, left
+// factors -> At (row-major, split) (after hmat_aca)
+mnpbem_status hmat_split(const HmatDev& h, bool values, cudaStream_t st);
 // y[q] = H_q x (x = x1 for q = 0, 1; x2 for q = 2, 3); x, y [n][N] in face order, N <= 16;
 // double-single arithmetic on the split values (FP32 pipe, ~1e-14 relative)
 // bytes: algorithmic bytes of the product (for the profiler)
