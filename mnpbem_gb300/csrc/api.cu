@@ -111,14 +111,16 @@ struct Lane {
   GJWork<double> gj64;
   LDUWork<float> lu32;   // block LDU factors of G1, G2, Sigma
   LDUWork<double> lu64;
+  LDUWork<float> lu32b;  // G1's factorisation, which runs beside G2's on the side stream
+  LDUWork<double> lu64b;
   DevBuf lu_status;      // LDU status words (see dense.cuh)
   DevBuf lu_ctl, lu_tmp; // control words and intermediate vectors of the triangular sweeps
-  TcGemmCtx tc;
-  int* status_host = nullptr;     // pinned: Gauss-Jordan (4), LDU (2), tensor-core error word (1), spare
+  TcGemmCtx tc, tcb;     // tcb: products queued on the side stream
+  int* status_host = nullptr;     // pinned: Gauss-Jordan (4), LDU (2), tensor-core error words (2)
   double* norms_host = nullptr;   // pinned: refinement norms (4)
   cudaEvent_t ev = nullptr;       // completion of the work last queued by the scheduler
-  cudaStream_t side = nullptr;    // work beside the lane's own (made by side_fork)
-  cudaEvent_t side_ev = nullptr;
+  cudaStream_t side[2] = {};      // work beside the lane's own (SideStream): 0 G1's chain, 1 H-matrices
+  cudaEvent_t side_ev[2] = {};
   struct Graphs {
     bool valid = false;
     int precision = -1, P = 0, ninf = 0;
@@ -213,7 +215,10 @@ mnpbem_status check_geom(const mnpbem_geom* g) {
 
 void lane_release(Lane& L) {
   if (L.st) cudaStreamSynchronize(L.st);
+  for (cudaStream_t q : L.side)
+    if (q) cudaStreamSynchronize(q);
   tc_release(L.tc);
+  tc_release(L.tcb);
   for (int q = 0; q < NSTAGES; ++q) {
     if (L.graphs.exec[q]) cudaGraphExecDestroy(L.graphs.exec[q]);
     L.graphs.exec[q] = nullptr;
@@ -229,37 +234,36 @@ void lane_release(Lane& L) {
   L.norms_host = nullptr;
   L.ev = nullptr;
   L.st = nullptr;
-  if (L.side) {
-    cudaStreamSynchronize(L.side);
-    cudaStreamDestroy(L.side);
+  for (int q = 0; q < 2; ++q) {
+    if (L.side[q]) cudaStreamDestroy(L.side[q]);
+    if (L.side_ev[q]) cudaEventDestroy(L.side_ev[q]);
+    L.side[q] = nullptr;
+    L.side_ev[q] = nullptr;
   }
-  if (L.side_ev) cudaEventDestroy(L.side_ev);
-  L.side = nullptr;
-  L.side_ev = nullptr;
 }
 
-// the lane's second stream, ordered after what the lane has queued; join orders the
-// lane after it.  An early return waits for it, as it uses buffers of the caller.
+// a second stream of the lane, ordered after what the lane has queued; join orders
+// the lane after it.  An early return waits for it, as it uses buffers of the caller.
 struct SideStream {
   Lane& L;
+  const int q;
   bool open = false;
-  explicit SideStream(Lane& l) : L(l) {}
+  SideStream(Lane& l, int which) : L(l), q(which) {}
+  cudaStream_t st() const { return L.side[q]; }
   mnpbem_status fork() {
-    if (!L.side) MNP_CUDA(cudaStreamCreateWithFlags(&L.side, cudaStreamNonBlocking));
-    if (!L.side_ev) MNP_CUDA(cudaEventCreateWithFlags(&L.side_ev, cudaEventDisableTiming));
-    MNP_CUDA(cudaEventRecord(L.side_ev, L.st));
-    MNP_CUDA(cudaStreamWaitEvent(L.side, L.side_ev, 0));
+    MNP_CUDA(cudaEventRecord(L.side_ev[q], L.st));
+    MNP_CUDA(cudaStreamWaitEvent(L.side[q], L.side_ev[q], 0));
     open = true;
     return MNPBEM_OK;
   }
   mnpbem_status join() {
-    MNP_CUDA(cudaEventRecord(L.side_ev, L.side));
-    MNP_CUDA(cudaStreamWaitEvent(L.st, L.side_ev, 0));
+    MNP_CUDA(cudaEventRecord(L.side_ev[q], L.side[q]));
+    MNP_CUDA(cudaStreamWaitEvent(L.st, L.side_ev[q], 0));
     open = false;
     return MNPBEM_OK;
   }
   ~SideStream() {
-    if (open) cudaStreamSynchronize(L.side);
+    if (open && !capturing_now()) cudaStreamSynchronize(L.side[q]);
   }
 };
 
@@ -274,6 +278,10 @@ mnpbem_status add_lane(mnpbem_geom* G) {
   cudaError_t e = cudaMallocHost(&L->status_host, LANE_NSTATUS * sizeof(int));
   if (e == cudaSuccess) e = cudaMallocHost(&L->norms_host, 4 * sizeof(double));
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&L->ev, cudaEventDisableTiming);
+  for (int q = 0; q < 2; ++q) {
+    if (e == cudaSuccess) e = cudaEventCreateWithFlags(&L->side_ev[q], cudaEventDisableTiming);
+    if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&L->side[q], cudaStreamNonBlocking);
+  }
   mnpbem_status s = MNPBEM_OK;
   if (e != cudaSuccess) {
     cudaGetLastError();
@@ -955,10 +963,10 @@ size_t lane_bytes_estimate(const mnpbem_geom* G, int precision, int P, int ninf)
   const size_t es = precision == MNPBEM_FP64 ? sizeof(double2) : sizeof(float2);
   size_t b = 5 * es * n * ld;
   // hi / lo planes, B' of the rank-1024 products and the LDU panels
-  if (precision == MNPBEM_MIXED) b += 4 * 2 * sizeof(float2) * n * ld + 3 * 8 * 1024 * n;
-  else b += 3 * 2048 * n;   // digit slices of the complex128 products
+  if (precision == MNPBEM_MIXED) b += 4 * 2 * sizeof(float2) * n * ld + 6 * 8 * 1024 * n;
+  else b += 6 * 2048 * n;   // digit slices of the complex128 products
   b += sizeof(double2) * n * P * 80 + sizeof(float2) * n * P * 56;
-  b += 3 * es * n * 256 + sizeof(double2) * (size_t)(P + ninf) * 6 * P + 64 * n;
+  b += 6 * es * n * 256 + sizeof(double2) * (size_t)(P + ninf) * 6 * P + 64 * n;
   return b;
 }
 
@@ -995,6 +1003,8 @@ uint64_t lane_sig(const mnpbem_geom* G, const Lane& L) {
   mixbuf(L.outbuf); mixbuf(L.bsplit); mixbuf(L.lp_dev); mixbuf(G->exbuf);
   mixbuf(L.tc.bexp); mixbuf(L.tc.err); mixbuf(L.tc.a16); mixbuf(L.tc.scales); mixbuf(L.tc.ctr);
   mixbuf(L.tc.a8); mixbuf(L.tc.b8); mixbuf(L.tc.exps);
+  mixbuf(L.tcb.bexp); mixbuf(L.tcb.err); mixbuf(L.tcb.a16); mixbuf(L.tcb.scales); mixbuf(L.tcb.ctr);
+  mixbuf(L.tcb.a8); mixbuf(L.tcb.b8); mixbuf(L.tcb.exps);
   auto gj = [&](const auto& w) {
     mixbuf(w.ccol); mixbuf(w.rrow); mixbuf(w.ncol); mixbuf(w.xblk); mixbuf(w.status); mixbuf(w.pan);
     mix(nullptr, (size_t)w.nb);
@@ -1012,6 +1022,8 @@ uint64_t lane_sig(const mnpbem_geom* G, const Lane& L) {
   };
   lu(L.lu32);
   lu(L.lu64);
+  lu(L.lu32b);
+  lu(L.lu64b);
   mixbuf(L.lu_status);
   mixbuf(L.lu_ctl); mixbuf(L.lu_tmp);
   mix(nullptr, (size_t)G->lu_steps);
@@ -1083,6 +1095,9 @@ template <typename R>
 LDUWork<R>& luw(Lane& L);
 template <> LDUWork<float>& luw<float>(Lane& L) { return L.lu32; }
 template <> LDUWork<double>& luw<double>(Lane& L) { return L.lu64; }
+template <typename R> LDUWork<R>& luwb(Lane& L);
+template <> LDUWork<float>& luwb<float>(Lane& L) { return L.lu32b; }
+template <> LDUWork<double>& luwb<double>(Lane& L) { return L.lu64b; }
 
 void* tc_ctx(mnpbem_geom* G, Lane& L) { return G->tc_enabled ? (void*)&L.tc : nullptr; }
 
@@ -1179,15 +1194,34 @@ mnpbem_status stage_initmat(mnpbem_geom* G, Lane& L, bool direct) {
   const FaceData fd = face_data(G, L);
   const LamParams* lp = L.lp_dev.as<LamParams>();
   // G1 = LDU per diagonal block, Sigma1 = H1 G1^-1 (H1 shares G1's blocks:
-  // its off-diagonal blocks are zero and stay zero)
+  // its off-diagonal blocks are zero and stay zero).  Independent of G2's chain
+  // below, and both are bound by the latency of their pivot blocks: on a second
+  // stream.  Single solves, before and now: 284 faces 1.57 and 1.37 ms, 2016
+  // (gradient) 18.8 and 16.7, two particles of 12 000 434 and 411; sweeps, whose
+  // lanes fill the chip already, 0 (4000 faces) to 15 % (1350, complex128).
+  SideStream side(L, 0);
+  const bool beside = !G->prof.enabled;
+  LDUWork<R>& lwb = beside ? luwb<R>(L) : lw;
+  void* ctxb = ctx;
+  if (beside) {
+    lwb.b = lw.b; lwb.m = lw.m; lwb.round_a = lw.round_a;
+    if (ctx) {
+      L.tcb.stages = L.tc.stages; L.tcb.max_ctas = L.tc.max_ctas; L.tcb.pair = L.tc.pair;
+      L.tcb.f16 = L.tc.f16; L.tcb.enabled = L.tc.enabled;
+      ctxb = &L.tcb;
+    }
+    MNP_TRY(side.fork());
+  }
+  const cudaStream_t stb = beside ? side.st() : L.st;
   for (size_t q = 0; q < G->g1_off.size(); ++q) {
     const int64_t o = G->g1_off[q], nq = G->g1_n[q];
-    MNP_TRY(ldu_factor<R>(M[0] + o * ld + o, nq, ld, lw, lus, gemm_w<R>, ctx, L.st));
-    MNP_TRY(ldu_rsolve<R>(M[2] + o * ld + o, nq, ld, M[0] + o * ld + o, ld, lw, gemm_w<R>, ctx, L.st));
+    MNP_TRY(ldu_factor<R>(M[0] + o * ld + o, nq, ld, lwb, lus, gemm_w<R>, ctxb, stb));
+    MNP_TRY(ldu_rsolve<R>(M[2] + o * ld + o, nq, ld, M[0] + o * ld + o, ld, lwb, gemm_w<R>, ctxb, stb));
   }
   // G2 = LDU, Sigma2 = H2 G2^-1
   MNP_TRY(ldu_factor<R>(M[1], n, ld, lw, lus, gemm_w<R>, ctx, L.st));
   MNP_TRY(ldu_rsolve<R>(M[3], n, ld, M[1], ld, lw, gemm_w<R>, ctx, L.st));
+  if (beside) MNP_TRY(side.join());
   // Delta -> M4, Sigma (partial) -> M3
   launch_delta_sigma<R>(n, M[2], M[3], M[4], ld, fd, L.st);
   MNP_CHECK_LAUNCH();
@@ -1205,6 +1239,7 @@ mnpbem_status stage_initmat(mnpbem_geom* G, Lane& L, bool direct) {
     }
   }
   if (direct && ctx) MNP_TRY(tc_check_error(L.tc, L.st));
+  if (direct && ctx && beside) MNP_TRY(tc_check_error(L.tcb, L.st));
   if (direct) MNP_TRY(sweep_check(L.st));
   return MNPBEM_OK;
 }
@@ -1469,8 +1504,8 @@ float status_cond(const Lane& L) {
 
 mnpbem_status check_pivots(Lane& L, int precision) {
   const int* h = L.status_host;
-  if (h[6]) {
-    set_error("tensor-core GEMM: a bounded pipeline wait expired (code %d)", h[6]);
+  if (h[6] | h[7]) {
+    set_error("tensor-core GEMM: a bounded pipeline wait expired (code %d)", h[6] | h[7]);
     L.tc.enabled = false;
     return MNPBEM_ERR_TIMEOUT;
   }
@@ -1503,6 +1538,7 @@ mnpbem_status status_copy(Lane& L, int precision) {
   }
   MNP_TRY(cp(L.lu_status, 4, 2));
   if (L.tc.err.ptr && L.tc.err_cleared) MNP_TRY(cp(L.tc.err, 6, 1));
+  if (L.tcb.err.ptr && L.tcb.err_cleared) MNP_TRY(cp(L.tcb.err, 7, 1));
   return MNPBEM_OK;
 }
 
@@ -1857,18 +1893,24 @@ mnpbem_status size_like(Lane& d, const Lane& s) {
   MNP_TRY(size_gj(d.gj64, s.gj64));
   MNP_TRY(size_lu(d.lu32, s.lu32));
   MNP_TRY(size_lu(d.lu64, s.lu64));
-  MNP_TRY(d.tc.bexp.ensure(s.tc.bexp.bytes));
-  MNP_TRY(d.tc.a16.ensure(s.tc.a16.bytes));
-  MNP_TRY(d.tc.scales.ensure(s.tc.scales.bytes));
-  MNP_TRY(d.tc.a8.ensure(s.tc.a8.bytes));
-  MNP_TRY(d.tc.b8.ensure(s.tc.b8.bytes));
-  MNP_TRY(d.tc.exps.ensure(s.tc.exps.bytes));
-  MNP_TRY(d.tc.err.ensure(s.tc.err.bytes));
-  MNP_TRY(d.tc.ctr.ensure(s.tc.ctr.bytes));
-  // the host reads the error word at the end of a call even if the lane ran nothing
-  if (d.tc.err.ptr) MNP_CUDA(cudaMemsetAsync(d.tc.err.ptr, 0, sizeof(int), d.st));
-  tc_device_ready(d.tc);
-  return MNPBEM_OK;
+  MNP_TRY(size_lu(d.lu32b, s.lu32b));
+  MNP_TRY(size_lu(d.lu64b, s.lu64b));
+  const auto tc = [&](TcGemmCtx& a, const TcGemmCtx& b) -> mnpbem_status {
+    MNP_TRY(a.bexp.ensure(b.bexp.bytes));
+    MNP_TRY(a.a16.ensure(b.a16.bytes));
+    MNP_TRY(a.scales.ensure(b.scales.bytes));
+    MNP_TRY(a.a8.ensure(b.a8.bytes));
+    MNP_TRY(a.b8.ensure(b.b8.bytes));
+    MNP_TRY(a.exps.ensure(b.exps.bytes));
+    MNP_TRY(a.err.ensure(b.err.bytes));
+    MNP_TRY(a.ctr.ensure(b.ctr.bytes));
+    // the host reads the error word at the end of a call even if the lane ran nothing
+    if (a.err.ptr) MNP_CUDA(cudaMemsetAsync(a.err.ptr, 0, sizeof(int), d.st));
+    tc_device_ready(a);
+    return MNPBEM_OK;
+  };
+  MNP_TRY(tc(d.tc, s.tc));
+  return tc(d.tcb, s.tcb);
 }
 
 // without graphs for this configuration on any lane, one lane runs a wavelength
@@ -2065,7 +2107,7 @@ __global__ void k_sw_next(JobCtl* jc, SweepCtl* sc, const LamParams* lps, LamPar
 
 // status words of the wavelength's initmat (the layout of Lane::status_host)
 __global__ void k_sw_status(const SweepCtl* sc, const int* gj, const int* gji, const int* lu, const int* tce,
-                            const SweepDst* dp) {
+                            const int* tcb, const SweepDst* dp) {
   if (threadIdx.x) return;
   atomicAdd(dp->stages + 0, 1ull);
   atomicAdd(dp->stages + 1, 1ull);
@@ -2077,6 +2119,7 @@ __global__ void k_sw_status(const SweepCtl* sc, const int* gj, const int* gji, c
   if (gji) { o[2] = gji[0]; o[3] = gji[1]; }
   if (lu) { o[4] = lu[0]; o[5] = lu[1]; }
   if (tce) o[6] = tce[0];
+  if (tcb) o[7] = tcb[0];
 }
 
 __global__ void k_ref_init(SweepCtl* sc, cudaGraphConditionalHandle h, int run, const SweepDst* dp) {
@@ -2184,6 +2227,7 @@ cudaError_t build_lane_branch(mnpbem_geom* G, Lane& L, const SolveCtx& c, const 
   cudaError_t e = cudaGraphConditionalHandleCreate(&hq, top, 0, 0);
   if (e != cudaSuccess) return e;
   const int* stc = (L.tc.err.ptr && L.tc.err_cleared) ? L.tc.err.as<int>() : nullptr;
+  const int* stcb = (L.tcb.err.ptr && L.tcb.err_cleared) ? L.tcb.err.as<int>() : nullptr;
   cudaGraphNode_t first, loop;
   void* a_next[] = {&jc, &sc, &lps, &lpd, &hq, &stc, &d};
   if ((e = add_kernel(&first, top, nullptr, 0, k_sw_next, 1, 32, a_next)) != cudaSuccess) return e;
@@ -2199,7 +2243,7 @@ cudaError_t build_lane_branch(mnpbem_geom* G, Lane& L, const SolveCtx& c, const 
   const int* sgji = f64 ? (g64.inner ? g64.inner->status.as<int>() : nullptr)
                         : (g32.inner ? g32.inner->status.as<int>() : nullptr);
   const int* slu = L.lu_status.as<int>();
-  void* a_st[] = {&sc, &sgj, &sgji, &slu, &stc, &d};
+  void* a_st[] = {&sc, &sgj, &sgji, &slu, &stc, &stcb, &d};
   if ((e = add_kernel(&nst, body, &n1, 1, k_sw_status, 1, 32, a_st)) != cudaSuccess) return e;
   if ((e = cudaGraphAddChildGraphNode(&n2, body, &nst, 1, gr.graph[2])) != cudaSuccess) return e;
   const bool refine = c.precision == MNPBEM_MIXED && s.ref.maxit > 0;
@@ -2527,7 +2571,10 @@ mnpbem_status job_finish(Job& j, bool failed) {
   for (int l = 0; l < j.nl; ++l) {
     Lane& L = *G->lanes[l];
     MNP_TRY(check_pivots(L, j.c.precision));
-    if (j.c.precision == MNPBEM_MIXED && G->tc_enabled) MNP_TRY(tc_check_error(L.tc, L.st));
+    if (j.c.precision == MNPBEM_MIXED && G->tc_enabled) {
+      MNP_TRY(tc_check_error(L.tc, L.st));
+      MNP_TRY(tc_check_error(L.tcb, L.st));
+    }
   }
   MNP_TRY(sweep_check(G->st));
   return MNPBEM_OK;
@@ -3812,11 +3859,11 @@ mnpbem_status iter_prepare(mnpbem_geom* G, Job& j, const double2* ext_pot, HmatH
   // The H-matrices (FP64 pipe) are independent of the dense preconditioner (chains
   // of short tensor-core kernels): they are filled beside it on a second stream
   // (6000 faces: 9.7 ms of kernels, 5 of which the chains hide)
-  SideStream side(L);
+  SideStream side(L, 1);
   const bool beside = o.precond == 1 && !keep && !G->prof.enabled;
   if (beside) {
     MNP_TRY(side.fork());
-    MNP_TRY(hmat_queue(G, L, H, true, L.side));
+    MNP_TRY(hmat_queue(G, L, H, true, side.st()));
   }
   if (o.precond == 1 && !keep) {
     MNP_TRY(run_stage(G, L, j.c, 0, true));   // per-face eps + dense matrices
