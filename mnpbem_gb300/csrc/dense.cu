@@ -1298,26 +1298,69 @@ void round_tf32(float* x, int64_t count, cudaStream_t st) {
   k_round_tf32<<<(unsigned)cdiv_up(count, 256), 256, 0, st>>>(x, count);
 }
 
-// Ccol[n][bw] <- A[:, k0 .. k0 + bw) with the rows k0 .. k0 + bw zeroed and,
-// if rna, rounded to TF32 (nearest): the A operand of the column-panel product
-// and of the rank update of one fused Gauss-Jordan step.
-__global__ void k_gj_take_col(const float2* __restrict__ A, int64_t lda, int64_t n, int64_t k0, int bw,
-                              float2* __restrict__ Ccol, int rna) {
+__device__ __forceinline__ float rna_tf32(float x) {
+  uint32_t r;
+  asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(r) : "f"(x));
+  return __uint_as_float(r);
+}
+// dst[rows][cols] (row stride ldd) <- src[rows][cols] (row stride lds),
+// rounded to TF32 (nearest) when rna: the A operand of a tensor-core product;
+// rows z0 .. z1 - 1 become zero
+template <typename R>
+__global__ void k_copy_panel(const cplx<R>* __restrict__ src, int64_t lds, int64_t rows, int cols,
+                             cplx<R>* __restrict__ dst, int64_t ldd, int rna, int64_t z0, int64_t z1) {
   const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= n * bw) return;
-  const int64_t i = idx / bw;
-  const int c = (int)(idx - i * bw);
-  float2 v = make_float2(0.f, 0.f);
-  if (i < k0 || i >= k0 + bw) {
-    v = A[i * lda + k0 + c];
-    if (rna) {
-      uint32_t x, y;
-      asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(x) : "f"(v.x));
-      asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(y) : "f"(v.y));
-      v = make_float2(__uint_as_float(x), __uint_as_float(y));
+  if (idx >= rows * cols) return;
+  const int64_t i = idx / cols;
+  const int c = (int)(idx - i * cols);
+  cplx<R> v = (i >= z0 && i < z1) ? mk<R>(0, 0) : src[i * lds + c];
+  if constexpr (sizeof(R) == 4)
+    if (rna) v = mk<R>(rna_tf32(v.x), rna_tf32(v.y));
+  dst[i * ldd + c] = v;
+}
+// The same for complex64 in 16-byte pieces (even strides and columns, aligned
+// bases): four loads in flight per thread.  Bound by HBM at 24 000 rows and by its
+// share of the SMs beside other wavelengths' kernels at 4000: the panels of a
+// 24 000-face solve 12.8 ms in single entries, 11.7 now; sweep of 4000 faces, eight
+// wavelengths in flight, 121 and 117 ms.
+__global__ void __launch_bounds__(256) k_copy_panel4(const float2* __restrict__ src, int64_t lds, unsigned total,
+                                                   unsigned cols2, float2* __restrict__ dst, int64_t ldd, int rna,
+                                                   int64_t z0, int64_t z1) {
+  float4 v[4];
+  unsigned row[4], col[4];
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    const unsigned idx = blockIdx.x * 1024u + 256u * u + threadIdx.x;
+    row[u] = idx / cols2;
+    col[u] = 2 * (idx - row[u] * cols2);
+    v[u] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (idx < total && (row[u] < z0 || row[u] >= z1))
+      v[u] = *reinterpret_cast<const float4*>(src + (int64_t)row[u] * lds + col[u]);
+  }
+#pragma unroll
+  for (int u = 0; u < 4; ++u) {
+    if (blockIdx.x * 1024u + 256u * u + threadIdx.x >= total) break;
+    if (rna) v[u] = make_float4(rna_tf32(v[u].x), rna_tf32(v[u].y), rna_tf32(v[u].z), rna_tf32(v[u].w));
+    *reinterpret_cast<float4*>(dst + (int64_t)row[u] * ldd + col[u]) = v[u];
+  }
+}
+
+template <typename R>
+static void copy_panel(const cplx<R>* src, int64_t lds, int64_t rows, int cols, cplx<R>* dst, int64_t ldd, bool rna,
+                       cudaStream_t st, int64_t z0 = 0, int64_t z1 = 0) {
+  if (rows <= 0 || cols <= 0) return;
+  ProfScope ps(PH_ELEMWISE, st, 0.0, 2.0 * sizeof(cplx<R>) * rows * cols, 1);
+  const int64_t cnt = rows * cols;
+  if constexpr (sizeof(R) == 4) {
+    const uintptr_t al = reinterpret_cast<uintptr_t>(src) | reinterpret_cast<uintptr_t>(dst);
+    if (!((lds | ldd | cols) & 1) && !(al & 15) && cnt < (1ll << 32)) {
+      k_copy_panel4<<<(unsigned)cdiv_up(cnt / 2, (int64_t)1024), 256, 0, st>>>(
+          src, lds, (unsigned)(cnt / 2), (unsigned)(cols / 2), dst, ldd, rna ? 1 : 0, z0, z1);
+      return;
     }
   }
-  Ccol[idx] = v;
+  k_copy_panel<R><<<(unsigned)cdiv_up(cnt, (int64_t)256), 256, 0, st>>>(src, lds, rows, cols, dst, ldd, rna ? 1 : 0, z0,
+                                                                        z1);
 }
 
 // --------------------------------------------------- blocked Gauss-Jordan
@@ -1388,12 +1431,10 @@ mnpbem_status gj_invert(cplx<R>* A, int64_t n, int64_t lda, GJWork<R>& w, GemmFn
                                      st));
           MNP_TRY(gj_invert<R>(X, bw, bw, *w.inner, big_gemm, ctx, st));
         }
-        {
-          ProfScope ps(PH_ELEMWISE, st, 0.0, 16.0 * n * bw, 1);
-          k_gj_take_col<<<(unsigned)cdiv_up(n * bw, (int64_t)256), 256, 0, st>>>(Af, lda, n, k0, bw, Cf,
-                                                                                 w.round_a ? 1 : 0);
-          MNP_CHECK_LAUNCH();
-        }
+        // the column panel without the pivot rows: the A operand of the column-panel
+        // product and of the rank update
+        copy_panel<float>(Af + k0, lda, n, bw, Cf, bw, w.round_a, st, k0, k0 + bw);
+        MNP_CHECK_LAUNCH();
         MNP_TRY(tc_gemm_c64(*tc, bw, n, bw, b1, Xf, bw, Af + k0 * lda, lda, b0, Af + k0 * lda, lda, st));
         MNP_TRY(tc_gemm_c64(*tc, n, bw, bw, make_float2(-1.f, 0.f), Cf, bw, Xf, bw, b0, Af + k0, lda, st));
         MNP_TRY(tc_gemm_c64(*tc, n, n, bw, make_float2(-1.f, 0.f), Cf, bw, Af + k0 * lda, lda, b1, Af, lda, st,
@@ -1455,36 +1496,6 @@ template mnpbem_status gj_invert<double>(double2*, int64_t, int64_t, GJWork<doub
                                          GemmFn<double>, void*, cudaStream_t, bool);
 
 // ------------------------------------------------------ block LDU factors
-// dst[rows][cols] (row stride ldd) <- src[rows][cols] (row stride lds),
-// rounded to TF32 (nearest) when rna: the A operand of a tensor-core product
-template <typename R>
-__global__ void k_copy_panel(const cplx<R>* __restrict__ src, int64_t lds, int64_t rows, int cols,
-                             cplx<R>* __restrict__ dst, int64_t ldd, int rna) {
-  const int64_t idx = (int64_t)blockIdx.x * blockDim.x + threadIdx.x;
-  if (idx >= rows * cols) return;
-  const int64_t i = idx / cols;
-  const int c = (int)(idx - i * cols);
-  cplx<R> v = src[i * lds + c];
-  if constexpr (sizeof(R) == 4) {
-    if (rna) {
-      uint32_t x, y;
-      asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(x) : "f"(v.x));
-      asm("cvt.rna.tf32.f32 %0, %1;" : "=r"(y) : "f"(v.y));
-      v = mk<R>(__uint_as_float(x), __uint_as_float(y));
-    }
-  }
-  dst[i * ldd + c] = v;
-}
-
-template <typename R>
-static void copy_panel(const cplx<R>* src, int64_t lds, int64_t rows, int cols, cplx<R>* dst, int64_t ldd, bool rna,
-                       cudaStream_t st) {
-  if (rows <= 0 || cols <= 0) return;
-  ProfScope ps(PH_ELEMWISE, st, 0.0, 2.0 * sizeof(cplx<R>) * rows * cols, 1);
-  const int64_t cnt = rows * cols;
-  k_copy_panel<R><<<(unsigned)cdiv_up(cnt, (int64_t)256), 256, 0, st>>>(src, lds, rows, cols, dst, ldd, rna ? 1 : 0);
-}
-
 // A_kk <- inv(A_kk) in place, with a copy in X (ld bw): 64-wide blocks with
 // partial pivoting, 256-wide complex64 blocks on a CTA cluster, whose copy in X
 // is rounded to TF32 (nearest) for the tensor-core products (the tensor cores
