@@ -457,7 +457,7 @@ def fp64_full(a, torch, mixed):
     err_sca = float(np.max(np.abs(rmx["sca"][0] - r64["sca"][0]) / np.abs(r64["sca"][0])))
     return {"value": 1.0 / t64, "unit": UNIT, "seconds": t64,
             "sample": "1 wavelength (%g nm) of the same %d-face workload through the FP64 path (block LU + "
-                      "triangular solves + Gauss-Jordan inverse on CUDA-core FP64 GEMMs), host wall clock "
+                      "triangular solves + Gauss-Jordan inverse on FP64-class GEMMs), host wall clock "
                       "around bemsolver.spectrum" % (lam, a.faces),
             "ext_rel_err_mixed_vs_fp64": err_ext, "sca_rel_err_mixed_vs_fp64": err_sca,
             "mixed_refine_tol": a.refine_tol}
