@@ -37,15 +37,28 @@ __device__ __forceinline__ void cis_load(CisTable& t, const CisTable* src) {
   __syncthreads();
 }
 
-// exp(i k d) for complex k (Im k >= 0 for passive media; any sign works)
+// exp(i k d) for complex k (Im k >= 0 for passive media; any sign works).  SHIFT:
+// j by adding 1.5 2^52, whose low word is j (two FP64 operations instead of a
+// product, a rounding and a conversion; the last bits may differ, as a phase next to
+// the middle of two table entries may go to the other)
+template <bool SHIFT = false>
 __device__ __forceinline__ double2 cis_exp(const CisTable& T, double2 k, double d) {
   const double th = k.x * d;
-  const double jf = rint(th * CIS_INV);
+  double jf;
+  int j;
+  if constexpr (SHIFT) {
+    const double jm = fma(th, CIS_INV, 6755399441055744.0);
+    j = __double2loint(jm);
+    jf = jm - 6755399441055744.0;
+  } else {
+    jf = rint(th * CIS_INV);
+    j = (int)((long long)jf & (CIS_N - 1));
+  }
   const double t = fma(-jf, CIS_C2, fma(-jf, CIS_C1, th));
   const double t2 = t * t;
   const double sn = t * fma(t2, fma(t2, fma(t2, -1.0 / 5040.0, 1.0 / 120.0), -1.0 / 6.0), 1.0);
   const double cn = fma(t2, fma(t2, fma(t2, fma(t2, 1.0 / 40320.0, -1.0 / 720.0), 1.0 / 24.0), -0.5), 1.0);
-  const double2 tb = T.cs[((long long)jf) & (CIS_N - 1)];
+  const double2 tb = T.cs[j & (CIS_N - 1)];
   double cr = tb.x * cn - tb.y * sn;
   double sr = fma(tb.y, cn, tb.x * sn);
   if (k.y != 0.0) {
