@@ -1,5 +1,6 @@
-// Dense complex kernels: SIMT GEMM, shared-memory block inversion and the
-// blocked Gauss-Jordan inversion that replaces MATLAB's inv() in
+// Dense complex kernels: SIMT products (general, few tiles, few columns), block
+// inverses, and the block LDU factors, their triangular sweeps and the blocked
+// Gauss-Jordan inversion that replace MATLAB's inv() in
 // BEM/@bemret/private/initmat.m:27-28,50,72.
 //
 // Gauss-Jordan without row interchanges: the matrices inverted by bemret
