@@ -259,8 +259,9 @@ MNPBEM_API mnpbem_status mnpbem_gemm_c64(int32_t device, int32_t path, int64_t M
 
 /* Complex128 GEMM C = alpha A B + beta C (row-major, interleaved complex, real
  * alpha and beta) on host buffers: path 0 = CUDA cores (FP64), path 1 = tensor
- * cores on FP16 digit slices with FP64-class results (alpha = +-1, beta 0 or 1,
- * 16 <= K <= 64, M, N >= 16; else MNPBEM_ERR_UNSUPPORTED).  The building block of the
+ * cores on FP16 digit slices, every entry within the error bound of an FP64 sum of
+ * its own terms (alpha = +-1, beta 0 or 1, 16 <= K <= 64, M, N >= 16; else
+ * MNPBEM_ERR_UNSUPPORTED).  The building block of the
  * FP64 factorisations and products of initmat.m.                              */
 MNPBEM_API mnpbem_status mnpbem_gemm_c128(int32_t device, int32_t path, int64_t M, int64_t N, int64_t K,
                                           double alpha, const double* A, int64_t lda, const double* B,

@@ -964,7 +964,7 @@ size_t lane_bytes_estimate(const mnpbem_geom* G, int precision, int P, int ninf)
   size_t b = 5 * es * n * ld;
   // hi / lo planes, B' of the rank-1024 products and the LDU panels
   if (precision == MNPBEM_MIXED) b += 4 * 2 * sizeof(float2) * n * ld + 6 * 8 * 1024 * n;
-  else b += 6 * 2048 * n;   // digit slices of the complex128 products
+  else b += 7 * 2048 * n;   // digit slices of the complex128 products
   b += sizeof(double2) * n * P * 80 + sizeof(float2) * n * P * 56;
   b += 6 * es * n * 256 + sizeof(double2) * (size_t)(P + ninf) * 6 * P + 64 * n;
   return b;

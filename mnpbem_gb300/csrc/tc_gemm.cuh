@@ -14,7 +14,7 @@ struct TcGemmCtx {
   bool f16 = false;       // FP16 operands with power-of-two row / column scaling (kind::f16)
   int f16_min_k = 512;    // ... for products with K >= f16_min_k
   int f16_min_mn = 512;   //     and M, N >= f16_min_mn
-  DevBuf a8, b8, exps;    // complex128 products: digit slices of A and B', row / column exponents
+  DevBuf a8, b8, exps;    // complex128 products: digit slices of A and B', their rows' / columns' exponents and sums
   DevBuf err;             // device error word of the bounded waits
   DevBuf ctr;             // tile counter of the persistent kernel (zeroed before each launch)
   int num_sms = 0;
@@ -39,8 +39,9 @@ mnpbem_status tc_gemm_c64(TcGemmCtx& c, int64_t M, int64_t N, int64_t K, float2 
                           float2* C, int64_t ldc, cudaStream_t st, int64_t bz0 = 0, int64_t bz1 = 0);
 // C = alpha A B + beta C in complex128 on the tensor cores (tc_gemm64.cu):
 // operands cut into eight 8-bit digits per row of A and column of B, exact
-// products, FP64-class results.  alpha = +-1, beta 0 or 1, K <= TC64_K; A and B are
-// copied before C is written, so C may overlap them.
+// products; entries that the digits may not hold to the accuracy of an FP64 sum are
+// computed in FP64 from A and a copy of B, so C may overlap B alone.  alpha = +-1,
+// beta 0 or 1, K <= TC64_K.
 constexpr int TC64_K = 64;
 bool tc_gemm64_eligible(TcGemmCtx& c, int64_t M, int64_t N, int64_t K, double2 alpha, double2 beta);
 mnpbem_status tc_gemm_c128(TcGemmCtx& c, int64_t M, int64_t N, int64_t K, double alpha, const double2* A, int64_t lda,
