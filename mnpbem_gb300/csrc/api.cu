@@ -622,6 +622,14 @@ mnpbem_status mnpbem_geom_set_option(mnpbem_geom* g, const char* key, int32_t va
     for (auto& L : g->lanes) L->tc.f16 = g->tc_f16;
     return MNPBEM_OK;
   }
+  if (k == "selftest_tc_error") {
+    // the error words of every lane as an expired wait leaves them (tests of the reports)
+    MNP_CUDA(cudaSetDevice(g->device));
+    for (auto& L : g->lanes)
+      for (TcGemmCtx* t : {&L->tc, &L->tcb})
+        if (t->err.ptr) MNP_CUDA(cudaMemcpy(t->err.ptr, &value, sizeof(int), cudaMemcpyHostToDevice));
+    return MNPBEM_OK;
+  }
   if (k == "tc_ctas" && value >= 0 && value <= 4096) {
     g->tc_ctas = value;
     for (auto& L : g->lanes) L->tc.max_ctas = value;
@@ -1038,6 +1046,7 @@ uint64_t lane_sig(const mnpbem_geom* G, const Lane& L) {
   mix(nullptr, (size_t)G->tf32_rna);
   mix(nullptr, (size_t)G->asm_ds);
   mix(nullptr, (size_t)G->gj_fused);
+  mix(nullptr, (size_t)L.tc.enabled + 2 * (size_t)L.tcb.enabled);   // off after an expired wait
   return h;
 }
 
@@ -1238,8 +1247,10 @@ mnpbem_status stage_initmat(mnpbem_geom* G, Lane& L, bool direct) {
       return MNPBEM_ERR_SINGULAR;
     }
   }
-  if (direct && ctx) MNP_TRY(tc_check_error(L.tc, L.st));
-  if (direct && ctx && beside) MNP_TRY(tc_check_error(L.tcb, L.st));
+  if (direct && ctx) {
+    const mnpbem_status s1 = tc_check_error(L.tc, L.st), s2 = tc_check_error(L.tcb, L.st);
+    MNP_TRY(s1 != MNPBEM_OK ? s1 : s2);
+  }
   if (direct) MNP_TRY(sweep_check(L.st));
   return MNPBEM_OK;
 }
@@ -1487,7 +1498,7 @@ mnpbem_status launch_stage(mnpbem_geom* G, Lane& L, const SolveCtx& c, int stage
 //   [0] [1]  Gauss-Jordan (Deltai): pivot flag, block condition proxy (float bits)
 //   [2] [3]  the same for its inner level (pivot blocks wider than 64)
 //   [4] [5]  block LDU factors (G1, G2, Sigma): pivot flag, condition proxy
-//   [6]      tensor-core GEMM error word (a bounded wait expired)
+//   [6] [7]  tensor-core GEMM error words, lane and side stream (a bounded wait expired)
 // The condition proxy of a diagonal block is max|A_kk| * max|inv(A_kk)|; above
 // these limits its inverse has lost (nearly) every digit of the precision.
 constexpr float COND_LIMIT_32 = 1e6f, COND_LIMIT_64 = 1e13f;
@@ -1506,7 +1517,7 @@ mnpbem_status check_pivots(Lane& L, int precision) {
   const int* h = L.status_host;
   if (h[6] | h[7]) {
     set_error("tensor-core GEMM: a bounded pipeline wait expired (code %d)", h[6] | h[7]);
-    L.tc.enabled = false;
+    L.tc.enabled = L.tcb.enabled = false;
     return MNPBEM_ERR_TIMEOUT;
   }
   if (h[0] | h[2] | h[4]) {
@@ -1537,8 +1548,8 @@ mnpbem_status status_copy(Lane& L, int precision) {
     if (L.gj32.inner) MNP_TRY(cp(L.gj32.inner->status, 2, 2));
   }
   MNP_TRY(cp(L.lu_status, 4, 2));
-  if (L.tc.err.ptr && L.tc.err_cleared) MNP_TRY(cp(L.tc.err, 6, 1));
-  if (L.tcb.err.ptr && L.tcb.err_cleared) MNP_TRY(cp(L.tcb.err, 7, 1));
+  MNP_TRY(cp(L.tc.err, 6, 1));
+  MNP_TRY(cp(L.tcb.err, 7, 1));
   return MNPBEM_OK;
 }
 
@@ -1902,10 +1913,8 @@ mnpbem_status size_like(Lane& d, const Lane& s) {
     MNP_TRY(a.a8.ensure(b.a8.bytes));
     MNP_TRY(a.b8.ensure(b.b8.bytes));
     MNP_TRY(a.exps.ensure(b.exps.bytes));
-    MNP_TRY(a.err.ensure(b.err.bytes));
+    if (b.err.ptr) MNP_TRY(tc_error_word(a, d.st));
     MNP_TRY(a.ctr.ensure(b.ctr.bytes));
-    // the host reads the error word at the end of a call even if the lane ran nothing
-    if (a.err.ptr) MNP_CUDA(cudaMemsetAsync(a.err.ptr, 0, sizeof(int), d.st));
     tc_device_ready(a);
     return MNPBEM_OK;
   };
@@ -2083,7 +2092,7 @@ struct SweepDst {
   int* iters;                       // [w]
   double* res;                      // [w]
   int* status;                      // [w][LANE_NSTATUS]
-  int* nan;                         // set when a refinement step produced NaN
+  int* nan;                         // bit 0: a refinement step produced NaN; 2: a lane found an expired wait
   unsigned long long* stages;       // [NSTAGES] stage runs (the launch accounting of the replays)
   int64_t n;
   int P;
@@ -2093,9 +2102,10 @@ struct SweepDst {
 // the lane once a bounded tensor-core wait has expired or a refinement step
 // produced NaN (the host reports either after the graph)
 __global__ void k_sw_next(JobCtl* jc, SweepCtl* sc, const LamParams* lps, LamParams* lp,
-                          cudaGraphConditionalHandle h, const int* tce, const SweepDst* dp) {
+                          cudaGraphConditionalHandle h, const int* tce, const int* tcb, const SweepDst* dp) {
   if (threadIdx.x) return;
-  const bool failed = (tce && *(volatile const int*)tce) || *(volatile const int*)dp->nan;
+  if ((tce && *(volatile const int*)tce) || (tcb && *(volatile const int*)tcb)) atomicOr(dp->nan, 4);
+  const bool failed = *(volatile const int*)dp->nan != 0;
   const int w = failed ? jc->nenei : atomicAdd(&jc->next, 1);
   const bool go = w < jc->nenei;
   if (go) {
@@ -2226,10 +2236,10 @@ cudaError_t build_lane_branch(mnpbem_geom* G, Lane& L, const SolveCtx& c, const 
   cudaGraphConditionalHandle hq;
   cudaError_t e = cudaGraphConditionalHandleCreate(&hq, top, 0, 0);
   if (e != cudaSuccess) return e;
-  const int* stc = (L.tc.err.ptr && L.tc.err_cleared) ? L.tc.err.as<int>() : nullptr;
-  const int* stcb = (L.tcb.err.ptr && L.tcb.err_cleared) ? L.tcb.err.as<int>() : nullptr;
+  const int* stc = L.tc.err.as<int>();     // null: no tensor-core product ran
+  const int* stcb = L.tcb.err.as<int>();
   cudaGraphNode_t first, loop;
-  void* a_next[] = {&jc, &sc, &lps, &lpd, &hq, &stc, &d};
+  void* a_next[] = {&jc, &sc, &lps, &lpd, &hq, &stc, &stcb, &d};
   if ((e = add_kernel(&first, top, nullptr, 0, k_sw_next, 1, 32, a_next)) != cudaSuccess) return e;
   cudaGraph_t body;
   if ((e = add_cond(&loop, top, &first, 1, hq, cudaGraphCondTypeWhile, 1, &body)) != cudaSuccess) return e;
@@ -2287,7 +2297,7 @@ cudaError_t build_lane_branch(mnpbem_geom* G, Lane& L, const SolveCtx& c, const 
   void* a_out[] = {&sc, &x1, &x2, &ob, &d};
   const unsigned ob_blocks = (unsigned)std::min<int64_t>(cdiv_up(G->g.n * 4 * c.P, (int64_t)256), 2048);
   if ((e = add_kernel(&no, body, &n4, 1, k_sw_out, ob_blocks, 256, a_out)) != cudaSuccess) return e;
-  void* a_nx[] = {&jc, &sc, &lps, &lpd, &hq, &stc, &d};
+  void* a_nx[] = {&jc, &sc, &lps, &lpd, &hq, &stc, &stcb, &d};
   return add_kernel(&nn, body, &no, 1, k_sw_next, 1, 32, a_nx);
 }
 
@@ -2401,6 +2411,10 @@ mnpbem_status sweep_finish(Job& j, SweepJobBufs& b, int w0) {
   std::vector<double> rv((size_t)nenei * (2 * P + 1));
   MNP_CUDA(cudaMemcpy(iv.data(), b.stage_i, sizeof(int) * iv.size(), cudaMemcpyDeviceToHost));
   MNP_CUDA(cudaMemcpy(rv.data(), b.stage_r, sizeof(double) * rv.size(), cudaMemcpyDeviceToHost));
+  if (iv.back() & 4) {
+    set_error("tensor-core GEMM: a bounded pipeline wait expired");
+    return MNPBEM_ERR_TIMEOUT;
+  }
   if (iv.back()) {
     set_error("refinement produced NaN");
     return MNPBEM_ERR_NOT_CONVERGED;
@@ -2555,7 +2569,15 @@ mnpbem_status job_finish(Job& j, bool failed) {
   mnpbem_geom* G = j.G;
   if (failed) {
     // leave nothing in flight that writes the caller's buffers
-    for (int l = 0; l < j.nl && l < (int)G->lanes.size(); ++l) cudaStreamSynchronize(G->lanes[l]->st);
+    for (int l = 0; l < j.nl && l < (int)G->lanes.size(); ++l) {
+      Lane& L = *G->lanes[l];
+      cudaStreamSynchronize(L.st);
+      // reported once: the lane goes on without the tensor cores, its words clear
+      for (TcGemmCtx* t : {&L.tc, &L.tcb}) tc_check_error(*t, L.st);
+      L.tc.enabled = L.tcb.enabled = L.tc.enabled && L.tcb.enabled;
+      for (int q = 0; q < LANE_NSTATUS; ++q) L.status_host[q] = 0;
+      L.state = Lane::IDLE;
+    }
     cudaGetLastError();
     G->prof.flush();
     return MNPBEM_OK;
@@ -2570,11 +2592,7 @@ mnpbem_status job_finish(Job& j, bool failed) {
   G->prof.flush();
   for (int l = 0; l < j.nl; ++l) {
     Lane& L = *G->lanes[l];
-    MNP_TRY(check_pivots(L, j.c.precision));
-    if (j.c.precision == MNPBEM_MIXED && G->tc_enabled) {
-      MNP_TRY(tc_check_error(L.tc, L.st));
-      MNP_TRY(tc_check_error(L.tcb, L.st));
-    }
+    MNP_TRY(check_pivots(L, j.c.precision));   // tensor-core products run in initmat alone, whose words these are
   }
   MNP_TRY(sweep_check(G->st));
   return MNPBEM_OK;
@@ -2900,7 +2918,6 @@ mnpbem_status mnpbem_cross_section_gradient(mnpbem_geom* G, const mnpbem_planewa
       adj_resid(n, y12, y12 + 4 * n, gs2, gh2, r64, r64 + n, r64 + 4 * n, r64 + 5 * n, nrm + 2, st);
       MNP_CHECK_LAUNCH();
     }
-    MNP_TRY(tc_check_error(L.tc, st));
     MNP_TRY(sweep_check(st));
   }
   // ---- weights, then G1 [sig1 h1], G2 [sig2 h2], H1 sig1 from freshly assembled FP64 matrices

@@ -1155,7 +1155,7 @@ static mnpbem_status tc_gemm_f16(TcGemmCtx& c, int64_t M, int64_t N, int64_t K, 
   MNP_TRY(c.bexp.ensure(sizeof(__half) * N2 * Kp));
   MNP_TRY(c.a16.ensure(sizeof(__half) * 2 * M * Kp));
   MNP_TRY(c.scales.ensure(sizeof(float) * (M + 2 * N)));
-  MNP_TRY(c.err.ensure(sizeof(int)));
+  MNP_TRY(tc_error_word(c, st));
   MNP_TRY(c.ctr.ensure(sizeof(int)));
   __half* Bp = c.bexp.as<__half>();
   __half* A16 = c.a16.as<__half>();
@@ -1181,10 +1181,6 @@ static mnpbem_status tc_gemm_f16(TcGemmCtx& c, int64_t M, int64_t N, int64_t K, 
       !make_map(enc, &mp, C, (uint64_t)N2, (uint64_t)M, (uint64_t)ldc * 8, TC_BM, false, TC_BN)) {
     set_error("cuTensorMapEncodeTiled failed");
     return MNPBEM_ERR_CUDA;
-  }
-  if (!c.err_cleared) {
-    MNP_CUDA(cudaMemsetAsync(c.err.ptr, 0, sizeof(int), st));
-    c.err_cleared = true;
   }
   const int64_t MT = cdiv_up(M, TC_BM), NT = cdiv_up(N2, TC_BN);
   if (MT * NT >= (1ll << 31)) { set_error("tc_gemm_c64: too many tiles"); return MNPBEM_ERR_INVALID_ARG; }
@@ -1222,7 +1218,7 @@ mnpbem_status tc_gemm_c64(TcGemmCtx& c, int64_t M, int64_t N, int64_t K, float2 
   const int64_t K2 = 2 * K, N2 = 2 * N;
   const int64_t K2p = round_up(K2, TC_BK);
   MNP_TRY(c.bexp.ensure(sizeof(float) * N2 * K2p));
-  MNP_TRY(c.err.ensure(sizeof(int)));
+  MNP_TRY(tc_error_word(c, st));
   MNP_TRY(c.ctr.ensure(sizeof(int)));
   float* Bp = c.bexp.as<float>();
   {
@@ -1245,10 +1241,6 @@ mnpbem_status tc_gemm_c64(TcGemmCtx& c, int64_t M, int64_t N, int64_t K, float2 
       !make_map(enc, &mp, C, (uint64_t)N2, (uint64_t)M, (uint64_t)ldc * 8, TC_BM, false, TC_BN)) {
     set_error("cuTensorMapEncodeTiled failed");
     return MNPBEM_ERR_CUDA;
-  }
-  if (!c.err_cleared) {
-    MNP_CUDA(cudaMemsetAsync(c.err.ptr, 0, sizeof(int), st));
-    c.err_cleared = true;
   }
   const int64_t MT = cdiv_up(M, pair ? TP_TILE : TC_BM), NT = cdiv_up(N2, pair ? TP_TILE : TC_BN);
   if (MT * NT >= (1ll << 31)) { set_error("tc_gemm_c64: too many tiles"); return MNPBEM_ERR_INVALID_ARG; }
@@ -1286,13 +1278,20 @@ mnpbem_status tc_gemm_c64(TcGemmCtx& c, int64_t M, int64_t N, int64_t K, float2 
   return MNPBEM_OK;
 }
 
+mnpbem_status tc_error_word(TcGemmCtx& c, cudaStream_t st) {
+  if (c.err.ptr) return MNPBEM_OK;
+  MNP_TRY(c.err.ensure(sizeof(int)));
+  MNP_CUDA(cudaMemsetAsync(c.err.ptr, 0, sizeof(int), st));
+  return MNPBEM_OK;
+}
+
 mnpbem_status tc_check_error(TcGemmCtx& c, cudaStream_t st) {
-  if (!c.err.ptr || !c.err_cleared) return MNPBEM_OK;
+  if (!c.err.ptr) return MNPBEM_OK;
   int h = 0;
   MNP_CUDA(cudaMemcpyAsync(&h, c.err.ptr, sizeof(int), cudaMemcpyDeviceToHost, st));
   MNP_CUDA(cudaStreamSynchronize(st));
-  c.err_cleared = false;
   if (h) {
+    MNP_CUDA(cudaMemsetAsync(c.err.ptr, 0, sizeof(int), st));
     set_error("tensor-core GEMM: a bounded pipeline wait expired (code %d)", h);
     c.enabled = false;
     return MNPBEM_ERR_TIMEOUT;

@@ -8,14 +8,13 @@ struct TcGemmCtx {
   bool checked = false;   // device capability probed
   bool usable = false;    // sm_103 device, driver entry point and kernel attributes available
   bool enabled = true;    // switched off after a device-side error
-  bool err_cleared = false;
   DevBuf bexp;            // expanded B operand [2N][2K] (real, K-major, tf32 or fp16)
   DevBuf a16, scales;     // FP16 path: A operand [M][2K] in fp16, row / column scales
   bool f16 = false;       // FP16 operands with power-of-two row / column scaling (kind::f16)
   int f16_min_k = 512;    // ... for products with K >= f16_min_k
   int f16_min_mn = 512;   //     and M, N >= f16_min_mn
   DevBuf a8, b8, exps;    // complex128 products: digit slices of A and B', their rows' / columns' exponents and sums
-  DevBuf err;             // device error word of the bounded waits
+  DevBuf err;             // device error word of the bounded waits (cleared when allocated and when reported)
   DevBuf ctr;             // tile counter of the persistent kernel (zeroed before each launch)
   int num_sms = 0;
   int stages = 4;         // pipeline depth of the persistent kernel (3 or 4)
@@ -40,8 +39,8 @@ mnpbem_status tc_gemm_c64(TcGemmCtx& c, int64_t M, int64_t N, int64_t K, float2 
 // C = alpha A B + beta C in complex128 on the tensor cores (tc_gemm64.cu):
 // operands cut into eight 8-bit digits per row of A and column of B, exact
 // products; entries that the digits may not hold to the accuracy of an FP64 sum are
-// computed in FP64 from A and a copy of B, so C may overlap B alone.  alpha = +-1,
-// beta 0 or 1, K <= TC64_K.
+// computed in FP64 from A and a copy of B, so C may overlap B alone.  alpha = +-1, beta 0 or
+// 1, K <= TC64_K.
 constexpr int TC64_K = 64;
 bool tc_gemm64_eligible(TcGemmCtx& c, int64_t M, int64_t N, int64_t K, double2 alpha, double2 beta);
 mnpbem_status tc_gemm_c128(TcGemmCtx& c, int64_t M, int64_t N, int64_t K, double alpha, const double2* A, int64_t lda,
@@ -51,7 +50,10 @@ bool tc_device_ready(TcGemmCtx& c);
 // CUtensorMap of a row-major fp16 matrix [rows][inner] (box_inner 32: 64-byte swizzle, 64: 128-byte)
 bool tc_f16_map(TcGemmCtx& c, void* map, const void* ptr, uint64_t inner, uint64_t rows, uint32_t box_inner,
                 uint32_t box_rows);
-// reads (and clears) the device error word; MNPBEM_ERR_TIMEOUT if a wait expired
+// allocates and clears the device error word, once per context
+mnpbem_status tc_error_word(TcGemmCtx& c, cudaStream_t st);
+// reads the device error word; if a wait expired MNPBEM_ERR_TIMEOUT, the word cleared
+// and the context's tensor-core products switched off
 mnpbem_status tc_check_error(TcGemmCtx& c, cudaStream_t st);
 void tc_release(TcGemmCtx& c);
 

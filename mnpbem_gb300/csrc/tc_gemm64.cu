@@ -593,7 +593,7 @@ mnpbem_status tc_gemm_c128(TcGemmCtx& c, int64_t M, int64_t N, int64_t K, double
   MNP_TRY(c.a8.ensure(sizeof(__half) * Z_S * M * Z_KR));
   MNP_TRY(c.b8.ensure(sizeof(__half) * Z_S * 2 * N * Z_KR + sizeof(double2) * K * N));
   MNP_TRY(c.exps.ensure(sizeof(SliceInfo) * (M + N)));
-  MNP_TRY(c.err.ensure(sizeof(int)));
+  MNP_TRY(tc_error_word(c, st));
   MNP_TRY(c.ctr.ensure(sizeof(int)));
   static bool attr = false;
   if (!attr) {
@@ -603,10 +603,6 @@ mnpbem_status tc_gemm_c128(TcGemmCtx& c, int64_t M, int64_t N, int64_t K, double
   __half *a8 = c.a8.as<__half>(), *b8 = c.b8.as<__half>();
   double2* bc = reinterpret_cast<double2*>(b8 + (int64_t)Z_S * 2 * N * Z_KR);
   SliceInfo *ea = c.exps.as<SliceInfo>(), *eb = ea + M;
-  if (!c.err_cleared) {
-    MNP_CUDA(cudaMemsetAsync(c.err.ptr, 0, sizeof(int), st));
-    c.err_cleared = true;
-  }
   {
     ProfScope ps(PH_ELEMWISE, st, 0.0, 16.0 * K * (M + 2.0 * N) + 2.0 * Z_S * Z_KR * (M + 2.0 * N));
     k_slice_a<<<(unsigned)cdiv_up(M, (int64_t)8), 256, 0, st>>>(A, lda, (int)M, (int)K, a8, ea, c.ctr.as<int>());
