@@ -11,6 +11,8 @@
 // matrix, so all O(n^3) work is a GEMM.  A pivot guard reports singular blocks.
 #include <cooperative_groups.h>
 
+#include <atomic>
+
 #include "dense.cuh"
 #include "ds_math.cuh"
 #include "mbarrier.cuh"
@@ -506,8 +508,18 @@ __global__ void __launch_bounds__(32 * DS_WARPS) k_gemm_thin_hi(int64_t M, int64
 
 __device__ int g_sweep_err;   // a bounded wait of the triangular sweeps expired
 
+// the current device's number, as an index into per-device tables (the last entry is
+// shared by all devices beyond it and never kept)
+constexpr int MAX_DEVICES = 64;
+static int device_index() {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) cudaGetLastError();
+  return dev >= 0 && dev < MAX_DEVICES ? dev : MAX_DEVICES;
+}
 static int num_sms() {
-  static int sms = 0;
+  static std::atomic<int> kept[MAX_DEVICES];
+  const int d = device_index();
+  int sms = d < MAX_DEVICES ? kept[d].load() : 0;
   if (!sms) {
     int dev = 0;
     cudaGetDevice(&dev);
@@ -515,6 +527,7 @@ static int num_sms() {
       cudaGetLastError();
       sms = 148;
     }
+    if (d < MAX_DEVICES) kept[d] = sms;
   }
   return sms;
 }
@@ -1793,12 +1806,15 @@ static mnpbem_status launch_sweep(SweepArgs<R> a, int maxblk, cudaStream_t st) {
   auto kern = k_ldu_sweep<R, NB, RW, CPL, LOWER>;
   const int smem = (int)sizeof(cplx<R>) * 2 * NB * (a.b + 4);
   constexpr int SMEM_MAX = (int)sizeof(cplx<R>) * 2 * NB * (32 * CPL + 4);
-  static int per_sm = -1;
-  if (per_sm < 0) {
+  // CTAs per SM, kept per device together with the kernel's shared-memory attribute
+  static std::atomic<int> kept[MAX_DEVICES];
+  const int d = device_index();
+  int per_sm = d < MAX_DEVICES ? kept[d].load() : 0;
+  if (!per_sm) {
     MNP_CUDA(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM_MAX));
-    int occ = 0;
-    MNP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kern, SWEEP_THREADS, SMEM_MAX));
-    per_sm = std::max(1, occ);
+    MNP_CUDA(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, SWEEP_THREADS, SMEM_MAX));
+    per_sm = std::max(1, per_sm);
+    if (d < MAX_DEVICES) kept[d] = per_sm;
   }
   const int S = (a.b + 8 * RW - 1) / (8 * RW);
   a.items = maxblk * S * a.nprob;

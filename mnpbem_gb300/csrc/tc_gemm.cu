@@ -1117,6 +1117,7 @@ bool tc_gemm_eligible(TcGemmCtx& c, int64_t M, int64_t N, int64_t K, const void*
     cudaDeviceGetAttribute(&major, cudaDevAttrComputeCapabilityMajor, dev);
     cudaDeviceGetAttribute(&minor, cudaDevAttrComputeCapabilityMinor, dev);
     c.usable = (major == 10 && minor == 3) && get_encode(c) != nullptr &&
+               tc_gemm64_prepare() &&
                cudaFuncSetAttribute(k_tc_gemm<3, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, tc_psmem(3)) == cudaSuccess &&
                cudaFuncSetAttribute(k_tc_gemm<4, 0>, cudaFuncAttributeMaxDynamicSharedMemorySize, tc_psmem(4)) == cudaSuccess &&
                cudaFuncSetAttribute(k_tc_gemm<3, 1>, cudaFuncAttributeMaxDynamicSharedMemorySize, tc_psmem(3)) == cudaSuccess &&

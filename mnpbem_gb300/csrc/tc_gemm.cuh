@@ -42,6 +42,7 @@ mnpbem_status tc_gemm_c64(TcGemmCtx& c, int64_t M, int64_t N, int64_t K, float2 
 // computed in FP64 from A and a copy of B, so C may overlap B alone.  alpha = +-1, beta 0 or
 // 1, K <= TC64_K.
 constexpr int TC64_K = 64;
+bool tc_gemm64_prepare();   // the kernel's shared memory on the current device (when a context is probed)
 bool tc_gemm64_eligible(TcGemmCtx& c, int64_t M, int64_t N, int64_t K, double2 alpha, double2 beta);
 mnpbem_status tc_gemm_c128(TcGemmCtx& c, int64_t M, int64_t N, int64_t K, double alpha, const double2* A, int64_t lda,
                            const double2* B, int64_t ldb, bool accumulate, double2* C, int64_t ldc, cudaStream_t st);

@@ -581,6 +581,10 @@ __global__ void __launch_bounds__(Z_THREADS, 1)
 }
 
 // --------------------------------------------------------------------- host
+bool tc_gemm64_prepare() {
+  return cudaFuncSetAttribute(k_tc_gemm64, cudaFuncAttributeMaxDynamicSharedMemorySize, Z_SMEM) == cudaSuccess;
+}
+
 bool tc_gemm64_eligible(TcGemmCtx& c, int64_t M, int64_t N, int64_t K, double2 alpha, double2 beta) {
   if (!tc_device_ready(c)) return false;
   if (alpha.y != 0.0 || (alpha.x != 1.0 && alpha.x != -1.0) || beta.y != 0.0 || (beta.x != 0.0 && beta.x != 1.0))
@@ -595,11 +599,6 @@ mnpbem_status tc_gemm_c128(TcGemmCtx& c, int64_t M, int64_t N, int64_t K, double
   MNP_TRY(c.exps.ensure(sizeof(SliceInfo) * (M + N)));
   MNP_TRY(tc_error_word(c, st));
   MNP_TRY(c.ctr.ensure(sizeof(int)));
-  static bool attr = false;
-  if (!attr) {
-    MNP_CUDA(cudaFuncSetAttribute(k_tc_gemm64, cudaFuncAttributeMaxDynamicSharedMemorySize, Z_SMEM));
-    attr = true;
-  }
   __half *a8 = c.a8.as<__half>(), *b8 = c.b8.as<__half>();
   double2* bc = reinterpret_cast<double2*>(b8 + (int64_t)Z_S * 2 * N * Z_KR);
   SliceInfo *ea = c.exps.as<SliceInfo>(), *eb = ea + M;
