@@ -140,6 +140,7 @@ struct Lane {
   int last_kind = 0;         // stage of the last refinement step
   bool ds_done = false;      // a double-single residual has been computed for this wavelength
   double bnorm2 = 0.0;       // ||b||^2 of the excitation (from the last full residual)
+  bool stalled = false;      // a refinement of this call ended far from its tolerance
   // preconditioner of the iterative solver kept for later wavelengths: the
   // dense chain matrices in mat[], the per-face data and parameters of the
   // wavelength it was built at (cleared whenever mat[] is overwritten)
@@ -187,6 +188,7 @@ struct mnpbem_geom {
   bool tc_f16 = true;       // tensor-core products with scaled FP16 operands (kind::f16) instead of TF32
   bool tc_enabled = true;
   bool use_graphs = true;
+  bool pivoted = false;      // 64-wide diagonal blocks with row interchanges, for the retry of a call (with_pivots)
   Profiler prof;
   // per-wavelength parameters: pinned host ring (one slot per wavelength)
   LamParams* lp_ring = nullptr;
@@ -1046,6 +1048,7 @@ uint64_t lane_sig(const mnpbem_geom* G, const Lane& L) {
   mix(nullptr, (size_t)G->tf32_rna);
   mix(nullptr, (size_t)G->asm_ds);
   mix(nullptr, (size_t)G->gj_fused);
+  mix(nullptr, (size_t)G->pivoted);
   mix(nullptr, (size_t)L.tc.enabled + 2 * (size_t)L.tcb.enabled);   // off after an expired wait
   return h;
 }
@@ -1110,11 +1113,17 @@ template <> LDUWork<double>& luwb<double>(Lane& L) { return L.lu64b; }
 
 void* tc_ctx(mnpbem_geom* G, Lane& L) { return G->tc_enabled ? (void*)&L.tc : nullptr; }
 
-// rows of the diagonal blocks of the LDU factors: 256 on the tensor-core path
-// (cluster block inverse), else 64 (single-CTA block inverse with pivoting)
+// rows of the diagonal blocks of the LDU factors: 256 in complex64 with the tensor
+// cores (cluster block inverse, no row interchanges), else 64 (pivoting inside the
+// block).  Up to 1023 faces a call whose wide blocks fail is run again with narrow
+// ones (with_pivots).
+template <typename R>
+bool wide_blocks(const mnpbem_geom* G, void* ctx) {
+  return sizeof(R) == 4 && ctx && G->g.n > 64 && !G->pivoted;
+}
 template <typename R>
 int lu_block(const mnpbem_geom* G, void* ctx) {
-  return (sizeof(R) == 4 && ctx && G->g.n > 64) ? 256 : 64;
+  return wide_blocks<R>(G, ctx) ? 256 : 64;
 }
 
 // Lane matrices after initmat: mat[0] LDU(G1), mat[1] LDU(G2), mat[2] Sigma1,
@@ -1191,7 +1200,7 @@ mnpbem_status stage_initmat(mnpbem_geom* G, Lane& L, bool direct) {
   // 512-wide Gauss-Jordan steps 1.365 against 1.265 wavelength-solves/s for
   // rank-512 / 256-wide; at 4000 faces the 256-wide steps were faster)
   const bool large = n >= 12000;
-  gjw<R>(L).nb = (sizeof(R) == 4 && ctx && n > 64) ? (G->gj_nb ? G->gj_nb : (large ? 512 : 256)) : 64;
+  gjw<R>(L).nb = wide_blocks<R>(G, ctx) ? (G->gj_nb ? G->gj_nb : (large ? 512 : 256)) : 64;
   gjw<R>(L).round_a = G->tf32_rna;
   gjw<R>(L).fused = G->gj_fused;
   LDUWork<R>& lw = luw<R>(L);
@@ -1592,6 +1601,12 @@ template <typename S>
 __host__ __device__ inline bool refine_converged(const S& s, const double* hn, double tol) {
   return s.ds_done && sqrt(hn[2]) <= tol * sqrt(hn[3]);
 }
+// ended far from the tolerance (or from the default one, if that is wider): not the
+// rounding level, but a factorisation that does not contract
+__host__ __device__ inline bool refine_far(const double* hn, double tol) {
+  return !(sqrt(hn[2]) <= (tol > 1e-10 ? tol : 1e-10) * sqrt(hn[3]));
+}
+constexpr int STALL_STEPS = 10;   // steps (the default limit) before that counts
 int next_step(const Lane& L) { return refine_next_kind(L); }
 void step_done(Lane& L, int kind, const double* hn) { refine_step_done(L, kind, hn); }
 bool step_converged(const Lane& L, const double* hn, double tol) { return refine_converged(L, hn, tol); }
@@ -1627,6 +1642,7 @@ mnpbem_status solve_one(mnpbem_geom* G, Lane& L, const SolveCtx& c, const Refine
       if (!(hn[2] == hn[2])) { set_error("refinement produced NaN"); return MNPBEM_ERR_NOT_CONVERGED; }
       if (step_converged(L, hn, ref.tol)) break;
     }
+    if (used >= STALL_STEPS && used >= ref.maxit && refine_far(hn, ref.tol)) L.stalled = true;
   }
   if (c.spectra) MNP_TRY(launch_stage(G, L, c, 4, graphs));
   MNP_CUDA(cudaStreamSynchronize(st));
@@ -1742,7 +1758,11 @@ mnpbem_status lane_advance(mnpbem_geom* G, Lane& L, const SolveCtx& c, const Swe
     const double* hn = L.norms_host;
     step_done(L, L.last_kind, hn);
     if (!(hn[2] == hn[2])) { set_error("refinement produced NaN"); return MNPBEM_ERR_NOT_CONVERGED; }
-    if (step_converged(L, hn, s.ref.tol) || L.iters >= s.ref.maxit) return queue_finish(G, L, c);
+    if (step_converged(L, hn, s.ref.tol)) return queue_finish(G, L, c);
+    if (L.iters >= s.ref.maxit) {
+      if (L.iters >= STALL_STEPS && refine_far(hn, s.ref.tol)) L.stalled = true;
+      return queue_finish(G, L, c);
+    }
     return queue_iter(G, L, c);
   }
   // DONE: results of L.w are in the lane; the stream is idle, so host-side
@@ -2092,7 +2112,8 @@ struct SweepDst {
   int* iters;                       // [w]
   double* res;                      // [w]
   int* status;                      // [w][LANE_NSTATUS]
-  int* nan;                         // bit 0: a refinement step produced NaN; 2: a lane found an expired wait
+  int* nan;                         // bit 0: a refinement step produced NaN; 1: one stalled; 2: a lane found an
+                                    // expired wait
   unsigned long long* stages;       // [NSTAGES] stage runs (the launch accounting of the replays)
   int64_t n;
   int P;
@@ -2105,7 +2126,7 @@ __global__ void k_sw_next(JobCtl* jc, SweepCtl* sc, const LamParams* lps, LamPar
                           cudaGraphConditionalHandle h, const int* tce, const int* tcb, const SweepDst* dp) {
   if (threadIdx.x) return;
   if ((tce && *(volatile const int*)tce) || (tcb && *(volatile const int*)tcb)) atomicOr(dp->nan, 4);
-  const bool failed = *(volatile const int*)dp->nan != 0;
+  const bool failed = (*(volatile const int*)dp->nan & 5) != 0;
   const int w = failed ? jc->nenei : atomicAdd(&jc->next, 1);
   const bool go = w < jc->nenei;
   if (go) {
@@ -2164,6 +2185,7 @@ __global__ void k_ref_decide(SweepCtl* sc, const double* hn, double tol, int max
   const bool nan = !(hn[2] == hn[2]);
   if (nan) atomicOr(d.nan, 1);
   const bool conv = refine_converged(*sc, hn, tol);
+  if (!conv && sc->iters >= maxit && sc->iters >= STALL_STEPS && refine_far(hn, tol)) atomicOr(d.nan, 2);
   d.iters[sc->w] = sc->iters;
   d.res[sc->w] = sc->res;
   cudaGraphSetConditional(h, (nan || conv || sc->iters >= maxit) ? 0u : 1u);
@@ -2415,11 +2437,12 @@ mnpbem_status sweep_finish(Job& j, SweepJobBufs& b, int w0) {
     set_error("tensor-core GEMM: a bounded pipeline wait expired");
     return MNPBEM_ERR_TIMEOUT;
   }
-  if (iv.back()) {
+  if (iv.back() & 1) {
     set_error("refinement produced NaN");
     return MNPBEM_ERR_NOT_CONVERGED;
   }
   Lane& L0 = *j.run[0];
+  if (iv.back() & 2) L0.stalled = true;
   // launch accounting: every stage run as a replay of lane 0's record, plus
   // the graph's control kernels (4 per wavelength, 2 per refinement step)
   {
@@ -2598,8 +2621,43 @@ mnpbem_status job_finish(Job& j, bool failed) {
   return MNPBEM_OK;
 }
 
-mnpbem_status run_jobs(std::vector<Job>& jobs) {
+// A mixed-precision call on particles of 65 to 1023 faces, run again with 64-wide
+// pivoted diagonal blocks when the 256-wide ones, which interchange no rows, met a
+// singular or ill-conditioned block or left a refinement that does not converge (a
+// metal with eps near minus its surroundings': the diagonal of Sigma vanishes).  From
+// 1024 faces on every block is 256 wide.  The handles are as before afterwards, so a
+// call's result does not depend on the calls before it.
+template <typename F>
+mnpbem_status with_pivots(const std::vector<mnpbem_geom*>& gs, int precision, const F& run) {
+  for (mnpbem_geom* G : gs)
+    for (auto& L : G->lanes) L->stalled = false;
+  const mnpbem_status st = run();
+  std::vector<mnpbem_geom*> small;
+  for (mnpbem_geom* G : gs)
+    if (precision == MNPBEM_MIXED && G->tc_enabled && G->g.n > 64 && G->g.n < 1024) small.push_back(G);
+  bool retry = st == MNPBEM_ERR_SINGULAR || st == MNPBEM_ERR_NOT_CONVERGED;
+  if (st == MNPBEM_OK)
+    for (mnpbem_geom* G : small)
+      for (auto& L : G->lanes) retry = retry || L->stalled;
+  if (!retry || small.empty()) return st;
+  const auto mode = [&](bool on) {
+    for (mnpbem_geom* G : small) {
+      G->pivoted = on;
+      for (auto& L : G->lanes) L->pc_valid = false;   // a kept preconditioner has the other blocks
+    }
+  };
+  mode(true);
+  const mnpbem_status s2 = run();
+  mode(false);
+  return s2;
+}
+
+mnpbem_status run_jobs_once(std::vector<Job>& jobs) {
   mnpbem_status st = MNPBEM_OK;
+  for (Job& j : jobs) {
+    j.next = j.active = 0;
+    j.run.clear();
+  }
   for (Job& j : jobs)
     for (auto& L : j.G->lanes) L->pc_valid = false;
   for (Job& j : jobs)
@@ -2618,6 +2676,11 @@ mnpbem_status run_jobs(std::vector<Job>& jobs) {
   }
   for (Job& j : jobs) MNP_TRY(job_finish(j, false));
   return MNPBEM_OK;
+}
+mnpbem_status run_jobs(std::vector<Job>& jobs) {
+  std::vector<mnpbem_geom*> gs;
+  for (Job& j : jobs) gs.push_back(j.G);
+  return with_pivots(gs, jobs[0].c.precision, [&] { return run_jobs_once(jobs); });
 }
 
 template <typename C>
@@ -2769,7 +2832,7 @@ mnpbem_status mnpbem_ext_gradient(mnpbem_geom* G, const mnpbem_planewave* exc, i
                                        eps_grad);
 }
 
-mnpbem_status mnpbem_cross_section_gradient(mnpbem_geom* G, const mnpbem_planewave* exc, int32_t ipol,
+static mnpbem_status cross_section_gradient_once(mnpbem_geom* G, const mnpbem_planewave* exc, int32_t ipol,
                                             int32_t which, double enei, const double* eps_media, int32_t nmed,
                                             int32_t precision, double* value, double* verts_grad,
                                             double* eps_grad) {
@@ -2950,7 +3013,17 @@ mnpbem_status mnpbem_cross_section_gradient(mnpbem_geom* G, const mnpbem_planewa
   return MNPBEM_OK;
 }
 
-mnpbem_status mnpbem_bem_matrices(mnpbem_geom* G, double enei, const double* eps_media,
+mnpbem_status mnpbem_cross_section_gradient(mnpbem_geom* G, const mnpbem_planewave* exc, int32_t ipol,
+                                            int32_t which, double enei, const double* eps_media, int32_t nmed,
+                                            int32_t precision, double* value, double* verts_grad,
+                                            double* eps_grad) {
+  MNP_TRY(check_geom(G));
+  return with_pivots({G}, precision, [&] {
+    return cross_section_gradient_once(G, exc, ipol, which, enei, eps_media, nmed, precision, value, verts_grad, eps_grad);
+  });
+}
+
+static mnpbem_status bem_matrices_once(mnpbem_geom* G, double enei, const double* eps_media,
                                   int32_t nmed, int32_t precision, double* G1i, double* G2i,
                                   double* Sigma1, double* Deltai, double* Sigmai) {
   MNP_TRY(check_geom(G));
@@ -3002,6 +3075,15 @@ mnpbem_status mnpbem_bem_matrices(mnpbem_geom* G, double enei, const double* eps
   }
   G->prof.flush();
   return MNPBEM_OK;
+}
+
+mnpbem_status mnpbem_bem_matrices(mnpbem_geom* G, double enei, const double* eps_media,
+                                  int32_t nmed, int32_t precision, double* G1i, double* G2i,
+                                  double* Sigma1, double* Deltai, double* Sigmai) {
+  MNP_TRY(check_geom(G));
+  return with_pivots({G}, precision, [&] {
+    return bem_matrices_once(G, enei, eps_media, nmed, precision, G1i, G2i, Sigma1, Deltai, Sigmai);
+  });
 }
 
 }  // extern "C"
@@ -3958,7 +4040,7 @@ void hmat_stats(const HmatHost& H, const std::vector<int>& ranks, int64_t n, mnp
 
 }  // namespace
 
-mnpbem_status mnpbem_solve_iter(mnpbem_geom* G, const mnpbem_cluster_tree* tree, const mnpbem_iter_options* op,
+static mnpbem_status solve_iter_once(mnpbem_geom* G, const mnpbem_cluster_tree* tree, const mnpbem_iter_options* op,
                                 const mnpbem_planewave* exc, const mnpbem_potentials* pot, double enei,
                                 const double* eps_media, int32_t nmed, int32_t precision, mnpbem_solution* out,
                                 mnpbem_iter_info* info) {
@@ -4026,6 +4108,16 @@ mnpbem_status mnpbem_solve_iter(mnpbem_geom* G, const mnpbem_cluster_tree* tree,
     hmat_stats(H, H.ranks, n, info);
   }
   return MNPBEM_OK;
+}
+
+mnpbem_status mnpbem_solve_iter(mnpbem_geom* G, const mnpbem_cluster_tree* tree, const mnpbem_iter_options* op,
+                                const mnpbem_planewave* exc, const mnpbem_potentials* pot, double enei,
+                                const double* eps_media, int32_t nmed, int32_t precision, mnpbem_solution* out,
+                                mnpbem_iter_info* info) {
+  MNP_TRY(check_geom(G));
+  return with_pivots({G}, precision, [&] {
+    return solve_iter_once(G, tree, op, exc, pot, enei, eps_media, nmed, precision, out, info);
+  });
 }
 
 mnpbem_status mnpbem_hmat_full(mnpbem_geom* G, const mnpbem_cluster_tree* tree, const mnpbem_iter_options* op,
