@@ -176,7 +176,7 @@ struct mnpbem_geom {
   int64_t ld = 0;
   std::vector<std::unique_ptr<Lane>> lanes;
   int lanes_req = 0;        // 0: automatic
-  int gj_nb = 0;            // Gauss-Jordan step width on the tensor-core path (256 or 512; 0: by size)
+  int gj_nb = 0;            // Gauss-Jordan step width on the tensor-core path (256 or 512; 0: width and operands by size)
   int lu_steps = 0;         // LDU steps of 256 per trailing update on the tensor-core path (1, 2 or 4; 0: by size)
   std::vector<int64_t> g1_off, g1_n;   // diagonal blocks of G1 (one block when G1 is full)
   bool tf32_rna = true;     // round tensor-core A operands to nearest TF32
@@ -1195,12 +1195,14 @@ mnpbem_status stage_initmat(mnpbem_geom* G, Lane& L, bool direct) {
   for (int q = 0; q < 5; ++q) M[q] = L.mat[q].as<Cx>();
   void* ctx = tc_ctx(G, L);
   // wider Gauss-Jordan steps when the rank-nb updates run on tensor cores:
-  // fewer passes over the n x n matrix (each step reads and writes it once)
-  // By size (measured on GB300, 24 000-face dimer: rank-1024 LDU updates and
-  // 512-wide Gauss-Jordan steps 1.365 against 1.265 wavelength-solves/s for
-  // rank-512 / 256-wide; at 4000 faces the 256-wide steps were faster)
+  // fewer passes over the n x n matrix (each step reads and writes it once).
+  // By size: rank-1024 LDU updates and 512-wide steps with FP16 operands from 12 000
+  // faces on (24 000-face dimer: 1.365 against 1.265 wavelength-solves/s for rank-512 /
+  // 256-wide); below, Delta's inverse keeps 32-bit operands (TF32) unless the option
+  // gj_block asks for a width, in 512-wide steps from 3500 faces on (sweeps: 8000 faces
+  // 230 ms against 241 with 256, 4000 123.4 and 124.3; 2016, gradient, 17.0 and 16.5)
   const bool large = n >= 12000;
-  gjw<R>(L).nb = wide_blocks<R>(G, ctx) ? (G->gj_nb ? G->gj_nb : (large ? 512 : 256)) : 64;
+  gjw<R>(L).nb = wide_blocks<R>(G, ctx) ? (G->gj_nb ? G->gj_nb : (n >= 3500 ? 512 : 256)) : 64;
   gjw<R>(L).round_a = G->tf32_rna;
   gjw<R>(L).fused = G->gj_fused;
   LDUWork<R>& lw = luw<R>(L);
@@ -1243,7 +1245,11 @@ mnpbem_status stage_initmat(mnpbem_geom* G, Lane& L, bool direct) {
   // Delta -> M4, Sigma (partial) -> M3
   launch_delta_sigma<R>(n, M[2], M[3], M[4], ld, fd, L.st);
   MNP_CHECK_LAUNCH();
-  MNP_TRY(gj_invert<R>(M[4], n, ld, gjw<R>(L), gemm_w<R>, ctx, L.st, direct));
+  const bool f16 = L.tc.f16;
+  L.tc.f16 = f16 && (large || G->gj_nb);
+  const mnpbem_status gs = gj_invert<R>(M[4], n, ld, gjw<R>(L), gemm_w<R>, ctx, L.st, direct);
+  L.tc.f16 = f16;
+  MNP_TRY(gs);
   launch_sigma_add<R>(n, M[3], M[4], ld, fd, lp, L.st);
   MNP_CHECK_LAUNCH();
   MNP_TRY(ldu_factor<R>(M[3], n, ld, lw, lus, gemm_w<R>, ctx, L.st));
