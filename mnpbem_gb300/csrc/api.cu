@@ -1182,6 +1182,24 @@ mnpbem_status stage_assemble(mnpbem_geom* G, Lane& L, int precision) {
   return assemble_launch(p, true, true, L.st);
 }
 
+// Is there memory for the second stream's panels and operand buffers (18 KB per row
+// of G1's largest block in complex64, 10 KB in complex128, beside 48 and 24 KB that the
+// lane's own may still need)?  Asked until they are allocated; a solve that fits without
+// them keeps one stream.
+template <typename R>
+bool side_fits(mnpbem_geom* G, Lane& L) {
+  if (luwb<R>(L).ccol.ptr) return true;
+  if (capturing_now()) return false;      // the direct run before it had no room
+  size_t rows = 0, fr = 0, tot = 0;
+  for (int64_t q : G->g1_n) rows = std::max(rows, (size_t)q);
+  if (cudaMemGetInfo(&fr, &tot) != cudaSuccess) {
+    cudaGetLastError();
+    return false;
+  }
+  const size_t kb = sizeof(R) == 4 ? 18 * rows + 48 * (size_t)G->g.n : 10 * rows + 24 * (size_t)G->g.n;
+  return fr >= 1024 * kb + ((size_t)16 << 20);
+}
+
 // ---------------------------------------------------------------- S1
 // initmat.m:27-72 with block LDU factors in place of the inverses of G1, G2
 // and Sigma (real FLOP per wavelength: 8/3 n^3 per factorisation, 8 n^3 per
@@ -1220,7 +1238,7 @@ mnpbem_status stage_initmat(mnpbem_geom* G, Lane& L, bool direct) {
   // (gradient) 18.8 and 16.7, two particles of 12 000 434 and 411; sweeps, whose
   // lanes fill the chip already, 0 (4000 faces) to 15 % (1350, complex128).
   SideStream side(L, 0);
-  const bool beside = !G->prof.enabled;
+  const bool beside = !G->prof.enabled && side_fits<R>(G, L);
   LDUWork<R>& lwb = beside ? luwb<R>(L) : lw;
   void* ctxb = ctx;
   if (beside) {
