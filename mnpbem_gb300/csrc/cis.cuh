@@ -37,7 +37,8 @@ __device__ __forceinline__ void cis_load(CisTable& t, const CisTable* src) {
   __syncthreads();
 }
 
-// exp(i k d) for complex k (Im k >= 0 for passive media; any sign works).  SHIFT:
+// exp(i k d) for complex k (Im k >= 0 for passive media; any sign works: 0 beyond a decay
+// of exp(-700), infinite where the growth leaves the range).  SHIFT:
 // j by adding 1.5 2^52, whose low word is j (two FP64 operations instead of a
 // product, a rounding and a conversion; the last bits may differ, as a phase next to
 // the middle of two table entries may go to the other)
@@ -75,8 +76,13 @@ __device__ __forceinline__ double2 cis_exp(const CisTable& T, double2 k, double 
       const long long yi = (long long)yf;
       const long long nn = yi >> 6;                 // floor(y / 64)
       const int m = (int)(yi - (nn << 6));
-      const double scale = __longlong_as_double((unsigned long long)(1023 - nn) << 52);   // 2^(-nn)
-      e = ev * T.e2[m] * scale;
+      e = ev * T.e2[m];
+      if (nn > -1000) {
+        e *= __longlong_as_double((unsigned long long)(1023 - nn) << 52);   // 2^(-nn)
+      } else {         // growth to the end of the range and beyond (infinity)
+        const long long up = nn < -2023 ? 1023 : -nn - 1000;
+        e = e * __longlong_as_double((long long)(1023 + 1000) << 52) * __longlong_as_double((1023 + up) << 52);
+      }
     }
     cr *= e;
     sr *= e;
