@@ -313,7 +313,9 @@ MNPBEM_API mnpbem_status mnpbem_geom_set_lanes(mnpbem_geom* g, int32_t lanes);
 
 /* Tuning options of a handle (the autotuner of mnpbem_gb300/autotune.py picks
  * them per problem size): "lanes" (0..16), "gj_block" (Gauss-Jordan step of
- * the tensor-core inversions: 256 or 512), "tc_stages" (TMA pipeline depth of
+ * the tensor-core inversion of Delta: 256 or 512, the latter with FP16 operands
+ * unless "tc_f16" is 0; unset, 256 below 3500 faces and 512 from there, with FP16
+ * operands from 12 000 faces), "tc_stages" (TMA pipeline depth of
  * the tensor-core GEMM: 3 or 4), "tc_ctas" (CTAs of the persistent
  * tensor-core GEMM, 0 = one per SM; fewer leave SMs to the pivot-block
  * clusters of other lanes), "tc_pair" (only 0: the CTA-pair tensor-core GEMM
@@ -323,8 +325,9 @@ MNPBEM_API mnpbem_status mnpbem_geom_set_lanes(mnpbem_geom* g, int32_t lanes);
  * on FP16 operands scaled per row / column by powers of two, kind::f16, 1 =
  * default, or on TF32 operands, 0), "tf32_round" (round A operands to nearest
  * TF32: 0/1), "assembly_ds" (mixed-precision assembly in double-single FP32
- * arithmetic: 0/1), "sweep_graph" (1 = default: the wavelengths of a sweep
- * after each lane's first run as one CUDA graph with a device-side
+ * arithmetic: 0/1), "selftest_tc_error" (the lanes' tensor-core error words as an
+ * expired wait leaves them, for tests: the next call returns MNPBEM_ERR_TIMEOUT),
+ * "sweep_graph" (1 = default: the wavelengths of a sweep after the first as one CUDA graph with a device-side
  * wavelength queue and device-side refinement decisions; 0: the host
  * scheduler polls the lanes and queues every stage; results are identical).
  * Unknown keys or values return MNPBEM_ERR_INVALID_ARG.

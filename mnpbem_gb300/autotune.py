@@ -8,8 +8,12 @@ rank-nb updates and the size of its pivot blocks), the number of 256-row LDU
 steps gathered into one trailing update of the factorisations (1, 2, 4: rank
 256, 512, 1024), the number of wavelengths in flight (lanes) -- and stores
 the fastest combination in ``data/tuned.json``
-keyed by the face count.  ``bemsolver`` applies the entry whose face count is
-closest (within a factor of 2) when it creates a mixed-precision solver.
+keyed by the face count that was measured.  ``bemsolver`` applies the entry whose face
+count is closest (by ratio, within a factor of 2) when it creates a mixed-precision
+solver, so the line between two entries lies at their geometric mean.
+
+A ``gj_block`` of 512 takes FP16 operands in the products of Delta's inverse; entries
+below 12 000 faces leave it to the library, which keeps 32-bit operands there.
 
     python -m mnpbem_gb300.autotune --faces 4000 [--device 0]
 """
@@ -23,7 +27,8 @@ import numpy as np
 
 _HERE = os.path.dirname(os.path.abspath(__file__))
 TUNED = os.path.join(_HERE, "data", "tuned.json")
-GRID = {"tc_stages": (3, 4), "gj_block": (256, 512), "lu_steps": (1, 2, 4), "lanes": (2, 4, 6, 8, 12, 16)}
+# gj_block 0: not set, the library's width and operands by size
+GRID = {"tc_stages": (3, 4), "gj_block": (0, 256, 512), "lu_steps": (1, 2, 4), "lanes": (2, 4, 6, 8, 12, 16)}
 
 
 def load():
@@ -72,6 +77,9 @@ def tune(faces, device=0, nw=16, repeats=2):
     for combo in itertools.product(*GRID.values()):
         opts = dict(zip(GRID.keys(), combo))
         solver = B.bemsolver(cp, B.bemoptions(precision="mixed", device=device, tuned=False))
+        opts = {k: v for k, v in opts.items() if v}
+        if faces < 12000 and opts.get("gj_block") == 512:
+            continue                                    # 16-bit operands only where the library takes them by itself
         for k, v in opts.items():
             solver.set_option(k, v)
         solver.spectrum(exc, enei)                      # sizes buffers, captures graphs

@@ -954,9 +954,9 @@ mnpbem_status mnpbem_geom_stream(const mnpbem_geom* G, void** stream) {
 //   S2 first solve     excitation + mldivide chain (+ conversions)
 //   S3 refinement step FP64 residual of the full operator + chain + update (MIXED)
 //   S4 spectra         far fields + extinction / scattering into a fixed slot
-// The first wavelength a lane runs for a configuration goes through the
-// stages directly (sizing every buffer); the lane then captures each stage as
-// a CUDA graph and replays the graphs for its later wavelengths.
+// The first wavelength of a configuration goes through the stages directly on one
+// lane (sizing every buffer); every lane, with buffers of those sizes, then captures
+// each stage as a CUDA graph and replays the graphs for its wavelengths.
 namespace {
 
 struct SolveCtx {
@@ -1026,7 +1026,7 @@ uint64_t lane_sig(const mnpbem_geom* G, const Lane& L) {
   gj(L.gj32);
   gj(L.gj64);
   auto lu = [&](const auto& w) {
-    mixbuf(w.ccol); mixbuf(w.rrow); mixbuf(w.xblk); mixbuf(w.tmp); mixbuf(w.pan);
+    mixbuf(w.ccol); mixbuf(w.rrow); mixbuf(w.xblk); mixbuf(w.pan);
     mix(nullptr, (size_t)w.b);
     mix(nullptr, (size_t)w.m);
   };
@@ -1940,7 +1940,6 @@ mnpbem_status size_lu(LDUWork<R>& d, const LDUWork<R>& s) {
   MNP_TRY(d.ccol.ensure(s.ccol.bytes));
   MNP_TRY(d.rrow.ensure(s.rrow.bytes));
   MNP_TRY(d.xblk.ensure(s.xblk.bytes));
-  MNP_TRY(d.tmp.ensure(s.tmp.bytes));
   return d.pan.ensure(s.pan.bytes);
 }
 mnpbem_status size_like(Lane& d, const Lane& s) {

@@ -62,14 +62,15 @@ mnpbem_status gj_status_copy(GJWork<R>& w, int* host2, cudaStream_t st);
 // blocks, U unit block-upper (stored above them: U_kj = X_k A_kj after the
 // updates of the steps before k).  Blocks of w.b rows; the trailing updates
 // of w.m consecutive steps are gathered into one product of rank w.b * w.m.
-// Each diagonal block is inverted with partial pivoting inside the block
-// (CUDA-core path, 64-wide blocks) or by the 256-wide cluster kernel.
+// Each diagonal block is inverted with partial pivoting inside the block (64-wide
+// blocks: complex128, and complex64 without the tensor cores or when a call is run
+// again for its pivots) or by the 256-wide cluster kernel, which interchanges no rows.
 // Status words (device, cleared by ldu_status_clear): [0] != 0 when a block
 // inverse met a zero or non-finite pivot; [1] the largest per-block condition
 // proxy max|A_kk| * max|X_k| as the bits of a non-negative float.
 template <typename R>
 struct LDUWork {
-  DevBuf ccol, rrow, xblk, tmp;
+  DevBuf ccol, rrow, xblk;
   DevBuf pan;            // panel scratch of the 256-wide block inverse
   int b = 64;
   int m = 1;
