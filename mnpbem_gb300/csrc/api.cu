@@ -140,7 +140,7 @@ struct Lane {
   int last_kind = 0;         // stage of the last refinement step
   bool ds_done = false;      // a double-single residual has been computed for this wavelength
   double bnorm2 = 0.0;       // ||b||^2 of the excitation (from the last full residual)
-  bool stalled = false;      // a refinement of this call ended far from its tolerance
+  double stalled = 0.0;      // largest residual of this call's refinements that ended far from their tolerance
   // preconditioner of the iterative solver kept for later wavelengths: the
   // dense chain matrices in mat[], the per-face data and parameters of the
   // wavelength it was built at (cleared whenever mat[] is overwritten)
@@ -1631,6 +1631,7 @@ __host__ __device__ inline bool refine_far(const double* hn, double tol) {
   return !(sqrt(hn[2]) <= (tol > 1e-10 ? tol : 1e-10) * sqrt(hn[3]));
 }
 constexpr int STALL_STEPS = 10;   // steps (the default limit) before that counts
+void note_stall(Lane& L, double res) { L.stalled = std::max(L.stalled, std::max(res, 1e-300)); }
 int next_step(const Lane& L) { return refine_next_kind(L); }
 void step_done(Lane& L, int kind, const double* hn) { refine_step_done(L, kind, hn); }
 bool step_converged(const Lane& L, const double* hn, double tol) { return refine_converged(L, hn, tol); }
@@ -1666,7 +1667,7 @@ mnpbem_status solve_one(mnpbem_geom* G, Lane& L, const SolveCtx& c, const Refine
       if (!(hn[2] == hn[2])) { set_error("refinement produced NaN"); return MNPBEM_ERR_NOT_CONVERGED; }
       if (step_converged(L, hn, ref.tol)) break;
     }
-    if (used >= STALL_STEPS && used >= ref.maxit && refine_far(hn, ref.tol)) L.stalled = true;
+    if (used >= STALL_STEPS && used >= ref.maxit && refine_far(hn, ref.tol)) note_stall(L, final_res);
   }
   if (c.spectra) MNP_TRY(launch_stage(G, L, c, 4, graphs));
   MNP_CUDA(cudaStreamSynchronize(st));
@@ -1784,7 +1785,7 @@ mnpbem_status lane_advance(mnpbem_geom* G, Lane& L, const SolveCtx& c, const Swe
     if (!(hn[2] == hn[2])) { set_error("refinement produced NaN"); return MNPBEM_ERR_NOT_CONVERGED; }
     if (step_converged(L, hn, s.ref.tol)) return queue_finish(G, L, c);
     if (L.iters >= s.ref.maxit) {
-      if (L.iters >= STALL_STEPS && refine_far(hn, s.ref.tol)) L.stalled = true;
+      if (L.iters >= STALL_STEPS && refine_far(hn, s.ref.tol)) note_stall(L, L.res);
       return queue_finish(G, L, c);
     }
     return queue_iter(G, L, c);
@@ -2465,7 +2466,9 @@ mnpbem_status sweep_finish(Job& j, SweepJobBufs& b, int w0) {
     return MNPBEM_ERR_NOT_CONVERGED;
   }
   Lane& L0 = *j.run[0];
-  if (iv.back() & 2) L0.stalled = true;
+  if (iv.back() & 2)
+    for (int w = w0; w < nenei; ++w)
+      if (iv[w] >= j.s.ref.maxit) note_stall(L0, rv[(size_t)nenei * 2 * P + w]);
   // launch accounting: every stage run as a replay of lane 0's record, plus
   // the graph's control kernels (4 per wavelength, 2 per refinement step)
   {
@@ -2648,20 +2651,29 @@ mnpbem_status job_finish(Job& j, bool failed) {
 // pivoted diagonal blocks when the 256-wide ones, which interchange no rows, met a
 // singular or ill-conditioned block or left a refinement that does not converge (a
 // metal with eps near minus its surroundings': the diagonal of Sigma vanishes).  From
-// 1024 faces on every block is 256 wide.  The handles are as before afterwards, so a
-// call's result does not depend on the calls before it.
+// 1024 faces on every block is 256 wide.  Where the pivoted blocks converge no better,
+// the call is run a third time for the outputs of the wide ones.  The handles are as
+// before afterwards, so a call's result does not depend on the calls before it.
 template <typename F>
 mnpbem_status with_pivots(const std::vector<mnpbem_geom*>& gs, int precision, const F& run) {
-  for (mnpbem_geom* G : gs)
-    for (auto& L : G->lanes) L->stalled = false;
-  const mnpbem_status st = run();
+  const auto once = [&](double& worst) {
+    for (mnpbem_geom* G : gs)
+      for (auto& L : G->lanes) L->stalled = 0.0;
+    const mnpbem_status s = run();
+    worst = 0.0;
+    for (mnpbem_geom* G : gs)
+      for (auto& L : G->lanes) worst = std::max(worst, L->stalled);
+    return s;
+  };
+  double wide = 0.0, narrow = 0.0;
+  const mnpbem_status st = once(wide);
   std::vector<mnpbem_geom*> small;
   for (mnpbem_geom* G : gs)
     if (precision == MNPBEM_MIXED && G->tc_enabled && G->g.n > 64 && G->g.n < 1024) small.push_back(G);
   bool retry = st == MNPBEM_ERR_SINGULAR || st == MNPBEM_ERR_NOT_CONVERGED;
   if (st == MNPBEM_OK)
     for (mnpbem_geom* G : small)
-      for (auto& L : G->lanes) retry = retry || L->stalled;
+      for (auto& L : G->lanes) retry = retry || L->stalled > 0.0;
   if (!retry || small.empty()) return st;
   const auto mode = [&](bool on) {
     for (mnpbem_geom* G : small) {
@@ -2670,8 +2682,9 @@ mnpbem_status with_pivots(const std::vector<mnpbem_geom*>& gs, int precision, co
     }
   };
   mode(true);
-  const mnpbem_status s2 = run();
+  const mnpbem_status s2 = once(narrow);
   mode(false);
+  if (st == MNPBEM_OK && (s2 != MNPBEM_OK || narrow > wide)) return once(wide);
   return s2;
 }
 

@@ -55,3 +55,17 @@ def test_batch(gpu_lib):
     r = m.spectrum_batch([(b, e, [550.0, 600.0]) for _, b, e in sets])
     for q in r:
         assert np.all(q["ir_resid"] < TOL)
+
+
+def test_better_of_both_is_kept(gpu_lib):
+    """Two spheres of sizes 1 : 300, whose areas differ by 10^5 inside a block: neither
+    converges in ten steps, the wide blocks end at a residual of 1e-8 and the pivoted
+    ones above 1."""
+    v, f = shapes.trisphere(144, 20.0)
+    vb, fb = shapes.trisphere(144, 6000.0)
+    drude = m.epsfun(lambda w: 10 - 9.065 ** 2 / (w * (w + 0.0708j)), "eV")
+    cp = m.comparticle([m.epsconst(1.77), drude], [m.particle(v, f), m.particle(vb + [3012.0, 0, 0], fb)],
+                       [[2, 1], [2, 1]], 1, 2)
+    bem = m.bemsolver(cp, m.bemoptions(precision="mixed"))
+    r = bem.spectrum(m.planewave([[1.0, 0, 0]], [[0, 0, 1.0]]), [550.0, 600.0])
+    assert np.all(r["ir_resid"] < 1e-4)
