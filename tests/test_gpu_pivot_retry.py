@@ -69,3 +69,19 @@ def test_better_of_both_is_kept(gpu_lib):
     bem = m.bemsolver(cp, m.bemoptions(precision="mixed"))
     r = bem.spectrum(m.planewave([[1.0, 0, 0]], [[0, 0, 1.0]]), [550.0, 600.0])
     assert np.all(r["ir_resid"] < 1e-4)
+
+
+def test_gradient_and_iterative_solver(gpu_lib):
+    """The other callers of the factorisation: the gradient's forward solve is run again
+    as a sweep's is, and the iterative solver takes its dense preconditioner from either.
+    Tolerance: the plane-wave solves' condition (1e5) times the refinement's 1e-10, and
+    the iterative solver's own residual."""
+    cp, bem, exc = solver()
+    val, gv, _ = bem.cross_section_gradient(exc, 600.0, 0, "ext", "mixed")
+    ref, rv, _ = bem.cross_section_gradient(exc, 600.0, 0, "ext", "fp64")
+    assert abs(val - ref) < 1e5 * TOL * abs(ref)
+    assert np.max(np.abs(gv - rv)) < 1e5 * TOL * np.max(np.abs(rv))
+    it = m.bemsolver(cp, m.bemoptions(precision="mixed", iter={"tol": 1e-9}))
+    for _ in range(2):
+        it.mldivide(exc(cp, 600.0))
+        assert it.info["flag"] == 0
